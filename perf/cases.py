@@ -17,6 +17,7 @@ from __future__ import annotations
 import math
 
 import torch
+import torch.nn.functional as F
 
 from state_space_models_neuron_b200 import parallel as nxd
 from state_space_models_neuron_b200.models import Mamba2Cache, Mamba2ForCausalLM, Mamba2HybridForCausalLM, get_config
@@ -136,8 +137,9 @@ def prepare(case, seed):
             # decoding keeps values made from the per-head parameters by address: a program that serves one model until
             # it ends never frees these, and the many models made here must not meet what was kept for another one
             _SERVED.extend(layer.mixer.dt_bias for layer in model.backbone.layers)
-            logits, cache = model.prefill(ids)
-            state["cache"], state["token"] = cache, logits[:, -1].argmax(-1, keepdim=True)
+            _, cache = model.prefill(ids)
+            state["cache"] = cache
+            state["token"] = torch.randint(0, config.vocab_size, (case["batch"], 1), device="cuda", generator=gen)
             if case["kind"] == "decode":
                 state["step"] = GraphedDecodeStep(model, cache, case["batch"])
     return state
@@ -214,3 +216,110 @@ def tolerance(case):
     # adds up); gradients of two runs of one implementation differ by 0.005 to 0.011 after three optimizer steps, because
     # AdamW's first steps move a weight by the sign of its gradient.  Largest single difference seen: 0.68.
     return {"rel": 0.03, "max": 0.9}
+
+
+def _norm(x, weight, eps, group=None):
+    grouped = x.unflatten(-1, (-1, group or x.shape[-1]))
+    return (grouped * torch.rsqrt(grouped.square().mean(-1, keepdim=True) + eps)).flatten(-2) * weight
+
+
+def _mixer(m, x, value, before):
+    """Mamba-2 mixer over x [B, L, D] behind the state `before` = (conv window [B, 4, C], SSM state [B, H, P, N]) or None."""
+    inner, bc, heads = m.intermediate_size_tp, m.n_groups_tp * STATE, m.num_heads_tp
+    batch, length = x.shape[:2]
+    z, xbc, dt = F.linear(x, value(m.in_proj.weight), value(m.in_proj.bias)).split([inner, inner + 2 * bc, heads], -1)
+    window, S = before or (x.new_zeros(batch, 4, inner + 2 * bc), x.new_zeros(batch, heads, m.head_dim, STATE))
+    window = torch.cat([window, xbc], 1)
+    taps = value(m.conv1d.weight)[:, 0]
+    pre = sum(window[:, k + 1:k + 1 + length] * taps[:, k] for k in range(4))
+    act = F.silu(pre if m.conv1d.bias is None else pre + value(m.conv1d.bias))
+    xs, Bm, Cm = (t.unflatten(-1, (n, -1)) for t, n in zip(act.split([inner, bc, bc], -1), (heads, m.n_groups_tp, m.n_groups_tp)))
+    dt = F.softplus(dt + value(m.dt_bias))
+    log_decay = -torch.exp(value(m.A_log)) * dt
+    parts = []
+    for t in range(0, length, 128):
+        part = slice(t, t + 128)
+        l = log_decay[:, part].cumsum(1).transpose(1, 2)                                       # [B, H, T]
+        u = (xs[:, part] * dt[:, part, :, None]).transpose(1, 2)
+        B, C = (v[:, part].transpose(1, 2).repeat_interleave(heads // m.n_groups_tp, 1) for v in (Bm, Cm))
+        within = (l[..., :, None] - l[..., None, :]).tril().exp().tril()
+        y = (C @ B.transpose(-1, -2) * within) @ u + l.exp()[..., None] * (C @ S.transpose(-1, -2))
+        S = l[..., -1:, None].exp() * S + (u * (l[..., -1:] - l).exp()[..., None]).transpose(-1, -2) @ B
+        parts.append(y.transpose(1, 2))
+    y = (torch.cat(parts, 1) + value(m.D)[:, None] * xs).flatten(-2)
+    y = _norm(y * F.silu(z), value(m.norm.weight), m.norm.eps, m.norm.group_size)
+    return F.linear(y, value(m.out_proj.weight), value(m.out_proj.bias)), (window[:, -4:], S)
+
+
+def _attention(a, x, value):
+    q, k, v = (F.linear(x, value(p.weight)).unflatten(-1, (-1, a.head_dim)).transpose(1, 2) for p in (a.q_proj, a.k_proj, a.v_proj))
+    if a.rotary_emb_dim:
+        half = a.rotary_emb_dim // 2
+        angle = torch.arange(x.shape[1], device=x.device, dtype=x.dtype)[:, None] * \
+            a.rope_theta ** (-torch.arange(half, device=x.device, dtype=x.dtype) / half)
+        cos, sin = angle.cos(), angle.sin()
+        q, k = (torch.cat([t[..., :half] * cos - t[..., half:2 * half] * sin, t[..., half:2 * half] * cos + t[..., :half] * sin,
+                           t[..., 2 * half:]], -1) for t in (q, k))
+    ratio = a.num_heads // a.num_kv_heads
+    out = [F.scaled_dot_product_attention(q[:, h], k[:, h // ratio], v[:, h // ratio], is_causal=True) for h in range(a.num_heads)]
+    return F.linear(torch.cat(out, -1), value(a.o_proj.weight))
+
+
+def _mlp(m, x, value):
+    h = F.linear(x, value(m.gate_up_proj.weight))
+    h = F.silu(h[..., :m.split_size]) * h[..., m.split_size:] if m.gated else F.gelu(h)
+    return F.linear(h, value(m.down_proj.weight))
+
+
+def _hidden(model, ids, value, before=None):
+    """(last hidden states, states of the mixers) of tokens behind the mixers' states `before`."""
+    x, states = F.embedding(ids, value(model.backbone.embeddings.weight)), []
+    for block in model.backbone.layers:
+        layer = block.mixer if hasattr(block, "mixer") else block.layer
+        normed = _norm(x, value(block.norm.weight), model.config.layer_norm_epsilon)
+        if hasattr(layer, "in_proj"):
+            out, after = _mixer(layer, normed, value, before[len(states)] if before else None)
+            states.append(after)
+        else:
+            out = (_attention if hasattr(layer, "q_proj") else _mlp)(layer, normed, value)
+        x = x + out
+    return _norm(x, value(model.backbone.norm_f.weight), model.config.layer_norm_epsilon), states
+
+
+def exact(case, seed):
+    """The first pass in 64 bits.  None for the captured training step, which stands behind two optimizer steps whose
+    first moves of a weight follow the sign of its gradient, and for weights after such a move; the same gradients are
+    those of the step launched op by op."""
+    kind = case["kind"]
+    if kind == "train" or case["batch"] * case["seq"] > 40000:
+        return None
+    state = prepare(case, seed)
+    model, ids, wide = state["model"], state["ids"], {}
+
+    def value(p):
+        if p is not None and p not in wide:
+            wide[p] = p.detach().double().requires_grad_(kind == "train_eager")
+        return None if p is None else wide[p]
+
+    def logits_of(hidden):
+        return F.linear(hidden, value(model.lm_head.weight))
+
+    def loss_of(logits):
+        return F.cross_entropy(logits[:, :-1].flatten(0, 1), ids[:, 1:].flatten())
+
+    if kind == "train_eager":
+        loss = loss_of(logits_of(_hidden(model, ids, value)[0]))
+        loss.backward()
+        flat = torch.zeros(state["opt"].flat_grads.shape, dtype=torch.float64, device="cuda")
+        for p, w in wide.items():
+            flat[p.main_grad.storage_offset():][:p.numel()] = w.grad.flatten()
+        clipped = flat * min(1.0, 1.0 / (float(flat.norm()) + 1e-6))
+        return {"loss": loss.detach(), "gradients": flat, "weights": None, "moments": [0.1 * clipped, 0.05 * clipped.square()]}
+    with torch.no_grad():
+        hidden, states = _hidden(model, ids, value)
+        if kind == "score":
+            logits = logits_of(hidden)
+            return {"loss": loss_of(logits), "logits": logits}
+        if kind != "prefill":
+            hidden, states = _hidden(model, state["token"], value, states)
+        return {"logits": logits_of(hidden[:, -1:]), "conv": [w.transpose(1, 2) for w, _ in states], "ssm": [S for _, S in states]}
