@@ -954,6 +954,9 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }
 
 // ------------------------------------------------------------------------------------ host
+bool gemm_skinny(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc,
+                 const void* bias, int* status, int sms, cudaStream_t stream, int* code);
+
 static int g_num_sms = 0;
 static unsigned long long* g_trace = nullptr;
 
@@ -1257,6 +1260,15 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  // few rows (decoding): kernels that stream the weights (gemm_skinny.cu), unless a test or a measurement forces a tiling
+  if (mode == 0 && act == 0 && !a_mn && !b_mn && comm == nullptr && extra == nullptr && M <= 128 && gemm_forced_bn() == 0 &&
+      gemm_pair_mode() == 1 && gemm_split_enabled() == 1 && g_trace == nullptr && !epilogue_direct()) {
+    int code = 0;
+    if (gemm_skinny(A, B, C, M, N, K, lda, ldb, ldc, bias, status, g_num_sms, stream, &code)) {
+      if (tiles_n_out) *tiles_n_out = 0;
+      return code;
+    }
   }
   // the collective variants walk the tiles block by block (rows of one shard / owner): pair tiles need whole blocks
   int allow_pair = gemm_pairs_enabled();
