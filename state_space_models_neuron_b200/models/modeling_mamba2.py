@@ -232,25 +232,37 @@ class Mamba2ForCausalLM(Mamba2PreTrainedModel, GenerationMixin):
         if labels is not None and not kwargs.get("return_logits", True):
             loss = self.loss_from_hidden(hidden, labels)
         else:
-            logits = self.lm_head(hidden).float()
-            if labels is not None:
-                shift_logits = logits[:, :-1, :]
-                shift_labels = labels[:, 1:].to(logits.device)
-                loss = parallel_cross_entropy(shift_logits, shift_labels).mean()
+            logits, loss = self.logits_and_loss(hidden, labels)
         if return_dict is False:
             return tuple(v for v in (loss, logits, out.cache_params, out.hidden_states) if v is not None)
         return Mamba2CausalLMOutput(loss=loss, logits=logits, cache_params=out.cache_params,
                                     hidden_states=out.hidden_states)
 
-    def loss_from_hidden(self, hidden, labels):
-        """Loss without materialising fp32 logits for the caller: labels are shifted instead of
-        the logits (position L-1 is ignored), the mean runs over the B*(L-1) real targets."""
+    def logits_and_loss(self, hidden, labels):
+        """(fp32 logits, loss or None).  Where the head's GEMM delivers the cross-entropy statistics of its rows, the loss
+        comes from them; a shifted copy of the fp32 logits and two passes over it took half of a scoring call."""
+        tp = ps.get_tensor_model_parallel_size() if self.backbone.sequence_parallel_enabled else 1
+        if (labels is not None and hidden.is_cuda and hidden.dtype == torch.bfloat16 and labels.device == hidden.device
+                and labels.dtype == torch.int64 and tuple(labels.shape) == (hidden.shape[0], hidden.shape[1] * tp)):
+            logits, loss = self._head_loss(hidden, labels)
+            return ops.widen(logits), loss
+        logits = ops.widen(self.lm_head(hidden))
+        if labels is None:
+            return logits, None
+        return logits, parallel_cross_entropy(logits[:, :-1, :], labels[:, 1:].to(logits.device)).mean()
+
+    def _head_loss(self, hidden, labels):
         shifted = torch.full_like(labels, -100)
         shifted[:, :-1] = labels[:, 1:]
         shifted = shifted.to(hidden.device)
         logits, stats = self.lm_head(hidden, ce_labels=shifted)
         per_tok = parallel_cross_entropy(logits, shifted, stats=stats)
-        return per_tok.sum() / (labels.shape[0] * (labels.shape[1] - 1))
+        return logits, per_tok.sum() / (labels.shape[0] * (labels.shape[1] - 1))
+
+    def loss_from_hidden(self, hidden, labels):
+        """Loss without materialising fp32 logits for the caller: labels are shifted instead of
+        the logits (position L-1 is ignored), the mean runs over the B*(L-1) real targets."""
+        return self._head_loss(hidden, labels)[1]
 
     @torch.no_grad()
     def prefill(self, input_ids, cache_params: Optional[Mamba2Cache] = None):
@@ -259,7 +271,7 @@ class Mamba2ForCausalLM(Mamba2PreTrainedModel, GenerationMixin):
             p = next(self.parameters())
             cache_params = Mamba2Cache(self.config, input_ids.shape[0], dtype=p.dtype, device=p.device)
         out = self.backbone(input_ids=input_ids, cache_params=cache_params, use_cache=True)
-        return self.lm_head(out.last_hidden_state[:, -1:, :]).float(), cache_params
+        return ops.widen(self.lm_head(out.last_hidden_state[:, -1:, :])), cache_params
 
     @torch.no_grad()
     def generate(self, inputs=None, max_new_tokens: Optional[int] = None, max_length: Optional[int] = None,
@@ -330,4 +342,4 @@ class Mamba2ForCausalLM(Mamba2PreTrainedModel, GenerationMixin):
     def step(self, input_ids, cache_params: Mamba2Cache):
         """Single-token decode: logits for the next token (mamba2/modeling_mamba2.py:523-531)."""
         hidden = self.backbone.step(input_ids, cache_params)
-        return self.lm_head(hidden).float()
+        return ops.widen(self.lm_head(hidden))

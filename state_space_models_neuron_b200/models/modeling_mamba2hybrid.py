@@ -15,7 +15,6 @@ from transformers import GenerationMixin
 
 from ..parallel import mappings as mp
 from ..parallel import state as ps
-from ..parallel.cross_entropy import parallel_cross_entropy
 from ..parallel.layers import ColumnParallelLinear, ParallelEmbedding, normal_init
 from .cache import Mamba2Cache
 from .configuration_mamba2hybrid import Mamba2HybridConfig
@@ -129,6 +128,8 @@ class Mamba2HybridForCausalLM(Mamba2HybridPreTrainedModel, GenerationMixin):
         return self.backbone.set_input_embeddings(new_embeddings)
 
     loss_from_hidden = Mamba2ForCausalLM.loss_from_hidden
+    logits_and_loss = Mamba2ForCausalLM.logits_and_loss
+    _head_loss = Mamba2ForCausalLM._head_loss
 
     def forward(self, input_ids=None, inputs_embeds=None, labels=None, output_hidden_states=None,
                 return_dict=None, **kwargs):
@@ -139,9 +140,7 @@ class Mamba2HybridForCausalLM(Mamba2HybridPreTrainedModel, GenerationMixin):
         if labels is not None and not kwargs.get("return_logits", True):
             loss = self.loss_from_hidden(hidden, labels)
         else:
-            logits = self.lm_head(hidden).float()
-            if labels is not None:
-                loss = parallel_cross_entropy(logits[:, :-1, :], labels[:, 1:].to(logits.device)).mean()
+            logits, loss = self.logits_and_loss(hidden, labels)
         if return_dict is False:
             return tuple(v for v in (loss, logits, out.hidden_states) if v is not None)
         return Mamba2CausalLMOutput(loss=loss, logits=logits, hidden_states=out.hidden_states)

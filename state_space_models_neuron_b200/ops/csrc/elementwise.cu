@@ -498,28 +498,73 @@ template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-template <typename T>
+// 16 bytes of a logit row as floats, and back
+template <typename T> struct LogitVec;
+template <> struct LogitVec<float> {
+  static constexpr int N = 4;
+  static __device__ __forceinline__ void load(const float* p, float (&f)[4]) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+  }
+  static __device__ __forceinline__ void store(float* p, const float (&f)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+  }
+};
+template <> struct LogitVec<__nv_bfloat16> {
+  static constexpr int N = 8;
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&f)[8]) { load8(p, f); }
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&f)[8]) { store8(p, f); }
+};
+template <typename T> __device__ __forceinline__ T from_f(float v);
+template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
+template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
+
+// what a running sum of exp(x - max) is relative to: a maximum of -inf (nothing finite yet) counts as 0, so that -inf adds
+// nothing and NaN stays NaN
+__device__ __forceinline__ float ce_ref(float m) { return m == -INFINITY ? 0.f : m; }
+
+// One pass over the logits, bound by reading them: 16-byte loads and an online softmax instead of one pass for the
+// maximum and one for the sum.  VEC: rows start on 16-byte boundaries (the tail of V is read one by one).
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 ce_partials_kernel(const T* __restrict__ logits, long long ld, const long long* __restrict__ labels, int V,
                    int vocab_start, float* __restrict__ omax, float* __restrict__ osum, float* __restrict__ otgt) {
   __shared__ float red[33];
   const long long row = blockIdx.x;
   const T* lr = logits + row * ld;
-  float m = -INFINITY;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) m = fmaxf(m, to_f<T>(lr[i]));
-  m = block_max(m, red);
-  float s = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) s += __expf(to_f<T>(lr[i]) - m);
-  s = block_sum(s, red);
+  float m = -INFINITY, s = 0.f;
+  constexpr int N = LogitVec<T>::N;
+  const int nv = VEC ? V / N : 0;
+  #pragma unroll 4
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    float f[N], mx = m;
+    LogitVec<T>::load(lr + (long long)i * N, f);
+    #pragma unroll
+    for (int e = 0; e < N; ++e) mx = fmaxf(mx, f[e]);
+    const float ref = ce_ref(mx);
+    s *= __expf(m - ref);
+    m = mx;
+    #pragma unroll
+    for (int e = 0; e < N; ++e) s += __expf(f[e] - ref);
+  }
+  for (int i = nv * N + threadIdx.x; i < V; i += blockDim.x) {
+    const float x = to_f<T>(lr[i]), mx = fmaxf(m, x), ref = ce_ref(mx);
+    s = s * __expf(m - ref) + __expf(x - ref);
+    m = mx;
+  }
+  const float gm = block_max(m, red);
+  s = block_sum(s * __expf(m - ce_ref(gm)), red);
   if (threadIdx.x == 0) {
     const long long loc = labels[row] - vocab_start;
-    omax[row] = m; osum[row] = s;
+    omax[row] = gm; osum[row] = s;
     otgt[row] = (loc >= 0 && loc < V) ? to_f<T>(lr[loc]) : 0.f;
   }
 }
 
 // grad[row, i] = (exp(l - gmax) / gsum - [i == label]) * g[row];  gmax/gsum are the global statistics.
-template <typename T>
+// Bound by reading and writing V values per row: 16-byte accesses where the rows of both start on 16-byte boundaries
+// (4608 x 50272 bf16: 442 us with 2-byte accesses, 149 us now, 141 us at copy bandwidth).
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 ce_backward_kernel(const T* __restrict__ logits, long long ld, const long long* __restrict__ labels, int V,
                    int vocab_start, long long ignore_index, const float* __restrict__ gmax,
@@ -528,14 +573,42 @@ ce_backward_kernel(const T* __restrict__ logits, long long ld, const long long* 
   const long long lab = labels[row];
   const float g = (lab == ignore_index) ? 0.f : grow[row];
   const float m = gmax[row], inv = 1.f / gsum[row];
-  const long long loc = lab - vocab_start;
+  const long long at = lab - vocab_start;
+  const int loc = at >= 0 && at < V ? (int)at : -1;
   const T* lr = logits + row * ld;
   T* gr = grad + row * gld;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
+  constexpr int N = LogitVec<T>::N;
+  const int nv = VEC ? V / N : 0;
+  #pragma unroll 4
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    float f[N];
+    LogitVec<T>::load(lr + (long long)i * N, f);
+    const int d = loc - i * N;
+    #pragma unroll
+    for (int e = 0; e < N; ++e) {
+      float p = __expf(f[e] - m) * inv;
+      if (d == e) p -= 1.f;
+      f[e] = p * g;
+    }
+    LogitVec<T>::store(gr + (long long)i * N, f);
+  }
+  for (int i = nv * N + threadIdx.x; i < V; i += blockDim.x) {
     float p = __expf(to_f<T>(lr[i]) - m) * inv;
     if (i == loc) p -= 1.f;
-    p *= g;
-    if constexpr (sizeof(T) == 2) gr[i] = __float2bfloat16(p); else gr[i] = p;
+    gr[i] = from_f<T>(p * g);
+  }
+}
+
+// bf16 rows (stride ld, 16-byte aligned, n a multiple of 8) to contiguous fp32 rows; bound by the 6 bytes per value
+__global__ void __launch_bounds__(256)
+widen_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restrict__ out, int n) {
+  const __nv_bfloat16* xr = x + (long long)blockIdx.y * ld;
+  float* o = out + (long long)blockIdx.y * n;
+  #pragma unroll 4
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 8; i += gridDim.x * blockDim.x) {
+    float f[8];
+    load8(xr + (long long)i * 8, f);
+    store8f(o + (long long)i * 8, f);
   }
 }
 
@@ -594,15 +667,32 @@ rope_kernel(const __nv_bfloat16* __restrict__ x, long long x_ld, __nv_bfloat16* 
 
 // Row statistics that a GEMM epilogue produced per column tile -> one (max, sum exp(x - max)) per row.
 // tmax / tsum: [tiles][rows].
+// Bound by latency (a few MB): the tiles of a row are dealt to eight thread groups, four loads in flight each, and the
+// groups' results meet in shared memory (one thread per row walking all tiles twice: 49 us for 8192 rows x 197 tiles).
 __global__ void __launch_bounds__(256)
 ce_merge_tiles_kernel(const float* __restrict__ tmax, const float* __restrict__ tsum, int tiles, long long rows,
                       float* __restrict__ omax, float* __restrict__ osum) {
-  const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  float m = -INFINITY;
-  for (int t = 0; t < tiles; ++t) m = fmaxf(m, tmax[(long long)t * rows + r]);
-  float s = 0.f;
-  for (int t = 0; t < tiles; ++t) s += tsum[(long long)t * rows + r] * __expf(tmax[(long long)t * rows + r] - m);
+  __shared__ float sm[8][33], ss[8][33];
+  const int tx = threadIdx.x & 31, tg = threadIdx.x >> 5;
+  const long long r = (long long)blockIdx.x * 32 + tx;
+  float m = -INFINITY, s = 0.f;
+  if (r < rows) {
+    #pragma unroll 4
+    for (int t = tg; t < tiles; t += 8) {
+      const float tm = tmax[(long long)t * rows + r], ts = tsum[(long long)t * rows + r];
+      const float mx = fmaxf(m, tm), ref = ce_ref(mx);
+      s = s * __expf(m - ref) + ts * __expf(tm - ref);
+      m = mx;
+    }
+  }
+  sm[tg][tx] = m; ss[tg][tx] = s;
+  __syncthreads();
+  if (tg != 0 || r >= rows) return;
+  #pragma unroll
+  for (int k = 1; k < 8; ++k) m = fmaxf(m, sm[k][tx]);
+  s = 0.f;
+  #pragma unroll
+  for (int k = 0; k < 8; ++k) s += ss[k][tx] * __expf(sm[k][tx] - ce_ref(m));
   omax[r] = m;
   osum[r] = s;
 }
@@ -993,8 +1083,11 @@ extern "C" int ssm_ce_partials(const void* logits, long long ld, int is_fp32, co
                                int vocab_start, void* omax, void* osum, void* otgt, cudaStream_t st) {
   auto lb = reinterpret_cast<const long long*>(labels);
   auto a = reinterpret_cast<float*>(omax); auto b = reinterpret_cast<float*>(osum); auto c = reinterpret_cast<float*>(otgt);
-  if (is_fp32) ce_partials_kernel<float><<<(unsigned)rows, 256, 0, st>>>(reinterpret_cast<const float*>(logits), ld, lb, V, vocab_start, a, b, c);
-  else ce_partials_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>(BF(logits), ld, lb, V, vocab_start, a, b, c);
+  const bool vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && ld % (is_fp32 ? 4 : 8) == 0;
+  #define CE_PARTIALS(T, VEC) ce_partials_kernel<T, VEC><<<(unsigned)rows, 256, 0, st>>>(reinterpret_cast<const T*>(logits), ld, lb, V, vocab_start, a, b, c)
+  if (is_fp32) { if (vec) CE_PARTIALS(float, true); else CE_PARTIALS(float, false); }
+  else { if (vec) CE_PARTIALS(__nv_bfloat16, true); else CE_PARTIALS(__nv_bfloat16, false); }
+  #undef CE_PARTIALS
   return (int)cudaGetLastError();
 }
 SSM_DEBUG_BOUNDS_GETTER(ssm_debug_bounds_elementwise)
@@ -1015,7 +1108,7 @@ extern "C" int ssm_rope(const void* x, long long x_ld, void* out, long long out_
 extern "C" int ssm_ce_merge_tiles(const void* tmax, const void* tsum, int tiles, long long rows, void* omax, void* osum,
                                   cudaStream_t st) {
   if (tiles < 1 || rows < 1) return -SSM_ERR_BAD_ARG;
-  ce_merge_tiles_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(
+  ce_merge_tiles_kernel<<<(unsigned)((rows + 31) / 32), 256, 0, st>>>(
       reinterpret_cast<const float*>(tmax), reinterpret_cast<const float*>(tsum), tiles, rows,
       reinterpret_cast<float*>(omax), reinterpret_cast<float*>(osum));
   return (int)cudaGetLastError();
@@ -1026,8 +1119,20 @@ extern "C" int ssm_ce_backward(const void* logits, long long ld, int is_fp32, co
   auto lb = reinterpret_cast<const long long*>(labels);
   auto a = reinterpret_cast<const float*>(gmax); auto b = reinterpret_cast<const float*>(gsum);
   auto c = reinterpret_cast<const float*>(grow);
-  if (is_fp32) ce_backward_kernel<float><<<(unsigned)rows, 256, 0, st>>>(reinterpret_cast<const float*>(logits), ld, lb, V, vocab_start, ignore_index, a, b, c, reinterpret_cast<float*>(grad), gld);
-  else ce_backward_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>(BF(logits), ld, lb, V, vocab_start, ignore_index, a, b, c, BFM(grad), gld);
+  const int per16 = is_fp32 ? 4 : 8;
+  const bool vec = ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0 && ld % per16 == 0 && gld % per16 == 0;
+  #define CE_BACKWARD(T, VEC) ce_backward_kernel<T, VEC><<<(unsigned)rows, 256, 0, st>>>(reinterpret_cast<const T*>(logits), ld, lb, V, vocab_start, ignore_index, a, b, c, reinterpret_cast<T*>(grad), gld)
+  if (is_fp32) { if (vec) CE_BACKWARD(float, true); else CE_BACKWARD(float, false); }
+  else { if (vec) CE_BACKWARD(__nv_bfloat16, true); else CE_BACKWARD(__nv_bfloat16, false); }
+  #undef CE_BACKWARD
+  return (int)cudaGetLastError();
+}
+
+extern "C" int ssm_widen(const void* x, long long ld, void* out, long long rows, int n, cudaStream_t st) {
+  if (rows < 1 || rows > 65535 || n < 8 || n % 8 || ld % 8 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return -SSM_ERR_BAD_ARG;
+  const int blocks = (n / 8 + 1023) / 1024;
+  widen_kernel<<<dim3((unsigned)blocks, (unsigned)rows), 256, 0, st>>>(BF(x), ld, reinterpret_cast<float*>(out), n);
   return (int)cudaGetLastError();
 }
 

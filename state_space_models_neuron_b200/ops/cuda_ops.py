@@ -560,6 +560,18 @@ def ce_backward(logits, labels, row_max, row_sum, grad_rows, vocab_start, ignore
     return grad
 
 
+def widen(x):
+    """fp32 copy of bf16 `x` [..., n] (rows may be padded); inference only, the gradient path keeps `x.float()`."""
+    n = x.shape[-1]
+    x2 = x.reshape(-1, n) if x.dim() != 2 else x
+    if (x.dtype != torch.bfloat16 or x2.shape[0] == 0 or x2.shape[0] > 65535 or n % 8 or n == 0 or x2.stride(1) != 1
+            or x2.stride(0) % 8 or x2.data_ptr() % 16):
+        return x.float()
+    out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    _run("ssm_widen", _p(x2), _ll(x2.stride(0)), _p(out), _ll(x2.shape[0]), n, _st())
+    return out
+
+
 # ======================================================================================
 # optimizer
 # ======================================================================================

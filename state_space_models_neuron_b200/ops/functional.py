@@ -211,6 +211,13 @@ def ce_partials(logits, labels, vocab_start: int):
     return oracle.ce_partials(logits, labels, vocab_start)
 
 
+def widen(x):
+    """x in fp32."""
+    if _native(x) and not (torch.is_grad_enabled() and x.requires_grad):
+        return _cuda().widen(x)
+    return x.float()
+
+
 def ce_backward(logits, labels, row_max, row_sum, grad_rows, vocab_start: int, ignore_index: int):
     """d loss / d logits for the local vocab shard: (softmax - onehot) * grad_rows."""
     if _native(logits):

@@ -1,0 +1,62 @@
+"""Cross-entropy kernels at the edges of their 16-byte path, and the loss taken in the LM head's GEMM."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("V", [1, 7, 8, 9, 255, 2048, 2055, 50288])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("pad", [0, 8, 5])          # extra elements per row: aligned rows, and rows that are not
+def test_partials_and_backward(V, dtype, pad):
+    from state_space_models_neuron_b200.ops import cuda_ops
+    rows, gen = 5, torch.Generator(device="cuda").manual_seed(V + pad)
+    store = (torch.randn(rows, (V + 7) // 8 * 8 + pad, device="cuda", generator=gen) * 30).to(dtype)
+    x = store[:, :V]
+    x[1] = -200.0                                   # far from zero: the exponent is relative to the maximum
+    x[2, : V // 2] = float("-inf")                  # masked entries
+    labels = torch.randint(0, V, (rows,), device="cuda", generator=gen)
+    labels[3], labels[4] = -100, V + 3              # ignored; another shard's id
+    m, s, t = cuda_ops.ce_partials(x, labels, 0)
+    ref = x.double()
+    assert torch.equal(m.double(), ref.max(1).values)
+    # fp32 exponentials (2 ulp) of arguments up to 2^8 (2^-24 relative each) and a sum of V terms
+    assert torch.allclose(s.double(), (ref - ref.max(1, keepdim=True).values).exp().sum(1), rtol=1e-4)
+    assert torch.equal(t[:3].double(), ref.gather(1, labels[:3, None])[:, 0]) and (t[3:] == 0).all()
+    g = torch.rand(rows, device="cuda", generator=gen)
+    grad = cuda_ops.ce_backward(x, labels, m, s, g, 0, -100)
+    p = torch.softmax(ref, 1)
+    p[torch.arange(3), labels[:3]] -= 1
+    want = p * torch.where(labels == -100, 0.0, g.double())[:, None]
+    assert torch.allclose(grad.double(), want, rtol=2 ** -8 if dtype == torch.bfloat16 else 2e-4, atol=2e-6)
+
+
+@pytest.mark.parametrize("V", [512, 1000])
+def test_loss_of_labelled_forward(V):
+    """forward(labels=...) returns fp32 logits and the mean loss of the shifted labels, with the same gradients as the
+    loss computed from those logits."""
+    from state_space_models_neuron_b200.models import Mamba2Config, Mamba2ForCausalLM
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    cfg = Mamba2Config(num_heads=8, head_dim=64, vocab_size=V, hidden_size=256, state_size=128, num_hidden_layers=1,
+                       n_groups=1, initializer_range=0.02, dtype=torch.bfloat16)
+    model = Mamba2ForCausalLM(cfg, device="cuda").to(torch.bfloat16)
+    ids = torch.randint(0, V, (2, 128), device="cuda")
+    ids[0, 5:9] = -100
+    inputs = ids.clamp(min=0)
+    out = model(input_ids=inputs, labels=ids)
+    valid = ids[:, 1:] != -100
+    per_token = torch.nn.functional.cross_entropy(out.logits[:, :-1].reshape(-1, V), ids[:, 1:].reshape(-1), reduction="none",
+                                                  ignore_index=-100)
+    want = per_token.sum() / valid.numel()
+    assert out.logits.dtype == torch.float32
+    assert abs(out.loss.item() - want.item()) < 1e-5 * abs(want.item())
+    w = model.lm_head.weight
+    grad, = torch.autograd.grad(out.loss, w, retain_graph=True)
+    ref, = torch.autograd.grad(want, w)
+    # both round d(logits) to bf16 once and accumulate in fp32
+    assert ((grad - ref).float().norm() / ref.float().norm()).item() < 2 ** -7
+    with torch.no_grad():
+        again = model(input_ids=inputs, labels=ids)
+    assert torch.equal(again.logits, out.logits)
