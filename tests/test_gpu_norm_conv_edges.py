@@ -1,0 +1,65 @@
+"""Norm and conv kernels at the edges of their thread and tile shapes, forward and backward, against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _near(got, want, steps=3):
+    # one bf16 rounding of the result; where a result is a difference, of its terms (the scale of the tensor)
+    bound = steps * 2.0 ** -8 * (want.abs() + want.abs().mean())
+    assert ((got.double() - want).abs() <= bound).all(), ((got.double() - want).abs() / bound).max().item()
+
+
+@pytest.mark.parametrize("d,groups", [(8, 1), (264, 1), (2048, 1), (2056, 1), (5120, 1), (8192, 1), (4096, 8)])
+@pytest.mark.parametrize("rows", [1, 297, 601])              # fewer rows than blocks, one more, an uneven share
+@pytest.mark.parametrize("gate", [True, False])
+def test_norms(d, groups, rows, gate):
+    from state_space_models_neuron_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(d + rows)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+    y, z, w, dout = make(rows, d), make(rows, d), make(d), make(rows, d)
+    for t in (y, z, w):
+        t.requires_grad_()
+    out = ops.gated_rmsnorm(y, z if gate else None, w, 1e-5, d // groups)
+    Y, Z, W = (t.detach().double().requires_grad_() for t in (y, z, w))
+    h = (Y * torch.nn.functional.silu(Z) if gate else Y).view(rows, groups, -1)
+    ref = (h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-5)).view(rows, d) * W
+    _near(out, ref)
+    out.backward(dout)
+    ref.backward(dout.double())
+    _near(y.grad, Y.grad)
+    _near(w.grad, W.grad)
+    if gate:
+        _near(z.grad, Z.grad)
+    elif groups == 1:
+        for rd in (torch.bfloat16, torch.float32):
+            x, res, dres = make(rows, d).requires_grad_(), torch.randn(rows, d, device="cuda", generator=gen).to(rd), make(rows, d).to(rd)
+            got, total = ops.add_rmsnorm(x, res, w, 1e-5, rd)
+            s = (x.detach().double() + res.double()).to(rd).double().requires_grad_()
+            want = s * torch.rsqrt(s.square().mean(-1, keepdim=True) + 1e-5) * W
+            _near(got, want)
+            gx, = torch.autograd.grad((got, total), x, (dout, dres))
+            gs, = torch.autograd.grad(want, s, dout.double())
+            _near(gx, gs + dres.double())
+
+
+@pytest.mark.parametrize("L", [1, 3, 8, 33, 35, 130])        # remainders of the token tiles and of the batches of four
+@pytest.mark.parametrize("C", [8, 520, 10240])
+@pytest.mark.parametrize("init", [True, False])
+def test_conv(L, C, init):
+    from state_space_models_neuron_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(L + C)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+    x, w, b, dy = make(2, L, C).requires_grad_(), make(C, 1, 4).requires_grad_(), make(C).requires_grad_(), make(2, L, C)
+    before = make(2, 3, C) if init else None
+    out = ops.causal_conv1d_silu(x, w, b, before)
+    X, W, Bs = (t.detach().double().requires_grad_() for t in (x, w, b))
+    pad = torch.cat([before.double() if init else X.new_zeros(2, 3, C), X], 1)
+    ref = torch.nn.functional.silu(sum(pad[:, k:k + L] * W[:, 0, k] for k in range(4)) + Bs)
+    _near(out, ref)
+    if not init:                                               # the backward kernel takes the tokens before the first as zeros
+        out.backward(dy)
+        ref.backward(dy.double())
+        for got, want in ((x, X), (w, W), (b, Bs)):
+            _near(got.grad, want.grad)
