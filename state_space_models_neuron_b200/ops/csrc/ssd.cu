@@ -206,6 +206,171 @@ ssd_state_pass_kernel(const float* __restrict__ local, const float* __restrict__
 }
 
 // =====================================================================================
+// chunk states and their recurrence in one kernel (the two kernels above without the fp32 states in between):
+//   in[c] = run ; run = exp(l_T[c]) * run + sum_j s_j W[j][n] V[j][p]       c ascending (mode 0) or descending (mode 1)
+// One CTA per (head slice, batch) walks the chunks; the running state stays in registers (256 threads: row n = tid & 127,
+// 32 of the 64 channels each).  Loads run three chunks ahead; the products of the next chunk run on tcgen05 (two TMEM
+// buffers) while this one's state is stored and updated.
+// Bound by latency per chunk (wait, scale V, products, update) at few heads, by HBM at many (V in, bf16 states out): the
+// fp32 states, written and read back, were two thirds of the bytes.
+// =====================================================================================
+struct StateWalkParams {
+  const float* dt; const float* l;       // [B, H, L]
+  const float* init; float* fin;         // fp32 [B, Hv, 128, 64] or null
+  int L, H, Hv, G, nc, w_col0, mode;
+  int* status;
+};
+constexpr int WALK_STAGES = 3;
+constexpr int WALK_STAGE_BYTES = TILE128 + TILE64;
+constexpr int WALK_SMEM = WALK_STAGES * WALK_STAGE_BYTES + 2 * TILE64 + 128 + 1024;
+
+__global__ void __launch_bounds__(256, 1)
+ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_v,
+                      const __grid_constant__ CUtensorMap tm_in, const StateWalkParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sOut = smem + WALK_STAGES * WALK_STAGE_BYTES;                 // two staging tiles for the bf16 states
+  uint64_t* full = reinterpret_cast<uint64_t*>(sOut + 2 * TILE64);       // [stage] loads landed
+  uint64_t* done = full + WALK_STAGES;                                   // [2] products of a TMEM buffer complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 2);
+  const int hv = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5;
+  const int row = tid & 127, half = tid >> 7;
+  const int h = hv / (p.Hv / p.H), g = h / (p.H / p.G);
+  const float* lh = p.l + ((long long)b * p.H + h) * p.L;
+  const float* dth = p.dt + ((long long)b * p.H + h) * p.L;
+  auto chunk = [&](int k) { return p.mode == 0 ? k : p.nc - 1 - k; };    // chunk of step k
+
+  if (tid == 0) {
+    for (int s = 0; s < WALK_STAGES; ++s) mbar_init(&full[s], 1);
+    mbar_init(&done[0], 1); mbar_init(&done[1], 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tm_w); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_in);
+  }
+  if (warp == 0) { tmem_alloc(tmem_slot, 128); tmem_relinquish(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+
+  auto load = [&](int k) {                                               // thread 0
+    const int st = k % WALK_STAGES, r = b * p.L + chunk(k) * CT;
+    uint8_t* sw = smem + st * WALK_STAGE_BYTES;
+    mbar_expect_tx(&full[st], WALK_STAGE_BYTES);
+    tma_load_2d(sw, &tm_w, p.w_col0 + g * NS, r, &full[st]);
+    tma_load_2d(sw + TILE128 / 2, &tm_w, p.w_col0 + g * NS + 64, r, &full[st]);
+    tma_load_2d(sw + TILE128, &tm_v, hv * PS, r, &full[st]);
+  };
+  int loaded = 0;                                                        // steps whose loads have been issued (thread 0)
+  if (tid == 0)
+    for (; loaded < WALK_STAGES && loaded < p.nc; ++loaded) load(loaded);
+  // scaling of a step: l_j, l_T and dt_j of this thread's row, fetched a step ahead
+  float lj = 0.f, lT = 0.f, dtj = 0.f;
+  auto fetch = [&](int k) {
+    if (k >= p.nc) return;
+    const long long o = (long long)chunk(k) * CT;
+    lj = lh[o + row]; lT = lh[o + CT - 1]; dtj = dth[o + row];
+  };
+  // V rows of step k scaled in place, then its products issued into TMEM buffer k & 1
+  bool ok = true;
+  auto scale_and_issue = [&](int k) {
+    const int st = k % WALK_STAGES;
+    uint8_t* sw = smem + st * WALK_STAGE_BYTES;
+    uint8_t* sv = sw + TILE128;
+    const float s = p.mode == 0 ? __expf(lT - lj) * dtj : __expf(lj);
+    ok = mbar_wait(&full[st], (k / WALK_STAGES) & 1, p.status);
+    if (ok) {
+      #pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint4* at = reinterpret_cast<uint4*>(sv + sw128_offset(row, half * 4 + q));
+        float f[8];
+        unpack8(*at, f);
+        #pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] *= s;
+        *at = pack8(f);
+      }
+    }
+    fence_proxy_async_smem();
+    ok = __syncthreads_and(ok);
+    if (tid == 0 && ok) {
+      tc_fence_after_sync();
+      const uint32_t idesc = make_idesc_bf16(128, PS, 1, 1);
+      const uint32_t aw = smem_u32(sw), av = smem_u32(sv);
+      #pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma_bf16(tmem + (k & 1) * 64, desc_mnmajor(aw, kk, TILE128 / 2), desc_mnmajor(av, kk, 0), idesc, kk != 0);
+      umma_commit(&done[k & 1]);
+    }
+    __syncwarp();
+  };
+
+  const long long state = ((long long)b * p.Hv + hv) * (NS * PS) + row * PS + half * 32;
+  float run[32];
+  #pragma unroll
+  for (int e = 0; e < 32; e += 4) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.init != nullptr) v = *reinterpret_cast<const float4*>(p.init + state + e);
+    run[e] = v.x; run[e + 1] = v.y; run[e + 2] = v.z; run[e + 3] = v.w;
+  }
+  fetch(0);
+  float dec = __expf(lT);                                                // of the step whose products are in flight
+  scale_and_issue(0);
+  fetch(1);
+  for (int k = 0; k < p.nc && ok; ++k) {
+    const float dec_k = dec;
+    // the state that enters step k's chunk
+    uint8_t* so = sOut + (k & 1) * TILE64;
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float f[8];
+      #pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = run[q * 8 + e];
+      *reinterpret_cast<uint4*>(so + sw128_offset(row, half * 4 + q)) = pack8(f);
+    }
+    if (k + 1 < p.nc) {
+      dec = __expf(lT);
+      scale_and_issue(k + 1);                                            // its barrier also covers the staging tile
+      if (!ok) break;
+      fetch(k + 2);
+    } else {
+      fence_proxy_async_smem();
+      __syncthreads();
+    }
+    if (tid == 0) {
+      tma_store_2d(&tm_in, so, 0, ((b * p.Hv + hv) * p.nc + chunk(k)) * NS);
+      tma_store_commit();
+    }
+    ok = mbar_wait(&done[k & 1], (k >> 1) & 1, p.status);
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after_sync();
+    if (tid == 0 && ok && loaded < p.nc) { load(loaded); ++loaded; }     // step k's stage is free again
+    if (ok) {
+      uint32_t v[32];
+      tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, (k & 1) * 64 + half * 32), v);
+      tmem_ld_wait();
+      #pragma unroll
+      for (int e = 0; e < 32; ++e) run[e] = dec_k * run[e] + __uint_as_float(v[e]);
+    }
+    tc_fence_before_sync();
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // step k - 1's tile has been read
+    ok = __syncthreads_and(ok);                                          // TMEM buffer and staging tile are free again
+  }
+  if (ok && p.fin != nullptr) {
+    #pragma unroll
+    for (int e = 0; e < 32; e += 4)
+      *reinterpret_cast<float4*>(p.fin + state + e) = make_float4(run[e], run[e + 1], run[e + 2], run[e + 3]);
+  }
+  if (tid == 0) {
+    tma_store_wait_all();
+    if (!ok)                                                             // copies still in flight land before the CTA goes
+      for (int k = loaded > WALK_STAGES ? loaded - WALK_STAGES : 0; k < loaded; ++k)
+        mbar_wait(&full[k % WALK_STAGES], (k / WALK_STAGES) & 1, nullptr);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 128);
+}
+
+// =====================================================================================
 // forward chunk scan.  grid (nc, Hv, B), 128 threads, 2 CTAs / SM.
 // TMEM: [0,128) CB^T product, [128,192) Y_diag, [192,256) Y_off.
 // smem: C tile | B tile | x tile | S_in tile ; the decay-weighted matrix reuses the C tile, the output
@@ -758,6 +923,30 @@ extern "C" int ssm_ssd_state_pass(const void* local, const void* l, const void* 
                                               reinterpret_cast<const float*>(init),
                                               reinterpret_cast<__nv_bfloat16*>(in16), reinterpret_cast<float*>(fin), L,
                                               H, Hv, L / CT, reverse);
+  return (int)cudaGetLastError();
+}
+
+// w_src as in ssm_ssd_chunk_state; v: bf16 [B*L, Hv*64] columns at v (row stride v_stride).  in16 bf16 [B,Hv,nc,128,64] is
+// written, init / fin fp32 [B,Hv,128,64] are optional.
+extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_cols, int w_col0, const void* v,
+                                  long long v_stride, const void* dt, const void* l, const void* init, void* in16, void* fin,
+                                  int B, int L, int H, int Hv, int G, int mode, int* status, cudaStream_t st) {
+  if (L % CT || Hv % H || H % G || w_stride % 8 || v_stride % 8 || B < 1 || B > 65535) return -SSM_ERR_BAD_ARG;
+  static bool cfg = false;
+  if (!cfg) { int e = smem_opt_in((const void*)ssd_state_walk_kernel, WALK_SMEM); if (e) return e; cfg = true; }
+  const int nc = L / CT;
+  CUtensorMap tw, tv, ti;
+  int r = make_tmap_2d_bf16(&tw, w_src, (uint64_t)w_cols, (uint64_t)B * L, (uint64_t)w_stride * 2, 64, 128);
+  if (r) return -100 - r;
+  r = make_tmap_2d_bf16(&tv, v, (uint64_t)Hv * PS, (uint64_t)B * L, (uint64_t)v_stride * 2, 64, 128);
+  if (r) return -200 - r;
+  r = make_tmap_2d_bf16(&ti, in16, 64, (uint64_t)B * Hv * nc * NS, 128, 64, 128);
+  if (r) return -300 - r;
+  StateWalkParams p;
+  p.dt = reinterpret_cast<const float*>(dt); p.l = reinterpret_cast<const float*>(l);
+  p.init = reinterpret_cast<const float*>(init); p.fin = reinterpret_cast<float*>(fin);
+  p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.w_col0 = w_col0; p.mode = mode; p.status = status;
+  ssd_state_walk_kernel<<<dim3(Hv, B), 256, WALK_SMEM, st>>>(tw, tv, ti, p);
   return (int)cudaGetLastError();
 }
 

@@ -608,6 +608,31 @@ def _ssd_dims(d_inner, head_dim, n_groups, d_state):
     return H, psplit, H * psplit
 
 
+def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, L, H, Hv, G, mode):
+    """(bf16 state [B, Hv, nc, 128, 64] on one side of every chunk, fp32 state behind the last one or None).  mode 0: states
+    entering the chunks; mode 1: gradients of the states leaving them (the recurrence runs backwards)."""
+    dev, nc, st = conv_out.device, L // _CT, status_tensor(conv_out.device)
+    states = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev)
+    final = torch.empty(B, Hv, 128, 64, dtype=torch.float32, device=dev) if want_final else None
+    if _walk_states(B * Hv, nc):
+        _run("ssm_ssd_state_walk", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(init),
+             _p(states), _p(final), B, L, H, Hv, G, mode, _p(st), _st())
+        return states, final
+    local = torch.empty(B, Hv, nc, 128, 64, dtype=torch.float32, device=dev)
+    _run("ssm_ssd_chunk_state", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(local),
+         B, L, H, Hv, G, mode, _p(st), _st())
+    _run("ssm_ssd_state_pass", _p(local), _p(l), _p(init), _p(states), _p(final), B, L, H, Hv, mode, _st())
+    return states, final
+
+
+def _walk_states(slices: int, nc: int) -> bool:
+    """One kernel that walks the chunks of a head slice, or one CTA per chunk and a recurrence kernel behind it.  A chunk of
+    the walk takes 1.4 us however few slices walk; the two kernels take 18 ns per slice and chunk (64 slices x 64 chunks:
+    89 us walking, 75 us separately; 128 x 16: 26 and 65; 1280 x 16: 243 and 640) and a second launch, which decides for
+    one or two chunks."""
+    return slices >= 80 or nc <= 2
+
+
 def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner, G, H, Hv, init_state=None,
                  want_final=False):
     """conv_out [B*L, C] bf16 contiguous.  Returns y [B*L, d_inner], dt, l, S_in, final (or None)."""
@@ -618,12 +643,7 @@ def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner,
     dt = torch.empty(B, H, L, dtype=torch.float32, device=dev)
     l = torch.empty_like(dt)
     _run("ssm_ssd_dt_prep", _p(dt_raw2), _ll(dt_raw_stride), _p(dt_bias), _p(A), _p(dt), _p(l), B, L, H, _st())
-    s_local = torch.empty(B, Hv, nc, 128, 64, dtype=torch.float32, device=dev)
-    _run("ssm_ssd_chunk_state", _p(conv_out), _ll(C), C, d_inner, _p(conv_out), _ll(C), _p(dt), _p(l), _p(s_local),
-         B, L, H, Hv, G, 0, _p(st), _st())
-    s_in = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev)
-    final = torch.empty(B, Hv, 128, 64, dtype=torch.float32, device=dev) if want_final else None
-    _run("ssm_ssd_state_pass", _p(s_local), _p(l), _p(init_state), _p(s_in), _p(final), B, L, H, Hv, 0, _st())
+    s_in, final = _chunk_states(conv_out, C, d_inner, conv_out, C, dt, l, init_state, want_final, B, L, H, Hv, G, 0)
     y = torch.empty(B * L, d_inner, dtype=torch.bfloat16, device=dev)
     _run("ssm_ssd_chunk_scan_fwd", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
          B, L, H, Hv, G, d_inner, _p(st), _st())
@@ -650,11 +670,7 @@ def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, 
     nc = L // _CT
     st = status_tensor(dev)
     psplit = Hv // H
-    ds_local = torch.empty(B, Hv, nc, 128, 64, dtype=torch.float32, device=dev)
-    _run("ssm_ssd_chunk_state", _p(conv_out), _ll(C), C, d_inner + G * 128, _p(dy2), _ll(dy2.stride(0)), _p(dt), _p(l),
-         _p(ds_local), B, L, H, Hv, G, 1, _p(st), _st())
-    ds_out = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev)
-    _run("ssm_ssd_state_pass", _p(ds_local), _p(l), _p(None), _p(ds_out), _p(None), B, L, H, Hv, 1, _st())
+    ds_out, _ = _chunk_states(conv_out, C, d_inner + G * 128, dy2, dy2.stride(0), dt, l, None, False, B, L, H, Hv, G, 1)
     dx = torch.empty(B * L, d_inner, dtype=torch.bfloat16, device=dev)
     dBC = torch.zeros(B * L, 2 * G * 128, dtype=torch.float32, device=dev)
     hpart = torch.empty(B * nc, Hv, 3, dtype=torch.float32, device=dev)
