@@ -40,162 +40,239 @@ struct AttnFwdParams {
   int* status;
 };
 
-__global__ void __launch_bounds__(128, 1)
+// Forward: 320 threads for a pair of query tiles (256 queries) of one head.
+//   warps 0-3, 4-7  softmax of the first / second query tile, thread = query row (the row's 128 scores in registers)
+//   warp 8          issues all products;  warp 9  loads K and V tiles through a ring of three
+// The two tiles take turns: while one group's exponentials keep the special-function units busy, the tensor cores work on
+// the other's products.  S and O of both tiles fill the 512 TMEM columns.  O is rescaled in TMEM only when a row's maximum
+// has grown by more than 2^8 since its last rescaling (the sums use the same stale maximum, so the quotient is exact);
+// P <= 2^8 keeps its relative precision in bf16.
+// Bound by the exponentials (16 per clock and SM: as long as the products of a tile) and the softmax arithmetic around them.
+// One 128-thread group doing everything in turn took 1541 us for 8192 queries of 32 heads, this 695 us (8192 x 16: 870 -> 424, 4096 x 32: 467 -> 248).
+constexpr int ATTN_FWD_THREADS = 320;
+constexpr int KV_RING = 3;
+constexpr int ATTN_FWD_SMEM = (4 + KV_RING) * ATILE + 256 + 1024;
+constexpr float RESCALE_LOG2 = 8.f;
+
+__global__ void __launch_bounds__(ATTN_FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                 const AttnFwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK0 = smem + ATILE;             // K stages at +1, +2 tiles; V stages at +3, +4 tiles
-  uint8_t* sV0 = smem + 3 * ATILE;
-  uint8_t* sP = smem + 5 * ATILE;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * ATILE);   // [0] q, [1..2] kv stage, [3] S ready, [4] PV ready
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5;
-  const int hk = h / (p.Hq / p.Hkv);
-  const int row0 = b * p.L + qt * AT;
+  uint8_t* sQ = smem;                                  // two query tiles
+  uint8_t* sP = smem + 2 * ATILE;                      // two probability tiles, output staging at the end
+  uint8_t* sKV = smem + 4 * ATILE;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (4 + KV_RING) * ATILE);
+  uint64_t *q_full = bars, *full = bars + 1, *empty = full + KV_RING, *s_full = empty + KV_RING, *p_ready = s_full + 2,
+           *o_done = p_ready + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.y, b = blockIdx.z, hk = h / (p.Hq / p.Hkv);
+  const int qtiles = p.L / AT;
+  const int q0 = 2 * ((int)gridDim.x - 1 - (int)blockIdx.x);           // longest walks first
+  const int n0 = q0 + 1, n1 = q0 + 1 < qtiles ? q0 + 2 : 0;            // key tiles of the two query tiles (n1 = 0: none)
+  const int n = n1 > 0 ? n1 : n0;
 
   if (tid == 0) {
-    for (int k = 0; k < 5; ++k) mbar_init(&bars[k], 1);
+    mbar_init(q_full, 1);
+    for (int k = 0; k < KV_RING; ++k) { mbar_init(&full[k], 1); mbar_init(&empty[k], 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_ready[t], 128); mbar_init(&o_done[t], 1); }
     mbar_fence_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_o);
   }
-  if (warp == 0) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  if (warp == 8) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = *tmem_slot;
-  const int ntiles = qt + 1;
+  const uint32_t tmem = *tmem_slot;                    // S of tile t at 128 t, O at 256 + 128 t
 
-  auto load_kv = [&](int j, int stage) {
-    mbar_expect_tx(&bars[1 + stage], 2 * ATILE);
-    const int r = b * p.L + j * AT;
-    uint8_t* dk = sK0 + stage * ATILE;
-    uint8_t* dv = sV0 + stage * ATILE;
-    tma_load_2d(dk, &tm_k, hk * AD, r, &bars[1 + stage]);
-    tma_load_2d(dk + ATILE / 2, &tm_k, hk * AD + 64, r, &bars[1 + stage]);
-    tma_load_2d(dv, &tm_v, hk * AD, r, &bars[1 + stage]);
-    tma_load_2d(dv + ATILE / 2, &tm_v, hk * AD + 64, r, &bars[1 + stage]);
-  };
-  if (tid == 0) {
-    mbar_expect_tx(&bars[0], ATILE);
-    tma_load_2d(sQ, &tm_q, h * AD, row0, &bars[0]);
-    tma_load_2d(sQ + ATILE / 2, &tm_q, h * AD + 64, row0, &bars[0]);
-    load_kv(0, 0);
-  }
-  float o[AD];
-  #pragma unroll
-  for (int d = 0; d < AD; ++d) o[d] = 0.f;
-  float m_run = -INFINITY, l_run = 0.f;
-  const float c = p.scale * LOG2E;
-  bool ok = true;
-  const uint32_t aQ = smem_u32(sQ), aP = smem_u32(sP);
-
-  for (int j = 0; j < ntiles && ok; ++j) {
-    const int st = j & 1;
-    const uint32_t kv_par = (j >> 1) & 1, par = j & 1;
-    if (tid == 0) {
-      if (j + 1 < ntiles) load_kv(j + 1, st ^ 1);        // stage st^1 was released by the barrier ending tile j-1
-      bool good = (j > 0) || mbar_wait(&bars[0], 0, p.status);
-      good = good && mbar_wait(&bars[1 + st], kv_par, p.status);
-      if (good) {
+  // K and V tiles in the order in which they are used: K0, K1, V0, K2, V1, ..., V(n-1)
+  if (warp == 9) {
+    if (lane == 0) {
+      const int qt_n = n1 > 0 ? 2 : 1;
+      mbar_expect_tx(q_full, qt_n * ATILE);
+      for (int t = 0; t < qt_n; ++t) {
+        tma_load_2d(sQ + t * ATILE, &tm_q, h * AD, b * p.L + (q0 + t) * AT, q_full);
+        tma_load_2d(sQ + t * ATILE + ATILE / 2, &tm_q, h * AD + 64, b * p.L + (q0 + t) * AT, q_full);
+      }
+      bool ok = true;
+      int i = 0;
+      for (; i < 2 * n && ok; ++i) {
+        const int s = i % KV_RING;
+        ok = mbar_wait(&empty[s], ((i / KV_RING) & 1) ^ 1, p.status);
+        if (!ok) break;
+        const bool is_v = i == 2 * n - 1 || (i > 0 && (i & 1) == 0);
+        const int j = i == 2 * n - 1 ? n - 1 : is_v ? i / 2 - 1 : (i + 1) / 2;
+        const CUtensorMap* tm = is_v ? &tm_v : &tm_k;
+        uint8_t* dst = sKV + s * ATILE;
+        mbar_expect_tx(&full[s], ATILE);
+        tma_load_2d(dst, tm, hk * AD, b * p.L + j * AT, &full[s]);
+        tma_load_2d(dst + ATILE / 2, tm, hk * AD + 64, b * p.L + j * AT, &full[s]);
+      }
+      if (!ok) {                                       // copies still in flight land before the CTA goes
+        mbar_wait(q_full, 0, nullptr);
+        for (int k = i > KV_RING ? i - KV_RING : 0; k < i; ++k) mbar_wait(&full[k % KV_RING], (k / KV_RING) & 1, nullptr);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 8) {
+    if (lane == 0) {
+      const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0), id_o = make_idesc_bf16(128, 128, 0, 1);
+      auto scores = [&](int t, int slot) {             // S_t = Q_t K^T
+        const uint32_t aq = smem_u32(sQ + t * ATILE), ak = smem_u32(sKV + slot * ATILE);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + t * 128, adesc_k(aq, kk), adesc_k(ak, kk), id_s, kk != 0);
+        umma_commit(&s_full[t]);
+      };
+      bool ok = mbar_wait(q_full, 0, p.status) && mbar_wait(&full[0], 0, p.status);
+      if (ok) {
         tc_fence_after_sync();
-        const uint32_t aK = smem_u32(sK0 + st * ATILE);
-        const uint32_t id = make_idesc_bf16(128, 128, 0, 0);
-        #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem, adesc_k(aQ, kk), adesc_k(aK, kk), id, kk != 0);
-        umma_commit(&bars[3]);
+        scores(0, 0);
+        if (n1 > 0) scores(1, 0);
+        umma_commit(&empty[0]);
       }
-    }
-    __syncwarp();
-    ok = __syncthreads_and(mbar_wait(&bars[3], par, p.status));
-    tc_fence_after_sync();
-    if (!ok) break;
-    // ---- online softmax, row = tid
-    const bool diag = (j == qt);
-    float m_new = m_run;
-    #pragma unroll 1
-    for (int jb = 0; jb < 4; ++jb) {
-      uint32_t v[32];
-      tmem_ld32(tmem_addr(tmem, warp * 32, jb * 32), v);
-      tmem_ld_wait();
-      #pragma unroll
-      for (int e = 0; e < 32; ++e)
-        if (!diag || jb * 32 + e <= tid) m_new = fmaxf(m_new, __uint_as_float(v[e]));
-    }
-    const float alpha = exp2f((m_run - m_new) * c);       // m_run = -inf on the first tile -> 0
-    float rsum = 0.f;
-    #pragma unroll 1
-    for (int jb = 0; jb < 4; ++jb) {
-      uint32_t v[32];
-      tmem_ld32(tmem_addr(tmem, warp * 32, jb * 32), v);
-      tmem_ld_wait();
-      #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        float f[8];
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int col = jb * 32 + ch * 8 + e;
-          const float pv = (!diag || col <= tid) ? exp2f((__uint_as_float(v[ch * 8 + e]) - m_new) * c) : 0.f;
-          f[e] = pv;
-          rsum += pv;
+      int used = 1;                                    // ring entries handed out so far
+      for (int j = 0; j < n && ok; ++j) {
+        const bool more = j + 1 < n;
+        const int ik = used, iv = used + (more ? 1 : 0);
+        used = iv + 1;
+        const int sk = ik % KV_RING, sv = iv % KV_RING;
+        bool k_here = false, v_here = false;
+        #pragma unroll 1
+        for (int t = 0; t < 2 && ok; ++t) {
+          const int nt = t == 0 ? n0 : n1;
+          if (j >= nt) continue;
+          ok = mbar_wait(&p_ready[t], j & 1, p.status);
+          if (ok && j + 1 < nt) {
+            if (!k_here) { ok = mbar_wait(&full[sk], (ik / KV_RING) & 1, p.status); k_here = true; }
+            tc_fence_after_sync();
+            if (ok) scores(t, sk);
+            if (ok && (t == 1 || n1 <= j + 1)) umma_commit(&empty[sk]);     // K(j+1) has no further reader
+          }
+          if (ok && !v_here) { ok = mbar_wait(&full[sv], (iv / KV_RING) & 1, p.status); v_here = true; }
+          if (ok) {
+            tc_fence_after_sync();
+            const uint32_t ap = smem_u32(sP + t * ATILE), av = smem_u32(sKV + sv * ATILE);
+            #pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_bf16(tmem + 256 + t * 128, adesc_k(ap, kk), adesc_mn(av, kk), id_o, (j | kk) != 0);
+            umma_commit(&o_done[t]);
+          }
         }
-        tile_store8(sP, tid, jb * 32 + ch * 8, f);
+        if (ok) umma_commit(&empty[sv]);
       }
     }
-    l_run = l_run * alpha + rsum;
-    m_run = m_new;
-    #pragma unroll
-    for (int d = 0; d < AD; ++d) o[d] *= alpha;
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after_sync();
-      const uint32_t aV = smem_u32(sV0 + st * ATILE);
-      const uint32_t id = make_idesc_bf16(128, 128, 0, 1);
-      #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 128, adesc_k(aP, kk), adesc_mn(aV, kk), id, kk != 0);
-      umma_commit(&bars[4]);
-    }
     __syncwarp();
-    ok = __syncthreads_and(mbar_wait(&bars[4], par, p.status));
-    tc_fence_after_sync();
-    if (!ok) break;
-    #pragma unroll
-    for (int db = 0; db < 4; ++db) {
-      uint32_t v[32];
-      tmem_ld32(tmem_addr(tmem, warp * 32, 128 + db * 32), v);
+  } else {
+    const int t = warp >> 2, row = tid & 127, nt = t == 0 ? n0 : n1;
+    const uint32_t lanes = (uint32_t)(warp & 3) * 32;
+    uint8_t* tile = sP + t * ATILE;
+    const float c = p.scale * LOG2E;
+    float m_run = 0.f, l_run = 0.f;
+    bool ok = true;
+    for (int j = 0; j < nt && ok; ++j) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], j & 1, p.status));
+      if (!ok) break;
+      tc_fence_after_sync();
+      uint32_t v[4][32];
+      #pragma unroll
+      for (int i = 0; i < 4; ++i) tmem_ld32(tmem_addr(tmem, lanes, t * 128 + i * 32), v[i]);
       tmem_ld_wait();
+      if (j == nt - 1) {                               // diagonal tile
+        #pragma unroll
+        for (int i = 0; i < 4; ++i)
+          #pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (i * 32 + e > row) v[i][e] = 0xff800000u;          // -inf
+      }
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
       #pragma unroll
-      for (int e = 0; e < 32; ++e) o[db * 32 + e] += __uint_as_float(v[e]);
-    }
-    tc_fence_before_sync();
-    __syncthreads();          // all reads of S / PV and of this K/V stage are done
-  }
-  if (ok) {
-    const float inv = 1.f / l_run;
-    #pragma unroll
-    for (int ch = 0; ch < 16; ++ch) {
-      float f[8];
+      for (int e = 0; e < 32; ++e) {
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], __uint_as_float(v[i][e]));
+      }
+      const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      float alpha = 1.f;
+      bool grow = false;
+      if (j == 0) m_run = top;
+      else if ((top - m_run) * c > RESCALE_LOG2) {
+        grow = true;
+        alpha = exp2f((m_run - top) * c);
+        m_run = top;
+      }
+      const float off = m_run * c;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t pk[64];
       #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = o[ch * 8 + e] * inv;
-      tile_store8(sP, tid, ch * 8, f);
+      for (int i = 0; i < 4; ++i) {
+        #pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          const float a0 = exp2f(fmaf(__uint_as_float(v[i][e]), c, -off));
+          const float a1 = exp2f(fmaf(__uint_as_float(v[i][e + 1]), c, -off));
+          sum[i] += a0 + a1;
+          pk[i * 16 + e / 2] = pack_bf16(a0, a1);
+        }
+      }
+      l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+      if (j > 0) {                                     // P and O are in use until the previous product is complete
+        ok = __all_sync(0xffffffffu, mbar_wait(&o_done[t], (j - 1) & 1, p.status));
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (__any_sync(0xffffffffu, grow)) {
+          #pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            uint32_t o[32];
+            tmem_ld32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 32), o);
+            tmem_ld_wait();
+            #pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+            tmem_st32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 32), o);
+          }
+          tmem_st_wait();
+        }
+      }
+      #pragma unroll
+      for (int q = 0; q < 16; ++q)
+        *reinterpret_cast<uint4*>(tile + (q >> 3) * (ATILE / 2) + sw128_offset(row, q & 7)) =
+            make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      mbar_arrive(&p_ready[t]);
     }
-    p.lse[((long long)b * p.Hq + h) * p.L + qt * AT + tid] = m_run * p.scale + logf(l_run);
+    if (nt > 0) {
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&o_done[t], (nt - 1) & 1, p.status));
+      if (ok) {
+        tc_fence_after_sync();
+        const float inv = 1.f / l_run;
+        #pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+          uint32_t o[32];
+          tmem_ld32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 32), o);
+          tmem_ld_wait();
+          #pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float f[8];
+            #pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(o[q * 8 + e]) * inv;
+            tile_store8(tile, row, i * 32 + q * 8, f);
+          }
+        }
+        p.lse[((long long)b * p.Hq + h) * p.L + (q0 + t) * AT + row] = m_run * p.scale + logf(l_run);
+        fence_proxy_async_smem();
+      }
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
+      if (row == 0 && ok) {
+        tma_store_2d(&tm_o, tile, h * AD, b * p.L + (q0 + t) * AT);
+        tma_store_2d(&tm_o, tile + ATILE / 2, h * AD + 64, b * p.L + (q0 + t) * AT);
+        tma_store_commit();
+        tma_store_wait_all();
+      }
+      tc_fence_before_sync();
+    }
   }
-  fence_proxy_async_smem();
   __syncthreads();
-  if (tid == 0 && ok) {
-    tma_store_2d(&tm_o, sP, h * AD, row0);
-    tma_store_2d(&tm_o, sP + ATILE / 2, h * AD + 64, row0);
-    tma_store_commit();
-    tma_store_wait_all();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256);
+  if (warp == 8) tmem_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -383,7 +460,7 @@ extern "C" int ssm_attn_fwd(const void* q, const void* k, const void* v, void* o
                             int Hkv, int D, float scale, int* status, cudaStream_t st) {
   if (D != AD || L % AT || Hq % Hkv) return -SSM_ERR_BAD_ARG;
   static bool cfg = false;
-  const int smem = 6 * ATILE + 128 + 1024;
+  const int smem = ATTN_FWD_SMEM;
   if (!cfg) {
     cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
@@ -394,8 +471,8 @@ extern "C" int ssm_attn_fwd(const void* q, const void* k, const void* v, void* o
   if (r) return r;
   AttnFwdParams p;
   p.lse = reinterpret_cast<float*>(lse); p.L = L; p.Hq = Hq; p.Hkv = Hkv; p.scale = scale; p.status = status;
-  dim3 grid(L / AT, Hq, B);
-  attn_fwd_kernel<<<grid, 128, smem, st>>>(tq, tk, tv, to, p);
+  dim3 grid((L / AT + 1) / 2, Hq, B);
+  attn_fwd_kernel<<<grid, ATTN_FWD_THREADS, smem, st>>>(tq, tk, tv, to, p);
   return (int)cudaGetLastError();
 }
 
