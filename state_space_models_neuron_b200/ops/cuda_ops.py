@@ -984,7 +984,8 @@ class _Attention(torch.autograd.Function):
         do2 = dout.reshape(B * L, Hq * D)
         if not do2.is_contiguous():
             do2 = do2.contiguous()
-        delta = (do2.view(B, L, Hq, D).float() * out.view(B, L, Hq, D).float()).sum(-1).permute(0, 2, 1).contiguous()
+        delta = torch.empty(B, Hq, L, dtype=torch.float32, device=dout.device)
+        _run("ssm_attn_delta", _p(do2), _p(out), _p(delta), B, L, Hq, D, _st())
         dq32 = torch.zeros(B * L, Hq * D, dtype=torch.float32, device=dout.device)
         dk, dv = torch.empty_like(k2), torch.empty_like(v2)
         _run("ssm_attn_bwd", _p(q2), _p(k2), _p(v2), _p(do2), _p(lse), _p(delta), _p(dq32), _p(dk), _p(dv), B, L, Hq, Hkv,
