@@ -10,6 +10,7 @@ import ctypes
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad as _forward_ad
 
 from . import native
 
@@ -43,7 +44,7 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def _st():
-    return _c.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _c.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ll(v):
@@ -51,6 +52,9 @@ def _ll(v):
 
 
 def status_tensor(device=None) -> torch.Tensor:
+    t = _status.get(device)                 # the device of a tensor carries its index: the key as it is stored
+    if t is not None:
+        return t
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     if device not in _status:
         _status[device] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -66,13 +70,38 @@ def check_status() -> None:
                                "(1: mbarrier wait timed out, 2: flag wait timed out, 3: bad argument)")
 
 
+_functions = {}
+
+
 def _run(name: str, *args):
-    fn = getattr(_lib(), name)
-    fn.restype = _c.c_int
+    fn = _functions.get(name)
+    if fn is None:
+        fn = getattr(_lib(), name)
+        fn.restype = _c.c_int
+        _functions[name] = fn
     code = fn(*args)
     _launches[0] += 1
     if code != 0:
         raise RuntimeError(f"{name} failed with code {code} (negative: argument check, positive: cudaError_t)")
+
+
+class _NoGrad:
+    """What a Function's forward gets in place of its context when nothing is recorded."""
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    def mark_non_differentiable(self, *tensors):
+        pass
+
+
+def _apply(function, *args):
+    """`function.apply`, or its forward alone where autograd would record nothing: entering and leaving an autograd
+    Function costs the host 5 to 10 us per call, half of a small kernel's launch.  Forward-mode differentiation and
+    functorch transforms keep `apply`, which answers them as before."""
+    if torch.is_grad_enabled() or _forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
+        return function.apply(*args)
+    return function.forward(_NoGrad(), *args)
 
 
 def _require_bf16(*ts):
@@ -248,14 +277,14 @@ class _Linear(torch.autograd.Function):
 
 def linear(x, w, bias=None):
     _require_bf16(x, w)
-    return _Linear.apply(x, w, bias)
+    return _apply(_Linear, x, w, bias)
 
 
 def linear_ce(x, w, labels, vocab_start: int = 0):
     """(x w^T, (row max, row sum-exp, target logit)): the LM head with the cross-entropy statistics taken in the
     GEMM epilogue (mamba2/modeling_mamba2.py:498-510 computes them in separate passes over fp32 logits)."""
     _require_bf16(x, w)
-    out = _Linear.apply(x, w, None, labels, int(vocab_start))
+    out = _apply(_Linear, x, w, None, labels, int(vocab_start))
     return out[0], tuple(out[1:])
 
 
@@ -314,7 +343,7 @@ def causal_conv1d_silu(x, weight, bias, initial_state=None):
     _require_bf16(x, weight, bias)
     if weight.shape[-1] != 4:
         raise ValueError("the conv kernel is written for 4 taps")
-    return _Conv.apply(x, weight, bias, initial_state)
+    return _apply(_Conv, x, weight, bias, initial_state)
 
 
 # ======================================================================================
@@ -374,7 +403,7 @@ class _GatedNorm(torch.autograd.Function):
 def gated_rmsnorm(y, z, w, eps, group_size=None):
     _require_bf16(y, z, w)
     gs = y.shape[-1] if group_size is None else group_size
-    return _GatedNorm.apply(y, z, w, eps, gs)
+    return _apply(_GatedNorm, y, z, w, eps, gs)
 
 
 class _AddRMSNorm(torch.autograd.Function):
@@ -419,7 +448,7 @@ class _AddRMSNorm(torch.autograd.Function):
 def add_rmsnorm(x, residual, w, eps, residual_dtype=None):
     _require_bf16(x, w)
     rd = residual_dtype or x.dtype
-    return _AddRMSNorm.apply(x, residual, w, eps, rd)
+    return _apply(_AddRMSNorm, x, residual, w, eps, rd)
 
 
 def rmsnorm(x, w, eps):
@@ -450,7 +479,7 @@ def gelu(x):
     _require_bf16(x)
     if x.numel() % 8:
         return torch.nn.functional.gelu(x)
-    return _Gelu.apply(x)
+    return _apply(_Gelu, x)
 
 
 class _Glu(torch.autograd.Function):
@@ -481,7 +510,7 @@ def glu(h, act: str = "silu"):
     _require_bf16(h)
     if h.shape[-1] % 16 or act not in ("gelu", "silu", "swish"):
         raise ValueError("glu kernel needs an even split into multiples of 8 columns and act in {gelu, silu}")
-    return _Glu.apply(h, 0 if act == "gelu" else 1)
+    return _apply(_Glu, h, 0 if act == "gelu" else 1)
 
 
 # ======================================================================================
@@ -532,7 +561,7 @@ def embedding(ids, w, vocab_start: int = 0):
         inside = (local >= 0) & (local < w.shape[0])
         return torch.nn.functional.embedding(torch.where(inside, local, torch.zeros_like(local)), w) \
             * inside[..., None].to(w.dtype)
-    return _Embedding.apply(ids, w, int(vocab_start))
+    return _apply(_Embedding, ids, w, int(vocab_start))
 
 
 # ======================================================================================
@@ -806,7 +835,7 @@ def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner
     if chunk_size != _CT:
         raise ValueError("the GPU kernels use 128-token chunks")
     gs = d_inner if norm_group_size is None else norm_group_size
-    res = _MixerCore.apply(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim,
+    res = _apply(_MixerCore, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim,
                            eps, gs, recompute, return_final_states)
     if return_final_states:
         return res[0], (res[1], res[2])
@@ -863,7 +892,7 @@ class _SSDScan(torch.autograd.Function):
 def ssd_chunk_scan(x, dt_raw, A, Bm, Cm, D, dt_bias, chunk_size, initial_state, return_final_state):
     if chunk_size != _CT:
         raise ValueError("the GPU kernels use 128-token chunks")
-    return _SSDScan.apply(x, dt_raw, A, Bm, Cm, D, dt_bias, return_final_state, initial_state)
+    return _apply(_SSDScan, x, dt_raw, A, Bm, Cm, D, dt_bias, return_final_state, initial_state)
 
 
 # ======================================================================================
@@ -955,7 +984,7 @@ def apply_rotary(x, cos, sin):
     rd = cos.shape[-1] * 2
     if x.shape[-1] % 8 or rd % 16 or cos.dtype != torch.float32 or cos.shape[0] != x.shape[1]:
         raise ValueError("rotary kernel needs head_dim % 8 == 0, rotary dim % 16 == 0 and fp32 tables of the sequence length")
-    return _Rope.apply(x, cos, sin)
+    return _apply(_Rope, x, cos, sin)
 
 
 # ======================================================================================
@@ -999,4 +1028,4 @@ def attention(q, k, v, causal=True):
         raise NotImplementedError("the GPU attention kernel is causal")
     if q.shape[-1] != 128 or q.shape[1] % 128 or q.shape[1] != k.shape[1]:
         raise ValueError("the GPU attention kernel needs head_dim 128 and equal q/k lengths that are multiples of 128")
-    return _Attention.apply(q, k, v)
+    return _apply(_Attention, q, k, v)
