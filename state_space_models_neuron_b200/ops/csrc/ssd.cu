@@ -40,6 +40,11 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return u;
 }
 
+__device__ __forceinline__ void load8f_smem(const float* p, float (&f)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+
 // block-wide helpers for 128 threads -----------------------------------------------------------------
 __device__ __forceinline__ float warp_sum128(float v) {
   #pragma unroll
@@ -216,7 +221,7 @@ ssd_state_pass_kernel(const float* __restrict__ local, const float* __restrict__
 // =====================================================================================
 struct StateWalkParams {
   const float* dt; const float* l;       // [B, H, L]
-  const float* init; float* fin;         // fp32 [B, Hv, 128, 64] or null
+  const float* init; float* fin;         // fp32 [B, Hv, 128 n, 64 p] in, [B, Hv, 64 p, 128 n] out, or null
   int L, H, Hv, G, nc, w_col0, mode;
   int* status;
 };
@@ -354,10 +359,10 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // step k - 1's tile has been read
     ok = __syncthreads_and(ok);                                          // TMEM buffer and staging tile are free again
   }
-  if (ok && p.fin != nullptr) {
+  if (ok && p.fin != nullptr) {                                          // channel rows, as a decoding cache holds them
+    float* fin = p.fin + ((long long)b * p.Hv + hv) * (NS * PS) + (half * 32) * NS + row;
     #pragma unroll
-    for (int e = 0; e < 32; e += 4)
-      *reinterpret_cast<float4*>(p.fin + state + e) = make_float4(run[e], run[e + 1], run[e + 2], run[e + 3]);
+    for (int e = 0; e < 32; ++e) fin[e * NS] = run[e];
   }
   if (tid == 0) {
     tma_store_wait_all();
@@ -521,6 +526,280 @@ ssd_chunk_scan_fwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __gr
   }
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 256);
+}
+
+// =====================================================================================
+// forward scan in one kernel: the state walk (ascending) and the chunk scan of the same chunk.  One CTA per (head slice,
+// batch); x, B and C of a chunk are read once, the state that enters it goes from registers through shared memory into the
+// product with C, and to HBM only where a backward pass will want it.
+//   warps 0-15  row = token / state row, a quarter of the columns each.  Chunk k:
+//                 c  decay-weighted C B^T                     -> M
+//                 e  state update, C S_in read back
+//                 a  of chunk k + 1: x scaled for the state, entering state to shared memory
+//                 f  y = M x + exp(l_i) C S_in + D x, in place of x
+//   warp 16     issues the products: state and C S_in of k + 1 behind a, M x of k and C B^T of k + 1 behind c
+//   warp 17     loads (two stages) and stores
+// so that every product runs under the arithmetic of another step.  Bound by that arithmetic (one exponential per pair of
+// tokens), the products' reads of shared memory and the hand-overs.  States and scan in kernels of their own wrote and read
+// the states and read x and B twice: 128 slices x 16 chunks 86 -> 51 us, 320 x 16 232 -> 158, 1280 x 16 808 -> 472.
+// TMEM: [0,128) and [128,256) C B^T by turns, [256,320) state, [320,384) C S_in, [384,448) M x.
+// =====================================================================================
+struct WalkScanParams {
+  const float* dt; const float* l; const float* D;    // [B, H, L]; D [H]
+  const float* init; float* fin;         // fp32 [B, Hv, 128 n, 64 p] in, [B, Hv, 64 p, 128 n] out, or null
+  int store_states;                      // write the bf16 state entering every chunk
+  int L, H, Hv, G, nc, d_in;
+  int* status;
+};
+constexpr int WS_THREADS = 18 * 32;
+constexpr int WS_STAGE = 2 * TILE128 + TILE64;                           // B | C | x
+constexpr int WS_USED = 2 * WS_STAGE + 2 * TILE64 + TILE128 + 2 * 2 * CT * 4 + 128;
+constexpr int WS_SMEM = 227 * 1024;                                      // all of it: what is left aligns the tiles
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+__global__ void __launch_bounds__(WS_THREADS, 1)
+ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_constant__ CUtensorMap tm_in,
+                     const __grid_constant__ CUtensorMap tm_y, const WalkScanParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sXs = smem + 2 * WS_STAGE;                  // scaled x [128 j][64 p]
+  uint8_t* sS = sXs + TILE64;                          // entering state [128 n][64 p]
+  uint8_t* sM = sS + TILE64;                           // M [128 i][128 j]
+  float* sLD = reinterpret_cast<float*>(sM + TILE128); // [2] l[128] | dt[128] of a stage's chunk
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sLD + 2 * 2 * CT);
+  uint64_t *full = bars, *cb_done = bars + 2, *st_done = bars + 4, *y_done = bars + 5, *xs_ready = bars + 6,
+           *m_ready = bars + 7, *y_ready = bars + 8, *s_free = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  if (smem - smem_raw > WS_SMEM - WS_USED) {           // uniform; cannot happen while dynamic shared memory starts on 1 KiB
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, SSM_ERR_BAD_ARG);
+    return;
+  }
+  const int hv = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = hv / (p.Hv / p.H), g = h / (p.H / p.G);
+
+  if (tid == 0) {
+    for (int k = 0; k < 6; ++k) mbar_init(&bars[k], 1);
+    for (int k = 6; k < 10; ++k) mbar_init(&bars[k], 16);
+    mbar_init(s_free, 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tm_xbc); tma_prefetch_desc(&tm_in); tma_prefetch_desc(&tm_y);
+  }
+  if (warp == 16) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 17) {
+    if (lane == 0) {
+      const long long lo = ((long long)b * p.H + h) * p.L;
+      auto load = [&](int k) {
+        uint8_t* sb = smem + (k & 1) * WS_STAGE;
+        uint64_t* bar = &full[k & 1];
+        const int r = b * p.L + k * CT, cB = p.d_in + g * NS, cC = p.d_in + p.G * NS + g * NS;
+        mbar_expect_tx(bar, WS_STAGE + 2 * CT * 4);
+        tma_load_2d(sb, &tm_xbc, cB, r, bar);
+        tma_load_2d(sb + TILE128 / 2, &tm_xbc, cB + 64, r, bar);
+        tma_load_2d(sb + TILE128, &tm_xbc, cC, r, bar);
+        tma_load_2d(sb + TILE128 + TILE128 / 2, &tm_xbc, cC + 64, r, bar);
+        tma_load_2d(sb + 2 * TILE128, &tm_xbc, hv * PS, r, bar);
+        bulk_load(sLD + (k & 1) * 2 * CT, p.l + lo + (long long)k * CT, CT * 4, bar);
+        bulk_load(sLD + (k & 1) * 2 * CT + CT, p.dt + lo + (long long)k * CT, CT * 4, bar);
+      };
+      int loaded = 0;
+      for (; loaded < 2 && loaded < p.nc; ++loaded) load(loaded);
+      bool ok = true;
+      for (int k = -1; k < p.nc && ok; ++k) {
+        if (p.store_states && k + 1 < p.nc) {          // the state entering chunk k + 1 is in shared memory
+          ok = mbar_wait(xs_ready, (k + 1) & 1, p.status);
+          if (!ok) break;
+          tma_store_2d(&tm_in, sS, 0, ((b * p.Hv + hv) * p.nc + k + 1) * NS);
+          tma_store_commit();
+          tma_store_wait_read();
+          mbar_arrive(s_free);
+        }
+        if (k >= 0) {                                  // y of chunk k stands in its x tile
+          ok = mbar_wait(&y_ready[k & 1], (k >> 1) & 1, p.status);
+          if (!ok) break;
+          tma_store_2d(&tm_y, smem + (k & 1) * WS_STAGE + 2 * TILE128, hv * PS, b * p.L + k * CT);
+          tma_store_commit();
+          if (loaded < p.nc) { tma_store_wait_read(); load(loaded); ++loaded; }
+        }
+      }
+      tma_store_wait_all();
+      if (!ok)                                         // copies still in flight land before the CTA goes
+        for (int k = loaded > 2 ? loaded - 2 : 0; k < loaded; ++k) mbar_wait(&full[k & 1], (k >> 1) & 1, nullptr);
+    }
+    __syncwarp();
+  } else if (warp == 16) {
+    if (lane == 0) {
+      const uint32_t id_cb = make_idesc_bf16(128, 128, 0, 0), id_st = make_idesc_bf16(128, PS, 1, 1),
+                     id_off = make_idesc_bf16(128, PS, 0, 1);
+      const uint64_t dXs = desc_mnmajor(smem_u32(sXs), 0, 0), dS = desc_mnmajor(smem_u32(sS), 0, 0);
+      // descriptor steps (16-byte units) of a k-step: 32 bytes inside an atom of 64, then the next atom; 16 rows
+      auto kstep = [](int kk) { return (uint64_t)((kk >> 2) * (TILE128 / 2 / 16) + (kk & 3) * 2); };
+      auto issue_cb = [&](int k) {
+        const uint32_t aB = smem_u32(smem + (k & 1) * WS_STAGE);
+        const uint64_t dC = desc_kmajor(aB + TILE128, 0, TILE128 / 2), dB = desc_kmajor(aB, 0, TILE128 / 2);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + (k & 1) * 128, dC + kstep(kk), dB + kstep(kk), id_cb, kk != 0);
+        umma_commit(&cb_done[k & 1]);
+      };
+      bool ok = mbar_wait(&full[0], 0, p.status);
+      if (ok) { tc_fence_after_sync(); issue_cb(0); }
+      auto issue_state = [&](int k) {
+        ok = mbar_wait(xs_ready, k & 1, p.status);
+        if (!ok) return;
+        tc_fence_after_sync();
+        const uint32_t aB = smem_u32(smem + (k & 1) * WS_STAGE);
+        const uint64_t dBm = desc_mnmajor(aB, 0, TILE128 / 2), dC = desc_kmajor(aB + TILE128, 0, TILE128 / 2);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                 // S_local[n][p] = sum_j B[j][n] xs[j][p]
+          umma_bf16(tmem + 256, dBm + (uint64_t)(kk * 128), dXs + (uint64_t)(kk * 128), id_st, kk != 0);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                 // Y_off[i][p] = sum_n C[i][n] S_in[n][p]
+          umma_bf16(tmem + 320, dC + kstep(kk), dS + (uint64_t)(kk * 128), id_off, kk != 0);
+        umma_commit(st_done);
+      };
+      if (ok) issue_state(0);
+      for (int k = 0; k < p.nc && ok; ++k) {
+        ok = mbar_wait(m_ready, k & 1, p.status);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint64_t dM = desc_kmajor(smem_u32(sM), 0, TILE128 / 2),
+                       dX = desc_mnmajor(smem_u32(smem + (k & 1) * WS_STAGE + 2 * TILE128), 0, 0);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                 // Y_diag[i][p] = sum_j M[i][j] x[j][p]
+          umma_bf16(tmem + 384, dM + kstep(kk), dX + (uint64_t)(kk * 128), id_off, kk != 0);
+        umma_commit(y_done);
+        if (k + 1 < p.nc) {
+          ok = mbar_wait(&full[(k + 1) & 1], ((k + 1) >> 1) & 1, p.status);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_cb(k + 1);
+          issue_state(k + 1);
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    const int rw = warp & 3, wq = warp >> 2, row = rw * 32 + lane;      // quarter wq: 16 channels, 32 tokens
+    const uint32_t lanes = (uint32_t)rw * 32;
+    const float Dh = p.D[h];
+    float run[16];
+    #pragma unroll
+    for (int e = 0; e < 16; e += 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.init != nullptr)
+        v = *reinterpret_cast<const float4*>(p.init + ((long long)b * p.Hv + hv) * (NS * PS) + row * PS + wq * 16 + e);
+      run[e] = v.x; run[e + 1] = v.y; run[e + 2] = v.z; run[e + 3] = v.w;
+    }
+    bool ok = true;
+    // what the other warps do with these writes starts when all sixteen warps have arrived
+    auto arrive = [&](uint64_t* bar) {
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto wait = [&](uint64_t* bar, int phase) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, p.status));
+      tc_fence_after_sync();
+    };
+    float li = 0.f, lT = 0.f;                          // of the chunk whose x has been scaled last
+    auto prepare = [&](int k) {                        // a
+      wait(&full[k & 1], k >> 1);
+      if (ok && p.store_states && k > 0) wait(s_free, k - 1);
+      if (!ok) return;
+      const float* sl = sLD + (k & 1) * 2 * CT;
+      li = sl[row]; lT = sl[CT - 1];
+      const float sx = __expf(lT - li) * sl[CT + row];
+      const uint8_t* sX = smem + (k & 1) * WS_STAGE + 2 * TILE128;
+      #pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t off = sw128_offset(row, wq * 2 + q);
+        float f[8];
+        unpack8(*reinterpret_cast<const uint4*>(sX + off), f);
+        #pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] *= sx;
+        *reinterpret_cast<uint4*>(sXs + off) = pack8(f);
+        #pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = run[q * 8 + e];
+        *reinterpret_cast<uint4*>(sS + off) = pack8(f);
+      }
+      arrive(xs_ready);
+    };
+    prepare(0);
+    for (int k = 0; k < p.nc && ok; ++k) {
+      const float lik = li, dec = __expf(lT);
+      const float* sl = sLD + (k & 1) * 2 * CT + wq * 32;
+      // ---- c
+      wait(&cb_done[k & 1], k >> 1);
+      if (!ok) break;
+      uint8_t* m_at = sM + (wq >> 1) * (TILE128 / 2);
+      if (wq > rw) {                                   // tokens j > i for every row of this warp
+        #pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+          *reinterpret_cast<uint4*>(m_at + sw128_offset(row, (wq & 1) * 4 + ch)) = make_uint4(0, 0, 0, 0);
+      } else {
+        uint32_t v[32];
+        tmem_ld32(tmem_addr(tmem, lanes, (k & 1) * 128 + wq * 32), v);
+        tmem_ld_wait();
+        #pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+          float lv[8], dv[8], f[8];
+          load8f_smem(sl + ch * 8, lv);
+          load8f_smem(sl + CT + ch * 8, dv);
+          #pragma unroll
+          for (int e = 0; e < 8; ++e)
+            f[e] = (wq * 32 + ch * 8 + e <= row) ? __uint_as_float(v[ch * 8 + e]) * __expf(lik - lv[e]) * dv[e] : 0.f;
+          *reinterpret_cast<uint4*>(m_at + sw128_offset(row, (wq & 1) * 4 + ch)) = pack8(f);
+        }
+      }
+      arrive(m_ready);
+      // ---- e
+      wait(st_done, k);
+      if (!ok) break;
+      uint32_t v[16], yo[16];
+      tmem_ld16(tmem_addr(tmem, lanes, 256 + wq * 16), v);
+      tmem_ld16(tmem_addr(tmem, lanes, 320 + wq * 16), yo);
+      tmem_ld_wait();
+      #pragma unroll
+      for (int e = 0; e < 16; ++e) run[e] = dec * run[e] + __uint_as_float(v[e]);
+      // ---- a of the next chunk
+      if (k + 1 < p.nc) { prepare(k + 1); if (!ok) break; }
+      // ---- f
+      wait(y_done, k);
+      if (!ok) break;
+      tmem_ld16(tmem_addr(tmem, lanes, 384 + wq * 16), v);
+      tmem_ld_wait();
+      const float al = __expf(lik);
+      uint8_t* sX = smem + (k & 1) * WS_STAGE + 2 * TILE128;
+      #pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint4* at = reinterpret_cast<uint4*>(sX + sw128_offset(row, wq * 2 + q));
+        float xv[8], f[8];
+        unpack8(*at, xv);
+        #pragma unroll
+        for (int e = 0; e < 8; ++e)
+          f[e] = __uint_as_float(v[q * 8 + e]) + al * __uint_as_float(yo[q * 8 + e]) + Dh * xv[e];
+        *at = pack8(f);
+      }
+      arrive(&y_ready[k & 1]);                         // two barriers: the store of a chunk may lag one chunk behind
+    }
+    if (ok && p.fin != nullptr) {                      // channel rows, as a decoding cache holds them
+      float* fin = p.fin + ((long long)b * p.Hv + hv) * (NS * PS) + (wq * 16) * NS + row;
+      #pragma unroll
+      for (int e = 0; e < 16; ++e) fin[e * NS] = run[e];
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 16) tmem_dealloc(tmem, 512);
 }
 
 // =====================================================================================
@@ -927,7 +1206,7 @@ extern "C" int ssm_ssd_state_pass(const void* local, const void* l, const void* 
 }
 
 // w_src as in ssm_ssd_chunk_state; v: bf16 [B*L, Hv*64] columns at v (row stride v_stride).  in16 bf16 [B,Hv,nc,128,64] is
-// written, init / fin fp32 [B,Hv,128,64] are optional.
+// written; init fp32 [B,Hv,128 n,64 p] and fin fp32 [B,Hv,64 p,128 n] are optional.
 extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_cols, int w_col0, const void* v,
                                   long long v_stride, const void* dt, const void* l, const void* init, void* in16, void* fin,
                                   int B, int L, int H, int Hv, int G, int mode, int* status, cudaStream_t st) {
@@ -947,6 +1226,35 @@ extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_c
   p.init = reinterpret_cast<const float*>(init); p.fin = reinterpret_cast<float*>(fin);
   p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.w_col0 = w_col0; p.mode = mode; p.status = status;
   ssd_state_walk_kernel<<<dim3(Hv, B), 256, WALK_SMEM, st>>>(tw, tv, ti, p);
+  return (int)cudaGetLastError();
+}
+
+// The whole forward scan.  xbc as in ssm_ssd_chunk_scan_fwd; s_in (bf16 [B,Hv,nc,128,64], written) or null; init fp32
+// [B,Hv,128 n,64 p] and fin fp32 [B,Hv,64 p,128 n] are optional; y as in ssm_ssd_chunk_scan_fwd.
+extern "C" int ssm_ssd_walk_scan(const void* xbc, long long xbc_stride, int xbc_cols, void* s_in, void* y, long long y_stride,
+                                 const void* dt, const void* l, const void* D, const void* init, void* fin, int B, int L,
+                                 int H, int Hv, int G, int d_in, int* status, cudaStream_t st) {
+  if (L % CT || Hv % H || H % G || xbc_stride % 8 || y_stride % 8 || B < 1 || B > 65535 ||
+      ((reinterpret_cast<uintptr_t>(dt) | reinterpret_cast<uintptr_t>(l)) & 15))
+    return -SSM_ERR_BAD_ARG;
+  static bool cfg = false;
+  if (!cfg) { int e = smem_opt_in((const void*)ssd_walk_scan_kernel, WS_SMEM); if (e) return e; cfg = true; }
+  const int nc = L / CT;
+  CUtensorMap tx, ts, ty;
+  int r = make_tmap_2d_bf16(&tx, xbc, (uint64_t)xbc_cols, (uint64_t)B * L, (uint64_t)xbc_stride * 2, 64, 128);
+  if (r) return -100 - r;
+  ts = tx;
+  if (s_in != nullptr) r = make_tmap_2d_bf16(&ts, s_in, 64, (uint64_t)B * Hv * nc * NS, 128, 64, 128);
+  if (r) return -200 - r;
+  r = make_tmap_2d_bf16(&ty, y, (uint64_t)Hv * PS, (uint64_t)B * L, (uint64_t)y_stride * 2, 64, 128);
+  if (r) return -300 - r;
+  WalkScanParams p;
+  p.dt = reinterpret_cast<const float*>(dt); p.l = reinterpret_cast<const float*>(l);
+  p.D = reinterpret_cast<const float*>(D);
+  p.init = reinterpret_cast<const float*>(init); p.fin = reinterpret_cast<float*>(fin);
+  p.store_states = s_in != nullptr;
+  p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.d_in = d_in; p.status = status;
+  ssd_walk_scan_kernel<<<dim3(Hv, B), WS_THREADS, WS_SMEM, st>>>(tx, ts, ty, p);
   return (int)cudaGetLastError();
 }
 

@@ -638,19 +638,22 @@ def _ssd_dims(d_inner, head_dim, n_groups, d_state):
 
 
 def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, L, H, Hv, G, mode):
-    """(bf16 state [B, Hv, nc, 128, 64] on one side of every chunk, fp32 state behind the last one or None).  mode 0: states
+    """(bf16 state [B, Hv, nc, 128, 64] on one side of every chunk, fp32 state [B, H, P, 128] behind the last one or None).  mode 0: states
     entering the chunks; mode 1: gradients of the states leaving them (the recurrence runs backwards)."""
     dev, nc, st = conv_out.device, L // _CT, status_tensor(conv_out.device)
     states = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev)
-    final = torch.empty(B, Hv, 128, 64, dtype=torch.float32, device=dev) if want_final else None
     if _walk_states(B * Hv, nc):
+        final = torch.empty(B, H, Hv // H * 64, 128, dtype=torch.float32, device=dev) if want_final else None
         _run("ssm_ssd_state_walk", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(init),
              _p(states), _p(final), B, L, H, Hv, G, mode, _p(st), _st())
         return states, final
+    final = torch.empty(B, Hv, 128, 64, dtype=torch.float32, device=dev) if want_final else None
     local = torch.empty(B, Hv, nc, 128, 64, dtype=torch.float32, device=dev)
     _run("ssm_ssd_chunk_state", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(local),
          B, L, H, Hv, G, mode, _p(st), _st())
     _run("ssm_ssd_state_pass", _p(local), _p(l), _p(init), _p(states), _p(final), B, L, H, Hv, mode, _st())
+    if want_final:
+        final = final.transpose(2, 3).reshape(B, H, Hv // H * 64, 128)
     return states, final
 
 
@@ -663,8 +666,9 @@ def _walk_states(slices: int, nc: int) -> bool:
 
 
 def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner, G, H, Hv, init_state=None,
-                 want_final=False):
-    """conv_out [B*L, C] bf16 contiguous.  Returns y [B*L, d_inner], dt, l, S_in, final (or None)."""
+                 want_final=False, want_states=True):
+    """conv_out [B*L, C] bf16 contiguous.  Returns y [B*L, d_inner], dt, l, S_in (None without want_states), final (or
+    None).  The backward pass wants S_in, the states entering the chunks."""
     dev = conv_out.device
     C = conv_out.shape[1]
     nc = L // _CT
@@ -672,8 +676,14 @@ def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner,
     dt = torch.empty(B, H, L, dtype=torch.float32, device=dev)
     l = torch.empty_like(dt)
     _run("ssm_ssd_dt_prep", _p(dt_raw2), _ll(dt_raw_stride), _p(dt_bias), _p(A), _p(dt), _p(l), B, L, H, _st())
-    s_in, final = _chunk_states(conv_out, C, d_inner, conv_out, C, dt, l, init_state, want_final, B, L, H, Hv, G, 0)
     y = torch.empty(B * L, d_inner, dtype=torch.bfloat16, device=dev)
+    if _walk_states(B * Hv, nc):
+        s_in = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev) if want_states else None
+        final = torch.empty(B, H, Hv // H * 64, 128, dtype=torch.float32, device=dev) if want_final else None
+        _run("ssm_ssd_walk_scan", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
+             _p(init_state), _p(final), B, L, H, Hv, G, d_inner, _p(st), _st())
+        return y, dt, l, s_in, final
+    s_in, final = _chunk_states(conv_out, C, d_inner, conv_out, C, dt, l, init_state, want_final, B, L, H, Hv, G, 0)
     _run("ssm_ssd_chunk_scan_fwd", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
          B, L, H, Hv, G, d_inner, _p(st), _st())
     return y, dt, l, s_in, final
@@ -718,13 +728,11 @@ def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, 
     return dx, dBC, hp[:, 0], hp[:, 1], hp[:, 2]
 
 
-def _final_states(final, xBC, H, psplit, K):
-    """kernel state layout [B,Hv,128 n,64 p] -> cache layout [B,H,P,N]; conv window [B,C,K]."""
-    B = final.shape[0]
-    ssm = final.reshape(B, H, psplit, 128, 64).permute(0, 1, 2, 4, 3).reshape(B, H, psplit * 64, 128).contiguous()
-    L = xBC.shape[1]
+def _conv_window(xBC, K):
+    """Last K inputs of the conv, [B, C, K]."""
+    B, L = xBC.shape[0], xBC.shape[1]
     tail = xBC[:, -K:, :] if L >= K else torch.cat([xBC.new_zeros(B, K - L, xBC.shape[2]), xBC], dim=1)
-    return tail.transpose(1, 2).contiguous(), ssm
+    return tail.transpose(1, 2).contiguous()
 
 
 def _mixer_params_fp32(A_log, D, dt_bias):
@@ -743,7 +751,7 @@ def _mixer_params_fp32(A_log, D, dt_bias):
 class _MixerCore(torch.autograd.Function):
     @staticmethod
     def forward(ctx, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, G, N, P, eps, gs, recompute,
-                want_final):
+                want_final, recorded):
         _require_bf16(zxBCdt, conv_w, conv_b, norm_w)
         H, psplit, Hv = _ssd_dims(d_inner, P, G, N)
         B, L, W = zxBCdt.shape
@@ -763,7 +771,7 @@ class _MixerCore(torch.autograd.Function):
         conv_out = _conv_fwd(xBC, w2, conv_b, None).view(B * L, C)
         A, Df, bf = _mixer_params_fp32(A_log, D, dt_bias)
         y, dt, l, s_in, final = _ssd_forward(conv_out, dt_raw2, ld, A, Df, bf, B, L, d_inner, G, H, Hv,
-                                             want_final=want_final)
+                                             want_final=want_final, want_states=recorded and not recompute)
         out = _gated_fwd(y, z2, norm_w, eps, gs)
         ctx.dims = (B, L, W, C, d_inner, G, N, P, H, Hv, eps, gs, recompute)
         if recompute:
@@ -774,9 +782,9 @@ class _MixerCore(torch.autograd.Function):
         ctx.conv_w_param = conv_w if conv_w.is_leaf else None
         out = out.view(B, L, d_inner)
         if want_final:
-            conv_state, ssm_state = _final_states(final, xBC, H, psplit, w2.shape[1])
-            ctx.mark_non_differentiable(conv_state, ssm_state)
-            return out, conv_state, ssm_state
+            conv_state = _conv_window(xBC, w2.shape[1])
+            ctx.mark_non_differentiable(conv_state, final)
+            return out, conv_state, final
         return out
 
     @staticmethod
@@ -818,7 +826,7 @@ class _MixerCore(torch.autograd.Function):
             _run("ssm_mixer_small_grads", _p(cpart), cpart.shape[0], C, _p(gpart), gpart.shape[0], d_inner, _p(hpart),
                  hpart.shape[0], Hv, H, _p(A), _p(mg[0]), _p(mg[1]), _p(mg[2]), _p(mg[3]), _p(mg[4]), _p(mg[5]),
                  mask, _st())
-            return (d_zx,) + (None,) * 14
+            return (d_zx,) + (None,) * 15
         dnorm_w = _gated_bwd(y, z2, norm_w, dout2, eps, gs, dy, dflat[:, :d_inner])
         dx, dBC, dA, dD, dbias = _ssd_backward(conv_out, dy, y, dt, l, s_in, dt_raw2, ld, A, Df, bf,
                                                dflat[:, d_inner + C:], ld, B, L, d_inner, G, H, Hv)
@@ -827,7 +835,7 @@ class _MixerCore(torch.autograd.Function):
         dA_log = (dA * A).to(A_log.dtype)
         return (d_zx, dw.to(w2.dtype).reshape(ctx.conv_w_shape), None if conv_b is None else db.to(conv_b.dtype),
                 dbias.to(dt_bias.dtype), dA_log, dD.to(D.dtype), dnorm_w.to(norm_w.dtype),
-                None, None, None, None, None, None, None, None)
+                None, None, None, None, None, None, None, None, None)
 
 
 def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim, eps,
@@ -836,7 +844,7 @@ def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner
         raise ValueError("the GPU kernels use 128-token chunks")
     gs = d_inner if norm_group_size is None else norm_group_size
     res = _apply(_MixerCore, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim,
-                           eps, gs, recompute, return_final_states)
+                 eps, gs, recompute, return_final_states, torch.is_grad_enabled())
     if return_final_states:
         return res[0], (res[1], res[2])
     return res
@@ -869,9 +877,8 @@ class _SSDScan(torch.autograd.Function):
         ctx.in_dtypes = (dt_raw.dtype, A.dtype, D.dtype, dt_bias.dtype)
         yv = y.view(Bsz, L, H, P)
         if want_final:
-            fin = final.reshape(Bsz, H, psplit, N, 64).permute(0, 1, 2, 4, 3).reshape(Bsz, H, P, N).contiguous()
-            ctx.mark_non_differentiable(fin)
-            return yv, fin
+            ctx.mark_non_differentiable(final)
+            return yv, final
         return yv
 
     @staticmethod

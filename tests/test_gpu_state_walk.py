@@ -32,3 +32,28 @@ def test_walk_equals_separate_kernels(monkeypatch, nc, H, P, G, mode):
     assert ((s0.float() - s1.float()).abs() <= 2.0 ** -7 * s0.float().abs() + 1e-6).all()
     if mode == 0:
         assert torch.allclose(f0, f1, rtol=1e-5, atol=1e-5 * f0.abs().max().item())
+
+
+@pytest.mark.parametrize("nc", [1, 2, 3, 4, 5, 9])             # two stages of loads, products of the next chunk ahead
+@pytest.mark.parametrize("H,P,G", [(4, 64, 1), (6, 128, 2)])
+def test_walk_scan_equals_separate_kernels(monkeypatch, nc, H, P, G):
+    from state_space_models_neuron_b200.ops import cuda_ops
+    B, L, d, Hv = 2, nc * 128, H * P, H * P // 64
+    gen = torch.Generator(device="cuda").manual_seed(nc * 10 + H)
+    xbc = torch.randn(B * L, d + 2 * G * 128, device="cuda", generator=gen).bfloat16()
+    raw = torch.randn(B * L, 8, device="cuda", generator=gen).bfloat16()
+    A, D, bias = -torch.rand(H, device="cuda", generator=gen) * 4, torch.rand(H, device="cuda"), torch.zeros(H, device="cuda")
+    init = torch.randn(B, Hv, 128, 64, device="cuda", generator=gen)
+    out = []
+    for walk in (False, True):
+        monkeypatch.setattr(cuda_ops, "_walk_states", lambda slices, n: walk)
+        out.append(cuda_ops._ssd_forward(xbc, raw, 8, A, D, bias, B, L, d, G, H, Hv, init, True))
+    bare = cuda_ops._ssd_forward(xbc, raw, 8, A, D, bias, B, L, d, G, H, Hv, init, True, want_states=False)
+    torch.cuda.synchronize()
+    cuda_ops.check_status()
+    (y0, _, _, s0, f0), (y1, _, _, s1, f1) = out
+    assert ((s0.float() - s1.float()).abs() <= 2.0 ** -7 * s0.float().abs() + 1e-6).all()
+    assert torch.allclose(f0, f1, rtol=1e-5, atol=1e-5 * f0.abs().max().item())
+    # y: one bf16 step of the result, and one of a state or a weight among the 128 terms of its sums
+    assert ((y0.float() - y1.float()).abs() <= 2.0 ** -7 * (y0.float().abs() + y0.float().abs().mean())).all()
+    assert bare[3] is None and torch.equal(bare[0], y1) and torch.equal(bare[4], f1)
