@@ -803,7 +803,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
 }
 
 // =====================================================================================
-// backward chunk scan.  grid (nc, G * splits, B), 256 threads (two warpgroups), 1 CTA / SM; the CTA walks `hpc` head slices
+// backward chunk scan.  grid (nc, G * splits, B), 1 CTA / SM; the CTA walks `hpc` head slices
 // of one group.  Given dY and, per chunk, S_in (state entering the chunk) and dS_out (gradient of the state
 // leaving the chunk):
 //   CB = C B^T ; dM = dY X^T ; M0 = CB o Lambda ; dCB = dM o Lambda o dt_j
@@ -814,344 +814,432 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
 //          W = dM o M0 o dt_j   (row sums in-thread, column sums by a warp butterfly; no cancellation of large terms)
 //   E = exp(l_T) <dS_out, S_in> + sum_j exp(l_T - l_j) dt_j sum_p x (B dS_out)
 //   dA += sum_j dt_j da_j ; dD += sum dY x ; d(dt_raw) = ddt sigmoid(dt_raw + bias)
+//   warps 0-15  row = token, a quarter of the columns each (16 channels, 32 tokens):
+//                 1  exp(l_T - l_j) dt_j x and exp(l_i) dY       2  M0, dCB and the row / column sums of W
+//                 3  dx and the per-token sums                   4  (warps 0-3, a thread per row) ddt, dA, dD, d dt_bias
+//   warp 16     issues the products: CB, dM behind the loads; dU, C S_in and then dB, dC behind 2
+//   warp 17     loads and the store of dx
+// The loads of the next head start as soon as the last product that reads a tile is complete, 3 runs under the products of
+// dB and dC, 4 under the next head's 1.  Bound by the per-pair arithmetic of 2 and the hand-overs between the steps: with
+// 128-token tiles and four operands per head in shared memory there is room for one head only.
 // TMEM: [0,128) CB then dU_diag | dU_state, [128,256) dM then C S_in, [256,384) dB, [384,512) dC
-// (dB, dC accumulate over the CTA's heads and are added to the fp32 output with red.add).
+// (dB, dC accumulate over the CTA's heads and are added to the fp32 output by bulk reductions).
 // =====================================================================================
 struct ScanBwdParams {
   const float* dt; const float* l; const float* D; const float* A; const float* dt_bias;
   const __nv_bfloat16* dt_raw; long long dt_raw_stride;     // [B*L rows], column h
   __nv_bfloat16* ddt_raw; long long ddt_stride;             // d(dt_raw): row (b*L+t)*stride + h  (bf16, atomic-free when psplit == 1)
   float* ddt32;                                             // [B, Hv, L] fp32 per head slice (summed on the host when psplit > 1)
-  float* dBC;                                               // fp32 [B*L, 2*G*128]
   float* hpart;                                             // fp32 [B*nc, Hv, 3]  (dA, dD, d dt_bias partials)
   int L, H, Hv, G, nc, d_in, hpc;
   int* status;
 };
 
-constexpr int BWD_SMEM = 2 * TILE128 /*C,B*/ + 4 * TILE64 /*X,dY,Sin,dSout*/ + 2 * TILE128 /*M0,dCB*/ + TILE64 /*dY'*/;
+constexpr int BWD_THREADS = 18 * 32;
+// C, B | x, dY, S_in, dS_out | M0, dCB | scaled x, scaled dY | l, dt | sums
+constexpr int BWD_USED = 2 * TILE128 + 4 * TILE64 + 2 * TILE128 + 2 * TILE64 + 2 * CT * 4 + 48 * 4 + 128;
+constexpr int BWD_SMEM = 227 * 1024;                 // all of it: what is left aligns the tiles
 
-// 256 threads = two warpgroups.  Row r = tid & 127 of every 128-row tile is shared by the two threads (r, wg = 0/1):
-// in the operand-building phase warpgroup wg handles the 32-column blocks jb with (jb & 1) == wg, in the scaling
-// and epilogue phases it handles channel half wg (32 of the 64 channels).  Two warps per scheduler hide the
-// TMEM-load / MUFU / shared-memory latencies that a single warpgroup leaves exposed.
-__device__ __forceinline__ float block_sum256(float v, float* red) {   // red: >= 8 floats; two __syncthreads
-  v = warp_sum128(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  return red[0] + red[1] + red[2] + red[3] + red[4] + red[5] + red[6] + red[7];
-}
-
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(BWD_THREADS, 1)
 ssd_chunk_scan_bwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_constant__ CUtensorMap tm_dy,
                           const __grid_constant__ CUtensorMap tm_sin, const __grid_constant__ CUtensorMap tm_dsout,
-                          const __grid_constant__ CUtensorMap tm_dx, const ScanBwdParams p) {
+                          const __grid_constant__ CUtensorMap tm_dx, const __grid_constant__ CUtensorMap tm_dbc,
+                          const ScanBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sC = smem;
   uint8_t* sB = sC + TILE128;
-  uint8_t* sX = sB + TILE128;          // x, later scaled in place, later dx staging
+  uint8_t* sX = sB + TILE128;
   uint8_t* sDY = sX + TILE64;
   uint8_t* sSin = sDY + TILE64;
   uint8_t* sDS = sSin + TILE64;
-  uint8_t* sM0 = sDS + TILE64;
+  uint8_t* sM0 = sDS + TILE64;         // M0; once dU is complete: dx staging | sums
   uint8_t* sDCB = sM0 + TILE128;
-  uint8_t* sDYs = sDCB + TILE128;      // exp(l_i) * dY
+  uint8_t* sXs = sDCB + TILE128;       // exp(l_T - l_j) dt_j x
+  uint8_t* sDYs = sXs + TILE64;        // exp(l_i) dY
   float* s_l = reinterpret_cast<float*>(sDYs + TILE64);
   float* s_dt = s_l + CT;
-  float* s_red = s_dt + CT;            // 16 floats
-  float* s_col = s_red + 16;           // [4 row-warps][128] column sums of W
-  float* s_pair = s_col + 4 * CT;      // [5][128] per-row partials handed from warpgroup 1 to warpgroup 0
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_pair + 5 * CT);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
-
+  float* s_red = s_dt + CT;            // [16] share of E per warp, [16] dD per warp, [4] suffix totals, [4] dA, [4] d dt_bias
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_red + 48);
+  uint64_t *cb_full = bars, *a_full = bars + 1, *b_full = bars + 2, *s_done = bars + 3, *u_done = bars + 4, *g_done = bars + 5,
+           *m0_free = bars + 6, *ops_ready = bars + 7, *e_done = bars + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  float* s_col = reinterpret_cast<float*>(sM0 + TILE64);               // [4 row-warps][128] column sums of W
+  float* s_part = s_col + 4 * CT;                                      // [4 sums][4 quarters][128 rows]
+  if (smem - smem_raw > BWD_SMEM - BWD_USED) {         // uniform; cannot happen while dynamic shared memory starts on 1 KiB
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, SSM_ERR_BAD_ARG);
+    return;
+  }
   const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = tid & 127, wg = tid >> 7, rw = warp & 3;      // tile row, warpgroup, row-warp (TMEM lane quarter)
   const int psplit = p.Hv / p.H;
   const int hv_per_group = (p.H / p.G) * psplit;
   const int splits = hv_per_group / p.hpc;
   const int g = blockIdx.y / splits;
   const int hv0 = g * hv_per_group + (blockIdx.y % splits) * p.hpc;
   const int row0 = b * p.L + c * CT;
+  const int GN = p.G * NS;
 
   if (tid == 0) {
-    for (int k = 0; k < 4; ++k) mbar_init(&bars[k], 1);
+    for (int k = 0; k < 7; ++k) mbar_init(&bars[k], 1);
+    mbar_init(ops_ready, 16); mbar_init(e_done, 16);
     mbar_fence_init();
     tma_prefetch_desc(&tm_xbc); tma_prefetch_desc(&tm_dy); tma_prefetch_desc(&tm_sin);
-    tma_prefetch_desc(&tm_dsout); tma_prefetch_desc(&tm_dx);
+    tma_prefetch_desc(&tm_dsout); tma_prefetch_desc(&tm_dx); tma_prefetch_desc(&tm_dbc);
   }
-  if (warp == 0) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 16) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t aC = smem_u32(sC), aB = smem_u32(sB), aX = smem_u32(sX), aDY = smem_u32(sDY), aSin = smem_u32(sSin),
-                 aDS = smem_u32(sDS), aM0 = smem_u32(sM0), aDCB = smem_u32(sDCB), aDYs = smem_u32(sDYs);
-  bool ok = true;
 
-  for (int it = 0; it < p.hpc && ok; ++it) {
-    const int hv = hv0 + it, h = hv / psplit;
-    const uint32_t par = it & 1;
-    // ---------------------------------------------------------------- loads
-    if (tid == 0) {
-      uint32_t bytes = 4 * TILE64;
-      if (it == 0) bytes += 2 * TILE128;
-      mbar_expect_tx(&bars[0], bytes);
-      if (it == 0) {
-        const int cB = p.d_in + g * NS, cC = p.d_in + p.G * NS + g * NS;
-        tma_load_2d(sC, &tm_xbc, cC, row0, &bars[0]);
-        tma_load_2d(sC + TILE128 / 2, &tm_xbc, cC + 64, row0, &bars[0]);
-        tma_load_2d(sB, &tm_xbc, cB, row0, &bars[0]);
-        tma_load_2d(sB + TILE128 / 2, &tm_xbc, cB + 64, row0, &bars[0]);
+  if (warp == 17) {
+    if (lane == 0) {
+      auto load_a = [&](int it) {                      // x, dY, l, dt
+        const int hv = hv0 + it, h = hv / psplit;
+        const long long lo = ((long long)b * p.H + h) * p.L + (long long)c * CT;
+        mbar_expect_tx(a_full, 2 * TILE64 + 2 * CT * 4);
+        tma_load_2d(sX, &tm_xbc, hv * PS, row0, a_full);
+        tma_load_2d(sDY, &tm_dy, hv * PS, row0, a_full);
+        bulk_load(s_l, p.l + lo, CT * 4, a_full);
+        bulk_load(s_dt, p.dt + lo, CT * 4, a_full);
+      };
+      auto load_b = [&](int it) {                      // S_in, dS_out
+        const int srow = ((b * p.Hv + hv0 + it) * p.nc + c) * NS;
+        mbar_expect_tx(b_full, 2 * TILE64);
+        tma_load_2d(sSin, &tm_sin, 0, srow, b_full);
+        tma_load_2d(sDS, &tm_dsout, 0, srow, b_full);
+      };
+      const int cB = p.d_in + g * NS, cC = p.d_in + GN + g * NS;
+      mbar_expect_tx(cb_full, 2 * TILE128);
+      tma_load_2d(sC, &tm_xbc, cC, row0, cb_full);
+      tma_load_2d(sC + TILE128 / 2, &tm_xbc, cC + 64, row0, cb_full);
+      tma_load_2d(sB, &tm_xbc, cB, row0, cb_full);
+      tma_load_2d(sB + TILE128 / 2, &tm_xbc, cB + 64, row0, cb_full);
+      load_a(0);
+      load_b(0);
+      bool ok = true;
+      int na = 1, nb = 1;
+      for (int it = 0; it < p.hpc; ++it) {
+        const bool more = it + 1 < p.hpc;
+        ok = mbar_wait(u_done, it & 1, p.status);
+        if (!ok) break;
+        if (more) { load_a(it + 1); ++na; }
+        ok = mbar_wait(g_done, it & 1, p.status);
+        if (!ok) break;
+        if (more) { load_b(it + 1); ++nb; }
+        ok = mbar_wait(e_done, it & 1, p.status);
+        if (!ok) break;
+        tma_store_2d(&tm_dx, sM0, (hv0 + it) * PS, row0);
+        tma_store_commit();
+        tma_store_wait_read();
+        mbar_arrive(m0_free);
       }
-      const int srow = ((b * p.Hv + hv) * p.nc + c) * NS;
-      tma_load_2d(sX, &tm_xbc, hv * PS, row0, &bars[0]);
-      tma_load_2d(sDY, &tm_dy, hv * PS, row0, &bars[0]);
-      tma_load_2d(sSin, &tm_sin, 0, srow, &bars[0]);
-      tma_load_2d(sDS, &tm_dsout, 0, srow, &bars[0]);
+      tma_store_wait_all();
+      if (!ok) {                                       // copies still in flight land before the CTA goes
+        mbar_wait(cb_full, 0, nullptr);
+        mbar_wait(a_full, (na - 1) & 1, nullptr);
+        mbar_wait(b_full, (nb - 1) & 1, nullptr);
+      }
     }
-    const long long lo = ((long long)b * p.H + h) * p.L + (long long)c * CT;
-    if (wg == 0) s_l[row] = p.l[lo + row];
-    else s_dt[row] = p.dt[lo + row];
-    __syncthreads();
-    // ---------------------------------------------------------------- phase 1: CB, dM
-    if (tid == 0) {
-      ok = mbar_wait(&bars[0], par, p.status);
-      if (ok) {
+    __syncwarp();
+  } else if (warp == 16) {
+    if (lane == 0) {
+      // descriptors of the tiles in the roles they have; a k-step adds to the address field: 32 bytes inside an atom of 64,
+      // then the next atom (kstep), or 16 rows (mstep)
+      const uint64_t dCk = desc_kmajor(smem_u32(sC), 0, TILE128 / 2), dBk = desc_kmajor(smem_u32(sB), 0, TILE128 / 2),
+                     dCm = desc_mnmajor(smem_u32(sC), 0, TILE128 / 2), dBm = desc_mnmajor(smem_u32(sB), 0, TILE128 / 2),
+                     dXk = desc_kmajor(smem_u32(sX), 0, 0), dYk = desc_kmajor(smem_u32(sDY), 0, 0),
+                     dYm = desc_mnmajor(smem_u32(sDY), 0, 0), dSink = desc_kmajor(smem_u32(sSin), 0, 0),
+                     dSinm = desc_mnmajor(smem_u32(sSin), 0, 0), dDSk = desc_kmajor(smem_u32(sDS), 0, 0),
+                     dDSm = desc_mnmajor(smem_u32(sDS), 0, 0), dM0m = desc_mnmajor(smem_u32(sM0), 0, TILE128 / 2),
+                     dCBm = desc_mnmajor(smem_u32(sDCB), 0, TILE128 / 2), dCBk = desc_kmajor(smem_u32(sDCB), 0, TILE128 / 2),
+                     dXsk = desc_kmajor(smem_u32(sXs), 0, 0), dYsk = desc_kmajor(smem_u32(sDYs), 0, 0);
+      auto kstep = [](int kk) { return (uint64_t)((kk >> 2) * (TILE128 / 2 / 16) + (kk & 3) * 2); };
+      auto mstep = [](int kk) { return (uint64_t)(kk * 128); };
+      const uint32_t id_cb = make_idesc_bf16(128, 128, 0, 0), id_u1 = make_idesc_bf16(128, PS, 1, 1),
+                     id_u2 = make_idesc_bf16(128, PS, 0, 1), id_b1 = make_idesc_bf16(128, 128, 1, 1),
+                     id_c1 = make_idesc_bf16(128, 128, 0, 1);
+      bool ok = mbar_wait(cb_full, 0, p.status);
+      for (int it = 0; it < p.hpc && ok; ++it) {
+        ok = mbar_wait(a_full, it & 1, p.status) && (it == 0 || mbar_wait(e_done, (it - 1) & 1, p.status));
+        if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t id_cb = make_idesc_bf16(128, 128, 0, 0);
         #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem, desc_kmajor(aC, kk, TILE128 / 2), desc_kmajor(aB, kk, TILE128 / 2), id_cb, kk != 0);
+        for (int kk = 0; kk < 8; ++kk)                            // CB[i][j] = sum_n C[i][n] B[j][n]
+          umma_bf16(tmem, dCk + kstep(kk), dBk + kstep(kk), id_cb, kk != 0);
         #pragma unroll
         for (int kk = 0; kk < 4; ++kk)                            // dM[i][j] = sum_p dY[i][p] x[j][p]
-          umma_bf16(tmem + 128, desc_kmajor(aDY, kk, 0), desc_kmajor(aX, kk, 0), id_cb, kk != 0);
-        umma_commit(&bars[1]);
+          umma_bf16(tmem + 128, dYk + kstep(kk), dXk + kstep(kk), id_cb, kk != 0);
+        umma_commit(s_done);
+        ok = mbar_wait(ops_ready, it & 1, p.status) && mbar_wait(b_full, it & 1, p.status);
+        if (!ok) break;
+        tc_fence_after_sync();
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                            // dU_diag[j][p] = sum_i M0[i][j] dY[i][p]
+          umma_bf16(tmem, dM0m + mstep(kk), dYm + mstep(kk), id_u1, kk != 0);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                            // dU_state[j][p] = sum_n B[j][n] dS_out[n][p]
+          umma_bf16(tmem + 64, dBk + kstep(kk), dDSm + mstep(kk), id_u2, kk != 0);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                            // Yoff[i][p] = sum_n C[i][n] S_in[n][p]
+          umma_bf16(tmem + 128, dCk + kstep(kk), dSinm + mstep(kk), id_u2, kk != 0);
+        umma_commit(u_done);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                            // dB[j][n] += sum_i dCB[i][j] C[i][n]
+          umma_bf16(tmem + 256, dCBm + mstep(kk), dCm + mstep(kk), id_b1, (it | kk) != 0);
+        #pragma unroll
+        for (int kk = 0; kk < 4; ++kk)                            // dB[j][n] += sum_p xs[j][p] dS_out[n][p]
+          umma_bf16(tmem + 256, dXsk + kstep(kk), dDSk + kstep(kk), id_cb, 1);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                            // dC[i][n] += sum_j dCB[i][j] B[j][n]
+          umma_bf16(tmem + 384, dCBk + kstep(kk), dBm + mstep(kk), id_c1, (it | kk) != 0);
+        #pragma unroll
+        for (int kk = 0; kk < 4; ++kk)                            // dC[i][n] += sum_p dYs[i][p] S_in[n][p]
+          umma_bf16(tmem + 384, dYsk + kstep(kk), dSink + kstep(kk), id_cb, 1);
+        umma_commit(g_done);
       }
     }
     __syncwarp();
-    ok = __syncthreads_and(mbar_wait(&bars[1], par, p.status));   // uniform outcome for the whole CTA
-    tc_fence_after_sync();
-    if (!ok) break;
-    // ---------------------------------------------------------------- thread-built operands
-    const float li = s_l[row], dti = s_dt[row], lT = s_l[CT - 1];
-    const float a_left = __expf(li), a_right = __expf(lT - li);
-    float r1 = 0.f;                      // this thread's share of sum_{j<i} W[i][j]
-    #pragma unroll 1
-    for (int jq = 0; jq < 2; ++jq) {
-      const int jb = wg + 2 * jq;        // 32-column block handled by this warpgroup
-      if (jb > rw) {                     // fully masked block (j > i for all rows of this warp)
-        #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          const int jc = jb * 32 + ch * 8;
-          const uint32_t off = (jc >> 6) * (TILE128 / 2) + sw128_offset(row, (jc & 63) >> 3);
-          *reinterpret_cast<uint4*>(sM0 + off) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(sDCB + off) = make_uint4(0, 0, 0, 0);
-        }
-        s_col[rw * CT + jb * 32 + lane] = 0.f;
-        continue;
-      }
-      uint32_t cb[32], dm[32];
-      float wv[32];
-      tmem_ld32(tmem_addr(tmem, rw * 32, jb * 32), cb);
-      tmem_ld32(tmem_addr(tmem, rw * 32, 128 + jb * 32), dm);
-      tmem_ld_wait();
-      #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        float m0[8], dc[8];
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int j = jb * 32 + ch * 8 + e;
-          const float lam = (j <= row) ? __expf(li - s_l[j]) : 0.f;
-          m0[e] = __uint_as_float(cb[ch * 8 + e]) * lam;
-          dc[e] = __uint_as_float(dm[ch * 8 + e]) * lam * s_dt[j];
-          // W[i][j] = dM[i][j] * (CB Lambda dt_j)[i][j], strictly below the diagonal
-          wv[ch * 8 + e] = (j < row) ? __uint_as_float(dm[ch * 8 + e]) * m0[e] * s_dt[j] : 0.f;
-        }
-        const int jc = jb * 32 + ch * 8;
-        const uint32_t off = (jc >> 6) * (TILE128 / 2) + sw128_offset(row, (jc & 63) >> 3);
-        *reinterpret_cast<uint4*>(sM0 + off) = pack8(m0);
-        *reinterpret_cast<uint4*>(sDCB + off) = pack8(dc);
-      }
-      #pragma unroll
-      for (int e = 0; e < 32; ++e) r1 += wv[e];
-      // column sums of this 32x32 block over the warp's rows: recursive halving, lane c ends with column c
-      #pragma unroll
-      for (int sft = 16; sft >= 1; sft >>= 1) {
-        const bool up = (lane & sft) != 0;
-        #pragma unroll
-        for (int k = 0; k < sft; ++k) {
-          const float keep = up ? wv[k + sft] : wv[k];
-          const float send = up ? wv[k] : wv[k + sft];
-          wv[k] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
-        }
-      }
-      s_col[rw * CT + jb * 32 + lane] = wv[0];
-    }
-    // scaled copies of this thread's channel half (4 chunks of 8): x in place, dY into its own tile
-    uint4 xrow[4];
-    float dot_ss = 0.f;                  // share of <dS_out, S_in> (row n = `row`, channel half wg)
-    {
-      const float sx = a_right * dti;
-      #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t off = sw128_offset(row, wg * 4 + q);
-        xrow[q] = *reinterpret_cast<const uint4*>(sX + off);
-        float f[8], f2[8];
-        unpack8(xrow[q], f);
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= sx;
-        *reinterpret_cast<uint4*>(sX + off) = pack8(f);
-        unpack8(*reinterpret_cast<const uint4*>(sDY + off), f);
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= a_left;
-        *reinterpret_cast<uint4*>(sDYs + off) = pack8(f);
-        unpack8(*reinterpret_cast<const uint4*>(sSin + off), f);
-        unpack8(*reinterpret_cast<const uint4*>(sDS + off), f2);
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) dot_ss += f[e] * f2[e];
-      }
-    }
-    if (wg == 1) s_pair[row] = r1;
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-    // ---------------------------------------------------------------- phase 2 MMAs
-    if (tid == 0) {
+  } else {
+    const int rw = warp & 3, wq = warp >> 2, row = rw * 32 + lane;
+    const uint32_t lanes = (uint32_t)rw * 32;
+    bool ok = true;
+    auto arrive = [&](uint64_t* bar) {
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto wait = [&](uint64_t* bar, int phase) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, p.status));
       tc_fence_after_sync();
-      const uint32_t id_u1 = make_idesc_bf16(128, PS, 1, 1);     // dU_diag[j][p] = sum_i M0[i][j] dY[i][p]
-      #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)
-        umma_bf16(tmem, desc_mnmajor(aM0, kk, TILE128 / 2), desc_mnmajor(aDY, kk, 0), id_u1, kk != 0);
-      const uint32_t id_u2 = make_idesc_bf16(128, PS, 0, 1);     // dU_state[j][p] = sum_n B[j][n] dS_out[n][p]
-      #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)
-        umma_bf16(tmem + 64, desc_kmajor(aB, kk, TILE128 / 2), desc_mnmajor(aDS, kk, 0), id_u2, kk != 0);
-      #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)                             // Yoff[i][p] = sum_n C[i][n] S_in[n][p]
-        umma_bf16(tmem + 128, desc_kmajor(aC, kk, TILE128 / 2), desc_mnmajor(aSin, kk, 0), id_u2, kk != 0);
-      const uint32_t id_b1 = make_idesc_bf16(128, 128, 1, 1);    // dB[j][n] += sum_i dCB[i][j] C[i][n]
-      #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)
-        umma_bf16(tmem + 256, desc_mnmajor(aDCB, kk, TILE128 / 2), desc_mnmajor(aC, kk, TILE128 / 2), id_b1,
-                  (it | kk) != 0);
-      const uint32_t id_kk = make_idesc_bf16(128, 128, 0, 0);    // dB[j][n] += sum_p xs[j][p] dS_out[n][p]
-      #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem + 256, desc_kmajor(aX, kk, 0), desc_kmajor(aDS, kk, 0), id_kk, 1);
-      const uint32_t id_c1 = make_idesc_bf16(128, 128, 0, 1);    // dC[i][n] += sum_j dCB[i][j] B[j][n]
-      #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)
-        umma_bf16(tmem + 384, desc_kmajor(aDCB, kk, TILE128 / 2), desc_mnmajor(aB, kk, TILE128 / 2), id_c1,
-                  (it | kk) != 0);
-      #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)                             // dC[i][n] += sum_p dYs[i][p] S_in[n][p]
-        umma_bf16(tmem + 384, desc_kmajor(aDYs, kk, 0), desc_kmajor(aSin, kk, 0), id_kk, 1);
-      umma_commit(&bars[2]);
-    }
-    __syncwarp();
-    ok = __syncthreads_and(mbar_wait(&bars[2], par, p.status));
-    tc_fence_after_sync();
-    if (!ok) break;
-    // ---------------------------------------------------------------- epilogue (row j = `row`, channel half wg)
-    const float Dh = p.D[h];
-    float ddt_direct = 0.f, r2 = 0.f, q = 0.f, dD = 0.f;
-    {
-      uint32_t ud[32], us[32], yo[32];
-      tmem_ld32(tmem_addr(tmem, rw * 32, wg * 32), ud);
-      tmem_ld32(tmem_addr(tmem, rw * 32, 64 + wg * 32), us);
-      tmem_ld32(tmem_addr(tmem, rw * 32, 128 + wg * 32), yo);
-      tmem_ld_wait();
-      #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        float xv[8], gy[8], o[8];
-        unpack8(xrow[ch], xv);
-        unpack8(*reinterpret_cast<const uint4*>(sDY + sw128_offset(row, wg * 4 + ch)), gy);
+    };
+    // barrier of the 512 threads; true where every one of them brings true
+    auto all_ok = [](bool mine) {
+      uint32_t all;
+      asm volatile(
+          "{\n\t"
+          ".reg .pred p, q;\n\t"
+          "setp.ne.u32 p, %1, 0;\n\t"
+          "bar.red.and.pred q, 1, 512, p;\n\t"
+          "selp.u32 %0, 1, 0, q;\n\t"
+          "}\n"
+          : "=r"(all) : "r"(mine ? 1u : 0u) : "memory");
+      return all != 0;
+    };
+    for (int it = 0; it < p.hpc; ++it) {
+      const int hv = hv0 + it, h = hv / psplit;
+      // dt_raw of this row: wanted in 4, on its way meanwhile
+      const float raw = wq == 0 ? __bfloat162float(p.dt_raw[(long long)(row0 + row) * p.dt_raw_stride + h]) : 0.f;
+      const float Dh = p.D[h];
+      float dti = 0.f, a_left = 0.f, a_right = 0.f;
+      do {                                             // a wait that ran out leaves here: all warps meet at the barrier
+        // ---- 1
+        wait(a_full, it);
+        if (!ok) break;
+        const float li = s_l[row], lT = s_l[CT - 1];
+        dti = s_dt[row]; a_left = __expf(li); a_right = __expf(lT - li);
+        uint4 xrow[2], grow[2];
         #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float usr = __uint_as_float(us[ch * 8 + e]);
-          const float dU = __uint_as_float(ud[ch * 8 + e]) + a_right * usr;
-          ddt_direct += xv[e] * dU;
-          q += xv[e] * usr;
-          r2 += gy[e] * __uint_as_float(yo[ch * 8 + e]);
-          dD += gy[e] * xv[e];
-          o[e] = dti * dU + Dh * gy[e];
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t off = sw128_offset(row, wq * 2 + q);
+          xrow[q] = *reinterpret_cast<const uint4*>(sX + off);
+          grow[q] = *reinterpret_cast<const uint4*>(sDY + off);
         }
-        *reinterpret_cast<uint4*>(sX + sw128_offset(row, wg * 4 + ch)) = pack8(o);   // dx staging (x tile is dead)
+        if (it > 0) { wait(g_done, it - 1); if (!ok) break; }      // the products of the head before have read what follows
+        #pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t off = sw128_offset(row, wq * 2 + q);
+          float f[8];
+          unpack8(xrow[q], f);
+          #pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] *= a_right * dti;
+          *reinterpret_cast<uint4*>(sXs + off) = pack8(f);
+          unpack8(grow[q], f);
+          #pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] *= a_left;
+          *reinterpret_cast<uint4*>(sDYs + off) = pack8(f);
+        }
+        wait(b_full, it);
+        if (!ok) break;
+        float dot_ss = 0.f;                  // share of <dS_out, S_in> (row n = `row`, 16 channels)
+        #pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t off = sw128_offset(row, wq * 2 + q);
+          float f[8], f2[8];
+          unpack8(*reinterpret_cast<const uint4*>(sSin + off), f);
+          unpack8(*reinterpret_cast<const uint4*>(sDS + off), f2);
+          #pragma unroll
+          for (int e = 0; e < 8; ++e) dot_ss += f[e] * f2[e];
+        }
+        // ---- 2: row i of M0 and dCB, columns 32 wq .. + 31
+        wait(s_done, it);
+        if (!ok) break;
+        if (it > 0) { wait(m0_free, it - 1); if (!ok) break; }
+        float r1 = 0.f, col[2] = {0.f, 0.f};             // this thread's share of sum_{j<i} W[i][j]; column sums over the warp
+        uint8_t* m_at = sM0 + (wq >> 1) * (TILE128 / 2);
+        uint8_t* d_at = sDCB + (wq >> 1) * (TILE128 / 2);
+        if (wq > rw) {                                   // tokens j > i for every row of this warp
+          #pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            const uint32_t off = sw128_offset(row, (wq & 1) * 4 + ch);
+            *reinterpret_cast<uint4*>(m_at + off) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(d_at + off) = make_uint4(0, 0, 0, 0);
+          }
+        } else {
+          #pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t cb[16], dm[16];
+            float wv[16];
+            tmem_ld16(tmem_addr(tmem, lanes, wq * 32 + half * 16), cb);
+            tmem_ld16(tmem_addr(tmem, lanes, 128 + wq * 32 + half * 16), dm);
+            tmem_ld_wait();
+            #pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+              const int j0 = wq * 32 + half * 16 + ch * 8;
+              float lv[8], dv[8], m0[8], dc[8];
+              load8f_smem(s_l + j0, lv);
+              load8f_smem(s_dt + j0, dv);
+              #pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float lam = (j0 + e <= row) ? __expf(li - lv[e]) : 0.f;
+                m0[e] = __uint_as_float(cb[ch * 8 + e]) * lam;
+                dc[e] = __uint_as_float(dm[ch * 8 + e]) * lam * dv[e];
+                // W[i][j] = dM[i][j] * (CB Lambda dt_j)[i][j], strictly below the diagonal
+                wv[ch * 8 + e] = (j0 + e < row) ? __uint_as_float(dm[ch * 8 + e]) * m0[e] * dv[e] : 0.f;
+              }
+              const uint32_t off = sw128_offset(row, (wq & 1) * 4 + half * 2 + ch);
+              *reinterpret_cast<uint4*>(m_at + off) = pack8(m0);
+              *reinterpret_cast<uint4*>(d_at + off) = pack8(dc);
+            }
+            #pragma unroll
+            for (int e = 0; e < 16; ++e) r1 += wv[e];
+            // column sums over the warp's rows: recursive halving, lanes l and l + 16 end with column l
+            #pragma unroll
+            for (int sft = 8; sft >= 1; sft >>= 1) {
+              const bool up = (lane & sft) != 0;
+              #pragma unroll
+              for (int k = 0; k < sft; ++k) {
+                const float keep = up ? wv[k + sft] : wv[k];
+                const float send = up ? wv[k] : wv[k + sft];
+                wv[k] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
+              }
+            }
+            col[half] = wv[0] + __shfl_xor_sync(0xffffffffu, wv[0], 16);
+          }
+        }
+        arrive(ops_ready);
+        // ---- 3: row j, 16 channels
+        wait(u_done, it);
+        if (!ok) break;
+        float ddt_direct = 0.f, r2 = 0.f, q = 0.f, dD = 0.f;
+        {
+          uint32_t ud[16], us[16], yo[16];
+          tmem_ld16(tmem_addr(tmem, lanes, wq * 16), ud);
+          tmem_ld16(tmem_addr(tmem, lanes, 64 + wq * 16), us);
+          tmem_ld16(tmem_addr(tmem, lanes, 128 + wq * 16), yo);
+          tmem_ld_wait();
+          #pragma unroll
+          for (int ch = 0; ch < 2; ++ch) {
+            float xv[8], gy[8], o[8];
+            unpack8(xrow[ch], xv);
+            unpack8(grow[ch], gy);
+            #pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float usr = __uint_as_float(us[ch * 8 + e]);
+              const float dU = __uint_as_float(ud[ch * 8 + e]) + a_right * usr;
+              ddt_direct += xv[e] * dU;
+              q += xv[e] * usr;
+              r2 += gy[e] * __uint_as_float(yo[ch * 8 + e]);
+              dD += gy[e] * xv[e];
+              o[e] = dti * dU + Dh * gy[e];
+            }
+            *reinterpret_cast<uint4*>(sM0 + sw128_offset(row, wq * 2 + ch)) = pack8(o);      // M0 is dead
+          }
+        }
+        if (lane < 16) {
+          s_col[rw * CT + wq * 32 + lane] = col[0];
+          s_col[rw * CT + wq * 32 + 16 + lane] = col[1];
+        }
+        s_part[wq * CT + row] = r1;
+        s_part[(4 + wq) * CT + row] = ddt_direct;
+        s_part[(8 + wq) * CT + row] = r2;
+        s_part[(12 + wq) * CT + row] = q;
+        // E = exp(l_T) <dS_out, S_in> + sum_j a_right dt_j q_j
+        const float e_share = warp_sum128(__expf(lT) * dot_ss + a_right * dti * q), d_share = warp_sum128(dD);
+        if (lane == 0) { s_red[warp] = e_share; s_red[16 + warp] = d_share; }
+      } while (false);
+      ok = all_ok(ok);
+      if (!ok) break;
+      if (wq != 0) { arrive(e_done); continue; }
+      // ---- 4
+      float E = 0.f;
+      #pragma unroll
+      for (int k = 0; k < 16; ++k) E += s_red[k];
+      float sum[4], c1 = 0.f;
+      #pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        sum[i] = (s_part[i * 4 * CT + row] + s_part[(i * 4 + 1) * CT + row]) + (s_part[(i * 4 + 2) * CT + row] + s_part[(i * 4 + 3) * CT + row]);
+        c1 += s_col[i * CT + row];
       }
-    }
-    fence_proxy_async_smem();
-    if (wg == 1) {                        // hand the per-row partials of the upper channel half to warpgroup 0
-      s_pair[CT + row] = ddt_direct;
-      s_pair[2 * CT + row] = r2;
-      s_pair[3 * CT + row] = q;
-    }
-    // E = exp(l_T) <dS_out, S_in> + sum_j a_right dt_j q_j   (both are plain sums over all 256 threads)
-    const float E = block_sum256(__expf(lT) * dot_ss + a_right * dti * q, s_red);
-    if (tid == 0) { tma_store_2d(&tm_dx, sX, hv * PS, row0); tma_store_commit(); }
-    float dl = 0.f;
-    if (wg == 0) {
-      r1 += s_pair[row];
-      ddt_direct += s_pair[CT + row];
-      r2 += s_pair[2 * CT + row];
-      q += s_pair[3 * CT + row];
-      const float c1 = s_col[row] + s_col[CT + row] + s_col[2 * CT + row] + s_col[3 * CT + row];
-      dl = r1 + a_left * r2 - c1 - a_right * dti * q;
-    }
-    // suffix sum of dl over the 128 rows (warpgroup 0; warpgroup 1 carries zeros through the same barriers)
-    float suf = dl;
-    #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float n = __shfl_down_sync(0xffffffffu, suf, o);
-      if (lane + o < 32) suf += n;
-    }
-    __syncthreads();
-    if (lane == 0 && wg == 0) s_red[8 + rw] = suf;      // warp totals
-    __syncthreads();
-    float ddr = 0.f, dta = 0.f;
-    if (wg == 0) {
+      arrive(e_done);                                  // nothing of M0 is read after this
+      // suffix sum of dl over the 128 rows
+      float suf = sum[0] + a_left * sum[2] - c1 - a_right * dti * sum[3];
+      #pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float n = __shfl_down_sync(0xffffffffu, suf, o);
+        if (lane + o < 32) suf += n;
+      }
+      if (lane == 0) s_red[32 + rw] = suf;
+      asm volatile("bar.sync 2, 128;" ::: "memory");
       float tail = 0.f;
-      for (int w = rw + 1; w < 4; ++w) tail += s_red[8 + w];
+      for (int w = rw + 1; w < 4; ++w) tail += s_red[32 + w];
       const float da = suf + tail + E;
-      const float ddt = ddt_direct + p.A[h] * da;
-      const float sig = sigmoid_f(__bfloat162float(p.dt_raw[(long long)(row0 + row) * p.dt_raw_stride + h]) + p.dt_bias[h]);
-      ddr = ddt * sig;
-      dta = dti * da;
+      const float ddt = sum[1] + p.A[h] * da;
+      const float ddr = ddt * sigmoid_f(raw + p.dt_bias[h]);
       if (p.ddt32 != nullptr) p.ddt32[((long long)b * p.Hv + hv) * p.L + (long long)c * CT + row] = ddr;
       else p.ddt_raw[(long long)(row0 + row) * p.ddt_stride + h] = __float2bfloat16(ddr);
+      const float a_share = warp_sum128(dti * da), b_share = warp_sum128(ddr);
+      if (lane == 0) { s_red[36 + rw] = a_share; s_red[40 + rw] = b_share; }
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      if (tid == 0) {
+        float sD = 0.f;
+        #pragma unroll
+        for (int k = 0; k < 16; ++k) sD += s_red[16 + k];
+        float* hp = p.hpart + (((long long)b * p.nc + c) * p.Hv + hv) * 3;
+        hp[0] = s_red[36] + s_red[37] + s_red[38] + s_red[39];
+        hp[1] = sD;
+        hp[2] = s_red[40] + s_red[41] + s_red[42] + s_red[43];
+      }
     }
-    const float sA = block_sum256(dta, s_red);
-    const float sD = block_sum256(dD, s_red);
-    const float sb = block_sum256(ddr, s_red);
-    if (tid == 0) {
-      float* hp = p.hpart + (((long long)b * p.nc + c) * p.Hv + hv) * 3;
-      hp[0] = sA; hp[1] = sD; hp[2] = sb;
-      tma_store_wait_read();      // the dx staging tile is reloaded as x by the next head
+    // ---- dB (quarters 0, 1) and dC (2, 3): 64 columns each, staged where C .. dS_out were
+    if (ok) wait(g_done, p.hpc - 1);
+    if (ok) {
+      #pragma unroll 1
+      for (int i = 0; i < 2; ++i) {
+        uint32_t v[32];
+        tmem_ld32(tmem_addr(tmem, lanes, 256 + wq * 64 + i * 32), v);
+        tmem_ld_wait();
+        uint8_t* blk = smem + (wq * 2 + i) * TILE64;   // [128 rows][32 fp32]
+        #pragma unroll
+        for (int k4 = 0; k4 < 8; ++k4)
+          *reinterpret_cast<uint4*>(blk + sw128_offset(row, k4)) = make_uint4(v[k4 * 4], v[k4 * 4 + 1], v[k4 * 4 + 2], v[k4 * 4 + 3]);
+      }
+    }
+    fence_proxy_async_smem();
+    ok = all_ok(ok);
+    if (tid == 0 && ok) {
+      for (int k = 0; k < 8; ++k)
+        asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+                     ::"l"(reinterpret_cast<uint64_t>(&tm_dbc)), "r"(smem_u32(smem + k * TILE64)),
+                     "r"((k >> 2) * GN + g * NS + (k & 3) * 32), "r"(row0) : "memory");
+      tma_store_commit();
+      tma_store_wait_all();
     }
     tc_fence_before_sync();
-    __syncthreads();
   }
-  // ---------------------------------------------------------------- flush dB (warpgroup 0), dC (warpgroup 1)
-  if (ok) {
-    tc_fence_after_sync();
-    const int GN = p.G * NS;
-    float* dst = p.dBC + (long long)(row0 + row) * (2 * GN) + wg * GN + g * NS;
-    #pragma unroll 1
-    for (int nb = 0; nb < 4; ++nb) {
-      uint32_t v[32];
-      tmem_ld32(tmem_addr(tmem, rw * 32, 256 + wg * 128 + nb * 32), v);
-      tmem_ld_wait();
-      #pragma unroll
-      for (int k4 = 0; k4 < 8; ++k4)
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + nb * 32 + k4 * 4),
-                     "f"(__uint_as_float(v[k4 * 4])), "f"(__uint_as_float(v[k4 * 4 + 1])),
-                     "f"(__uint_as_float(v[k4 * 4 + 2])), "f"(__uint_as_float(v[k4 * 4 + 3])) : "memory");
-    }
-  }
-  if (tid == 0) tma_store_wait_all();
-  tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (warp == 16) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace ssm
@@ -1294,13 +1382,13 @@ extern "C" int ssm_ssd_chunk_scan_bwd(const void* xbc, long long xbc_stride, int
                                       long long dt_raw_stride, const void* dt_bias, const void* A, const void* dt,
                                       const void* l, const void* D, int B, int L, int H, int Hv, int G, int d_in,
                                       int hpc, int* status, cudaStream_t st) {
-  if (L % CT || Hv % H || H % G || xbc_stride % 8 || dy_stride % 8 || dx_stride % 8)
+  if (L % CT || Hv % H || H % G || xbc_stride % 8 || dy_stride % 8 || dx_stride % 8 ||
+      ((reinterpret_cast<uintptr_t>(dt) | reinterpret_cast<uintptr_t>(l) | reinterpret_cast<uintptr_t>(dBC)) & 15))
     return -SSM_ERR_BAD_ARG;
   const int hv_per_group = Hv / G;
   if (hpc <= 0 || hv_per_group % hpc) return -SSM_ERR_BAD_ARG;
   static bool cfg = false;
-  const int smem = BWD_SMEM + (11 * CT + 16) * 4 + 64 + 1024;
-  if (!cfg) { int e = smem_opt_in((const void*)ssd_chunk_scan_bwd_kernel, smem); if (e) return e; cfg = true; }
+  if (!cfg) { int e = smem_opt_in((const void*)ssd_chunk_scan_bwd_kernel, BWD_SMEM); if (e) return e; cfg = true; }
   const int nc = L / CT;
   CUtensorMap tx, tdy, ts, tds, tdx;
   int r = make_tmap_2d_bf16(&tx, xbc, (uint64_t)xbc_cols, (uint64_t)B * L, (uint64_t)xbc_stride * 2, 64, 128);
@@ -1313,6 +1401,9 @@ extern "C" int ssm_ssd_chunk_scan_bwd(const void* xbc, long long xbc_stride, int
   if (r) return -400 - r;
   r = make_tmap_2d_bf16(&tdx, dx, (uint64_t)Hv * PS, (uint64_t)B * L, (uint64_t)dx_stride * 2, 64, 128);
   if (r) return -500 - r;
+  CUtensorMap tdbc;
+  r = make_tmap_2d(&tdbc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dBC, (uint64_t)2 * G * NS, (uint64_t)B * L, (uint64_t)2 * G * NS * 4, 32, 128);
+  if (r) return -600 - r;
   ScanBwdParams p;
   p.dt = reinterpret_cast<const float*>(dt); p.l = reinterpret_cast<const float*>(l);
   p.D = reinterpret_cast<const float*>(D); p.A = reinterpret_cast<const float*>(A);
@@ -1320,9 +1411,9 @@ extern "C" int ssm_ssd_chunk_scan_bwd(const void* xbc, long long xbc_stride, int
   p.dt_raw = reinterpret_cast<const __nv_bfloat16*>(dt_raw); p.dt_raw_stride = dt_raw_stride;
   p.ddt_raw = reinterpret_cast<__nv_bfloat16*>(ddt_raw); p.ddt_stride = ddt_stride;
   p.ddt32 = reinterpret_cast<float*>(ddt32);
-  p.dBC = reinterpret_cast<float*>(dBC); p.hpart = reinterpret_cast<float*>(hpart);
+  p.hpart = reinterpret_cast<float*>(hpart);
   p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.d_in = d_in; p.hpc = hpc; p.status = status;
   dim3 grid(nc, G * (hv_per_group / hpc), B);
-  ssd_chunk_scan_bwd_kernel<<<grid, 256, smem, st>>>(tx, tdy, ts, tds, tdx, p);
+  ssd_chunk_scan_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(tx, tdy, ts, tds, tdx, tdbc, p);
   return (int)cudaGetLastError();
 }
