@@ -689,15 +689,13 @@ def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner,
     return y, dt, l, s_in, final
 
 
-def _pick_hpc(hv_per_group, nc, G, B, target=296):
-    best = hv_per_group
-    for splits in range(1, hv_per_group + 1):
-        if hv_per_group % splits:
-            continue
-        best = hv_per_group // splits
-        if nc * G * B * splits >= target:
-            break
-    return best
+def _pick_hpc(hv_per_group, chunks, sms=148):
+    """Head slices that one CTA of the backward scan walks (a divisor of the group's).  One CTA fits an SM and spends about
+    one and a half heads on its set-up, B, C and the reduction of dB and dC, so the time is waves x (heads + 1.5): 64 chunks x
+    80 slices take 350 us with 16 heads per CTA (three waves) and 313 us with 40 (one)."""
+    def cost(hpc):
+        return -(-chunks * (hv_per_group // hpc) // sms) * (hpc + 1.5)
+    return min((d for d in range(1, hv_per_group + 1) if hv_per_group % d == 0), key=cost)
 
 
 def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, dt_bias, ddt_out, ddt_stride,
@@ -714,7 +712,7 @@ def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, 
     dBC = torch.zeros(B * L, 2 * G * 128, dtype=torch.float32, device=dev)
     hpart = torch.empty(B * nc, Hv, 3, dtype=torch.float32, device=dev)
     ddt32 = torch.empty(B, Hv, L, dtype=torch.float32, device=dev) if psplit > 1 else None
-    hpc = _pick_hpc(Hv // G, nc, G, B)
+    hpc = _pick_hpc(Hv // G, nc * G * B)
     _run("ssm_ssd_chunk_scan_bwd", _p(conv_out), _ll(C), C, _p(dy2), _ll(dy2.stride(0)),
          _p(s_in), _p(ds_out), _p(dx), _ll(d_inner), _p(dBC), _p(hpart), _p(ddt_out), _ll(ddt_stride), _p(ddt32),
          _p(dt_raw2), _ll(dt_raw_stride), _p(dt_bias), _p(A), _p(dt), _p(l), _p(D), B, L, H, Hv, G, d_inner, hpc,
