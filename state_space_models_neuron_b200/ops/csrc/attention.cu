@@ -275,12 +275,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // the diagonal.  Everything is transposed, TMEM lane = key (or channel for dQ): S^T = K Q^T and dP^T = V dO^T take 64
 // columns each, which leaves room for dQ^T (64), dV and dK (128 each) without sharing, and a query tile is small enough for
 // two stages of Q / dO and of P / dS in shared memory.
-//   warps 0-7   P and dS of a tile (row = key, 32 queries per warpgroup)
-//   warps 8-11  read dQ^T back and add it to fp32 dQ with one bulk reduction per tile
-//   warp 12     issues all products;  warp 13  loads
+//   warps 0-15   P and dS of a tile (row = key, 16 queries per warpgroup)
+//   warps 16-19  read dQ^T back and add it to fp32 dQ with one bulk reduction per tile
+//   warp 20      issues all products;  warp 21  loads
 // The scores of the next tile are issued before the three gradient products of this one, so the arithmetic of a tile and the
 // products of the tile before it overlap.  Bound by these two in turn.  One 128-thread group doing everything in turn, with a
-// reduction instruction per 16 bytes of dQ, took 3569 us for 8192 queries of 32 heads, this 2863 us (with the row sums: 8192 x 16 1867 -> 1555, 4096 x 32 1416 -> 877).
+// reduction instruction per 16 bytes of dQ, took 3569 us for 8192 queries of 32 heads, this 2670 us (2863 with eight warps for P and dS).
 struct AttnBwdParams {
   const float* lse; const float* delta;     // [B, Hq, L]
   __nv_bfloat16* dk; __nv_bfloat16* dv;     // [B*L, Hkv*128]
@@ -292,7 +292,7 @@ constexpr int AQ = 64;                               // queries of a tile
 constexpr int QTILE = AQ * AD * 2;                   // [64][128] bf16: two 8 KiB swizzle blocks
 constexpr int PTILE = AT * AQ * 2;                   // [128 keys][64 queries] bf16
 constexpr int BWD_STAGE = 2 * QTILE;                 // Q and dO
-constexpr int ATTN_BWD_THREADS = 14 * 32;
+constexpr int ATTN_BWD_THREADS = 22 * 32;
 constexpr int ATTN_BWD_SMEM = 2 * ATILE + 2 * BWD_STAGE + 4 * PTILE + AQ * AD * 4 + 2 * 2 * AQ * 4 + 256 + 1024;
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -324,18 +324,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (tid == 0) {
     mbar_init(kv_full, 1);
     for (int k = 0; k < 2; ++k) { mbar_init(&full[k], 1); mbar_init(&empty[k], 1); mbar_init(&done[k], 1); }
-    mbar_init(s_full, 1); mbar_init(ds_ready, 256); mbar_init(dq_full, 1); mbar_init(dq_free, 128);
+    mbar_init(s_full, 1); mbar_init(ds_ready, 16); mbar_init(dq_full, 1); mbar_init(dq_free, 128);
     mbar_fence_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_dq);
   }
-  if (warp == 12) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 20) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;                    // S^T 0, dP^T 64, dQ^T 128, dV 256, dK 384
 
-  if (warp == 13) {
+  if (warp == 21) {
     if (lane == 0) {
       mbar_expect_tx(kv_full, 2 * ATILE);
       tma_load_2d(sK, &tm_k, hk * AD, krow0, kv_full);
@@ -364,23 +364,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
     __syncwarp();
-  } else if (warp == 12) {
+  } else if (warp == 20) {
     if (lane == 0) {
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
       const uint32_t id_s = make_idesc_bf16(128, AQ, 0, 0), id_g = make_idesc_bf16(128, AD, 0, 1),
                      id_q = make_idesc_bf16(128, AQ, 1, 1);
-      auto qdesc_k = [](uint32_t base, int kk) {       // [64 rows][128], K-major
-        return make_smem_desc_sw128(base + (kk >> 2) * (QTILE / 2) + (kk & 3) * 32, 16, 1024);
-      };
-      auto qdesc_mn = [](uint32_t base, int kk) {      // the same tile as [64 k][128 n]
-        return make_smem_desc_sw128(base + kk * 2048, QTILE / 2, 1024);
-      };
+      // descriptors of whole tiles; a k-step adds to the address field (16-byte units): 32 bytes inside an atom of 64 and
+      // then the next atom (of 128 or of 64 rows), or 16 rows
+      auto kstep = [](int kk) { return (uint64_t)((kk >> 2) * (ATILE / 2 / 16) + (kk & 3) * 2); };
+      auto qstep = [](int kk) { return (uint64_t)((kk >> 2) * (QTILE / 2 / 16) + (kk & 3) * 2); };
+      auto mstep = [](int kk) { return (uint64_t)(kk * 128); };
+      const uint64_t dKk = adesc_k(aK, 0), dVk = adesc_k(aV, 0), dKm = adesc_mn(aK, 0);
       auto scores = [&](int it) {
-        const uint32_t aQ = smem_u32(sStage + (it & 1) * BWD_STAGE), aDO = aQ + QTILE;
+        const uint32_t aQ = smem_u32(sStage + (it & 1) * BWD_STAGE);
+        const uint64_t dQk = make_smem_desc_sw128(aQ, 16, 1024), dOk = make_smem_desc_sw128(aQ + QTILE, 16, 1024);
         #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem, adesc_k(aK, kk), qdesc_k(aQ, kk), id_s, kk != 0);
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem, dKk + kstep(kk), dQk + qstep(kk), id_s, kk != 0);
         #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 64, adesc_k(aV, kk), qdesc_k(aDO, kk), id_s, kk != 0);
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 64, dVk + kstep(kk), dOk + qstep(kk), id_s, kk != 0);
         umma_commit(s_full);
       };
       bool ok = mbar_wait(kv_full, 0, p.status) && mbar_wait(&full[0], 0, p.status);
@@ -395,46 +396,45 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (ok && it > 0) ok = mbar_wait(dq_free, (it - 1) & 1, p.status);
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t aQ = smem_u32(sStage + (it & 1) * BWD_STAGE), aDO = aQ + QTILE;
-        const uint32_t aP = smem_u32(sPS + (it & 1) * 2 * PTILE), aDS = aP + PTILE;
+        const uint32_t aQ = smem_u32(sStage + (it & 1) * BWD_STAGE), aP = smem_u32(sPS + (it & 1) * 2 * PTILE);
+        const uint64_t dQm = make_smem_desc_sw128(aQ, QTILE / 2, 1024), dOm = make_smem_desc_sw128(aQ + QTILE, QTILE / 2, 1024);
+        const uint64_t dP = make_smem_desc_sw128(aP, 16, 1024), dDS = make_smem_desc_sw128(aP + PTILE, 16, 1024);
         #pragma unroll
         for (int kk = 0; kk < 8; ++kk)      // dQ^T[d][i] = sum_key K[key][d] dS^T[key][i]
-          umma_bf16(tmem + 128, adesc_mn(aK, kk), make_smem_desc_sw128(aDS + kk * 2048, 16, 1024), id_q, kk != 0);
+          umma_bf16(tmem + 128, dKm + mstep(kk), dDS + mstep(kk), id_q, kk != 0);
         umma_commit(dq_full);
         #pragma unroll
         for (int kk = 0; kk < 4; ++kk)      // dV[key][d] += sum_i P^T[key][i] dO[i][d]
-          umma_bf16(tmem + 256, make_smem_desc_sw128(aP + kk * 32, 16, 1024), qdesc_mn(aDO, kk), id_g, (it | kk) != 0);
+          umma_bf16(tmem + 256, dP + kstep(kk), dOm + mstep(kk), id_g, (it | kk) != 0);
         #pragma unroll
         for (int kk = 0; kk < 4; ++kk)      // dK[key][d] += sum_i dS^T[key][i] Q[i][d]
-          umma_bf16(tmem + 384, make_smem_desc_sw128(aDS + kk * 32, 16, 1024), qdesc_mn(aQ, kk), id_g, (it | kk) != 0);
+          umma_bf16(tmem + 384, dDS + kstep(kk), dQm + mstep(kk), id_g, (it | kk) != 0);
         umma_commit(&done[it & 1]);
         umma_commit(&empty[it & 1]);
       }
     }
     __syncwarp();
-  } else if (warp >= 8) {
+  } else if (warp >= 16) {
     // ---- dQ^T: thread = channel; [query][channel] rows in shared memory, one bulk reduction per tile
-    const int d = tid - 256;
+    const int d = tid - 512;
     bool ok = true;
     for (int it = 0; it < n && ok; ++it) {
       const int h = hk * ratio + it / per_head, q = (2 * kt + it % per_head) * AQ;
       ok = __all_sync(0xffffffffu, mbar_wait(dq_full, it & 1, p.status));
       tc_fence_after_sync();
-      uint32_t v[2][32];
-      if (ok) {
-        tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, 128), v[0]);
-        tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, 160), v[1]);
-        tmem_ld_wait();
-        tc_fence_before_sync();
-        mbar_arrive(dq_free);
-      }
       if (d == 0) tma_store_wait_read();               // the previous tile has left the staging rows
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (ok) {
         #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 2; ++i) {
+          uint32_t v[32];
+          tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, 128 + i * 32), v);
+          tmem_ld_wait();
           #pragma unroll
-          for (int e = 0; e < 32; ++e) sdQ[(i * 32 + e) * AD + d] = __uint_as_float(v[i][e]);
+          for (int e = 0; e < 32; ++e) sdQ[(i * 32 + e) * AD + d] = __uint_as_float(v[e]);
+        }
+        tc_fence_before_sync();
+        mbar_arrive(dq_free);
       }
       fence_proxy_async_smem();
       {
@@ -468,19 +468,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       ok = __all_sync(0xffffffffu, mbar_wait(s_full, it & 1, p.status));
       if (!ok) break;
       tc_fence_after_sync();
-      uint32_t sv[32], dp[32];
-      tmem_ld32(tmem_addr(tmem, lanes, wg * 32), sv);
-      tmem_ld32(tmem_addr(tmem, lanes, 64 + wg * 32), dp);
+      uint32_t sv[16], dp[16];
+      tmem_ld16(tmem_addr(tmem, lanes, wg * 16), sv);
+      tmem_ld16(tmem_addr(tmem, lanes, 64 + wg * 16), dp);
       // the loads of this stage (statistics included) have completed on `full`, which the products of s_full waited for;
       // this thread observes the same phase before it reads what they wrote
       ok = __all_sync(0xffffffffu, mbar_wait(&full[st], (it >> 1) & 1, p.status));
       tmem_ld_wait();
       if (!ok) break;
-      const float* lse = sStat + st * 2 * AQ + wg * 32;
+      const float* lse = sStat + st * 2 * AQ + wg * 16;
       const float* delta = lse + AQ;
-      uint32_t pk[16], dk[16];
+      uint32_t pk[8], dk[8];
       #pragma unroll
-      for (int e4 = 0; e4 < 8; ++e4) {
+      for (int e4 = 0; e4 < 4; ++e4) {
         const float4 ls = *reinterpret_cast<const float4*>(lse + e4 * 4), de = *reinterpret_cast<const float4*>(delta + e4 * 4);
         const float lv[4] = {ls.x, ls.y, ls.z, ls.w}, dv[4] = {de.x, de.y, de.z, de.w};
         float pv[4], ds[4];
@@ -488,7 +488,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int e = 0; e < 4; ++e) {
           const int i = e4 * 4 + e;
           pv[e] = exp2f(fmaf(__uint_as_float(sv[i]), c, -lv[e] * LOG2E));
-          if (rel + wg * 32 + i < row) pv[e] = 0.f;            // the query lies before the key
+          if (rel + wg * 16 + i < row) pv[e] = 0.f;            // the query lies before the key
           ds[e] = pv[e] * (__uint_as_float(dp[i]) - dv[e]) * p.scale;
         }
         pk[e4 * 2] = pack_bf16(pv[0], pv[1]); pk[e4 * 2 + 1] = pack_bf16(pv[2], pv[3]);
@@ -500,23 +500,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       uint8_t* sp = sPS + st * 2 * PTILE;
       #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t off = sw128_offset(row, wg * 4 + q);
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t off = sw128_offset(row, wg * 2 + q);
         *reinterpret_cast<uint4*>(sp + off) = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
         *reinterpret_cast<uint4*>(sp + PTILE + off) = make_uint4(dk[q * 4], dk[q * 4 + 1], dk[q * 4 + 2], dk[q * 4 + 3]);
       }
       fence_proxy_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(ds_ready);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_ready);
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&done[(n - 1) & 1], ((n - 1) >> 1) & 1, p.status));
     if (ok) {
       tc_fence_after_sync();
-      __nv_bfloat16* dst = (wg == 0 ? p.dv : p.dk) + (long long)(krow0 + row) * (p.Hkv * AD) + hk * AD;
+      __nv_bfloat16* dst = (wg < 2 ? p.dv : p.dk) + (long long)(krow0 + row) * (p.Hkv * AD) + hk * AD + (wg & 1) * 64;
       #pragma unroll 1
-      for (int db = 0; db < 4; ++db) {
+      for (int db = 0; db < 2; ++db) {
         uint32_t v[32];
-        tmem_ld32(tmem_addr(tmem, lanes, 256 + wg * 128 + db * 32), v);
+        tmem_ld32(tmem_addr(tmem, lanes, 256 + wg * 64 + db * 32), v);
         tmem_ld_wait();
         #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
@@ -530,7 +531,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tc_fence_before_sync();
   }
   __syncthreads();
-  if (warp == 12) tmem_dealloc(tmem, 512);
+  if (warp == 20) tmem_dealloc(tmem, 512);
 }
 
 // delta[b, h, t] = sum_d dout * out of a row; one warp per (row, head), bound by reading both once
