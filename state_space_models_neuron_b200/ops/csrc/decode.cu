@@ -12,6 +12,8 @@ __global__ void __launch_bounds__(256)
 decode_conv_step_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __nv_bfloat16* __restrict__ state,
                         const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
                         float* __restrict__ act, int C) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (c >= C) return;
@@ -37,6 +39,8 @@ decode_ssm_step_kernel(const float* __restrict__ act, const __nv_bfloat16* __res
                        const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
                        float* __restrict__ state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G,
                        int d_in) {
+  pdl_trigger();
+  pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = h / (H / G);
@@ -98,12 +102,9 @@ SSM_DEBUG_BOUNDS_GETTER(ssm_debug_bounds_decode)
 extern "C" int ssm_decode_conv_step(const void* xnew, long long xs, void* state, const void* w, const void* bias,
                                     void* act, int B, int C, cudaStream_t st) {
   dim3 grid((C + 255) / 256, B);
-  decode_conv_step_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(xnew), xs,
-                                                reinterpret_cast<__nv_bfloat16*>(state),
-                                                reinterpret_cast<const __nv_bfloat16*>(w),
-                                                reinterpret_cast<const __nv_bfloat16*>(bias),
-                                                reinterpret_cast<float*>(act), C);
-  return (int)cudaGetLastError();
+  return launch_dependent(decode_conv_step_kernel, grid, dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16*>(xnew), xs,
+                          reinterpret_cast<__nv_bfloat16*>(state), reinterpret_cast<const __nv_bfloat16*>(w),
+                          reinterpret_cast<const __nv_bfloat16*>(bias), reinterpret_cast<float*>(act), C);
 }
 
 extern "C" int ssm_decode_ssm_step(const void* act, const void* dt_raw, long long dts, const void* dt_bias,
@@ -111,11 +112,8 @@ extern "C" int ssm_decode_ssm_step(const void* act, const void* dt_raw, long lon
                                    int N, int G, int d_in, cudaStream_t st) {
   if (N % 4 || H % G) return -SSM_ERR_BAD_ARG;
   dim3 grid(H, B);
-  decode_ssm_step_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const float*>(act),
-                                               reinterpret_cast<const __nv_bfloat16*>(dt_raw), dts,
-                                               reinterpret_cast<const float*>(dt_bias),
-                                               reinterpret_cast<const float*>(A), reinterpret_cast<const float*>(D),
-                                               reinterpret_cast<float*>(state), reinterpret_cast<__nv_bfloat16*>(y), C, H,
-                                               P, N, G, d_in);
-  return (int)cudaGetLastError();
+  return launch_dependent(decode_ssm_step_kernel, grid, dim3(128), 0, st, reinterpret_cast<const float*>(act),
+                          reinterpret_cast<const __nv_bfloat16*>(dt_raw), dts, reinterpret_cast<const float*>(dt_bias),
+                          reinterpret_cast<const float*>(A), reinterpret_cast<const float*>(D),
+                          reinterpret_cast<float*>(state), reinterpret_cast<__nv_bfloat16*>(y), C, H, P, N, G, d_in);
 }

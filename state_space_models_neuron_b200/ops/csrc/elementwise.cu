@@ -289,6 +289,8 @@ gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ y, long long ys, cons
                          long long zs, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                          long long os, int gs, float eps) {
   __shared__ float red[33];
+  pdl_trigger();
+  pdl_wait();
   const long long row = blockIdx.x;
   const int g = blockIdx.y;
   const int nvec = gs / 8;
@@ -430,6 +432,8 @@ __global__ void __launch_bounds__(1024 / NORM_MAXV)
 add_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const RT* __restrict__ res, const __nv_bfloat16* __restrict__ w,
                        __nv_bfloat16* __restrict__ out, RT* __restrict__ res_out, int D, float eps) {
   __shared__ float red[33];
+  pdl_trigger();
+  pdl_wait();
   const long long row = blockIdx.x;
   const int nvec = D / 8;
   float r[NORM_MAXV][8];
@@ -961,11 +965,6 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ p
 
 // ------------------------------------------------------------------------------------ C API
 using namespace ssm;
-#define LAUNCH_MV(kern, T, grid, t, st, ...)                                     \
-  do {                                                                          \
-    if (mv == 1) kern<T, 1><<<grid, t, 0, st>>>(__VA_ARGS__);                   \
-    else kern<T, 2><<<grid, t, 0, st>>>(__VA_ARGS__);                           \
-  } while (0)
 #define BF(p) reinterpret_cast<const __nv_bfloat16*>(p)
 #define BFM(p) reinterpret_cast<__nv_bfloat16*>(p)
 
@@ -1027,9 +1026,8 @@ extern "C" int ssm_gated_rmsnorm_fwd(const void* y, long long ys, const void* z,
   const int t = norm_threads(gs, &mv, false);
   if (gs % 8 || d % gs || t < 0 || ys % 8 || zs % 8 || os % 8) return -SSM_ERR_BAD_ARG;
   dim3 grid((unsigned)rows, d / gs);
-  if (mv == 1) gated_rmsnorm_fwd_kernel<1><<<grid, t, 0, st>>>(BF(y), ys, BF(z), zs, BF(w), BFM(out), os, gs, eps);
-  else gated_rmsnorm_fwd_kernel<2><<<grid, t, 0, st>>>(BF(y), ys, BF(z), zs, BF(w), BFM(out), os, gs, eps);
-  return (int)cudaGetLastError();
+  return launch_dependent(mv == 1 ? gated_rmsnorm_fwd_kernel<1> : gated_rmsnorm_fwd_kernel<2>, grid, dim3(t), 0, st, BF(y), ys,
+                          BF(z), zs, BF(w), BFM(out), os, gs, eps);
 }
 // dwpart must hold row_slices * d floats.
 extern "C" int ssm_gated_rmsnorm_bwd(const void* y, long long ys, const void* z, long long zs, const void* w,
@@ -1051,11 +1049,11 @@ extern "C" int ssm_add_rmsnorm_fwd(const void* x, const void* res, const void* w
   const int t = norm_threads(D, &mv, false);
   if (D % 8 || t < 0) return -SSM_ERR_BAD_ARG;
   if (res_fp32)
-    LAUNCH_MV(add_rmsnorm_fwd_kernel, float, (unsigned)rows, t, st, BF(x), reinterpret_cast<const float*>(res), BF(w), BFM(out),
-                                                                reinterpret_cast<float*>(res_out), D, eps);
-  else
-    LAUNCH_MV(add_rmsnorm_fwd_kernel, __nv_bfloat16, (unsigned)rows, t, st, BF(x), BF(res), BF(w), BFM(out), BFM(res_out), D, eps);
-  return (int)cudaGetLastError();
+    return launch_dependent(mv == 1 ? add_rmsnorm_fwd_kernel<float, 1> : add_rmsnorm_fwd_kernel<float, 2>, dim3((unsigned)rows),
+                            dim3(t), 0, st, BF(x), reinterpret_cast<const float*>(res), BF(w), BFM(out),
+                            reinterpret_cast<float*>(res_out), D, eps);
+  return launch_dependent(mv == 1 ? add_rmsnorm_fwd_kernel<__nv_bfloat16, 1> : add_rmsnorm_fwd_kernel<__nv_bfloat16, 2>,
+                          dim3((unsigned)rows), dim3(t), 0, st, BF(x), BF(res), BF(w), BFM(out), BFM(res_out), D, eps);
 }
 extern "C" int ssm_add_rmsnorm_bwd(const void* res, const void* w, const void* dout, const void* dres_out, void* dsum,
                                    void* dwpart, int row_slices, long long rows, int D, float eps, int res_fp32,

@@ -58,6 +58,13 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_
   const __nv_bfloat16* xr[NT];
   #pragma unroll
   for (int i = 0; i < NT; ++i) xr[i] = x + (long long)(i * 8 + g < M ? i * 8 + g : 0) * ldx + t * 8;
+  pdl_trigger();
+  {
+    // this warp's first weights on their way to L2 while the predecessor finishes: a 128-byte line per row and chunk
+    const int k = (warp + (lane >> 4) * ROWS_WARPS) * ROWS_CHUNK, r = n0 + (lane & 15);
+    if (k < K && r < N) prefetch_l2(w + (long long)r * ldw + k);
+  }
+  pdl_wait();
   float acc[NT][4];
   #pragma unroll
   for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -160,11 +167,15 @@ gemm_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     mbar_fence_init();
     tma_prefetch_desc(&tm_w); tma_prefetch_desc(&tm_x);
   }
+  pdl_trigger();
+  if (tid == 0)
+    for (int kb = kb0; kb < kb1 && kb < kb0 + STAGES; ++kb) tma_prefetch_l2_2d(&tm_w, kb * 64, n0);
   if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -300,13 +311,15 @@ static int launch_cols(const void* X, long long ldx, const void* W, long long ld
   cfg.blockDim = dim3(128, 1, 1);
   cfg.dynamicSmemBytes = S::TOTAL;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)p.split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tx, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -325,13 +338,8 @@ bool gemm_skinny(const void* X, const void* W, void* C, int M, int N, int K, lon
     const auto* w = reinterpret_cast<const __nv_bfloat16*>(W);
     const unsigned grid = (unsigned)((N + 15) / 16);
     // chunks in flight per warp: four hide more latency, two waste less of a short K
-    if (M <= 8 && K > 2 * ROWS_WARPS * ROWS_CHUNK)
-      gemm_rows_kernel<1, 4><<<grid, ROWS_WARPS * 32, 0, stream>>>(x, ldx, w, ldw, b, out, ldc, M, N, K);
-    else if (M <= 8)
-      gemm_rows_kernel<1, 2><<<grid, ROWS_WARPS * 32, 0, stream>>>(x, ldx, w, ldw, b, out, ldc, M, N, K);
-    else
-      gemm_rows_kernel<2, 2><<<grid, ROWS_WARPS * 32, 0, stream>>>(x, ldx, w, ldw, b, out, ldc, M, N, K);
-    *code = (int)cudaGetLastError();
+    auto kern = M > 8 ? gemm_rows_kernel<2, 2> : K > 2 * ROWS_WARPS * ROWS_CHUNK ? gemm_rows_kernel<1, 4> : gemm_rows_kernel<1, 2>;
+    *code = launch_dependent(kern, dim3(grid), dim3(ROWS_WARPS * 32), 0, stream, x, ldx, w, ldw, b, out, ldc, M, N, K);
     return true;
   }
   ColsParams p;
