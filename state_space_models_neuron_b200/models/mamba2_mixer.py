@@ -155,11 +155,17 @@ class Mamba2Mixer(nn.Module):
             raise ValueError(f"sequence length {zxBCdt.shape[1]} must be a multiple of {self.chunk_size}")
         kw = self._core_kwargs()
         if cache_params is not None:
+            # the kernels write into the plain cache's tensors where they can; a cache class of its own gets its updates
+            into = None
+            if type(cache_params) is Mamba2Cache:
+                into = (cache_params.conv_states[self.layer_idx], cache_params.ssm_states[self.layer_idx])
             y, (conv_state, ssm_state) = ops.mamba2_mixer_core(
                 zxBCdt, self.conv1d.weight, self.conv1d.bias, self.dt_bias, self.A_log, self.D, self.norm.weight,
-                chunk_size=self.chunk_size, return_final_states=True, **kw)
-            cache_params.update_conv_state(self.layer_idx, conv_state)
-            cache_params.update_ssm_state(self.layer_idx, ssm_state)
+                chunk_size=self.chunk_size, return_final_states=True, state_out=into, **kw)
+            if into is None or conv_state is not into[0]:
+                cache_params.update_conv_state(self.layer_idx, conv_state)
+            if into is None or ssm_state is not into[1]:
+                cache_params.update_ssm_state(self.layer_idx, ssm_state)
         else:
             y = ops.mamba2_mixer_core(
                 zxBCdt, self.conv1d.weight, self.conv1d.bias, self.dt_bias, self.A_log, self.D, self.norm.weight,

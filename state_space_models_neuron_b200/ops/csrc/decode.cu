@@ -1,8 +1,10 @@
 // Single-token decode over cached states for sm_100a (memory-bound: one pass over the SSM state).
+//   mixer step: both of the following in one kernel per (head, batch), the form that decoding takes
 //   conv step : roll the [C][4] window, depthwise conv + bias + SiLU for x, B and C alike
 //   ssm step  : S <- S exp(A dt) + (dt x) (x) B ;  y = S C + D x ;  dt = softplus(dt_raw + bias) fused
 // State layouts as in the cache: conv_state [B, C, 4] (oldest first), ssm_state [B, H, P, N] fp32, both
-// updated in place.  Reference: mamba2/mamba2_kernel_inference.py:13-23,26-104 (grid over batch only, softplus
+// updated in place.  The two separate steps serve heads that do not fit shared memory and parameters of other types.
+// Reference: mamba2/mamba2_kernel_inference.py:13-23,26-104 (grid over batch only, softplus
 // and gated norm outside); here the grid is (head, batch) and the state makes exactly one round trip.
 #include "common.cuh"
 
@@ -33,26 +35,11 @@ decode_conv_step_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __
   act[(long long)b * C + c] = silu_f(pre);
 }
 
-// grid (H, B), 128 threads: warp w owns rows p = 4w .. 4w+3, 4w+16 .., ...; lanes own n = 4*lane + 128*r.
-__global__ void __launch_bounds__(128)
-decode_ssm_step_kernel(const float* __restrict__ act, const __nv_bfloat16* __restrict__ dt_raw, long long dts,
-                       const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
-                       float* __restrict__ state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G,
-                       int d_in) {
-  pdl_trigger();
-  pdl_wait();
-  const int h = blockIdx.x, b = blockIdx.y;
+// State update and read-out of one head by 128 threads: warp w owns rows p = 4w .. 4w+3, 4w+16 .., ...; lanes own
+// n = 4*lane + 128*r.  xh [P], Bv / Cv [N]: activations of the head (global or shared memory).
+__device__ __forceinline__ void decode_ssm_head(const float* xh, const float* Bv, const float* Cv, float dt, float decay,
+                                                float Dh, float* __restrict__ S, __nv_bfloat16* __restrict__ y, int P, int N) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = h / (H / G);
-  const float dt = softplus_f(__bfloat162float(dt_raw[(long long)b * dts + h]) + dt_bias[h]);
-  const float decay = __expf(A[h] * dt);
-  const float Dh = D[h];
-  const float* ab = act + (long long)b * C;
-  const float* Bv = ab + d_in + g * N;
-  const float* Cv = ab + d_in + G * N + g * N;
-  // the activation row [x | B | C] must hold d_in + 2 G N values and the head's x slice must lie inside d_in
-  if (!SSM_INDEX_OK(d_in + 2 * G * N - 1, C) || !SSM_INDEX_OK(h * P + P - 1, d_in)) return;
-  float* S = state + (((long long)b * H + h) * P) * N;
   // four rows per warp iteration: four independent 16-byte loads per lane are in flight before any arithmetic,
   // and the four row sums are reduced together (the state makes one round trip; this loop is latency-bound otherwise)
   for (int p0 = warp * 4; p0 < P; p0 += 16) {
@@ -61,7 +48,7 @@ decode_ssm_step_kernel(const float* __restrict__ act, const __nv_bfloat16* __res
     #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int pp = p0 + r;
-      xs[r] = pp < P ? ab[h * P + pp] : 0.f;
+      xs[r] = pp < P ? xh[pp] : 0.f;
       acc[r] = 0.f;
     }
     for (int n = lane * 4; n < N; n += 128) {
@@ -89,9 +76,67 @@ decode_ssm_step_kernel(const float* __restrict__ act, const __nv_bfloat16* __res
     if (lane < 4 && p0 + lane < P) {
       const float a = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
       const float x = lane == 0 ? xs[0] : lane == 1 ? xs[1] : lane == 2 ? xs[2] : xs[3];
-      y[(long long)b * d_in + h * P + p0 + lane] = __float2bfloat16(a + Dh * x);
+      y[p0 + lane] = __float2bfloat16(a + Dh * x);
     }
   }
+}
+
+// grid (H, B), 128 threads, behind decode_conv_step_kernel
+__global__ void __launch_bounds__(128)
+decode_ssm_step_kernel(const float* __restrict__ act, const __nv_bfloat16* __restrict__ dt_raw, long long dts,
+                       const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
+                       float* __restrict__ state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G,
+                       int d_in) {
+  pdl_trigger();
+  pdl_wait();
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int g = h / (H / G);
+  const float dt = softplus_f(__bfloat162float(dt_raw[(long long)b * dts + h]) + dt_bias[h]);
+  const float* ab = act + (long long)b * C;
+  // the activation row [x | B | C] must hold d_in + 2 G N values and the head's x slice must lie inside d_in
+  if (!SSM_INDEX_OK(d_in + 2 * G * N - 1, C) || !SSM_INDEX_OK(h * P + P - 1, d_in)) return;
+  decode_ssm_head(ab + h * P, ab + d_in + g * N, ab + d_in + G * N + g * N, dt, __expf(A[h] * dt), D[h],
+                  state + (((long long)b * H + h) * P) * N, y + (long long)b * d_in + h * P, P, N);
+}
+
+// Conv and state update of one head in one kernel.  Every head computes the conv of its group's B and C channels for itself
+// (2 N short dot products next to a 4 P N byte state) and rolls the windows of its own x channels; the B and C windows,
+// which other heads still read, are rolled by the kernel behind this one (gated norm).  Bound by the state's round trip at
+// large batches and by latency at small ones, where the conv kernel alone cost as much as this (130M, batch 1: 470 -> 450 us
+// per token).
+struct DecodeParams { const void* A_log; const void* D; const void* dt_bias; int bf16_mask; };
+__device__ __forceinline__ float decode_param(const void* p, int h, bool bf16) {
+  return bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[h]) : reinterpret_cast<const float*>(p)[h];
+}
+__global__ void __launch_bounds__(128)
+decode_mixer_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __nv_bfloat16* __restrict__ window,
+                    const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias, const DecodeParams prm,
+                    float* __restrict__ state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G, int d_in) {
+  extern __shared__ __align__(16) float act[];         // B [N] | C [N] | x [P]
+  pdl_trigger();
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int g = h / (H / G);
+  float* S = state + (((long long)b * H + h) * P) * N;
+  // the state on its way to L2 while the predecessor finishes and the conv is computed
+  for (int i = threadIdx.x * 32; i < P * N; i += 128 * 32) prefetch_l2(S + i);
+  pdl_wait();
+  if (!SSM_INDEX_OK(d_in + 2 * G * N - 1, C) || !SSM_INDEX_OK(h * P + P - 1, d_in) || !SSM_INDEX_OK(C + h, xs)) return;
+  const __nv_bfloat16* xr = xnew + (long long)b * xs;
+  for (int i = threadIdx.x; i < 2 * N + P; i += 128) {
+    const bool own = i >= 2 * N;
+    const int c = own ? h * P + i - 2 * N : i < N ? d_in + g * N + i : d_in + G * N + g * N + i - N;
+    uint2* sp = reinterpret_cast<uint2*>(window + ((long long)b * C + c) * 4);
+    const uint2 s = *sp, wv = *reinterpret_cast<const uint2*>(w + (long long)c * 4);
+    const float x1 = bf16_hi(s.x), x2 = bf16_lo(s.y), x3 = bf16_hi(s.y), x4 = __bfloat162float(xr[c]);
+    if (own) *sp = make_uint2(pack_bf16(x1, x2), pack_bf16(x3, x4));
+    float pre = bias ? __bfloat162float(bias[c]) : 0.f;
+    pre += bf16_lo(wv.x) * x1 + bf16_hi(wv.x) * x2 + bf16_lo(wv.y) * x3 + bf16_hi(wv.y) * x4;
+    act[i] = silu_f(pre);
+  }
+  const float dt = softplus_f(__bfloat162float(xr[C + h]) + decode_param(prm.dt_bias, h, prm.bf16_mask & 4));
+  const float A = -expf(decode_param(prm.A_log, h, prm.bf16_mask & 1));
+  __syncthreads();
+  decode_ssm_head(act + 2 * N, act, act + N, dt, __expf(A * dt), decode_param(prm.D, h, prm.bf16_mask & 2), S, y + (long long)b * d_in + h * P, P, N);
 }
 
 }  // namespace ssm
@@ -116,4 +161,19 @@ extern "C" int ssm_decode_ssm_step(const void* act, const void* dt_raw, long lon
                           reinterpret_cast<const __nv_bfloat16*>(dt_raw), dts, reinterpret_cast<const float*>(dt_bias),
                           reinterpret_cast<const float*>(A), reinterpret_cast<const float*>(D),
                           reinterpret_cast<float*>(state), reinterpret_cast<__nv_bfloat16*>(y), C, H, P, N, G, d_in);
+}
+
+// One token of a mixer up to the gated norm.  xnew: bf16 [B, C + H] (x | B | C | dt) with row stride xs; window bf16 [B,C,4]:
+// the x channels are rolled, the rest is left for ssm_gated_rmsnorm_roll; A_log, D, dt_bias: bf16 where bit 0, 1, 2 of the
+// mask is set, else fp32; state fp32 [B,H,P,N]; y bf16 [B, d_in].
+extern "C" int ssm_decode_mixer_step(const void* xnew, long long xs, void* window, const void* w, const void* bias,
+                                     const void* A_log, const void* D, const void* dt_bias, int bf16_mask, void* state, void* y,
+                                     int B, int C, int H, int P, int N, int G, int d_in, cudaStream_t st) {
+  const size_t smem = (size_t)(2 * N + P) * sizeof(float);
+  if (N % 4 || H % G || smem > 48 * 1024 || B < 1 || B > 65535 || C != d_in + 2 * G * N) return -SSM_ERR_BAD_ARG;
+  DecodeParams prm{A_log, D, dt_bias, bf16_mask};
+  return launch_dependent(decode_mixer_kernel, dim3(H, B), dim3(128), smem, st, reinterpret_cast<const __nv_bfloat16*>(xnew), xs,
+                          reinterpret_cast<__nv_bfloat16*>(window), reinterpret_cast<const __nv_bfloat16*>(w),
+                          reinterpret_cast<const __nv_bfloat16*>(bias), prm, reinterpret_cast<float*>(state),
+                          reinterpret_cast<__nv_bfloat16*>(y), C, H, P, N, G, d_in);
 }

@@ -283,11 +283,15 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float2* red, int 
   return t;
 }
 
-template <int NORM_MAXV>
+// conv windows [rows][C][4] whose channels [c0, C) take the new token x [rows, C] (stride xs): what a decoding step leaves
+// for the kernel behind its state update
+struct WindowRoll { __nv_bfloat16* window; const __nv_bfloat16* x; long long xs; int c0, C; };
+
+template <int NORM_MAXV, bool ROLL>
 __global__ void __launch_bounds__(1024 / NORM_MAXV)
 gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ y, long long ys, const __nv_bfloat16* __restrict__ z,
                          long long zs, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
-                         long long os, int gs, float eps) {
+                         long long os, int gs, float eps, const WindowRoll roll) {
   __shared__ float red[33];
   pdl_trigger();
   pdl_wait();
@@ -321,6 +325,14 @@ gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ y, long long ys, cons
       }
       #pragma unroll
       for (int e = 0; e < 8; ++e) { h[i][e] = a[e]; ss += a[e] * a[e]; }
+    }
+  }
+  if (ROLL && g == 0) {
+    for (int c = roll.c0 + threadIdx.x; c < roll.C; c += blockDim.x) {
+      uint2* sp = reinterpret_cast<uint2*>(roll.window + (row * roll.C + c) * 4);
+      const uint2 s = *sp;
+      const uint32_t x = __bfloat16_as_ushort(roll.x[row * roll.xs + c]);
+      *sp = make_uint2((s.x >> 16) | (s.y << 16), (s.y >> 16) | (x << 16));
     }
   }
   const float rstd = rsqrtf(block_sum(ss, red) / gs + eps);
@@ -881,19 +893,6 @@ struct SmallGradArgs {
 
 __device__ __forceinline__ void put(float* dst, float v, bool acc) { *dst = acc ? *dst + v : v; }
 
-// fp32 copies of the per-head mixer parameters in one launch: out[0:H] = -exp(A_log), out[H:2H] = D,
-// out[2H:3H] = dt_bias (the three parameters may be bf16 or fp32)
-__global__ void mixer_param_prep_kernel(const void* A_log, const void* D, const void* dt_bias, int bf16_mask, int H,
-                                        float* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * H) return;
-  const int which = i / H, h = i % H;
-  const void* src = which == 0 ? A_log : which == 1 ? D : dt_bias;
-  const float v = (bf16_mask >> which) & 1 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(src)[h])
-                                           : reinterpret_cast<const float*>(src)[h];
-  out[i] = which == 0 ? -expf(v) : v;
-}
-
 // Column sums with the rows split over 8 thread groups: block = 32 columns x 8 row groups, each thread adds
 // every 8th row of its column (coalesced 128-byte row reads), the 8 partial sums meet in shared memory.
 // A one-thread-per-column loop over all rows is latency-bound on these small matrices.
@@ -1020,14 +1019,25 @@ static int norm_threads(int n, int* maxv, bool backward) {
   return t < 32 ? 32 : t;
 }
 
-extern "C" int ssm_gated_rmsnorm_fwd(const void* y, long long ys, const void* z, long long zs, const void* w,
-                                     void* out, long long os, long long rows, int d, int gs, float eps, cudaStream_t st) {
+template <bool ROLL>
+static int gated_fwd(const void* y, long long ys, const void* z, long long zs, const void* w, void* out, long long os,
+                     long long rows, int d, int gs, float eps, const WindowRoll& roll, cudaStream_t st) {
   int mv = 1;
   const int t = norm_threads(gs, &mv, false);
   if (gs % 8 || d % gs || t < 0 || ys % 8 || zs % 8 || os % 8) return -SSM_ERR_BAD_ARG;
   dim3 grid((unsigned)rows, d / gs);
-  return launch_dependent(mv == 1 ? gated_rmsnorm_fwd_kernel<1> : gated_rmsnorm_fwd_kernel<2>, grid, dim3(t), 0, st, BF(y), ys,
-                          BF(z), zs, BF(w), BFM(out), os, gs, eps);
+  return launch_dependent(mv == 1 ? gated_rmsnorm_fwd_kernel<1, ROLL> : gated_rmsnorm_fwd_kernel<2, ROLL>, grid, dim3(t), 0, st,
+                          BF(y), ys, BF(z), zs, BF(w), BFM(out), os, gs, eps, roll);
+}
+extern "C" int ssm_gated_rmsnorm_fwd(const void* y, long long ys, const void* z, long long zs, const void* w,
+                                     void* out, long long os, long long rows, int d, int gs, float eps, cudaStream_t st) {
+  return gated_fwd<false>(y, ys, z, zs, w, out, os, rows, d, gs, eps, WindowRoll{}, st);
+}
+// The same behind ssm_decode_mixer_step: also rolls channels [c0, C) of the conv windows.
+extern "C" int ssm_gated_rmsnorm_roll(const void* y, long long ys, const void* z, long long zs, const void* w, void* out,
+                                      long long os, long long rows, int d, int gs, float eps, void* window, const void* x,
+                                      long long xs, int c0, int C, cudaStream_t st) {
+  return gated_fwd<true>(y, ys, z, zs, w, out, os, rows, d, gs, eps, WindowRoll{BFM(window), BF(x), xs, c0, C}, st);
 }
 // dwpart must hold row_slices * d floats.
 extern "C" int ssm_gated_rmsnorm_bwd(const void* y, long long ys, const void* z, long long zs, const void* w,
@@ -1203,6 +1213,25 @@ extern "C" int ssm_ce_backward(const void* logits, long long ld, int is_fp32, co
   return (int)cudaGetLastError();
 }
 
+// last four inputs of the conv, [B, C, 4], from x [B, L, C] (row stride xs), L >= 4
+namespace ssm {
+__global__ void __launch_bounds__(256)
+conv_window_kernel(const __nv_bfloat16* __restrict__ x, long long xs, uint2* __restrict__ out, int L, int C) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+  if (c >= C) return;
+  const __nv_bfloat16* p = x + ((long long)b * L + L - 4) * xs + c;
+  uint32_t v[4];
+  #pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = __bfloat16_as_ushort(p[k * xs]);
+  out[(long long)b * C + c] = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+}
+}  // namespace ssm
+extern "C" int ssm_conv_window(const void* x, long long xs, void* out, int B, int L, int C, cudaStream_t st) {
+  if (L < 4 || B < 1 || B > 65535 || C < 1 || (reinterpret_cast<uintptr_t>(out) & 7)) return -SSM_ERR_BAD_ARG;
+  conv_window_kernel<<<dim3((C + 255) / 256, B), 256, 0, st>>>(BF(x), xs, reinterpret_cast<uint2*>(out), L, C);
+  return (int)cudaGetLastError();
+}
+
 extern "C" int ssm_widen(const void* x, long long ld, void* out, long long rows, int n, cudaStream_t st) {
   if (rows < 1 || rows > 65535 || n < 8 || n % 8 || ld % 8 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15))
     return -SSM_ERR_BAD_ARG;
@@ -1328,12 +1357,6 @@ extern "C" int ssm_sumsq_ranges(const void* g, const void* ranges, int nranges, 
   dim3 grid(148 * 8, nranges);       // with 148 * 2 blocks too few loads were in flight (824 MB: 210 us)
   sumsq_ranges_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const float*>(g), reinterpret_cast<const long long*>(ranges),
                                             reinterpret_cast<float*>(total));
-  return (int)cudaGetLastError();
-}
-extern "C" int ssm_mixer_param_prep(const void* A_log, const void* D, const void* dt_bias, int bf16_mask, int H,
-                                    void* out, cudaStream_t st) {
-  mixer_param_prep_kernel<<<(3 * H + 127) / 128, 128, 0, st>>>(A_log, D, dt_bias, bf16_mask, H,
-                                                              reinterpret_cast<float*>(out));
   return (int)cudaGetLastError();
 }
 extern "C" int ssm_colsum(const void* part, int S, int n, void* dst, int acc, cudaStream_t st) {

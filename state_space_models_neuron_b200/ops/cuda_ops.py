@@ -95,11 +95,16 @@ class _NoGrad:
         pass
 
 
+def _recording() -> bool:
+    """True where autograd, forward-mode differentiation or a functorch transform may want to see the call."""
+    return torch.is_grad_enabled() or _forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+
+
 def _apply(function, *args):
     """`function.apply`, or its forward alone where autograd would record nothing: entering and leaving an autograd
     Function costs the host 5 to 10 us per call, half of a small kernel's launch.  Forward-mode differentiation and
     functorch transforms keep `apply`, which answers them as before."""
-    if torch.is_grad_enabled() or _forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
+    if _recording():
         return function.apply(*args)
     return function.forward(_NoGrad(), *args)
 
@@ -665,28 +670,51 @@ def _walk_states(slices: int, nc: int) -> bool:
     return slices >= 80 or nc <= 2
 
 
+def _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a):
+    """dt = softplus(dt_raw + dt_bias) and the running sums of A dt inside every chunk (fp32 [B, H, L]), and (A, D, dt_bias)
+    in fp32.  log_a: A is A_log, of which the kernel takes -exp; the three may then be bf16 or fp32."""
+    dev = dt_raw2.device
+    if log_a:
+        mask = _head_param_mask(A, D, dt_bias, H)
+        if mask is None:
+            return _dt_prep(dt_raw2, dt_raw_stride, -torch.exp(A.float()).contiguous(), D.float().contiguous(),
+                            dt_bias.float().contiguous(), B, L, H, False)
+        params = torch.empty(3, H, dtype=torch.float32, device=dev)
+    else:
+        mask, params = 0, None
+    dt = torch.empty(B, H, L, dtype=torch.float32, device=dev)
+    l = torch.empty_like(dt)
+    _run("ssm_ssd_dt_prep", _p(dt_raw2), _ll(dt_raw_stride), _p(dt_bias), _p(A), _p(D), mask | (8 if log_a else 0), _p(params),
+         _p(dt), _p(l), B, L, H, _st())
+    return dt, l, (A, D, dt_bias) if params is None else params.unbind(0)
+
+
 def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner, G, H, Hv, init_state=None,
-                 want_final=False, want_states=True):
+                 want_final=False, want_states=True, log_a=False, final_out=None):
     """conv_out [B*L, C] bf16 contiguous.  Returns y [B*L, d_inner], dt, l, S_in (None without want_states), final (or
-    None).  The backward pass wants S_in, the states entering the chunks."""
+    None), and (A, D, dt_bias) in fp32.  The backward pass wants S_in, the states entering the chunks.  final_out: contiguous
+    fp32 [B, H, P, 128] that receives the final state."""
     dev = conv_out.device
     C = conv_out.shape[1]
     nc = L // _CT
     st = status_tensor(dev)
-    dt = torch.empty(B, H, L, dtype=torch.float32, device=dev)
-    l = torch.empty_like(dt)
-    _run("ssm_ssd_dt_prep", _p(dt_raw2), _ll(dt_raw_stride), _p(dt_bias), _p(A), _p(dt), _p(l), B, L, H, _st())
+    dt, l, params = _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a)
+    D = params[1]
     y = torch.empty(B * L, d_inner, dtype=torch.bfloat16, device=dev)
     if _walk_states(B * Hv, nc):
         s_in = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev) if want_states else None
-        final = torch.empty(B, H, Hv // H * 64, 128, dtype=torch.float32, device=dev) if want_final else None
+        final = None
+        if want_final:
+            final = torch.empty(B, H, Hv // H * 64, 128, dtype=torch.float32, device=dev) if final_out is None else final_out
         _run("ssm_ssd_walk_scan", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
              _p(init_state), _p(final), B, L, H, Hv, G, d_inner, _p(st), _st())
-        return y, dt, l, s_in, final
+        return y, dt, l, s_in, final, params
     s_in, final = _chunk_states(conv_out, C, d_inner, conv_out, C, dt, l, init_state, want_final, B, L, H, Hv, G, 0)
+    if final_out is not None and want_final:
+        final = final_out.copy_(final)
     _run("ssm_ssd_chunk_scan_fwd", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
          B, L, H, Hv, G, d_inner, _p(st), _st())
-    return y, dt, l, s_in, final
+    return y, dt, l, s_in, final, params
 
 
 def _pick_hpc(hv_per_group, chunks, sms=148):
@@ -726,30 +754,35 @@ def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, 
     return dx, dBC, hp[:, 0], hp[:, 1], hp[:, 2]
 
 
-def _conv_window(xBC, K):
+def _conv_window(xBC, K, out=None):
     """Last K inputs of the conv, [B, C, K]."""
-    B, L = xBC.shape[0], xBC.shape[1]
-    tail = xBC[:, -K:, :] if L >= K else torch.cat([xBC.new_zeros(B, K - L, xBC.shape[2]), xBC], dim=1)
+    B, L, C = xBC.shape
+    if K == 4 and L >= 4:
+        if out is None:
+            out = torch.empty(B, C, 4, dtype=xBC.dtype, device=xBC.device)
+        _run("ssm_conv_window", _p(xBC), _ll(xBC.stride(1)), _p(out), B, L, C, _st())
+        return out
+    tail = xBC[:, -K:, :] if L >= K else torch.cat([xBC.new_zeros(B, K - L, C), xBC], dim=1)
     return tail.transpose(1, 2).contiguous()
 
 
-def _mixer_params_fp32(A_log, D, dt_bias):
-    """(-exp(A_log), D, dt_bias) as fp32 [H] views of one buffer, one launch."""
-    H = A_log.numel()
-    ok = all(t.dtype in (torch.bfloat16, torch.float32) and t.is_contiguous() and t.numel() == H
-             for t in (A_log, D, dt_bias))
-    if not ok:
-        return -torch.exp(A_log.float()), D.float(), dt_bias.float()
-    out = torch.empty(3, H, dtype=torch.float32, device=A_log.device)
-    mask = sum(1 << i for i, t in enumerate((A_log, D, dt_bias)) if t.dtype == torch.bfloat16)
-    _run("ssm_mixer_param_prep", _P(A_log), _P(D), _P(dt_bias), mask, H, _P(out), _st())
-    return out[0], out[1], out[2]
+def _head_param_mask(A, D, dt_bias, H):
+    """Bit i set: parameter i is bf16.  None where the kernels cannot read one of them as it is."""
+    mask = 0
+    for i, t in enumerate((A, D, dt_bias)):
+        if t.dtype == torch.bfloat16:
+            mask |= 1 << i
+        elif t.dtype != torch.float32:
+            return None
+        if not t.is_contiguous() or t.numel() != H:
+            return None
+    return mask
 
 
 class _MixerCore(torch.autograd.Function):
     @staticmethod
     def forward(ctx, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, G, N, P, eps, gs, recompute,
-                want_final, recorded):
+                want_final, recorded, state_out):
         _require_bf16(zxBCdt, conv_w, conv_b, norm_w)
         H, psplit, Hv = _ssd_dims(d_inner, P, G, N)
         B, L, W = zxBCdt.shape
@@ -767,9 +800,10 @@ class _MixerCore(torch.autograd.Function):
         z2, xBC, dt_raw2 = flat[:, :d_inner], zxBCdt[..., d_inner:d_inner + C], flat[:, d_inner + C:]
         w2 = conv_w.reshape(C, -1).contiguous()
         conv_out = _conv_fwd(xBC, w2, conv_b, None).view(B * L, C)
-        A, Df, bf = _mixer_params_fp32(A_log, D, dt_bias)
-        y, dt, l, s_in, final = _ssd_forward(conv_out, dt_raw2, ld, A, Df, bf, B, L, d_inner, G, H, Hv,
-                                             want_final=want_final, want_states=recorded and not recompute)
+        window_out, final_out = state_out or (None, None)
+        y, dt, l, s_in, final, (A, Df, bf) = _ssd_forward(
+            conv_out, dt_raw2, ld, A_log, D, dt_bias, B, L, d_inner, G, H, Hv, want_final=want_final,
+            want_states=recorded and not recompute, log_a=True, final_out=final_out)
         out = _gated_fwd(y, z2, norm_w, eps, gs)
         ctx.dims = (B, L, W, C, d_inner, G, N, P, H, Hv, eps, gs, recompute)
         if recompute:
@@ -780,7 +814,7 @@ class _MixerCore(torch.autograd.Function):
         ctx.conv_w_param = conv_w if conv_w.is_leaf else None
         out = out.view(B, L, d_inner)
         if want_final:
-            conv_state = _conv_window(xBC, w2.shape[1])
+            conv_state = _conv_window(xBC, w2.shape[1], window_out)
             ctx.mark_non_differentiable(conv_state, final)
             return out, conv_state, final
         return out
@@ -795,7 +829,7 @@ class _MixerCore(torch.autograd.Function):
         z2, xBC, dt_raw2 = flat[:, :d_inner], zxBCdt[..., d_inner:d_inner + C], flat[:, d_inner + C:]
         if recompute:
             conv_out = _conv_fwd(xBC, w2, conv_b, None).view(B * L, C)
-            y, dt, l, s_in, _ = _ssd_forward(conv_out, dt_raw2, ld, A, Df, bf, B, L, d_inner, G, H, Hv)
+            y, dt, l, s_in, _, _ = _ssd_forward(conv_out, dt_raw2, ld, A, Df, bf, B, L, d_inner, G, H, Hv)
         else:
             conv_out, y, dt, l, s_in = saved[10:]
         dflat = torch.empty(B * L, ld, dtype=zxBCdt.dtype, device=zxBCdt.device)[:, :W]
@@ -824,7 +858,7 @@ class _MixerCore(torch.autograd.Function):
             _run("ssm_mixer_small_grads", _p(cpart), cpart.shape[0], C, _p(gpart), gpart.shape[0], d_inner, _p(hpart),
                  hpart.shape[0], Hv, H, _p(A), _p(mg[0]), _p(mg[1]), _p(mg[2]), _p(mg[3]), _p(mg[4]), _p(mg[5]),
                  mask, _st())
-            return (d_zx,) + (None,) * 15
+            return (d_zx,) + (None,) * 16
         dnorm_w = _gated_bwd(y, z2, norm_w, dout2, eps, gs, dy, dflat[:, :d_inner])
         dx, dBC, dA, dD, dbias = _ssd_backward(conv_out, dy, y, dt, l, s_in, dt_raw2, ld, A, Df, bf,
                                                dflat[:, d_inner + C:], ld, B, L, d_inner, G, H, Hv)
@@ -833,16 +867,23 @@ class _MixerCore(torch.autograd.Function):
         dA_log = (dA * A).to(A_log.dtype)
         return (d_zx, dw.to(w2.dtype).reshape(ctx.conv_w_shape), None if conv_b is None else db.to(conv_b.dtype),
                 dbias.to(dt_bias.dtype), dA_log, dD.to(D.dtype), dnorm_w.to(norm_w.dtype),
-                None, None, None, None, None, None, None, None, None)
+                None, None, None, None, None, None, None, None, None, None)
 
 
 def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim, eps,
-                      norm_group_size, chunk_size, recompute, return_final_states):
+                      norm_group_size, chunk_size, recompute, return_final_states, state_out=None):
     if chunk_size != _CT:
         raise ValueError("the GPU kernels use 128-token chunks")
     gs = d_inner if norm_group_size is None else norm_group_size
+    if state_out is not None:
+        B, H, C = zxBCdt.shape[0], d_inner // head_dim, d_inner + 2 * n_groups * d_state
+        window, state = state_out
+        if _recording() or not (window.dtype == zxBCdt.dtype and state.dtype == torch.float32 and window.is_contiguous()
+                                and state.is_contiguous() and window.device == state.device == zxBCdt.device
+                                and tuple(window.shape) == (B, C, 4) and tuple(state.shape) == (B, H, head_dim, d_state)):
+            state_out = None
     res = _apply(_MixerCore, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim,
-                 eps, gs, recompute, return_final_states, torch.is_grad_enabled())
+                 eps, gs, recompute, return_final_states, torch.is_grad_enabled(), state_out)
     if return_final_states:
         return res[0], (res[1], res[2])
     return res
@@ -868,7 +909,7 @@ class _SSDScan(torch.autograd.Function):
         if init_state is not None:   # [B,H,P,N] -> [B,Hv,128,64]
             init = init_state.float().reshape(Bsz, H, psplit, 64, N).permute(0, 1, 2, 4, 3).reshape(
                 Bsz, Hv, N, 64).contiguous()
-        y, dt, l, s_in, final = _ssd_forward(conv_out, dtr, Hp, Af, Df, bf, Bsz, L, d_inner, G, H, Hv, init,
+        y, dt, l, s_in, final, _ = _ssd_forward(conv_out, dtr, Hp, Af, Df, bf, Bsz, L, d_inner, G, H, Hv, init,
                                              want_final)
         ctx.save_for_backward(conv_out, y, dt, l, s_in, dtr, Af, Df, bf)
         ctx.dims = (Bsz, L, H, P, G, N, Hv, Hp)
@@ -903,21 +944,6 @@ def ssd_chunk_scan(x, dt_raw, A, Bm, Cm, D, dt_bias, chunk_size, initial_state, 
 # ======================================================================================
 # decode
 # ======================================================================================
-_DECODE_PARAMS = {}
-
-
-def _decode_params_fp32(A_log, D, dt_bias):
-    """(-exp(A_log), D, dt_bias) in fp32 for the decode kernel, prepared once per parameter version instead of three
-    casts per layer and token (inference leaves the parameters untouched, so this is once per model)."""
-    key = (A_log.data_ptr(), D.data_ptr(), dt_bias.data_ptr())
-    ver = (A_log._version, D._version, dt_bias._version)
-    hit = _DECODE_PARAMS.get(key)
-    if hit is None or hit[0] != ver:
-        hit = (ver, _mixer_params_fp32(A_log.detach(), D.detach(), dt_bias.detach()))
-        _DECODE_PARAMS[key] = hit
-    return hit[1]
-
-
 @torch.no_grad()
 def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups,
                     d_state, head_dim, eps, norm_group_size):
@@ -932,15 +958,23 @@ def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_lo
     if zxBCdt.stride(1) != 1:
         zxBCdt = zxBCdt.contiguous()
     dev = zxBCdt.device
-    act = torch.empty(B, C, dtype=torch.float32, device=dev)
-    xBC = zxBCdt[:, d_inner:d_inner + C]
-    _run("ssm_decode_conv_step", _p(xBC), _ll(zxBCdt.stride(0)), _p(conv_state), _p(conv_w.reshape(C, 4).contiguous()),
-         _p(conv_b), _p(act), B, C, _st())
     y = torch.empty(B, d_inner, dtype=torch.bfloat16, device=dev)
-    A, Df, bf = _decode_params_fp32(A_log, D, dt_bias)
-    _run("ssm_decode_ssm_step", _p(act), _p(zxBCdt[:, d_inner + C:]), _ll(zxBCdt.stride(0)), _p(bf),
-         _p(A), _p(Df), _p(ssm_state), _p(y), B, C, H, head_dim, d_state, n_groups, d_inner, _st())
+    xBC, ld = zxBCdt[:, d_inner:], zxBCdt.stride(0)                     # x | B | C | dt
+    w = conv_w.reshape(C, 4).contiguous()
     gs = d_inner if norm_group_size is None else norm_group_size
+    mask = _head_param_mask(A_log, D, dt_bias, H)
+    if mask is not None and W == d_inner + C + H and 2 * d_state + head_dim <= 12288:
+        _run("ssm_decode_mixer_step", _p(xBC), _ll(ld), _p(conv_state), _p(w), _p(conv_b), _p(A_log), _p(D), _p(dt_bias), mask,
+             _p(ssm_state), _p(y), B, C, H, head_dim, d_state, n_groups, d_inner, _st())
+        out = torch.empty(B, d_inner, dtype=torch.bfloat16, device=dev)
+        _run("ssm_gated_rmsnorm_roll", _p(y), _ll(d_inner), _p(zxBCdt), _ll(ld), _p(norm_w), _p(out), _ll(d_inner), _ll(B),
+             d_inner, gs, _c.c_float(eps), _p(conv_state), _p(xBC), _ll(ld), d_inner, C, _st())
+        return out
+    act = torch.empty(B, C, dtype=torch.float32, device=dev)
+    _run("ssm_decode_conv_step", _p(xBC), _ll(ld), _p(conv_state), _p(w), _p(conv_b), _p(act), B, C, _st())
+    _run("ssm_decode_ssm_step", _p(act), _p(zxBCdt[:, d_inner + C:]), _ll(ld), _p(dt_bias.float().contiguous()),
+         _p(-torch.exp(A_log.float()).contiguous()), _p(D.float().contiguous()), _p(ssm_state), _p(y), B, C, H, head_dim, d_state,
+         n_groups, d_inner, _st())
     return _gated_fwd(y, zxBCdt[:, :d_inner], norm_w, eps, gs)
 
 

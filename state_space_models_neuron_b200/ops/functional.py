@@ -109,7 +109,7 @@ def ssd_chunk_scan(x, dt_raw, A, Bm, Cm, D, dt_bias, chunk_size: int = 128,
 def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, *, d_inner: int,
                       n_groups: int, d_state: int, head_dim: int, eps: float,
                       norm_group_size: Optional[int], chunk_size: int = 128,
-                      recompute: bool = False, return_final_states: bool = False):
+                      recompute: bool = False, return_final_states: bool = False, state_out=None):
     """Everything between in_proj and out_proj of a Mamba-2 mixer.
 
     zxBCdt [B, L, d_inner + (d_inner + 2 G N) + H] is split into z | xBC | dt; then
@@ -117,12 +117,13 @@ def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, *, d_in
     The counterpart of the reference's fused driver kernels (mamba2/fused_kernel.py:251-282 fwd,
     285-420 bwd); `recompute` chooses between its two autograd variants (fused_kernel.py:423-471):
     keep the intermediates of the forward pass, or rebuild them from zxBCdt in backward.
-    Returns out [B,L,d_inner] and optionally (conv_state [B,C,K], ssm_state [B,H,P,N]).
+    Returns out [B,L,d_inner] and optionally (conv_state [B,C,K], ssm_state [B,H,P,N]).  `state_out` = two tensors that may
+    receive these states; the returned ones are those tensors where they did.
     """
     if _native(zxBCdt):
         return _cuda().mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner,
                                          n_groups, d_state, head_dim, eps, norm_group_size, chunk_size,
-                                         recompute, return_final_states)
+                                         recompute, return_final_states, state_out)
     Bsz, L, _ = zxBCdt.shape
     conv_dim = d_inner + 2 * n_groups * d_state
     H = d_inner // head_dim

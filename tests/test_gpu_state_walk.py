@@ -51,9 +51,38 @@ def test_walk_scan_equals_separate_kernels(monkeypatch, nc, H, P, G):
     bare = cuda_ops._ssd_forward(xbc, raw, 8, A, D, bias, B, L, d, G, H, Hv, init, True, want_states=False)
     torch.cuda.synchronize()
     cuda_ops.check_status()
-    (y0, _, _, s0, f0), (y1, _, _, s1, f1) = out
+    (y0, _, _, s0, f0, _), (y1, _, _, s1, f1, _) = out
     assert ((s0.float() - s1.float()).abs() <= 2.0 ** -7 * s0.float().abs() + 1e-6).all()
     assert torch.allclose(f0, f1, rtol=1e-5, atol=1e-5 * f0.abs().max().item())
     # y: one bf16 step of the result, and one of a state or a weight among the 128 terms of its sums
     assert ((y0.float() - y1.float()).abs() <= 2.0 ** -7 * (y0.float().abs() + y0.float().abs().mean())).all()
     assert bare[3] is None and torch.equal(bare[0], y1) and torch.equal(bare[4], f1)
+
+
+@pytest.mark.parametrize("B,H,P,G,fp32", [(1, 8, 64, 1, False), (3, 24, 64, 8, True), (5, 16, 128, 2, False)])
+def test_decode_step_equals_separate_kernels(monkeypatch, B, H, P, G, fp32):
+    """Conv, state update and window roll in the fused decoding kernels against one kernel each."""
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    d, N = H * P, 128
+    C = d + 2 * G * N
+    gen = torch.Generator(device="cuda").manual_seed(B + H)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    kind = torch.float32 if fp32 else torch.bfloat16
+    p = [make(C, 1, 4).bfloat16(), make(C).bfloat16(), make(H).to(kind), make(H).abs().to(kind), make(H).to(kind), make(d).bfloat16()]
+    kw = dict(d_inner=d, n_groups=G, d_state=N, head_dim=P, eps=1e-5, norm_group_size=d // G)
+    window, state = make(B, C, 4).bfloat16(), make(B, H, P, N)
+    out = []
+    mask = cuda_ops._head_param_mask
+    for fused in (True, False):
+        monkeypatch.setattr(cuda_ops, "_head_param_mask", mask if fused else (lambda *a: None))
+        w, s = window.clone(), state.clone()
+        ys = [ops.ssm_decode_step(torch.nn.functional.pad(make(B, d + C + H) * 0 + k + 1, (0, (-(d + C + H)) % 8)).bfloat16()[:, :d + C + H],
+                                  w, s, *p, **kw) for k in range(3)]
+        out.append((ys, w, s))
+    torch.cuda.synchronize()
+    cuda_ops.check_status()
+    assert torch.equal(out[0][1], out[1][1])                    # windows are moved, not computed
+    assert torch.allclose(out[0][2], out[1][2], rtol=1e-5, atol=1e-6)
+    for a, b in zip(out[0][0], out[1][0]):
+        assert ((a.float() - b.float()).abs() <= 2.0 ** -7 * (b.float().abs() + b.float().abs().mean())).all()
