@@ -4,6 +4,7 @@
 // all arithmetic fp32.  Reference counterparts: mamba2/conv1d_grouped.py:65-194 (conv),
 // mamba2/fused_kernel.py:76-175 (gated norm), mamba2/modeling_mamba2.py:94-103 (RMSNorm).
 #include "common.cuh"
+#include <type_traits>
 
 namespace ssm {
 
@@ -68,7 +69,7 @@ constexpr int CONV_K = 4;
 
 // Each thread owns 4 channels and walks a tile of tokens.  Both directions are bound by the bytes in flight: the loads of
 // the next four tokens are issued before the arithmetic of the present four (2048 x 10240: forward 34.5 -> 22.4 us,
-// backward 81.5 -> 68.9 us; 32768 x 5376: forward 264 -> 145 us).
+// backward 81.5 -> 55.3 us; 32768 x 5376: forward 264 -> 145 us).
 constexpr int CONV_CPT = 4;
 
 __device__ __forceinline__ void unpack4(const uint2 u, float (&f)[4]) {
@@ -138,12 +139,80 @@ conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
   }
 }
 
+// Backward of one thread's tile: tokens t0 .. t0 + TOK - 1 of 4 channels and three more behind it, whose pre-activation
+// gradients reach back into the tile.  T16: dy is bf16, else fp32; `dy` points at token t0 of these channels.
+template <int TOK, bool T16>
+__device__ __forceinline__ void conv_bwd_tile(const __nv_bfloat16* __restrict__ xb, long long xs, const void* __restrict__ dy,
+                                              long long ds, const float (&wt)[CONV_K][CONV_CPT], const float (&bs)[CONV_CPT],
+                                              __nv_bfloat16* __restrict__ dx, long long dxs, int t0, int L,
+                                              float (&dw)[CONV_K][CONV_CPT], float (&db)[CONV_CPT]) {
+  using Raw = typename std::conditional<T16, uint2, uint4>::type;
+  uint2 xn[4];
+  Raw gn[4];
+  auto fetch = [&](int i, int n) {
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      xn[k] = make_uint2(0, 0);
+      gn[k] = Raw{};
+      if (k < n && t0 + i + k < L) {
+        xn[k] = *reinterpret_cast<const uint2*>(xb + (long long)(t0 + i + k) * xs);
+        if constexpr (T16) gn[k] = *reinterpret_cast<const Raw*>(reinterpret_cast<const __nv_bfloat16*>(dy) + (long long)(i + k) * ds);
+        else gn[k] = *reinterpret_cast<const Raw*>(reinterpret_cast<const float*>(dy) + (long long)(i + k) * ds);
+      }
+    }
+  };
+  fetch(0, 4);
+  float xw[3][CONV_CPT], dp[3][CONV_CPT];              // x and pre-activation gradients of the three tokens before
+  #pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int t = t0 - 3 + k;
+    unpack4(t >= 0 ? *reinterpret_cast<const uint2*>(xb + (long long)t * xs) : make_uint2(0, 0), xw[k]);
+    #pragma unroll
+    for (int e = 0; e < CONV_CPT; ++e) dp[k][e] = 0.f;
+  }
+  auto token = [&](const uint2 xr, const Raw gr, int i, bool inside, bool store) {
+    const bool valid = t0 + i < L;
+    float cur[CONV_CPT], g[CONV_CPT], d[CONV_CPT];
+    unpack4(xr, cur);
+    if constexpr (T16) unpack4(gr, g);
+    else { g[0] = __uint_as_float(gr.x); g[1] = __uint_as_float(gr.y); g[2] = __uint_as_float(gr.z); g[3] = __uint_as_float(gr.w); }
+    #pragma unroll
+    for (int e = 0; e < CONV_CPT; ++e) {
+      const float pre = bs[e] + wt[0][e] * xw[0][e] + wt[1][e] * xw[1][e] + wt[2][e] * xw[2][e] + wt[3][e] * cur[e];
+      const float sg = sigmoid_f(pre);
+      const float dpre = valid ? g[e] * sg * (1.f + pre * (1.f - sg)) : 0.f;
+      if (inside) {
+        dw[0][e] += xw[0][e] * dpre; dw[1][e] += xw[1][e] * dpre; dw[2][e] += xw[2][e] * dpre;
+        dw[3][e] += cur[e] * dpre; db[e] += dpre;
+      }
+      // dx[t-3] = w3*dpre[t-3] + w2*dpre[t-2] + w1*dpre[t-1] + w0*dpre[t]
+      d[e] = wt[3][e] * dp[0][e] + wt[2][e] * dp[1][e] + wt[1][e] * dp[2][e] + wt[0][e] * dpre;
+      dp[0][e] = dp[1][e]; dp[1][e] = dp[2][e]; dp[2][e] = dpre;
+      xw[0][e] = xw[1][e]; xw[1][e] = xw[2][e]; xw[2][e] = cur[e];
+    }
+    if (store && t0 + i - 3 < L)
+      *reinterpret_cast<uint2*>(dx + (long long)(i - 3) * dxs) = make_uint2(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]));
+  };
+  #pragma unroll 1
+  for (int i = 0; i < TOK; i += 4) {
+    uint2 xr[4];
+    Raw gr[4];
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) { xr[k] = xn[k]; gr[k] = gn[k]; }
+    fetch(i + 4, i + 4 < TOK ? 4 : 3);
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) token(xr[k], gr[k], i + k, t0 + i + k < L, i > 0 || k == 3);
+  }
+  #pragma unroll
+  for (int k = 0; k < 3; ++k) token(xn[k], gn[k], TOK + k, false, true);
+}
+
 // Backward.  dy for channels [0, c_split) comes from dy16 (bf16, row stride ds16); channels >= c_split from
 // dy32 (fp32, row stride ds32, indexed by channel - c_split).  dx is written with row stride dxs.
 // part [gridDim.z * gridDim.y, C, 5] receives per-tile partial sums (dw[0..3], db).
-// A tile walks its tokens and three more behind it.
+// Three blocks per SM: with four the registers of a tile spill (2048 x 10240: 64.7 us, three 55.3; 8192 x 5376: 112.7 and 105.5).
 template <int TOK>
-__global__ void __launch_bounds__(128, 4)
+__global__ void __launch_bounds__(128, 3)
 conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const __nv_bfloat16* __restrict__ w,
                        const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ dy16, long long ds16,
                        const float* __restrict__ dy32, long long ds32, int c_split,
@@ -152,97 +221,19 @@ conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
   if (c0 >= C) return;
   const int t0 = blockIdx.y * TOK;
   const int b = blockIdx.z;
-  float wt[CONV_K][CONV_CPT], bs[CONV_CPT];
+  float wt[CONV_K][CONV_CPT], bs[CONV_CPT], dw[CONV_K][CONV_CPT], db[CONV_CPT];
   conv_params(w, bias, c0, wt, bs);
-  const __nv_bfloat16* xb = x + (long long)b * L * xs + c0;
-  const bool lo = c0 < c_split;
-  float xw[3][CONV_CPT], dp[CONV_K][CONV_CPT], dw[CONV_K][CONV_CPT], db[CONV_CPT];
   #pragma unroll
   for (int e = 0; e < CONV_CPT; ++e) {
     db[e] = 0.f;
     #pragma unroll
-    for (int k = 0; k < CONV_K; ++k) { dw[k][e] = 0.f; dp[k][e] = 0.f; }
+    for (int k = 0; k < CONV_K; ++k) dw[k][e] = 0.f;
   }
-  #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const int t = t0 - 3 + k;
-    if (t >= 0) unpack4(*reinterpret_cast<const uint2*>(xb + (long long)t * xs), xw[k]);
-    else {
-      #pragma unroll
-      for (int e = 0; e < CONV_CPT; ++e) xw[k][e] = 0.f;
-    }
-  }
-  constexpr int NSTEP = TOK + 3;
-  constexpr int NB = (NSTEP + 3) / 4;
-  uint2 xn[4];
-  uint4 gn[4];                       // four gradients: 8 bytes of bf16 or 16 bytes of fp32
-  auto fetch = [&](int ib) {
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int t = t0 + ib * 4 + k;
-      if (t < L && ib * 4 + k < NSTEP) {
-        xn[k] = *reinterpret_cast<const uint2*>(xb + (long long)t * xs);
-        if (lo) {
-          const uint2 u = *reinterpret_cast<const uint2*>(dy16 + ((long long)b * L + t) * ds16 + c0);
-          gn[k].x = u.x; gn[k].y = u.y;
-        } else {
-          gn[k] = *reinterpret_cast<const uint4*>(dy32 + ((long long)b * L + t) * ds32 + (c0 - c_split));
-        }
-      }
-    }
-  };
-  #pragma unroll
-  for (int k = 0; k < 4; ++k) { xn[k] = make_uint2(0, 0); gn[k] = make_uint4(0, 0, 0, 0); }
-  fetch(0);
-  #pragma unroll 1
-  for (int ib = 0; ib < NB; ++ib) {
-    uint2 xr[4];
-    uint4 gr[4];
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) { xr[k] = xn[k]; gr[k] = gn[k]; }
-    if (ib + 1 < NB) fetch(ib + 1);
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = ib * 4 + k;
-      const int t = t0 + i;
-      if (i >= NSTEP) break;
-      const bool valid = t < L;
-      float cur[CONV_CPT], g[CONV_CPT], d[CONV_CPT];
-      if (valid) {
-        unpack4(xr[k], cur);
-        if (lo) unpack4(make_uint2(gr[k].x, gr[k].y), g);
-        else {
-          g[0] = __uint_as_float(gr[k].x); g[1] = __uint_as_float(gr[k].y);
-          g[2] = __uint_as_float(gr[k].z); g[3] = __uint_as_float(gr[k].w);
-        }
-      }
-      #pragma unroll
-      for (int e = 0; e < CONV_CPT; ++e) {
-        float dpre = 0.f;
-        if (valid) {
-          const float pre = bs[e] + wt[0][e] * xw[0][e] + wt[1][e] * xw[1][e] + wt[2][e] * xw[2][e] + wt[3][e] * cur[e];
-          const float sg = sigmoid_f(pre);
-          dpre = g[e] * sg * (1.f + pre * (1.f - sg));
-          if (i < TOK) {
-            dw[0][e] += xw[0][e] * dpre; dw[1][e] += xw[1][e] * dpre; dw[2][e] += xw[2][e] * dpre;
-            dw[3][e] += cur[e] * dpre; db[e] += dpre;
-          }
-        } else {
-          cur[e] = 0.f;
-        }
-        dp[0][e] = dp[1][e]; dp[1][e] = dp[2][e]; dp[2][e] = dp[3][e]; dp[3][e] = dpre;
-        // dx[t-3] = w3*dpre[t-3] + w2*dpre[t-2] + w1*dpre[t-1] + w0*dpre[t]
-        d[e] = wt[3][e] * dp[0][e] + wt[2][e] * dp[1][e] + wt[1][e] * dp[2][e] + wt[0][e] * dp[3][e];
-        xw[0][e] = xw[1][e]; xw[1][e] = xw[2][e]; xw[2][e] = cur[e];
-      }
-      const int td = t - 3;
-      if (i >= 3 && td < L) {
-        uint2 o;
-        o.x = pack_bf16(d[0], d[1]); o.y = pack_bf16(d[2], d[3]);
-        *reinterpret_cast<uint2*>(dx + ((long long)b * L + td) * dxs + c0) = o;
-      }
-    }
-  }
+  const long long first = (long long)b * L + t0;
+  const __nv_bfloat16* xb = x + (long long)b * L * xs + c0;
+  __nv_bfloat16* dxt = dx + first * dxs + c0;
+  if (c0 < c_split) conv_bwd_tile<TOK, true>(xb, xs, dy16 + first * ds16 + c0, ds16, wt, bs, dxt, dxs, t0, L, dw, db);
+  else conv_bwd_tile<TOK, false>(xb, xs, dy32 + first * ds32 + (c0 - c_split), ds32, wt, bs, dxt, dxs, t0, L, dw, db);
   float* pp = part + ((long long)(blockIdx.z * gridDim.y + blockIdx.y) * C + c0) * 5;
   #pragma unroll
   for (int e = 0; e < CONV_CPT; ++e) {
