@@ -225,8 +225,8 @@ ssd_state_pass_kernel(const float* __restrict__ local, const float* __restrict__
 }
 
 // =====================================================================================
-// chunk states and their recurrence in one kernel (the two kernels above without the fp32 states in between):
-//   in[c] = run ; run = exp(l_T[c]) * run + sum_j s_j W[j][n] V[j][p]       c ascending (mode 0) or descending (mode 1)
+// the backward pass's states in one kernel (mode 1 of the two kernels above without the fp32 states in between):
+//   in[c] = run ; run = exp(l_T[c]) * run + sum_j exp(l_j) C[j][n] dY[j][p]       c descending
 // One CTA per (head slice, batch) walks the chunks; the running state stays in registers (256 threads: row n = tid & 127,
 // 32 of the 64 channels each).  Loads run three chunks ahead; the products of the next chunk run on tcgen05 (two TMEM
 // buffers) while this one's state is stored and updated.
@@ -234,9 +234,8 @@ ssd_state_pass_kernel(const float* __restrict__ local, const float* __restrict__
 // fp32 states, written and read back, were two thirds of the bytes.
 // =====================================================================================
 struct StateWalkParams {
-  const float* dt; const float* l;       // [B, H, L]
-  const float* init; float* fin;         // fp32 [B, Hv, 128 n, 64 p] in, [B, Hv, 64 p, 128 n] out, or null
-  int L, H, Hv, G, nc, w_col0, mode;
+  const float* l;                        // [B, H, L]
+  int L, H, Hv, G, nc, w_col0;
   int* status;
 };
 constexpr int WALK_STAGES = 3;
@@ -256,8 +255,7 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   const int row = tid & 127, half = tid >> 7;
   const int h = hv / (p.Hv / p.H), g = h / (p.H / p.G);
   const float* lh = p.l + ((long long)b * p.H + h) * p.L;
-  const float* dth = p.dt + ((long long)b * p.H + h) * p.L;
-  auto chunk = [&](int k) { return p.mode == 0 ? k : p.nc - 1 - k; };    // chunk of step k
+  auto chunk = [&](int k) { return p.nc - 1 - k; };                      // chunk of step k
 
   if (tid == 0) {
     for (int s = 0; s < WALK_STAGES; ++s) mbar_init(&full[s], 1);
@@ -282,12 +280,12 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   int loaded = 0;                                                        // steps whose loads have been issued (thread 0)
   if (tid == 0)
     for (; loaded < WALK_STAGES && loaded < p.nc; ++loaded) load(loaded);
-  // scaling of a step: l_j, l_T and dt_j of this thread's row, fetched a step ahead
-  float lj = 0.f, lT = 0.f, dtj = 0.f;
+  // scaling of a step: l_j of this thread's row and l_T, fetched a step ahead
+  float lj = 0.f, lT = 0.f;
   auto fetch = [&](int k) {
     if (k >= p.nc) return;
     const long long o = (long long)chunk(k) * CT;
-    lj = lh[o + row]; lT = lh[o + CT - 1]; dtj = dth[o + row];
+    lj = lh[o + row]; lT = lh[o + CT - 1];
   };
   // V rows of step k scaled in place, then its products issued into TMEM buffer k & 1
   bool ok = true;
@@ -295,7 +293,7 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     const int st = k % WALK_STAGES;
     uint8_t* sw = smem + st * WALK_STAGE_BYTES;
     uint8_t* sv = sw + TILE128;
-    const float s = p.mode == 0 ? __expf(lT - lj) * dtj : __expf(lj);
+    const float s = __expf(lj);
     ok = mbar_wait(&full[st], (k / WALK_STAGES) & 1, p.status);
     if (ok) {
       #pragma unroll
@@ -322,14 +320,9 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     __syncwarp();
   };
 
-  const long long state = ((long long)b * p.Hv + hv) * (NS * PS) + row * PS + half * 32;
   float run[32];
   #pragma unroll
-  for (int e = 0; e < 32; e += 4) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.init != nullptr) v = *reinterpret_cast<const float4*>(p.init + state + e);
-    run[e] = v.x; run[e + 1] = v.y; run[e + 2] = v.z; run[e + 3] = v.w;
-  }
+  for (int e = 0; e < 32; ++e) run[e] = 0.f;
   fetch(0);
   float dec = __expf(lT);                                                // of the step whose products are in flight
   scale_and_issue(0);
@@ -372,11 +365,6 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     tc_fence_before_sync();
     if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // step k - 1's tile has been read
     ok = __syncthreads_and(ok);                                          // TMEM buffer and staging tile are free again
-  }
-  if (ok && p.fin != nullptr) {                                          // channel rows, as a decoding cache holds them
-    float* fin = p.fin + ((long long)b * p.Hv + hv) * (NS * PS) + (half * 32) * NS + row;
-    #pragma unroll
-    for (int e = 0; e < 32; ++e) fin[e * NS] = run[e];
   }
   if (tid == 0) {
     tma_store_wait_all();
@@ -1308,11 +1296,11 @@ extern "C" int ssm_ssd_state_pass(const void* local, const void* l, const void* 
   return (int)cudaGetLastError();
 }
 
-// w_src as in ssm_ssd_chunk_state; v: bf16 [B*L, Hv*64] columns at v (row stride v_stride).  in16 bf16 [B,Hv,nc,128,64] is
-// written; init fp32 [B,Hv,128 n,64 p] and fin fp32 [B,Hv,64 p,128 n] are optional.
+// mode 1 of ssm_ssd_chunk_state (w_src: C) and ssm_ssd_state_pass in one; v: bf16 [B*L, Hv*64] (row stride v_stride).  in16 bf16
+// [B,Hv,nc,128,64] is written.
 extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_cols, int w_col0, const void* v,
-                                  long long v_stride, const void* dt, const void* l, const void* init, void* in16, void* fin,
-                                  int B, int L, int H, int Hv, int G, int mode, int* status, cudaStream_t st) {
+                                  long long v_stride, const void* l, void* in16, int B, int L, int H, int Hv, int G,
+                                  int* status, cudaStream_t st) {
   if (L % CT || Hv % H || H % G || w_stride % 8 || v_stride % 8 || B < 1 || B > 65535) return -SSM_ERR_BAD_ARG;
   static bool cfg = false;
   if (!cfg) { int e = smem_opt_in((const void*)ssd_state_walk_kernel, WALK_SMEM); if (e) return e; cfg = true; }
@@ -1325,9 +1313,8 @@ extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_c
   r = make_tmap_2d_bf16(&ti, in16, 64, (uint64_t)B * Hv * nc * NS, 128, 64, 128);
   if (r) return -300 - r;
   StateWalkParams p;
-  p.dt = reinterpret_cast<const float*>(dt); p.l = reinterpret_cast<const float*>(l);
-  p.init = reinterpret_cast<const float*>(init); p.fin = reinterpret_cast<float*>(fin);
-  p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.w_col0 = w_col0; p.mode = mode; p.status = status;
+  p.l = reinterpret_cast<const float*>(l);
+  p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.w_col0 = w_col0; p.status = status;
   ssd_state_walk_kernel<<<dim3(Hv, B), 256, WALK_SMEM, st>>>(tw, tv, ti, p);
   return (int)cudaGetLastError();
 }

@@ -647,11 +647,10 @@ def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, 
     entering the chunks; mode 1: gradients of the states leaving them (the recurrence runs backwards)."""
     dev, nc, st = conv_out.device, L // _CT, status_tensor(conv_out.device)
     states = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev)
-    if _walk_states(B * Hv, nc):
-        final = torch.empty(B, H, Hv // H * 64, 128, dtype=torch.float32, device=dev) if want_final else None
-        _run("ssm_ssd_state_walk", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(init),
-             _p(states), _p(final), B, L, H, Hv, G, mode, _p(st), _st())
-        return states, final
+    if mode == 1 and _walk_states(B * Hv, nc):         # forwards, ssm_ssd_walk_scan walks and scans at once
+        _run("ssm_ssd_state_walk", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(l), _p(states), B, L, H, Hv, G,
+             _p(st), _st())
+        return states, None
     final = torch.empty(B, Hv, 128, 64, dtype=torch.float32, device=dev) if want_final else None
     local = torch.empty(B, Hv, nc, 128, 64, dtype=torch.float32, device=dev)
     _run("ssm_ssd_chunk_state", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(local),
