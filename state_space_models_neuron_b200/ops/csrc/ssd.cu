@@ -821,6 +821,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
 //                 3  dx and the per-token sums                   4  (warps 0-3, a thread per row) ddt, dA, dD, d dt_bias
 //   warp 16     issues the products: CB, dM behind the loads; dU, C S_in and then dB, dC behind 2
 //   warp 17     loads and the store of dx
+// The arithmetic of 2 goes two values at a time (fma.rn.f32x2 and the like): 124 -> 116 us at 128 slices x 16 chunks.
 // The loads of the next head start as soon as the last product that reads a tile is complete, 3 runs under the products of
 // dB and dC, 4 under the next head's 1.  Bound by the per-pair arithmetic of 2 and the hand-overs between the steps: with
 // 128-token tiles and four operands per head in shared memory there is room for one head only.
@@ -1103,12 +1104,25 @@ ssd_chunk_scan_bwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __gr
               load8f_smem(s_l + j0, lv);
               load8f_smem(s_dt + j0, dv);
               #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float lam = (j0 + e <= row) ? __expf(li - lv[e]) : 0.f;
-                m0[e] = __uint_as_float(cb[ch * 8 + e]) * lam;
-                dc[e] = __uint_as_float(dm[ch * 8 + e]) * lam * dv[e];
+              for (int e = 0; e < 8; e += 2) {
+                const int i = ch * 8 + e;
+                float lam0, lam1;
+                unpack2(exp_diff2(pack2(li, li), pack2(lv[e], lv[e + 1])), lam0, lam1);
+                if (wq == rw) {                        // the diagonal block
+                  lam0 = half * 16 + i <= lane ? lam0 : 0.f;
+                  lam1 = half * 16 + i + 1 <= lane ? lam1 : 0.f;
+                }
+                const uint64_t lam = pack2(lam0, lam1);
+                const uint64_t mm = mul2(pack2(__uint_as_float(cb[i]), __uint_as_float(cb[i + 1])), lam);
+                const uint64_t dd = mul2(pack2(__uint_as_float(dm[i]), __uint_as_float(dm[i + 1])), pack2(dv[e], dv[e + 1]));
+                unpack2(mm, m0[e], m0[e + 1]);
+                unpack2(mul2(dd, lam), dc[e], dc[e + 1]);
                 // W[i][j] = dM[i][j] * (CB Lambda dt_j)[i][j], strictly below the diagonal
-                wv[ch * 8 + e] = (j0 + e < row) ? __uint_as_float(dm[ch * 8 + e]) * m0[e] * dv[e] : 0.f;
+                unpack2(mul2(dd, mm), wv[i], wv[i + 1]);
+                if (wq == rw) {
+                  wv[i] = half * 16 + i < lane ? wv[i] : 0.f;
+                  wv[i + 1] = half * 16 + i + 1 < lane ? wv[i + 1] : 0.f;
+                }
               }
               const uint32_t off = sw128_offset(row, (wq & 1) * 4 + half * 2 + ch);
               *reinterpret_cast<uint4*>(m_at + off) = pack8(m0);
