@@ -43,7 +43,8 @@ struct AttnFwdParams {
 // has grown by more than 2^8 since its last rescaling (the sums use the same stale maximum, so the quotient is exact);
 // P <= 2^8 keeps its relative precision in bf16.
 // Bound by the exponentials (16 per clock and SM: as long as the products of a tile) and the softmax arithmetic around them.
-// One 128-thread group doing everything in turn took 1541 us for 8192 queries of 32 heads, this 695 us (8192 x 16: 870 -> 424, 4096 x 32: 467 -> 248).
+// One 128-thread group doing everything in turn took 1541 us for 8192 queries of 32 heads, this 647 us (8192 x 16: 870 -> 402,
+// 4096 x 32: 467 -> 232).
 constexpr int ATTN_FWD_THREADS = 320;
 constexpr int KV_RING = 3;
 constexpr int ATTN_FWD_SMEM = (4 + KV_RING) * ATILE + 256 + 1024;
@@ -197,17 +198,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         m_run = top;
       }
       const float off = m_run * c;
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint64_t c2 = pack2(c, c), off2 = pack2(-off, -off);
+      uint64_t sum2[4] = {0, 0, 0, 0};
       uint32_t pk[64];
       #pragma unroll
       for (int i = 0; i < 4; ++i) {
         #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          const float a0 = exp2f(fmaf(__uint_as_float(v[i][e]), c, -off));
-          const float a1 = exp2f(fmaf(__uint_as_float(v[i][e + 1]), c, -off));
-          sum[i] += a0 + a1;
+          float a0, a1;
+          unpack2(fma2(pack2(__uint_as_float(v[i][e]), __uint_as_float(v[i][e + 1])), c2, off2), a0, a1);
+          a0 = exp2f(a0); a1 = exp2f(a1);
+          sum2[i] = add2(sum2[i], pack2(a0, a1));
           pk[i * 16 + e / 2] = pack_bf16(a0, a1);
         }
+      }
+      float sum[4];
+      #pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float a0, a1;
+        unpack2(sum2[i], a0, a1);
+        sum[i] = a0 + a1;
       }
       l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       if (j > 0) {                                     // P and O are in use until the previous product is complete
@@ -280,7 +290,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 //   warp 20      issues all products;  warp 21  loads
 // The scores of the next tile are issued before the three gradient products of this one, so the arithmetic of a tile and the
 // products of the tile before it overlap.  Bound by these two in turn.  One 128-thread group doing everything in turn, with a
-// reduction instruction per 16 bytes of dQ, took 3569 us for 8192 queries of 32 heads, this 2670 us (2863 with eight warps for P and dS).
+// reduction instruction per 16 bytes of dQ, took 3569 us for 8192 queries of 32 heads, this 2131 us (2863 with eight warps for P and dS, 2670 without
+// packed arithmetic and with masks on every tile).
 struct AttnBwdParams {
   const float* lse; const float* delta;     // [B, Hq, L]
   __nv_bfloat16* dk; __nv_bfloat16* dv;     // [B*L, Hkv*128]
@@ -482,14 +493,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       #pragma unroll
       for (int e4 = 0; e4 < 4; ++e4) {
         const float4 ls = *reinterpret_cast<const float4*>(lse + e4 * 4), de = *reinterpret_cast<const float4*>(delta + e4 * 4);
-        const float lv[4] = {ls.x, ls.y, ls.z, ls.w}, dv[4] = {de.x, de.y, de.z, de.w};
+        const uint64_t lv[2] = {pack2(ls.x, ls.y), pack2(ls.z, ls.w)}, dv[2] = {pack2(de.x, de.y), pack2(de.z, de.w)};
         float pv[4], ds[4];
         #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < 4; e += 2) {
           const int i = e4 * 4 + e;
-          pv[e] = exp2f(fmaf(__uint_as_float(sv[i]), c, -lv[e] * LOG2E));
-          if (rel + wg * 16 + i < row) pv[e] = 0.f;            // the query lies before the key
-          ds[e] = pv[e] * (__uint_as_float(dp[i]) - dv[e]) * p.scale;
+          unpack2(fma2(pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), pack2(c, c), mul2(lv[e / 2], pack2(-LOG2E, -LOG2E))),
+                  pv[e], pv[e + 1]);
+          pv[e] = exp2f(pv[e]); pv[e + 1] = exp2f(pv[e + 1]);
+          if (rel < AT) {                                      // a tile on the diagonal: queries before the key
+            pv[e] = rel + wg * 16 + i < row ? 0.f : pv[e];
+            pv[e + 1] = rel + wg * 16 + i + 1 < row ? 0.f : pv[e + 1];
+          }
+          const uint64_t g = fma2(dv[e / 2], pack2(-1.f, -1.f), pack2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])));
+          unpack2(mul2(mul2(pack2(pv[e], pv[e + 1]), g), pack2(p.scale, p.scale)), ds[e], ds[e + 1]);
         }
         pk[e4 * 2] = pack_bf16(pv[0], pv[1]); pk[e4 * 2 + 1] = pack_bf16(pv[2], pv[3]);
         dk[e4 * 2] = pack_bf16(ds[0], ds[1]); dk[e4 * 2 + 1] = pack_bf16(ds[2], ds[3]);
