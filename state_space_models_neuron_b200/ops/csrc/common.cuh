@@ -341,6 +341,19 @@ __device__ __forceinline__ uint64_t exp_diff2(uint64_t a, uint64_t b) {
   unpack2(mul2(fma2(b, pack2(-1.f, -1.f), a), pack2(1.4426950408889634f, 1.4426950408889634f)), x, y);
   return pack2(exp2f(x), exp2f(y));
 }
+__device__ __forceinline__ uint64_t bf16x2_pair(uint32_t v) { return pack2(bf16_lo(v), bf16_hi(v)); }
+__device__ __forceinline__ uint32_t pack_bf16_pair(uint64_t v) {
+  float a, b;
+  unpack2(v, a, b);
+  return pack_bf16(a, b);
+}
+// 1 / (1 + exp(-x)) of a pair
+__device__ __forceinline__ uint64_t sigmoid2(uint64_t x) {
+  float a, b;
+  unpack2(mul2(x, pack2(-1.4426950408889634f, -1.4426950408889634f)), a, b);
+  unpack2(add2(pack2(exp2f(a), exp2f(b)), pack2(1.f, 1.f)), a, b);
+  return pack2(1.f / a, 1.f / b);
+}
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : log1pf(__expf(x)); }

@@ -69,21 +69,22 @@ constexpr int CONV_K = 4;
 
 // Each thread owns 4 channels and walks a tile of tokens.  Both directions are bound by the bytes in flight: the loads of
 // the next four tokens are issued before the arithmetic of the present four (2048 x 10240: forward 34.5 -> 22.4 us,
-// backward 81.5 -> 55.3 us; 32768 x 5376: forward 264 -> 145 us).
+// backward 81.5 -> 51.2 us; 32768 x 5376: forward 264 -> 145 us).
 constexpr int CONV_CPT = 4;
 
-__device__ __forceinline__ void unpack4(const uint2 u, float (&f)[4]) {
-  f[0] = bf16_lo(u.x); f[1] = bf16_hi(u.x); f[2] = bf16_lo(u.y); f[3] = bf16_hi(u.y);
-}
+constexpr int CONV_PAIRS = CONV_CPT / 2;             // the arithmetic goes two channels at a time
+
+__device__ __forceinline__ void unpack4(const uint2 u, uint64_t (&f)[CONV_PAIRS]) { f[0] = bf16x2_pair(u.x); f[1] = bf16x2_pair(u.y); }
 
 // taps and bias of this thread's channels (the taps of a channel are 8 contiguous bytes)
 __device__ __forceinline__ void conv_params(const __nv_bfloat16* w, const __nv_bfloat16* bias, int c0,
-                                            float (&wt)[CONV_K][CONV_CPT], float (&bs)[CONV_CPT]) {
+                                            uint64_t (&wt)[CONV_K][CONV_PAIRS], uint64_t (&bs)[CONV_PAIRS]) {
   #pragma unroll
-  for (int e = 0; e < CONV_CPT; ++e) {
+  for (int e = 0; e < CONV_PAIRS; ++e) {
+    const int c = c0 + 2 * e;
     #pragma unroll
-    for (int k = 0; k < CONV_K; ++k) wt[k][e] = __bfloat162float(w[(c0 + e) * CONV_K + k]);
-    bs[e] = bias ? __bfloat162float(bias[c0 + e]) : 0.f;
+    for (int k = 0; k < CONV_K; ++k) wt[k][e] = pack2(__bfloat162float(w[c * CONV_K + k]), __bfloat162float(w[(c + 1) * CONV_K + k]));
+    bs[e] = bias ? pack2(__bfloat162float(bias[c]), __bfloat162float(bias[c + 1])) : 0;
   }
 }
 
@@ -98,7 +99,7 @@ conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
   if (!SSM_INDEX_OK(c0 + CONV_CPT - 1, C) || !SSM_INDEX_OK(C - 1, xs) || !SSM_INDEX_OK(C - 1, os)) return;   // whole vectors inside a row
   const int t0 = blockIdx.y * TOK;
   const int b = blockIdx.z;
-  float wt[CONV_K][CONV_CPT], bs[CONV_CPT];
+  uint64_t wt[CONV_K][CONV_PAIRS], bs[CONV_PAIRS];
   const __nv_bfloat16* xb = x + (long long)b * L * xs + c0;
   __nv_bfloat16* ob = out + (long long)b * L * os + c0;
   uint2 next[4];
@@ -107,7 +108,7 @@ conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
     for (int k = 0; k < 4; ++k) next[k] = t + k < L ? *reinterpret_cast<const uint2*>(xb + (long long)(t + k) * xs) : make_uint2(0, 0);
   };
   fetch(t0);
-  float h[3][CONV_CPT];   // x[t-3], x[t-2], x[t-1]
+  uint64_t h[3][CONV_PAIRS];   // x[t-3], x[t-2], x[t-1]
   #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int t = t0 - 3 + k;
@@ -127,14 +128,15 @@ conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
     for (int k = 0; k < 4; ++k) {
       const int t = t0 + i + k;
       if (t >= L) return;
-      float cur[CONV_CPT], o[CONV_CPT];
+      uint64_t cur[CONV_PAIRS], o[CONV_PAIRS];
       unpack4(now[k], cur);
       #pragma unroll
-      for (int e = 0; e < CONV_CPT; ++e) {
-        o[e] = silu_f(bs[e] + wt[0][e] * h[0][e] + wt[1][e] * h[1][e] + wt[2][e] * h[2][e] + wt[3][e] * cur[e]);
+      for (int e = 0; e < CONV_PAIRS; ++e) {
+        const uint64_t pre = fma2(wt[3][e], cur[e], fma2(wt[2][e], h[2][e], fma2(wt[1][e], h[1][e], fma2(wt[0][e], h[0][e], bs[e]))));
+        o[e] = mul2(pre, sigmoid2(pre));
         h[0][e] = h[1][e]; h[1][e] = h[2][e]; h[2][e] = cur[e];
       }
-      *reinterpret_cast<uint2*>(ob + (long long)t * os) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+      *reinterpret_cast<uint2*>(ob + (long long)t * os) = make_uint2(pack_bf16_pair(o[0]), pack_bf16_pair(o[1]));
     }
   }
 }
@@ -143,9 +145,9 @@ conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
 // gradients reach back into the tile.  T16: dy is bf16, else fp32; `dy` points at token t0 of these channels.
 template <int TOK, bool T16>
 __device__ __forceinline__ void conv_bwd_tile(const __nv_bfloat16* __restrict__ xb, long long xs, const void* __restrict__ dy,
-                                              long long ds, const float (&wt)[CONV_K][CONV_CPT], const float (&bs)[CONV_CPT],
+                                              long long ds, const uint64_t (&wt)[CONV_K][CONV_PAIRS], const uint64_t (&bs)[CONV_PAIRS],
                                               __nv_bfloat16* __restrict__ dx, long long dxs, int t0, int L,
-                                              float (&dw)[CONV_K][CONV_CPT], float (&db)[CONV_CPT]) {
+                                              uint64_t (&dw)[CONV_K][CONV_PAIRS], uint64_t (&db)[CONV_PAIRS]) {
   using Raw = typename std::conditional<T16, uint2, uint4>::type;
   uint2 xn[4];
   Raw gn[4];
@@ -162,36 +164,42 @@ __device__ __forceinline__ void conv_bwd_tile(const __nv_bfloat16* __restrict__ 
     }
   };
   fetch(0, 4);
-  float xw[3][CONV_CPT], dp[3][CONV_CPT];              // x and pre-activation gradients of the three tokens before
+  uint64_t xw[3][CONV_PAIRS], dp[3][CONV_PAIRS];              // x and pre-activation gradients of the three tokens before
   #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int t = t0 - 3 + k;
     unpack4(t >= 0 ? *reinterpret_cast<const uint2*>(xb + (long long)t * xs) : make_uint2(0, 0), xw[k]);
     #pragma unroll
-    for (int e = 0; e < CONV_CPT; ++e) dp[k][e] = 0.f;
+    for (int e = 0; e < CONV_PAIRS; ++e) dp[k][e] = 0;
   }
   auto token = [&](const uint2 xr, const Raw gr, int i, bool inside, bool store) {
     const bool valid = t0 + i < L;
-    float cur[CONV_CPT], g[CONV_CPT], d[CONV_CPT];
+    const uint64_t one = pack2(1.f, 1.f), minus = pack2(-1.f, -1.f);
+    uint64_t cur[CONV_PAIRS], g[CONV_PAIRS], d[CONV_PAIRS];
     unpack4(xr, cur);
     if constexpr (T16) unpack4(gr, g);
-    else { g[0] = __uint_as_float(gr.x); g[1] = __uint_as_float(gr.y); g[2] = __uint_as_float(gr.z); g[3] = __uint_as_float(gr.w); }
+    else {
+      g[0] = pack2(__uint_as_float(gr.x), __uint_as_float(gr.y));
+      g[1] = pack2(__uint_as_float(gr.z), __uint_as_float(gr.w));
+    }
     #pragma unroll
-    for (int e = 0; e < CONV_CPT; ++e) {
-      const float pre = bs[e] + wt[0][e] * xw[0][e] + wt[1][e] * xw[1][e] + wt[2][e] * xw[2][e] + wt[3][e] * cur[e];
-      const float sg = sigmoid_f(pre);
-      const float dpre = valid ? g[e] * sg * (1.f + pre * (1.f - sg)) : 0.f;
+    for (int e = 0; e < CONV_PAIRS; ++e) {
+      const uint64_t pre = fma2(wt[3][e], cur[e], fma2(wt[2][e], xw[2][e], fma2(wt[1][e], xw[1][e], fma2(wt[0][e], xw[0][e], bs[e]))));
+      const uint64_t sg = sigmoid2(pre);
+      // g sg (1 + pre (1 - sg))
+      const uint64_t dpre = valid ? mul2(mul2(g[e], sg), fma2(pre, fma2(sg, minus, one), one)) : 0;
       if (inside) {
-        dw[0][e] += xw[0][e] * dpre; dw[1][e] += xw[1][e] * dpre; dw[2][e] += xw[2][e] * dpre;
-        dw[3][e] += cur[e] * dpre; db[e] += dpre;
+        dw[0][e] = fma2(xw[0][e], dpre, dw[0][e]); dw[1][e] = fma2(xw[1][e], dpre, dw[1][e]);
+        dw[2][e] = fma2(xw[2][e], dpre, dw[2][e]); dw[3][e] = fma2(cur[e], dpre, dw[3][e]);
+        db[e] = add2(db[e], dpre);
       }
       // dx[t-3] = w3*dpre[t-3] + w2*dpre[t-2] + w1*dpre[t-1] + w0*dpre[t]
-      d[e] = wt[3][e] * dp[0][e] + wt[2][e] * dp[1][e] + wt[1][e] * dp[2][e] + wt[0][e] * dpre;
+      d[e] = fma2(wt[0][e], dpre, fma2(wt[1][e], dp[2][e], fma2(wt[2][e], dp[1][e], mul2(wt[3][e], dp[0][e]))));
       dp[0][e] = dp[1][e]; dp[1][e] = dp[2][e]; dp[2][e] = dpre;
       xw[0][e] = xw[1][e]; xw[1][e] = xw[2][e]; xw[2][e] = cur[e];
     }
     if (store && t0 + i - 3 < L)
-      *reinterpret_cast<uint2*>(dx + (long long)(i - 3) * dxs) = make_uint2(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]));
+      *reinterpret_cast<uint2*>(dx + (long long)(i - 3) * dxs) = make_uint2(pack_bf16_pair(d[0]), pack_bf16_pair(d[1]));
   };
   #pragma unroll 1
   for (int i = 0; i < TOK; i += 4) {
@@ -210,7 +218,8 @@ __device__ __forceinline__ void conv_bwd_tile(const __nv_bfloat16* __restrict__ 
 // Backward.  dy for channels [0, c_split) comes from dy16 (bf16, row stride ds16); channels >= c_split from
 // dy32 (fp32, row stride ds32, indexed by channel - c_split).  dx is written with row stride dxs.
 // part [gridDim.z * gridDim.y, C, 5] receives per-tile partial sums (dw[0..3], db).
-// Three blocks per SM: with four the registers of a tile spill (2048 x 10240: 64.7 us, three 55.3; 8192 x 5376: 112.7 and 105.5).
+// Three blocks per SM: with four the registers of a tile spilled (2048 x 10240: 64.7 us, three 55.3; 8192 x 5376: 112.7 and
+// 105.5; with the arithmetic in packed pairs 51.2 and 92.2).
 template <int TOK>
 __global__ void __launch_bounds__(128, 3)
 conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const __nv_bfloat16* __restrict__ w,
@@ -221,13 +230,13 @@ conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
   if (c0 >= C) return;
   const int t0 = blockIdx.y * TOK;
   const int b = blockIdx.z;
-  float wt[CONV_K][CONV_CPT], bs[CONV_CPT], dw[CONV_K][CONV_CPT], db[CONV_CPT];
+  uint64_t wt[CONV_K][CONV_PAIRS], bs[CONV_PAIRS], dw[CONV_K][CONV_PAIRS], db[CONV_PAIRS];
   conv_params(w, bias, c0, wt, bs);
   #pragma unroll
-  for (int e = 0; e < CONV_CPT; ++e) {
-    db[e] = 0.f;
+  for (int e = 0; e < CONV_PAIRS; ++e) {
+    db[e] = 0;
     #pragma unroll
-    for (int k = 0; k < CONV_K; ++k) dw[k][e] = 0.f;
+    for (int k = 0; k < CONV_K; ++k) dw[k][e] = 0;
   }
   const long long first = (long long)b * L + t0;
   const __nv_bfloat16* xb = x + (long long)b * L * xs + c0;
@@ -236,9 +245,10 @@ conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
   else conv_bwd_tile<TOK, false>(xb, xs, dy32 + first * ds32 + (c0 - c_split), ds32, wt, bs, dxt, dxs, t0, L, dw, db);
   float* pp = part + ((long long)(blockIdx.z * gridDim.y + blockIdx.y) * C + c0) * 5;
   #pragma unroll
-  for (int e = 0; e < CONV_CPT; ++e) {
-    pp[e * 5 + 0] = dw[0][e]; pp[e * 5 + 1] = dw[1][e]; pp[e * 5 + 2] = dw[2][e]; pp[e * 5 + 3] = dw[3][e];
-    pp[e * 5 + 4] = db[e];
+  for (int e = 0; e < CONV_PAIRS; ++e) {
+    #pragma unroll
+    for (int k = 0; k < CONV_K; ++k) unpack2(dw[k][e], pp[e * 10 + k], pp[e * 10 + 5 + k]);
+    unpack2(db[e], pp[e * 10 + 4], pp[e * 10 + 9]);
   }
 }
 
