@@ -2,9 +2,9 @@
 // Both kernels are bound by reading the weights once from HBM, so the work is cut for bytes in flight on every SM and
 // not for tensor throughput: the 128-row tiles of gemm.cu leave most SMs idle here (N / 192 tiles) and pay a read-back
 // of K slices through global memory.
-//   M <= 8    (16 with few weights) gemm_rows_kernel: 16 weight rows per CTA, its eight warps share K and add up in shared memory; operands
-//             go from global memory straight into mma.sync fragments (no descriptors, barriers or TMEM to set up:
-//             at these sizes set-up latency is as long as the transfer).
+//   M <= 8    (16 with few weights) gemm_rows_kernel: 16 weight rows per CTA, its eight warps share K and add up in shared
+//             memory; operands go from global memory straight into mma.sync fragments (no descriptors, barriers or TMEM
+//             to set up: at these sizes set-up latency is as long as the transfer).
 //   M <= 128  gemm_cols_kernel: the weight rows are the 128-row side of a tcgen05 tile and X the 32-, 64- or 128-column
 //             side; a cluster of up to eight CTAs shares K and adds the partial tiles over distributed shared memory.
 // Sums run in a fixed order, so results are reproducible.
@@ -16,7 +16,7 @@
 
 namespace ssm {
 
-// ------------------------------------------------------------------------------------------------ M <= 16
+// ------------------------------------------------------------------------------------------------ M <= 8 (16)
 constexpr int ROWS_WARPS = 8;
 constexpr int ROWS_CHUNK = 64;       // K elements of one warp step: 128 bytes of every weight row
 

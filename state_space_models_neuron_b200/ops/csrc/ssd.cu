@@ -6,7 +6,7 @@
 //             S_local = sum_j exp(l_T - l_j) dt_j B_j (x) x_j ;  S_in[c+1] = exp(l_T) S_in[c] + S_local[c]
 //   backward  see ssd_chunk_scan_bwd_kernel.
 // All 128x128x{64,128} products run on tcgen05 with fp32 accumulators in TMEM; operands come straight from
-// TMA (B, C, x, dY, states) or are built by the 128 threads of the CTA in the 128-byte-swizzled layout
+// TMA (B, C, x, dY, states) or are built by the arithmetic warps in the 128-byte-swizzled layout
 // (decay-weighted CB^T, scaled x / dY).  The decay factors are always formed as exp of a difference of
 // cumulative sums, never as a ratio of exponentials.
 // Reference math: mamba2/mamba2_kernel.py:15-62,138-169 (forward), :358-480 (backward).

@@ -662,11 +662,12 @@ def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, 
 
 
 def _walk_states(slices: int, nc: int) -> bool:
-    """One kernel that walks the chunks of a head slice, or one CTA per chunk and a recurrence kernel behind it.  A chunk of
-    the walk takes 1.4 us however few slices walk; the two kernels take 18 ns per slice and chunk (64 slices x 64 chunks:
-    89 us walking, 75 us separately; 128 x 16: 26 and 65; 1280 x 16: 243 and 640) and a second launch, which decides for
-    one or two chunks."""
-    return slices >= 80 or nc <= 2
+    """Kernels that walk the chunks of a head slice, or one CTA per chunk and a recurrence kernel between.  A chunk of the
+    forward walk takes 2.7 us, of the backward states 1.4 us, for up to 148 slices; the separate kernels take 58 and 35 ns per
+    slice and chunk (us at 64 chunks, forward / backward states: 32 slices walk 207 / 97, separate 168 / 91; 48 slices
+    210 / 99, 226 / 122; 64 slices 215 / 99, 279 / 145; 160 slices, the start of a second wave, 414 / 186, 638 / 366).  Up to
+    four chunks the launches saved decide."""
+    return slices >= 44 or nc <= 4
 
 
 def _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a):
