@@ -95,15 +95,22 @@ class _NoGrad:
         pass
 
 
+def _observed() -> bool:
+    """True where forward-mode differentiation, a functorch transform or `torch.jit.trace` wants to see the call: a tracer
+    that saw the tensors made inside would record them without the kernel that fills them through their addresses."""
+    return (_forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+            or torch._C._get_tracing_state() is not None)
+
+
 def _recording() -> bool:
-    """True where autograd, forward-mode differentiation or a functorch transform may want to see the call."""
-    return torch.is_grad_enabled() or _forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+    """True where autograd or one of the observers above may want to see the call."""
+    return torch.is_grad_enabled() or _observed()
 
 
 def _apply(function, *args):
     """`function.apply`, or its forward alone where autograd would record nothing: entering and leaving an autograd
-    Function costs the host 5 to 10 us per call, half of a small kernel's launch.  Forward-mode differentiation and
-    functorch transforms keep `apply`, which answers them as before."""
+    Function costs the host 5 to 10 us per call, half of a small kernel's launch.  Forward-mode differentiation, functorch
+    transforms and tracing keep `apply`, which answers them."""
     if _recording():
         return function.apply(*args)
     return function.forward(_NoGrad(), *args)
@@ -596,6 +603,8 @@ def ce_backward(logits, labels, row_max, row_sum, grad_rows, vocab_start, ignore
 
 def widen(x):
     """fp32 copy of bf16 `x` [..., n] (rows may be padded); inference only, the gradient path keeps `x.float()`."""
+    if _observed():
+        return x.float()
     n = x.shape[-1]
     x2 = x.reshape(-1, n) if x.dim() != 2 else x
     if (x.dtype != torch.bfloat16 or x2.shape[0] == 0 or x2.shape[0] > 65535 or n % 8 or n == 0 or x2.stride(1) != 1

@@ -51,3 +51,26 @@ def test_function_where_something_may_record():
             assert "_NoGrad" not in _Double.contexts
         with pytest.raises(RuntimeError):                     # no vmap rule: refused, as before
             torch.vmap(lambda t: cuda_ops._apply(_Double, t))(torch.ones(2, 3))
+
+
+class _Filled(torch.autograd.Function):
+    """As the kernels: the output is made inside and filled through its address."""
+
+    @staticmethod
+    def forward(ctx, x):
+        out = torch.empty_like(x)
+        out.numpy()[:] = 2 * x.numpy()
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        return 2 * g
+
+
+def test_traced_without_grad():
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda x: cuda_ops._apply(_Filled, x) + 1, torch.ones(4), check_trace=False)
+        assert torch.equal(traced(torch.full((4,), 5.0)), torch.full((4,), 11.0))
+        # the widening of logits takes the operation that a tracer can record
+        traced = torch.jit.trace(lambda x: cuda_ops.widen(x) + 1, torch.ones(2, 8).bfloat16(), check_trace=False)
+        assert torch.equal(traced(torch.full((2, 8), 5.0).bfloat16()), torch.full((2, 8), 6.0))
