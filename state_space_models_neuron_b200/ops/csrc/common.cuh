@@ -300,7 +300,10 @@ __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk) {
 // ---------------------------------------------------------------- programmatic dependent launch
 // A kernel launched with launch_dependent() may start while its predecessor in the stream still runs.  It touches global
 // memory only behind pdl_wait(), which returns when the predecessor has completed and its writes are visible (hints that
-// bring weights into L2 may go first: they deliver no values).  pdl_trigger() lets the successor start in the same way.
+// bring weights into L2 may go first: they deliver no values).  As any kernel in front of it may still write what it reads
+// while it is resident, the pointers that it reads through are not __restrict__ (through const __restrict__ the compiler may
+// load with ld.global.nc, which is defined only for data that nobody writes while the grid lives, and may move loads across
+// the wait), and it issues no ld.global.nc itself.  pdl_trigger() lets the successor start in the same way.
 // What this saves is the launch and set-up latency between the kernels of a decoding step, which are 2 to 5 us long.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -11,9 +11,8 @@
 namespace ssm {
 
 __global__ void __launch_bounds__(256)
-decode_conv_step_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __nv_bfloat16* __restrict__ state,
-                        const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
-                        float* __restrict__ act, int C) {
+decode_conv_step_kernel(const __nv_bfloat16* xnew, long long xs, __nv_bfloat16* state, const __nv_bfloat16* w,
+                        const __nv_bfloat16* bias, float* __restrict__ act, int C) {
   pdl_trigger();
   pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -38,7 +37,7 @@ decode_conv_step_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __
 // State update and read-out of one head by 128 threads: warp w owns rows p = 4w .. 4w+3, 4w+16 .., ...; lanes own
 // n = 4*lane + 128*r.  xh [P], Bv / Cv [N]: activations of the head (global or shared memory).
 __device__ __forceinline__ void decode_ssm_head(const float* xh, const float* Bv, const float* Cv, float dt, float decay,
-                                                float Dh, float* __restrict__ S, __nv_bfloat16* __restrict__ y, int P, int N) {
+                                                float Dh, float* S, __nv_bfloat16* __restrict__ y, int P, int N) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // four rows per warp iteration: four independent 16-byte loads per lane are in flight before any arithmetic,
   // and the four row sums are reduced together (the state makes one round trip; this loop is latency-bound otherwise)
@@ -83,10 +82,8 @@ __device__ __forceinline__ void decode_ssm_head(const float* xh, const float* Bv
 
 // grid (H, B), 128 threads, behind decode_conv_step_kernel
 __global__ void __launch_bounds__(128)
-decode_ssm_step_kernel(const float* __restrict__ act, const __nv_bfloat16* __restrict__ dt_raw, long long dts,
-                       const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
-                       float* __restrict__ state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G,
-                       int d_in) {
+decode_ssm_step_kernel(const float* act, const __nv_bfloat16* dt_raw, long long dts, const float* dt_bias, const float* A,
+                       const float* D, float* state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G, int d_in) {
   pdl_trigger();
   pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y;
@@ -109,9 +106,9 @@ __device__ __forceinline__ float decode_param(const void* p, int h, bool bf16) {
   return bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[h]) : reinterpret_cast<const float*>(p)[h];
 }
 __global__ void __launch_bounds__(128)
-decode_mixer_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __nv_bfloat16* __restrict__ window,
-                    const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias, const DecodeParams prm,
-                    float* __restrict__ state, __nv_bfloat16* __restrict__ y, int C, int H, int P, int N, int G, int d_in) {
+decode_mixer_kernel(const __nv_bfloat16* xnew, long long xs, __nv_bfloat16* window, const __nv_bfloat16* w,
+                    const __nv_bfloat16* bias, const DecodeParams prm, float* state, __nv_bfloat16* __restrict__ y, int C, int H,
+                    int P, int N, int G, int d_in) {
   extern __shared__ __align__(16) float act[];         // B [N] | C [N] | x [P]
   pdl_trigger();
   const int h = blockIdx.x, b = blockIdx.y;
@@ -122,21 +119,38 @@ decode_mixer_kernel(const __nv_bfloat16* __restrict__ xnew, long long xs, __nv_b
   pdl_wait();
   if (!SSM_INDEX_OK(d_in + 2 * G * N - 1, C) || !SSM_INDEX_OK(h * P + P - 1, d_in) || !SSM_INDEX_OK(C + h, xs)) return;
   const __nv_bfloat16* xr = xnew + (long long)b * xs;
-  for (int i = threadIdx.x; i < 2 * N + P; i += 128) {
-    const bool own = i >= 2 * N;
-    const int c = own ? h * P + i - 2 * N : i < N ? d_in + g * N + i : d_in + G * N + g * N + i - N;
-    uint2* sp = reinterpret_cast<uint2*>(window + ((long long)b * C + c) * 4);
-    const uint2 s = *sp, wv = *reinterpret_cast<const uint2*>(w + (long long)c * 4);
-    const float x1 = bf16_hi(s.x), x2 = bf16_lo(s.y), x3 = bf16_hi(s.y), x4 = __bfloat162float(xr[c]);
-    if (own) *sp = make_uint2(pack_bf16(x1, x2), pack_bf16(x3, x4));
-    float pre = bias ? __bfloat162float(bias[c]) : 0.f;
-    pre += bf16_lo(wv.x) * x1 + bf16_hi(wv.x) * x2 + bf16_lo(wv.y) * x3 + bf16_hi(wv.y) * x4;
-    act[i] = silu_f(pre);
+  const float raw = __bfloat162float(xr[C + h]), bias_h = decode_param(prm.dt_bias, h, prm.bf16_mask & 4),
+              log_a = decode_param(prm.A_log, h, prm.bf16_mask & 1), Dh = decode_param(prm.D, h, prm.bf16_mask & 2);
+  // three channels per thread at a time (all of them at N = 128 and P <= 128): their loads go out together, in front of the
+  // stores to the window, which they must not pass (2.7B, 64 sequences, us per token: 1218 one by one, 1184)
+  for (int i0 = threadIdx.x; i0 < 2 * N + P; i0 += 3 * 128) {
+    uint2 s[3], wv[3];
+    float x4[3], pre[3];
+    #pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int i = i0 + k * 128;
+      if (i >= 2 * N + P) break;
+      const int c = i >= 2 * N ? h * P + i - 2 * N : i < N ? d_in + g * N + i : d_in + G * N + g * N + i - N;
+      s[k] = *reinterpret_cast<const uint2*>(window + ((long long)b * C + c) * 4);
+      wv[k] = *reinterpret_cast<const uint2*>(w + (long long)c * 4);
+      x4[k] = __bfloat162float(xr[c]);
+      pre[k] = bias ? __bfloat162float(bias[c]) : 0.f;
+    }
+    #pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int i = i0 + k * 128;
+      if (i >= 2 * N + P) break;
+      const float x1 = bf16_hi(s[k].x), x2 = bf16_lo(s[k].y), x3 = bf16_hi(s[k].y);
+      if (i >= 2 * N)                                    // this head's own x channels
+        *reinterpret_cast<uint2*>(window + ((long long)b * C + h * P + i - 2 * N) * 4) = make_uint2(pack_bf16(x1, x2), pack_bf16(x3, x4[k]));
+      pre[k] += bf16_lo(wv[k].x) * x1 + bf16_hi(wv[k].x) * x2 + bf16_lo(wv[k].y) * x3 + bf16_hi(wv[k].y) * x4[k];
+      act[i] = silu_f(pre[k]);
+    }
   }
-  const float dt = softplus_f(__bfloat162float(xr[C + h]) + decode_param(prm.dt_bias, h, prm.bf16_mask & 4));
-  const float A = -expf(decode_param(prm.A_log, h, prm.bf16_mask & 1));
+  const float dt = softplus_f(raw + bias_h);
+  const float A = -expf(log_a);
   __syncthreads();
-  decode_ssm_head(act + 2 * N, act, act + N, dt, __expf(A * dt), decode_param(prm.D, h, prm.bf16_mask & 2), S, y + (long long)b * d_in + h * P, P, N);
+  decode_ssm_head(act + 2 * N, act, act + N, dt, __expf(A * dt), Dh, S, y + (long long)b * d_in + h * P, P, N);
 }
 
 }  // namespace ssm

@@ -28,7 +28,7 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // volatile: the loads of a step stay in front of its products (the compiler would otherwise sink each load to its use
-// and leave two of them in flight)
+// and leave two of them in flight).  Ordinary loads, for X and the weights: see pdl_wait().
 __device__ __forceinline__ uint4 ld8_if(bool in, const __nv_bfloat16* p) {
   uint4 u;
   asm volatile(
@@ -36,9 +36,9 @@ __device__ __forceinline__ uint4 ld8_if(bool in, const __nv_bfloat16* p) {
       ".reg .pred q;\n\t"
       "setp.ne.s32 q, %5, 0;\n\t"
       "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
-      "@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
+      "@q ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
       "}\n"
-      : "=&r"(u.x), "=&r"(u.y), "=&r"(u.z), "=&r"(u.w) : "l"(p), "r"((int)in));
+      : "=&r"(u.x), "=&r"(u.y), "=&r"(u.z), "=&r"(u.w) : "l"(p), "r"((int)in) : "memory");
   return u;
 }
 
@@ -46,9 +46,8 @@ __device__ __forceinline__ uint4 ld8_if(bool in, const __nv_bfloat16* p) {
 // {0,1} and {2,3} of the eight are the two k pairs of one 16-wide step and {4..7} those of the next, for both operands.
 template <int NT, int UNROLL>         // NT tiles of 8 rows of X, UNROLL chunks in flight
 __global__ void __launch_bounds__(ROWS_WARPS * 32)
-gemm_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w, long long ldw,
-                 const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, long long ldo, int M, int N,
-                 int K) {
+gemm_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, long long ldw, const __nv_bfloat16* bias,
+                 __nv_bfloat16* __restrict__ out, long long ldo, int M, int N, int K) {
   __shared__ float red[ROWS_WARPS][NT * 8][16 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * 16;
