@@ -357,6 +357,9 @@ __device__ __forceinline__ uint64_t sigmoid2(uint64_t x) {
   unpack2(add2(pack2(exp2f(a), exp2f(b)), pack2(1.f, 1.f)), a, b);
   return pack2(1.f / a, 1.f / b);
 }
+// what a running sum of exp(x - max) is relative to: a maximum of -inf (nothing finite yet) counts as 0, so that -inf adds
+// nothing and NaN stays NaN
+__device__ __forceinline__ float ce_ref(float m) { return m == -INFINITY ? 0.f : m; }
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : log1pf(__expf(x)); }

@@ -619,10 +619,6 @@ template <typename T> __device__ __forceinline__ T from_f(float v);
 template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
 
-// what a running sum of exp(x - max) is relative to: a maximum of -inf (nothing finite yet) counts as 0, so that -inf adds
-// nothing and NaN stays NaN
-__device__ __forceinline__ float ce_ref(float m) { return m == -INFINITY ? 0.f : m; }
-
 // One pass over the logits, bound by reading them: 16-byte loads and an online softmax instead of one pass for the
 // maximum and one for the sum.  VEC: rows start on 16-byte boundaries (the tail of V is read one by one).
 template <typename T, bool VEC>

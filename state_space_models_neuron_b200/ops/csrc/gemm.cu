@@ -770,12 +770,13 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                       if (col < p.N) mx = fmaxf(mx, x);
                     }
                     if (mx > ce_m) { ce_s *= __expf(ce_m - mx); ce_m = mx; }
+                    const float ref = ce_ref(ce_m);
                     #pragma unroll
                     for (int e = 0; e < 8; ++e) {
                       const int col = nb + h * 32 + c * 8 + e;
                       const float x = (e & 1) ? bf16_hi(pk[e >> 1]) : bf16_lo(pk[e >> 1]);
                       if (col < p.N) {
-                        ce_s += __expf(x - ce_m);
+                        ce_s += __expf(x - ref);
                         if ((long long)col == ce_lbl) p.ce_tgt[m0 + row] = x;
                       }
                     }

@@ -60,3 +60,30 @@ def test_loss_of_labelled_forward(V):
     with torch.no_grad():
         again = model(input_ids=inputs, labels=ids)
     assert torch.equal(again.logits, out.logits)
+
+
+@pytest.mark.parametrize("M,V,K", [(5, 1000, 64), (300, 3004, 128)])
+def test_statistics_of_rows_with_infinite_logits(M, V, K):
+    """Row statistics out of the LM head's GEMM where the first logits of a row (a vector, a tile, all but one, all) are -inf."""
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    from state_space_models_neuron_b200.parallel.cross_entropy import parallel_cross_entropy
+    gen = torch.Generator(device="cuda").manual_seed(V)
+    for first in (3, 8, 40, 520, V - 1, V):
+        x, w = (torch.randn(*s, device="cuda", generator=gen).bfloat16() for s in ((M, K), (V, K)))
+        x[:, 0] = 0
+        x[1], x[1, 0], w[:, 0] = 0.5, 1e30, 0            # row 1 meets -1e60 in the first columns
+        w[:first, 0] = -1e30
+        labels = torch.randint(0, V, (M,), device="cuda", generator=gen)
+        labels[1] = V - 1
+        with torch.no_grad():
+            y, (m, s, t) = ops.linear_ce(x, w, labels)
+            loss = parallel_cross_entropy(y, labels, stats=(m, s, t))
+        cuda_ops.check_status()
+        ref = y.double()
+        assert torch.equal(torch.isinf(ref).sum(1), torch.tensor([0, first] + [0] * (M - 2), device="cuda"))
+        m2, s2, t2 = cuda_ops.ce_partials(y, labels, 0)          # the pass over the logits
+        assert torch.equal(m, m2) and torch.equal(t, t2) and torch.allclose(s, s2, rtol=1e-5)
+        want = torch.nn.functional.cross_entropy(ref, labels, reduction="none")
+        assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5, equal_nan=True)
+        assert torch.isfinite(loss[1]) == (first < V)
