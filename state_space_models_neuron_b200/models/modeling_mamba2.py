@@ -13,6 +13,7 @@ from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
+from torch.nn.modules.module import _has_any_global_hook
 from transformers import GenerationMixin, PreTrainedModel
 from transformers.utils import ModelOutput
 
@@ -185,6 +186,24 @@ class Mamba2Model(Mamba2PreTrainedModel):
         return hidden
 
 
+def _delivers_statistics(head) -> bool:
+    """True for the plain head, whose GEMM can take the cross-entropy statistics along.  Any other module, a bias or a
+    gathered output has no such form; a hook, or a forward set on the module, gets the tensor that the head returns."""
+    return (type(head) is ColumnParallelLinear and head.bias is None and not head.gather_output and "forward" not in vars(head)
+            and not (head._forward_hooks or head._forward_pre_hooks or head._backward_hooks or head._backward_pre_hooks
+                     or _has_any_global_hook()))
+
+
+def _shift_labels(labels):
+    shifted = torch.full_like(labels, -100)
+    shifted[:, :-1] = labels[:, 1:]
+    return shifted
+
+
+def _mean_loss(logits, shifted, stats):
+    return parallel_cross_entropy(logits, shifted, stats=stats).sum() / (shifted.shape[0] * (shifted.shape[1] - 1))
+
+
 class Mamba2ForCausalLM(Mamba2PreTrainedModel, GenerationMixin):
     _tied_weights_keys = {"lm_head.weight": "backbone.embeddings.weight"}
 
@@ -239,30 +258,28 @@ class Mamba2ForCausalLM(Mamba2PreTrainedModel, GenerationMixin):
                                     hidden_states=out.hidden_states)
 
     def logits_and_loss(self, hidden, labels):
-        """(fp32 logits, loss or None).  Where the head's GEMM delivers the cross-entropy statistics of its rows, the loss
-        comes from them; a shifted copy of the fp32 logits and two passes over it took half of a scoring call."""
+        """(fp32 logits, loss or None); the loss is a function of these logits in autograd.  Where the head's GEMM delivers
+        the cross-entropy statistics of its rows the loss comes from them; a shifted copy of the fp32 logits and two passes
+        over it took half of a scoring call."""
         tp = ps.get_tensor_model_parallel_size() if self.backbone.sequence_parallel_enabled else 1
-        if (labels is not None and hidden.is_cuda and hidden.dtype == torch.bfloat16 and labels.device == hidden.device
-                and labels.dtype == torch.int64 and tuple(labels.shape) == (hidden.shape[0], hidden.shape[1] * tp)):
-            logits, loss = self._head_loss(hidden, labels)
-            return ops.widen(logits), loss
+        if (labels is not None and _delivers_statistics(self.lm_head) and hidden.is_cuda and hidden.dtype == torch.bfloat16
+                and labels.device == hidden.device and labels.dtype == torch.int64
+                and tuple(labels.shape) == (hidden.shape[0], hidden.shape[1] * tp)):
+            shifted = _shift_labels(labels)
+            logits, stats = self.lm_head(hidden, ce_labels=shifted)
+            logits = ops.widen(logits)
+            return logits, _mean_loss(logits, shifted, stats)
         logits = ops.widen(self.lm_head(hidden))
         if labels is None:
             return logits, None
         return logits, parallel_cross_entropy(logits[:, :-1, :], labels[:, 1:].to(logits.device)).mean()
 
-    def _head_loss(self, hidden, labels):
-        shifted = torch.full_like(labels, -100)
-        shifted[:, :-1] = labels[:, 1:]
-        shifted = shifted.to(hidden.device)
-        logits, stats = self.lm_head(hidden, ce_labels=shifted)
-        per_tok = parallel_cross_entropy(logits, shifted, stats=stats)
-        return logits, per_tok.sum() / (labels.shape[0] * (labels.shape[1] - 1))
-
     def loss_from_hidden(self, hidden, labels):
         """Loss without materialising fp32 logits for the caller: labels are shifted instead of
         the logits (position L-1 is ignored), the mean runs over the B*(L-1) real targets."""
-        return self._head_loss(hidden, labels)[1]
+        shifted = _shift_labels(labels).to(hidden.device)
+        logits, stats = self.lm_head(hidden, ce_labels=shifted)
+        return _mean_loss(logits, shifted, stats)
 
     @torch.no_grad()
     def prefill(self, input_ids, cache_params: Optional[Mamba2Cache] = None):

@@ -129,7 +129,6 @@ class Mamba2HybridForCausalLM(Mamba2HybridPreTrainedModel, GenerationMixin):
 
     loss_from_hidden = Mamba2ForCausalLM.loss_from_hidden
     logits_and_loss = Mamba2ForCausalLM.logits_and_loss
-    _head_loss = Mamba2ForCausalLM._head_loss
 
     def forward(self, input_ids=None, inputs_embeds=None, labels=None, output_hidden_states=None,
                 return_dict=None, **kwargs):
