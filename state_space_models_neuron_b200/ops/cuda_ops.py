@@ -719,8 +719,8 @@ def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner,
              _p(init_state), _p(final), B, L, H, Hv, G, d_inner, _p(st), _st())
         return y, dt, l, s_in, final, params
     s_in, final = _chunk_states(conv_out, C, d_inner, conv_out, C, dt, l, init_state, want_final, B, L, H, Hv, G, 0)
-    if final_out is not None and want_final:
-        final = final_out.copy_(final)
+    if want_final:
+        final = final.contiguous() if final_out is None else final_out.copy_(final)
     _run("ssm_ssd_chunk_scan_fwd", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
          B, L, H, Hv, G, d_inner, _p(st), _st())
     return y, dt, l, s_in, final, params

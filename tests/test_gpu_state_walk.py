@@ -81,3 +81,22 @@ def test_decode_step_equals_separate_kernels(monkeypatch, B, H, P, G, fp32):
     assert torch.allclose(out[0][2], out[1][2], rtol=1e-5, atol=1e-6)
     for a, b in zip(out[0][0], out[1][0]):
         assert ((a.float() - b.float()).abs() <= 2.0 ** -7 * (b.float().abs() + b.float().abs().mean())).all()
+
+
+@pytest.mark.parametrize("nc", [1, 4, 5])                      # walked, walked, a CTA per chunk
+@pytest.mark.parametrize("H,P,G", [(8, 64, 1), (8, 128, 2)])
+def test_decoding_takes_the_final_state(nc, H, P, G):
+    from state_space_models_neuron_b200 import ops
+    B, L, N, d = 2, nc * 128, 128, H * P
+    C = d + 2 * G * N
+    gen = torch.Generator(device="cuda").manual_seed(nc + H)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+    head = [make(H), make(H).abs(), make(H)]                   # dt_bias, A_log, D
+    y, state = ops.ssd_chunk_scan(make(B, L, H, P), make(B, L, H), -head[1].float().exp(), make(B, L, G, N), make(B, L, G, N),
+                                  head[2], head[0], chunk_size=128, return_final_state=True)
+    assert state.shape == (B, H, P, N) and state.is_contiguous()
+    before = state.clone()
+    ops.ssm_decode_step(make(B, d + C + H), make(B, C, 4), state, make(C, 1, 4), make(C), *head, make(d), d_inner=d, n_groups=G,
+                        d_state=N, head_dim=P, eps=1e-5, norm_group_size=None)
+    torch.cuda.synchronize()
+    assert not torch.equal(state, before)
