@@ -888,7 +888,8 @@ def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner
         B, H, C = zxBCdt.shape[0], d_inner // head_dim, d_inner + 2 * n_groups * d_state
         window, state = state_out
         if _recording() or not (window.dtype == zxBCdt.dtype and state.dtype == torch.float32 and window.is_contiguous()
-                                and state.is_contiguous() and window.device == state.device == zxBCdt.device
+                                and state.is_contiguous() and window.data_ptr() % 8 == 0     # the kernel stores whole windows
+                                and window.device == state.device == zxBCdt.device
                                 and tuple(window.shape) == (B, C, 4) and tuple(state.shape) == (B, H, head_dim, d_state)):
             state_out = None
     res = _apply(_MixerCore, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim,
