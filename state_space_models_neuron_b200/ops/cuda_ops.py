@@ -895,6 +895,8 @@ def mamba2_mixer_core(zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner
     res = _apply(_MixerCore, zxBCdt, conv_w, conv_b, dt_bias, A_log, D, norm_w, d_inner, n_groups, d_state, head_dim,
                  eps, gs, recompute, return_final_states, torch.is_grad_enabled(), state_out)
     if return_final_states:
+        if state_out is not None:          # written through their addresses: autograd learns of it here
+            torch.autograd.graph.increment_version(state_out)
         return res[0], (res[1], res[2])
     return res
 

@@ -31,3 +31,14 @@ def test_cache_tensors_anywhere_in_memory(offset, shift_state):
     assert same is cache and torch.equal(logits, want)
     for k in plain.conv_states:
         assert torch.equal(cache.conv_states[k], plain.conv_states[k]) and torch.equal(cache.ssm_states[k], plain.ssm_states[k])
+
+
+def test_gradient_through_an_overwritten_state_is_refused():
+    model, ids = _model_and_ids()
+    _, cache = model.prefill(ids)
+    for states in (cache.conv_states, cache.ssm_states):
+        scale = torch.ones((), device="cuda", requires_grad=True)
+        y = (scale.to(states[1].dtype) * states[1]).sum()       # saves the state
+        model.prefill(ids.flip(1), cache)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            y.backward()
