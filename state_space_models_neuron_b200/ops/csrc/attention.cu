@@ -39,16 +39,17 @@ struct AttnFwdParams {
 //   warps 0-3, 4-7  softmax of the first / second query tile, thread = query row (the row's 128 scores in registers)
 //   warp 8          issues all products;  warp 9  loads K and V tiles through a ring of three
 // The two tiles take turns: while one group's exponentials keep the special-function units busy, the tensor cores work on
-// the other's products.  S and O of both tiles fill the 512 TMEM columns.  O is rescaled in TMEM only when a row's maximum
-// has grown by more than 2^8 since its last rescaling (the sums use the same stale maximum, so the quotient is exact);
-// P <= 2^8 keeps its relative precision in bf16.
+// the other's products.  S and O of both tiles fill the 512 TMEM columns.  The online softmax and the turns of two tiles are
+// those of FlashAttention (Dao et al., 2022; Shah et al., 2024).  O is rescaled in TMEM for the warps in which a row's maximum
+// has grown: the largest P of a row is then 1, which bf16 holds exactly.  Rescaling only past a growth of 2^8 took 652 us
+// instead of 671 for 8192 queries of 32 heads, but put a rounding on that largest P: an error against 64 bits 1.5 % higher at
+// 1024 queries.
 // Bound by the exponentials (16 per clock and SM: as long as the products of a tile) and the softmax arithmetic around them.
-// One 128-thread group doing everything in turn took 1541 us for 8192 queries of 32 heads, this 647 us (8192 x 16: 870 -> 402,
-// 4096 x 32: 467 -> 232).
+// One 128-thread group doing everything in turn took 1537 us for 8192 queries of 32 heads, this 671 us (8192 x 16: 834 -> 386,
+// 4096 x 32 with 8 key heads: 436 -> 213, 4 x 1024 x 16: 77.5 -> 47.2; one box, called back to back).
 constexpr int ATTN_FWD_THREADS = 320;
 constexpr int KV_RING = 3;
 constexpr int ATTN_FWD_SMEM = (4 + KV_RING) * ATILE + 256 + 1024;
-constexpr float RESCALE_LOG2 = 8.f;
 
 __global__ void __launch_bounds__(ATTN_FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -192,7 +193,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       float alpha = 1.f;
       bool grow = false;
       if (j == 0) m_run = top;
-      else if ((top - m_run) * c > RESCALE_LOG2) {
+      else if (top > m_run) {
         grow = true;
         alpha = exp2f((m_run - top) * c);
         m_run = top;
@@ -225,14 +226,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (!ok) break;
         tc_fence_after_sync();
         if (__any_sync(0xffffffffu, grow)) {
+          const uint64_t al2 = pack2(alpha, alpha);
           #pragma unroll 1
-          for (int i = 0; i < 4; ++i) {
-            uint32_t o[32];
-            tmem_ld32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 32), o);
+          for (int i = 0; i < 2; ++i) {
+            uint32_t o[2][32];
+            tmem_ld32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 64), o[0]);
+            tmem_ld32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 64 + 32), o[1]);
             tmem_ld_wait();
             #pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-            tmem_st32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 32), o);
+            for (int k = 0; k < 2; ++k)
+              #pragma unroll
+              for (int e = 0; e < 32; e += 2) {
+                float a0, a1;
+                unpack2(mul2(pack2(__uint_as_float(o[k][e]), __uint_as_float(o[k][e + 1])), al2), a0, a1);
+                o[k][e] = __float_as_uint(a0); o[k][e + 1] = __float_as_uint(a1);
+              }
+            tmem_st32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 64), o[0]);
+            tmem_st32(tmem_addr(tmem, lanes, 256 + t * 128 + i * 64 + 32), o[1]);
           }
           tmem_st_wait();
         }
