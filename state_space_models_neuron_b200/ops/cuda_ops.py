@@ -729,10 +729,14 @@ def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner,
 def _pick_hpc(hv_per_group, chunks, sms=148):
     """Head slices that one CTA of the backward scan walks (a divisor of the group's).  One CTA fits an SM and spends about
     one and a half heads on its set-up, B, C and the reduction of dB and dC, so the time is waves x (heads + 1.5): 64 chunks x
-    80 slices take 350 us with 16 heads per CTA (three waves) and 313 us with 40 (one)."""
+    80 slices take 350 us with 16 heads per CTA (three waves) and 313 us with 40 (one).
+    The CTAs of a group add to the same dB and dC in the order in which they finish; with at most two of them the sums are
+    the same in every run.  Where one or two per group fill the chip there are no more (by the count above five instead of
+    two would save 9 % at 384 chunks x 80 slices)."""
     def cost(hpc):
         return -(-chunks * (hv_per_group // hpc) // sms) * (hpc + 1.5)
-    return min((d for d in range(1, hv_per_group + 1) if hv_per_group % d == 0), key=cost)
+    most = 2 if chunks >= 2 * sms or (chunks >= sms and hv_per_group % 2 == 0) else hv_per_group
+    return min((d for d in range(1, hv_per_group + 1) if hv_per_group % d == 0 and hv_per_group // d <= most), key=cost)
 
 
 def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, dt_bias, ddt_out, ddt_stride,

@@ -1,12 +1,24 @@
 """Head slices per CTA of the backward scan."""
+import pytest
+
 from state_space_models_neuron_b200.ops.cuda_ops import _pick_hpc
+
+GROUPS, CHUNKS = (1, 2, 3, 7, 8, 16, 24, 40, 48, 64, 80, 128), (1, 9, 16, 64, 128, 147, 148, 149, 256, 295, 296, 384, 512, 4096)
 
 
 def test_divides_and_never_takes_more_waves_than_one_head_each():
-    for group in (1, 2, 3, 7, 8, 16, 24, 80, 128):
-        for chunks in (1, 9, 16, 64, 128, 147, 148, 149, 512, 4096):
+    for group in GROUPS:
+        for chunks in CHUNKS:
             hpc = _pick_hpc(group, chunks)
-            assert group % hpc == 0
-            cost = lambda h: -(-chunks * (group // h) // 148) * (h + 1.5)
-            assert all(cost(hpc) <= cost(h) for h in range(1, group + 1) if group % h == 0)
+            assert 1 <= hpc <= group and group % hpc == 0
+            assert -(-chunks * (group // hpc) // 148) <= -(-chunks * group // 148)
+            assert hpc == 1 or chunks * group > 148              # heads are walked only when CTAs would queue
     assert _pick_hpc(80, 64) == 40 and _pick_hpc(16, 128) == 16 and _pick_hpc(16, 16) == 2
+
+
+@pytest.mark.parametrize("group", GROUPS)
+def test_sums_of_at_most_two_where_that_fills_the_chip(group):
+    """More than two CTAs per group add to dB and dC in an order that changes from run to run."""
+    for chunks in CHUNKS:
+        if chunks >= 296 or (chunks >= 148 and group % 2 == 0):
+            assert group // _pick_hpc(group, chunks) <= 2
