@@ -8,8 +8,6 @@
 
 namespace ssm {
 
-struct alignas(16) bf16x8 { __nv_bfloat162 v[4]; };
-
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
   f[0] = bf16_lo(u.x); f[1] = bf16_hi(u.x); f[2] = bf16_lo(u.y); f[3] = bf16_hi(u.y);
@@ -64,7 +62,6 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // =====================================================================================
 // causal depthwise conv1d (4 taps) + SiLU, channels-last
 // =====================================================================================
-constexpr int CONV_TOK = 32;   // tokens per thread at full size; small problems use shorter tiles (more CTAs)
 constexpr int CONV_K = 4;
 
 // Each thread owns 4 channels and walks a tile of tokens.  Both directions are bound by the bytes in flight: the loads of

@@ -67,17 +67,18 @@ def test_decode_step_equals_separate_kernels(monkeypatch, B, H, P, G, fp32):
     p = [make(C, 1, 4).bfloat16(), make(C).bfloat16(), make(H).to(kind), make(H).abs().to(kind), make(H).to(kind), make(d).bfloat16()]
     kw = dict(d_inner=d, n_groups=G, d_state=N, head_dim=P, eps=1e-5, norm_group_size=d // G)
     window, state = make(B, C, 4).bfloat16(), make(B, H, P, N)
+    tokens = [torch.nn.functional.pad(make(B, d + C + H), (0, (-(d + C + H)) % 8)).bfloat16()[:, :d + C + H] for _ in range(3)]
     out = []
     mask = cuda_ops._head_param_mask
     for fused in (True, False):
         monkeypatch.setattr(cuda_ops, "_head_param_mask", mask if fused else (lambda *a: None))
         w, s = window.clone(), state.clone()
-        ys = [ops.ssm_decode_step(torch.nn.functional.pad(make(B, d + C + H) * 0 + k + 1, (0, (-(d + C + H)) % 8)).bfloat16()[:, :d + C + H],
-                                  w, s, *p, **kw) for k in range(3)]
+        ys = [ops.ssm_decode_step(t, w, s, *p, **kw) for t in tokens]
         out.append((ys, w, s))
     torch.cuda.synchronize()
     cuda_ops.check_status()
-    assert torch.equal(out[0][1], out[1][1])                    # windows are moved, not computed
+    assert torch.equal(out[0][1], out[1][1])                    # windows are moved, not computed: the last token, of four
+    assert torch.equal(out[0][1], torch.stack([window[..., 3]] + [t[:, d:d + C] for t in tokens], -1))
     assert torch.allclose(out[0][2], out[1][2], rtol=1e-5, atol=1e-6)
     for a, b in zip(out[0][0], out[1][0]):
         assert ((a.float() - b.float()).abs() <= 2.0 ** -7 * (b.float().abs() + b.float().abs().mean())).all()
@@ -100,3 +101,52 @@ def test_decoding_takes_the_final_state(nc, H, P, G):
                         d_state=N, head_dim=P, eps=1e-5, norm_group_size=None)
     torch.cuda.synchronize()
     assert not torch.equal(state, before)
+
+
+def _scan64(x, dt, A, Bm, Cm, D, bias):
+    """The scan chunk by chunk in the precision of its inputs."""
+    H, G = x.shape[2], Bm.shape[2]
+    dt = torch.nn.functional.softplus(dt + bias)
+    S, out = x.new_zeros(x.shape[0], H, 128, x.shape[3]), []
+    Be, Ce = (t.repeat_interleave(H // G, 2) for t in (Bm, Cm))
+    for t0 in range(0, x.shape[1], 128):
+        at = slice(t0, t0 + 128)
+        l, u = (A * dt)[:, at].cumsum(1).transpose(1, 2), (x[:, at] * dt[:, at, :, None]).transpose(1, 2)
+        b, c = Be[:, at].transpose(1, 2), Ce[:, at].transpose(1, 2)
+        decay = (l[..., :, None] - l[..., None, :]).tril().exp().tril()
+        out.append(((c @ b.transpose(-1, -2) * decay) @ u + l.exp()[..., None] * (c @ S)).transpose(1, 2))
+        S = l[..., -1:, None].exp() * S + b.transpose(-1, -2) @ (u * (l[..., -1:] - l).exp()[..., None])
+    return torch.cat(out, 1) + D[:, None] * x
+
+
+# a CTA of the backward scan walks one, some or all heads of a group; five and more chunks with few slices take the kernels
+# of one CTA per chunk, the others walk
+@pytest.mark.parametrize("B,L,H,P,G", [(1, 640, 6, 64, 1), (2, 256, 8, 64, 2), (1, 128, 4, 128, 1), (1, 768, 8, 128, 2)])
+def test_scan_gradients_for_any_number_of_heads_per_cta(monkeypatch, B, L, H, P, G):
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    gen = torch.Generator(device="cuda").manual_seed(L + H)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    ins = [make(B, L, H, P).bfloat16(), make(B, L, H).bfloat16(), -make(H).abs() * 4 - 1, make(B, L, G, 128).bfloat16(),
+           make(B, L, G, 128).bfloat16(), make(H), make(H) - 3]
+    dy = make(B, L, H, P).bfloat16()
+    wide = [t.double().requires_grad_() for t in ins]
+    want = _scan64(*wide)
+    want = (want,) + torch.autograd.grad(want, wide, dy.double())
+    group, first = H * P // 64 // G, None
+    for hpc in [h for h in (1, 2, 3, group) if group % h == 0]:
+        monkeypatch.setattr(cuda_ops, "_pick_hpc", lambda slices, chunks: hpc)
+        leaf = [t.detach().clone().requires_grad_() for t in ins]
+        y = ops.ssd_chunk_scan(*leaf, chunk_size=128)
+        got = (y.detach(),) + torch.autograd.grad(y, leaf, dy)
+        torch.cuda.synchronize()
+        cuda_ops.check_status()
+        # operands of the products and results are rounded to bf16 (2^-9 each at most, independent): three such roundings
+        for a, b in zip(got, want):
+            assert ((a.double() - b).norm() / b.norm()).item() < 3 * 2.0 ** -9
+        first = first or got
+        for i, (a, b) in enumerate(zip(got, first)):
+            if i in (4, 5):                                    # dB and dC: another order of fp32 sums, rounded to bf16
+                assert ((a - b).float().abs() <= 2.0 ** -7 * (b.float().abs() + 1e-3 * b.float().abs().mean())).all()
+            else:                                              # a head's own
+                assert torch.equal(a, b)
