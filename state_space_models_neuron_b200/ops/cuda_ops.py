@@ -671,11 +671,12 @@ def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, 
 
 
 def _walk_states(slices: int, nc: int) -> bool:
-    """Kernels that walk the chunks of a head slice, or one CTA per chunk and a recurrence kernel between.  A chunk of the
-    forward walk takes 2.7 us, of the backward states 1.4 us, for up to 148 slices; the separate kernels take 58 and 35 ns per
-    slice and chunk (us at 64 chunks, forward / backward states: 32 slices walk 207 / 97, separate 168 / 91; 48 slices
-    210 / 99, 226 / 122; 64 slices 215 / 99, 279 / 145; 160 slices, the start of a second wave, 414 / 186, 638 / 366).  Up to
-    four chunks the launches saved decide."""
+    """Kernels that walk the chunks of a head slice, or one CTA per chunk and a recurrence kernel between.  Walking takes 3.3 us
+    per chunk forwards and 1.5 us for the backward states, for up to 148 slices at once; the separate kernels take about 50
+    and 23 us and 57 and 34 ns per slice and chunk (us at 64 chunks, forward / backward states: 32 slices walk 207 / 97, separate
+    168 / 91; 48 slices 210 / 99, 226 / 122; 64 slices 215 / 99, 279 / 145; 160 slices, the start of a second wave, 414 / 186,
+    638 / 366).  They cross at 44 slices forwards and 35 for the backward states, which follow the forward's line: between the
+    two they lose up to a sixth.  Up to four chunks the launches saved decide."""
     return slices >= 44 or nc <= 4
 
 
