@@ -316,11 +316,6 @@ constexpr int BWD_STAGE = 2 * QTILE;                 // Q and dO
 constexpr int ATTN_BWD_THREADS = 22 * 32;
 constexpr int ATTN_BWD_SMEM = 2 * ATILE + 2 * BWD_STAGE + 4 * PTILE + AQ * AD * 4 + 2 * 2 * AQ * 4 + 256 + 1024;
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
 __global__ void __launch_bounds__(ATTN_BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -458,22 +453,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         mbar_arrive(dq_free);
       }
       fence_proxy_async_smem();
-      {
-        uint32_t all;
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p, q;\n\t"
-            "setp.ne.u32 p, %1, 0;\n\t"
-            "bar.red.and.pred q, 1, 128, p;\n\t"
-            "selp.u32 %0, 1, 0, q;\n\t"
-            "}\n"
-            : "=r"(all) : "r"(ok ? 1u : 0u) : "memory");
-        ok = all != 0;                                 // the four warps meet at barriers: they leave together
-      }
+      ok = barrier_and<1, 128>(ok);                    // the four warps meet at barriers: they leave together
       if (d == 0 && ok) {
-        asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-                     ::"l"(reinterpret_cast<uint64_t>(&tm_dq)), "r"(smem_u32(sdQ)), "r"(h * AD), "r"(b * p.L + q)
-                     : "memory");
+        tma_add_2d(&tm_dq, sdQ, h * AD, b * p.L + q);
         tma_store_commit();
       }
     }

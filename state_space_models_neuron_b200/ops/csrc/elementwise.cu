@@ -9,9 +9,7 @@
 namespace ssm {
 
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
-  f[0] = bf16_lo(u.x); f[1] = bf16_hi(u.x); f[2] = bf16_lo(u.y); f[3] = bf16_hi(u.y);
-  f[4] = bf16_lo(u.z); f[5] = bf16_hi(u.z); f[6] = bf16_lo(u.w); f[7] = bf16_hi(u.w);
+  unpack8(*reinterpret_cast<const uint4*>(p), f);
 }
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   uint4 u;
@@ -262,10 +260,6 @@ conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
 // The forward kernels also fetch the weights in front of the sum, since ordinary loads behind pdl_wait() are not moved there
 // by the compiler (130M, one sequence, 49 norms and gates per token: 467 -> 433 us with all weights fetched there).
 
-__device__ __forceinline__ void unpack8(const uint4 u, float (&f)[8]) {
-  f[0] = bf16_lo(u.x); f[1] = bf16_hi(u.x); f[2] = bf16_lo(u.y); f[3] = bf16_hi(u.y);
-  f[4] = bf16_lo(u.z); f[5] = bf16_hi(u.z); f[6] = bf16_lo(u.w); f[7] = bf16_hi(u.w);
-}
 __device__ __forceinline__ uint4 load_raw8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
 
 // Sums of two values over the block, to every thread, behind ONE barrier: `red` (64 float2) is used in halves by turns,

@@ -30,10 +30,6 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int kk, uint32_t
   return make_smem_desc_sw128(base + kk * 2048, block_bytes, 1024);
 }
 
-__device__ __forceinline__ void unpack8(const uint4 u, float (&f)[8]) {
-  f[0] = bf16_lo(u.x); f[1] = bf16_hi(u.x); f[2] = bf16_lo(u.y); f[3] = bf16_hi(u.y);
-  f[4] = bf16_lo(u.z); f[5] = bf16_hi(u.z); f[6] = bf16_lo(u.w); f[7] = bf16_hi(u.w);
-}
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   uint4 u;
   u.x = pack_bf16(f[0], f[1]); u.y = pack_bf16(f[2], f[3]); u.z = pack_bf16(f[4], f[5]); u.w = pack_bf16(f[6], f[7]);
@@ -558,11 +554,6 @@ constexpr int WS_STAGE = 2 * TILE128 + TILE64;                           // B | 
 constexpr int WS_USED = 2 * WS_STAGE + 2 * TILE64 + TILE128 + 2 * 2 * CT * 4 + 128;
 constexpr int WS_SMEM = 227 * 1024;                                      // all of it: what is left aligns the tiles
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
 __global__ void __launch_bounds__(WS_THREADS, 1)
 ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_constant__ CUtensorMap tm_in,
                      const __grid_constant__ CUtensorMap tm_y, const WalkScanParams p) {
@@ -1017,19 +1008,7 @@ ssd_chunk_scan_bwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __gr
       ok = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, p.status));
       tc_fence_after_sync();
     };
-    // barrier of the 512 threads; true where every one of them brings true
-    auto all_ok = [](bool mine) {
-      uint32_t all;
-      asm volatile(
-          "{\n\t"
-          ".reg .pred p, q;\n\t"
-          "setp.ne.u32 p, %1, 0;\n\t"
-          "bar.red.and.pred q, 1, 512, p;\n\t"
-          "selp.u32 %0, 1, 0, q;\n\t"
-          "}\n"
-          : "=r"(all) : "r"(mine ? 1u : 0u) : "memory");
-      return all != 0;
-    };
+    auto all_ok = [](bool mine) { return barrier_and<1, 512>(mine); };
     for (int it = 0; it < p.hpc; ++it) {
       const int hv = hv0 + it, h = hv / psplit;
       // dt_raw of this row: wanted in 4, on its way meanwhile
@@ -1246,9 +1225,7 @@ ssd_chunk_scan_bwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __gr
     ok = all_ok(ok);
     if (tid == 0 && ok) {
       for (int k = 0; k < 8; ++k)
-        asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-                     ::"l"(reinterpret_cast<uint64_t>(&tm_dbc)), "r"(smem_u32(smem + k * TILE64)),
-                     "r"((k >> 2) * GN + g * NS + (k & 3) * 32), "r"(row0) : "memory");
+        tma_add_2d(&tm_dbc, smem + k * TILE64, (k >> 2) * GN + g * NS + (k & 3) * 32, row0);
       tma_store_commit();
       tma_store_wait_all();
     }
