@@ -300,8 +300,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 //   warp 20      issues all products;  warp 21  loads
 // The scores of the next tile are issued before the three gradient products of this one, so the arithmetic of a tile and the
 // products of the tile before it overlap.  Bound by these two in turn.  One 128-thread group doing everything in turn, with a
-// reduction instruction per 16 bytes of dQ, took 3569 us for 8192 queries of 32 heads, this 2131 us (2863 with eight warps for P and dS, 2670 without
-// packed arithmetic and with masks on every tile).
+// reduction instruction per 16 bytes of dQ, took 3390 us with its fills and conversions for 8192 queries of 32 heads, this
+// 2343 (4096 x 32: 1046 -> 647; one box, back to back).  The kernel alone takes 2131 us (2863 with eight warps for P and dS, 2670
+// without packed arithmetic and with masks on every tile).
 struct AttnBwdParams {
   const float* lse; const float* delta;     // [B, Hq, L]
   __nv_bfloat16* dk; __nv_bfloat16* dv;     // [B*L, Hkv*128]
