@@ -170,6 +170,49 @@ __device__ __forceinline__ float gelu_f(float x) {
   return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
 }
 
+// One block of 64 columns of a row joins the row's cross-entropy statistics (max, sum exp(x - max)).  pk: the bf16-rounded
+// logits that the consumer of C will read, `valid` of them inside N; staged: the shared-memory block that already holds them;
+// label: column of the target inside the block, else outside [0, 64).
+// One warp per scheduler works here, so what counts are dependent chains: the block's maximum comes first, and the
+// exponentials then run in pairs with no rescaling or label test between them.  (With both per 8 columns the epilogue took
+// 15 us a tile, twice the main loop at K = 1024; us before -> now: 4608 x 50272 x 768 764 -> 375, 8192 x 50288 x 1024
+// 1334 -> 676, 8192 x 50288 x 2560 1637 -> 1380, 2688 x 50288 x 1536 509 -> 293.)
+__device__ __forceinline__ void ce_block(uint4 (&pk)[2][4], int valid, long long label, const __nv_bfloat16* staged, int row,
+                                         float& m, float& s, float* target) {
+  uint32_t x[32];
+  #pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint4 u = pk[i >> 2][i & 3];
+    x[4 * i] = u.x; x[4 * i + 1] = u.y; x[4 * i + 2] = u.z; x[4 * i + 3] = u.w;
+  }
+  if (valid < 64) {                                  // columns beyond N count as -inf
+    #pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if (2 * i >= valid) x[i] = 0xff80ff80u;
+      else if (2 * i + 1 >= valid) x[i] = (x[i] & 0xffffu) | 0xff800000u;
+    }
+  }
+  __nv_bfloat162 mx[4];
+  #pragma unroll
+  for (int i = 0; i < 4; ++i) mx[i] = *reinterpret_cast<const __nv_bfloat162*>(&x[i]);
+  #pragma unroll
+  for (int i = 4; i < 32; ++i) mx[i & 3] = __hmax2(mx[i & 3], *reinterpret_cast<const __nv_bfloat162*>(&x[i]));
+  const __nv_bfloat162 t = __hmax2(__hmax2(mx[0], mx[1]), __hmax2(mx[2], mx[3]));
+  const float now = fmaxf(m, fmaxf(__low2float(t), __high2float(t)));
+  const float ref = ce_ref(now);
+  const uint64_t ref2 = pack2(ref, ref);
+  uint64_t sum[4] = {0, 0, 0, 0};
+  #pragma unroll
+  for (int i = 0; i < 32; ++i) sum[i & 3] = add2(sum[i & 3], exp_diff2(bf16x2_pair(x[i]), ref2));
+  float a, b;
+  unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
+  s = s * __expf(m - ref) + (a + b);
+  m = now;
+  if (label >= 0 && label < 64 && label < valid)
+    *target = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(reinterpret_cast<const uint8_t*>(staged) +
+                                                                       sw128_offset(row, (uint32_t)label >> 3) + (label & 7) * 2));
+}
+
 struct Work { int tile, kb0, kb1, slice, nslices, tail; };
 
 __device__ __forceinline__ bool get_work(const GemmParams& p, int unit, int it, int kblocks, Work& w) {
@@ -749,6 +792,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               // plain output (every GEMM of the training step except the MLP up-projection): convert and stage only;
               // keeping the bias / GELU arithmetic out of this loop matters, the compiler otherwise evaluates it
               // for every element and selects
+              uint4 pk[2][4];
               #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 #pragma unroll
@@ -759,30 +803,11 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                   o.z = pack_bf16(__uint_as_float(v[h][c * 8 + 4]), __uint_as_float(v[h][c * 8 + 5]));
                   o.w = pack_bf16(__uint_as_float(v[h][c * 8 + 6]), __uint_as_float(v[h][c * 8 + 7]));
                   *reinterpret_cast<uint4*>(buf + sw128_offset(row, h * 4 + c)) = o;
-                  if (p.ce_labels != nullptr) {
-                    // statistics of the values the consumer of C will read: the bf16-rounded logits
-                    const uint32_t pk[4] = {o.x, o.y, o.z, o.w};
-                    float mx = ce_m;
-                    #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                      const int col = nb + h * 32 + c * 8 + e;
-                      const float x = (e & 1) ? bf16_hi(pk[e >> 1]) : bf16_lo(pk[e >> 1]);
-                      if (col < p.N) mx = fmaxf(mx, x);
-                    }
-                    if (mx > ce_m) { ce_s *= __expf(ce_m - mx); ce_m = mx; }
-                    const float ref = ce_ref(ce_m);
-                    #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                      const int col = nb + h * 32 + c * 8 + e;
-                      const float x = (e & 1) ? bf16_hi(pk[e >> 1]) : bf16_lo(pk[e >> 1]);
-                      if (col < p.N) {
-                        ce_s += __expf(x - ref);
-                        if ((long long)col == ce_lbl) p.ce_tgt[m0 + row] = x;
-                      }
-                    }
-                  }
+                  pk[h][c] = o;
                 }
               }
+              if (p.ce_labels != nullptr)
+                ce_block(pk, p.N - nb, ce_lbl - nb, reinterpret_cast<const __nv_bfloat16*>(buf), row, ce_m, ce_s, p.ce_tgt + m0 + row);
             } else {
               #pragma unroll
               for (int h = 0; h < 2; ++h) {

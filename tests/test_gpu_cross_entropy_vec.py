@@ -87,3 +87,23 @@ def test_statistics_of_rows_with_infinite_logits(M, V, K):
         want = torch.nn.functional.cross_entropy(ref, labels, reduction="none")
         assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5, equal_nan=True)
         assert torch.isfinite(loss[1]) == (first < V)
+
+
+@pytest.mark.parametrize("N", [1, 2, 63, 64, 65, 191, 256, 257, 1001])
+def test_statistics_at_the_edges_of_a_column_block(N):
+    """Statistics out of the GEMM where N ends inside, at and just behind a 64-column block, with the labels of the rows at
+    every column, and shards that begin at another id."""
+    from state_space_models_neuron_b200.ops import cuda_ops
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    M, K, start = 300, 64, 1000
+    a, b = (torch.randn(*s, device="cuda", generator=gen).bfloat16() for s in ((M, K), (N, K)))
+    labels = start - 1 + torch.arange(M, device="cuda") * (N + 1) // (M - 1)         # one before the shard .. one behind it
+    y, (m, s, t) = cuda_ops.gemm_ce(a, b, labels, start)
+    cuda_ops.check_status()
+    ref, at = y.double(), labels - start
+    inside = (at >= 0) & (at < N)
+    assert torch.equal(m.double(), ref.max(1).values)
+    assert torch.equal(t.double(), torch.where(inside, ref.gather(1, at.clamp(0, N - 1)[:, None])[:, 0], 0.0))
+    # exponentials within 2 ulp and an argument below 2^7 rounded to 2^-24 of itself; sums of at most 1001 positive terms in
+    # chains of at most 16 per block and 16 blocks
+    assert torch.allclose(s.double(), (ref - ref.max(1, keepdim=True).values).exp().sum(1), rtol=2 ** -17 + 40 * 2 ** -24)
