@@ -21,10 +21,10 @@ from .. import ops
 from ..parallel import mappings as mp
 from ..parallel import state as ps
 from ..parallel.cross_entropy import parallel_argmax, parallel_cross_entropy
-from ..parallel.layers import ColumnParallelLinear, ParallelEmbedding, normal_init
+from ..parallel.layers import ColumnParallelLinear, ParallelEmbedding, RowParallelLinear, normal_init
 from .cache import Mamba2Cache
 from .configuration_mamba2 import Mamba2Config
-from .mamba2_mixer import Mamba2Mixer
+from .mamba2_mixer import Mamba2Mixer, MambaRMSNormGated
 
 
 class Mamba2RMSNorm(nn.Module):
@@ -48,6 +48,13 @@ class Mamba2RMSNorm(nn.Module):
         return ops.add_rmsnorm(hidden_states, residual, self.weight, self.variance_epsilon, residual_dtype)
 
 
+def _is_untouched(module, cls) -> bool:
+    """True for a module of exactly this class, with no hook and no forward of its own: calling it is its class's forward."""
+    return (type(module) is cls and "forward" not in vars(module)
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                     or _has_any_global_hook()))
+
+
 class Mamba2Block(nn.Module):
     """Pre-norm residual block: h <- h + mixer(norm(h)).
 
@@ -66,6 +73,15 @@ class Mamba2Block(nn.Module):
                                   dtype=config.dtype or torch.float32, device=device)
         self.mixer = Mamba2Mixer(config, layer_idx=layer_idx, device=device)
 
+    def _is_plain(self) -> bool:
+        """True where the block is made of the plain modules on one rank, so that one native call can stand for theirs: any other
+        class, a hook, a method set on a module, or a bias behind out_proj keeps the calls one by one."""
+        m = self.mixer
+        return (type(m) is Mamba2Mixer and type(self.norm) is Mamba2RMSNorm and type(m.norm) is MambaRMSNormGated
+                and m.out_proj.bias is None and _is_untouched(m.in_proj, ColumnParallelLinear)
+                and _is_untouched(m.out_proj, RowParallelLinear) and "step" not in vars(m) and "forward_add" not in vars(self.norm)
+                and ps.get_tensor_model_parallel_size() == 1)
+
     def forward(self, hidden_states, residual=None, cache_params=None):
         rd = torch.float32 if self.residual_in_fp32 else None
         normed, residual = self.norm.forward_add(hidden_states, residual, rd)
@@ -73,6 +89,13 @@ class Mamba2Block(nn.Module):
 
     def step(self, hidden_states, residual, cache_params):
         rd = torch.float32 if self.residual_in_fp32 else None
+        if self._is_plain() and hidden_states.dim() == 3 and hidden_states.shape[1] == 1:
+            m, i = self.mixer, self.layer_idx
+            done = ops.decode_block(hidden_states, residual, rd, cache_params.conv_states[i], cache_params.ssm_states[i],
+                                    self.norm.weight, self.norm.variance_epsilon, m.in_proj.weight, m.in_proj.bias, m.conv1d.weight,
+                                    m.conv1d.bias, m.dt_bias, m.A_log, m.D, m.norm.weight, m.out_proj.weight, **m._core_kwargs())
+            if done is not None:
+                return done
         normed, residual = self.norm.forward_add(hidden_states, residual, rd)
         return self.mixer.step(normed, cache_params), residual
 
@@ -189,9 +212,7 @@ class Mamba2Model(Mamba2PreTrainedModel):
 def _delivers_statistics(head) -> bool:
     """True for the plain head, whose GEMM can take the cross-entropy statistics along.  Any other module, a bias or a
     gathered output has no such form; a hook, or a forward set on the module, gets the tensor that the head returns."""
-    return (type(head) is ColumnParallelLinear and head.bias is None and not head.gather_output and "forward" not in vars(head)
-            and not (head._forward_hooks or head._forward_pre_hooks or head._backward_hooks or head._backward_pre_hooks
-                     or _has_any_global_hook()))
+    return _is_untouched(head, ColumnParallelLinear) and head.bias is None and not head.gather_output
 
 
 def _shift_labels(labels):

@@ -321,8 +321,8 @@ gated_rmsnorm_fwd_kernel(const __nv_bfloat16* y, long long ys, const __nv_bfloat
       for (int e = 0; e < 8; ++e) { h[i][e] = a[e]; ss += a[e] * a[e]; }
     }
   }
-  if (ROLL && g == 0) {
-    for (int c = roll.c0 + threadIdx.x; c < roll.C; c += blockDim.x) {
+  if (ROLL) {                                          // the row's blocks (one per group) share its channels
+    for (int c = roll.c0 + g * blockDim.x + threadIdx.x; c < roll.C; c += gridDim.y * blockDim.x) {
       uint2* sp = reinterpret_cast<uint2*>(roll.window + (row * roll.C + c) * 4);
       const uint2 s = *sp;
       const uint32_t x = __bfloat16_as_ushort(roll.x[row * roll.xs + c]);

@@ -8,7 +8,7 @@
 //   M <= 128  gemm_cols_kernel: the weight rows are the 128-row side of a tcgen05 tile and X the 32-, 64- or 128-column
 //             side; a cluster of up to eight CTAs shares K and adds the partial tiles over distributed shared memory.
 // Sums run in a fixed order, so results are reproducible.
-// Measured (weights from HBM, us; tiled kernel of gemm.cu -> these): 1 x 3352 x 768 11.5 -> 3.2, 1 x 50288 x 768
+// Measured (weights from HBM, us; tiled kernel of gemm.cu -> these, single launches): 1 x 3352 x 768 11.5 -> 3.2, 1 x 50288 x 768
 // 25.6 -> 17.2, 5 x 1024 x 2048 18.0 -> 5.9, 64 x 10576 x 2560 27.4 -> 16.1 (8.3 at copy bandwidth), 64 x 2560 x 5120
 // 24.0 -> 12.1, 64 x 50288 x 2560 62.6 -> 48.2 (39.3), 128 x 768 x 1536 18.7 -> 8.0, 128 x 10576 x 2560 29.7 -> 19.8,
 // 128 x 4096 x 8192 32.4 -> 21.6.
@@ -28,7 +28,9 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // volatile: the loads of a step stay in front of its products (the compiler would otherwise sink each load to its use
-// and leave two of them in flight).  Ordinary loads, for X and the weights: see pdl_wait().
+// and leave two of them in flight).  The assembler does the same unless a __syncwarp() stands behind the loads: with it (us per
+// call behind another call, one row) 768 x 1536 4.1 -> 2.7, 2560 x 5120 12.2 -> 7.2, 4096 x 8192 19.7 -> 12.3, 18560 x 4096
+// 31.0 -> 24.8 (23.2 at copy bandwidth).  Ordinary loads, for X and the weights: see pdl_wait().
 __device__ __forceinline__ uint4 ld8_if(bool in, const __nv_bfloat16* p) {
   uint4 u;
   asm volatile(
@@ -40,6 +42,12 @@ __device__ __forceinline__ uint4 ld8_if(bool in, const __nv_bfloat16* p) {
       "}\n"
       : "=&r"(u.x), "=&r"(u.y), "=&r"(u.z), "=&r"(u.w) : "l"(p), "r"((int)in) : "memory");
   return u;
+}
+
+// Chunks that a warp fetches at once: its share of K in equal turns of at most four, so that no turn is nearly empty
+static int rows_unroll(int per_warp) {
+  const int turns = (per_warp + 3) / 4;
+  return (per_warp + turns - 1) / turns;
 }
 
 // A lane holds 8 consecutive k of row lane / 4 (16 bytes); as the order of k inside a product does not matter, elements
@@ -83,6 +91,7 @@ gemm_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, 
         for (int i = 0; i < NT; ++i) b[u][s][i] = ld8_if(in, xr[i] + k);
       }
     }
+    __syncwarp();                             // all loads go out in front of it
     #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
       #pragma unroll
@@ -112,6 +121,174 @@ gemm_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, 
     if (bias != nullptr) v += __bfloat162float(bias[n0 + r]);
     out[(long long)m * ldo + n0 + r] = __float2bfloat16(v);
   }
+}
+
+// ------------------------------------------------------------------------------------------------ norm and product, M <= 8
+// A norm in front of a product with at most eight rows: out[m, n] = sum_g rstd[m, g] sum_{k in g} bf16(h[m, k] wn[k]) W[n, k].
+// The factor rstd of a row (and group) is known only when the whole row has been read, but it can be applied to the sums, so
+// every warp forms the operand of its own k from the inputs of the norm while it waits for its weights, and neither a kernel
+// nor a barrier stands in front of the product.  One rounding to bf16 per operand, as with a norm kernel of its own.
+//   add    h = x + residual, the new residual is stored by the blocks in turn (chunk c by block c mod gridDim.x)
+//   gated  h = y silu(z); also rolls the conv windows of a decoding step (see WindowRoll in elementwise.cu)
+// Every block reads the M rows for itself (from L2) next to 32 K bytes of weights, so this pays for narrow products, where a
+// kernel's start and end cost more than its work (us per call behind another call, norm and product -> this: one row, gated
+// 768 x 1536 4.4 -> 3.3, 2048 x 4096 7.8 -> 7.2, add 4384 x 1024 4.1 -> 3.8), and not for wide ones (add 10576 x 2560 12.9 ->
+// 19.8); the caller has the rule.
+enum { NORM_ADD_BF16 = 0, NORM_ADD_FP32 = 1, NORM_GATED = 2 };
+
+struct NormLinearParams {
+  const __nv_bfloat16* a; long long lda;      // x, or y
+  const void* b; long long ldb;               // residual (bf16 or fp32) or null, or z
+  const __nv_bfloat16* wn;
+  void* res_out;                              // add: [M, K] contiguous
+  const __nv_bfloat16* w; long long ldw;
+  const __nv_bfloat16* bias;
+  __nv_bfloat16* out; long long ldo;
+  int M, N, K, groups;                        // groups: 1, 2, 4 or 8 equal parts of K, each a multiple of ROWS_CHUNK if more than one
+  float eps;
+  __nv_bfloat16* window; const __nv_bfloat16* xnew; long long xs; int c0, C;      // gated: windows [M][C][4], channels [c0, C)
+};
+
+__device__ __forceinline__ uint4 ld16_if(bool in, const void* p) { return ld8_if(in, reinterpret_cast<const __nv_bfloat16*>(p)); }
+
+template <int KIND, int UNROLL>
+__global__ void __launch_bounds__(ROWS_WARPS * 32)
+norm_linear_kernel(const NormLinearParams p) {
+  __shared__ float red[ROWS_WARPS][8][16 + 1];
+  __shared__ float sums[ROWS_WARPS][8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * 16;
+  // the warps of a group share its chunks
+  const int per_group = ROWS_WARPS / p.groups, width = p.K / p.groups;
+  const int k_first = (warp / per_group) * width + (warp % per_group) * ROWS_CHUNK, k_end = (warp / per_group + 1) * width;
+  const int k_step = per_group * ROWS_CHUNK;
+  const __nv_bfloat16* wl = p.w + (long long)(n0 + g < p.N ? n0 + g : 0) * p.ldw + t * 8;
+  const __nv_bfloat16* wh = p.w + (long long)(n0 + g + 8 < p.N ? n0 + g + 8 : 0) * p.ldw + t * 8;
+  const bool mine = g < p.M;                  // lanes of rows beyond M bring zeros
+  const int row = mine ? g : 0;
+  pdl_trigger();
+  {
+    // this warp's first weights on their way to L2 while the predecessor finishes: a 128-byte line per row and chunk
+    const int r = n0 + (lane & 15);
+    if (r < p.N) {
+      #pragma unroll
+      for (int u = 0; u < UNROLL; u += 2) {
+        const int k = k_first + (u + (lane >> 4)) * k_step;
+        if (k < k_end) prefetch_l2(p.w + (long long)r * p.ldw + k);
+      }
+    }
+  }
+  pdl_wait();
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.f;
+  for (int k0 = k_first; k0 < k_end; k0 += k_step * UNROLL) {
+    uint4 wa[UNROLL][2], wb[UNROLL][2], xa[UNROLL][2], xb[UNROLL][2], xc[UNROLL][2], nw[UNROLL][2];
+    #pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      #pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int k = k0 + u * k_step + s * 32, kk = k + t * 8;
+        const bool in = kk < k_end;           // a group's width is a multiple of 8
+        xa[u][s] = ld16_if(in && mine, p.a + row * p.lda + kk);
+        if (KIND == NORM_ADD_FP32) {
+          const float* r = reinterpret_cast<const float*>(p.b) + row * p.ldb + kk;
+          xb[u][s] = ld16_if(in && mine && p.b != nullptr, r);
+          xc[u][s] = ld16_if(in && mine && p.b != nullptr, r + 4);
+        } else {
+          xb[u][s] = ld16_if(in && mine && p.b != nullptr, reinterpret_cast<const __nv_bfloat16*>(p.b) + row * p.ldb + kk);
+        }
+        nw[u][s] = ld16_if(in && mine, p.wn + kk);
+        wa[u][s] = ld8_if(in, wl + k);
+        wb[u][s] = ld8_if(in, wh + k);
+      }
+    }
+    __syncwarp();                             // all loads go out in front of it
+    #pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      #pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        float h[8], n[8];
+        unpack8(xa[u][s], h);
+        unpack8(nw[u][s], n);
+        if (KIND == NORM_GATED) {
+          float z[8];
+          unpack8(xb[u][s], z);
+          #pragma unroll
+          for (int e = 0; e < 8; ++e) h[e] *= silu_f(z[e]);
+        } else {
+          float r[8];
+          if (KIND == NORM_ADD_FP32) {
+            const uint4 lo = xb[u][s], hi = xc[u][s];
+            r[0] = __uint_as_float(lo.x); r[1] = __uint_as_float(lo.y); r[2] = __uint_as_float(lo.z); r[3] = __uint_as_float(lo.w);
+            r[4] = __uint_as_float(hi.x); r[5] = __uint_as_float(hi.y); r[6] = __uint_as_float(hi.z); r[7] = __uint_as_float(hi.w);
+          } else {
+            unpack8(xb[u][s], r);
+          }
+          #pragma unroll
+          for (int e = 0; e < 8; ++e) h[e] += r[e];
+          const int kk = k0 + u * k_step + s * 32 + t * 8;
+          if (mine && kk < k_end && (kk / ROWS_CHUNK) % gridDim.x == blockIdx.x) {
+            if (KIND == NORM_ADD_FP32) {
+              float* o = reinterpret_cast<float*>(p.res_out) + (long long)row * p.K + kk;
+              *reinterpret_cast<float4*>(o) = make_float4(h[0], h[1], h[2], h[3]);
+              *reinterpret_cast<float4*>(o + 4) = make_float4(h[4], h[5], h[6], h[7]);
+            } else {
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.res_out) + (long long)row * p.K + kk) =
+                  make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
+            }
+          }
+        }
+        #pragma unroll
+        for (int e = 0; e < 8; ++e) ss += h[e] * h[e];
+        const uint4 q = wa[u][s], v = wb[u][s];
+        mma_16x8x16(acc, q.x, v.x, q.y, v.y, pack_bf16(h[0] * n[0], h[1] * n[1]), pack_bf16(h[2] * n[2], h[3] * n[3]));
+        mma_16x8x16(acc, q.z, v.z, q.w, v.w, pack_bf16(h[4] * n[4], h[5] * n[5]), pack_bf16(h[6] * n[6], h[7] * n[7]));
+      }
+    }
+  }
+  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+  if (t == 0) sums[warp][g] = ss;
+  red[warp][2 * t][g] = acc[0];
+  red[warp][2 * t + 1][g] = acc[1];
+  red[warp][2 * t][g + 8] = acc[2];
+  red[warp][2 * t + 1][g + 8] = acc[3];
+  if (KIND == NORM_GATED) {
+    const long long channels = p.C - p.c0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.M * channels; i += (long long)gridDim.x * blockDim.x) {
+      const int r = (int)(i / channels), c = p.c0 + (int)(i % channels);
+      uint2* sp = reinterpret_cast<uint2*>(p.window + ((long long)r * p.C + c) * 4);
+      const uint2 s = *sp;
+      const uint32_t x = __bfloat16_as_ushort(p.xnew[r * p.xs + c]);
+      *sp = make_uint2((s.x >> 16) | (s.y << 16), (s.y >> 16) | (x << 16));
+    }
+  }
+  __syncthreads();
+  const int m = threadIdx.x >> 4, r = threadIdx.x & 15;
+  if (m < p.M && n0 + r < p.N) {
+    float v = 0.f;
+    for (int i = 0; i < ROWS_WARPS; i += per_group) {
+      float part = red[i][m][r], square = sums[i][m];
+      for (int k = 1; k < per_group; ++k) { part += red[i + k][m][r]; square += sums[i + k][m]; }
+      v += part * rsqrtf(square / width + p.eps);
+    }
+    if (p.bias != nullptr) v += __bfloat162float(p.bias[n0 + r]);
+    p.out[(long long)m * p.ldo + n0 + r] = __float2bfloat16(v);
+  }
+}
+
+template <int KIND>
+static int launch_norm_linear(const NormLinearParams& p, bool fp32, int sms, cudaStream_t stream) {
+  // bases and strides of 16-byte vectors, groups that whole warps can share
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.b) | reinterpret_cast<uintptr_t>(p.wn) |
+                      reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.res_out);
+  if (p.M < 1 || p.M > 8 || p.N < 1 || p.K < 8 || p.K % 8 || (a & 15) || p.lda % 8 || p.ldw % 8 || p.ldb % (fp32 ? 4 : 8) ||
+      !(p.groups == 1 || ((p.groups == 2 || p.groups == 4 || p.groups == 8) && p.K % (p.groups * ROWS_CHUNK) == 0)))
+    return -SSM_ERR_BAD_ARG;
+  const unsigned grid = (unsigned)((p.N + 15) / 16);
+  const int unroll = rows_unroll(((p.K + ROWS_CHUNK - 1) / ROWS_CHUNK + ROWS_WARPS - 1) / ROWS_WARPS);
+  auto kern = unroll == 1 ? norm_linear_kernel<KIND, 1> : unroll == 2 || grid > (unsigned)sms ? norm_linear_kernel<KIND, 2>
+            : norm_linear_kernel<KIND, 3>;
+  return launch_dependent(kern, dim3(grid), dim3(ROWS_WARPS * 32), 0, stream, p);
 }
 
 // ------------------------------------------------------------------------------------------------ M <= 128
@@ -336,8 +513,9 @@ bool gemm_skinny(const void* X, const void* W, void* C, int M, int N, int K, lon
     const auto* x = reinterpret_cast<const __nv_bfloat16*>(X);
     const auto* w = reinterpret_cast<const __nv_bfloat16*>(W);
     const unsigned grid = (unsigned)((N + 15) / 16);
-    // chunks in flight per warp: four hide more latency, two waste less of a short K
-    auto kern = M > 8 ? gemm_rows_kernel<2, 2> : K > 2 * ROWS_WARPS * ROWS_CHUNK ? gemm_rows_kernel<1, 4> : gemm_rows_kernel<1, 2>;
+    const int unroll = rows_unroll(((K + ROWS_CHUNK - 1) / ROWS_CHUNK + ROWS_WARPS - 1) / ROWS_WARPS);
+    auto kern = M > 8 ? gemm_rows_kernel<2, 2> : unroll == 4 ? gemm_rows_kernel<1, 4> : unroll == 3 ? gemm_rows_kernel<1, 3>
+              : gemm_rows_kernel<1, 2>;
     *code = launch_dependent(kern, dim3(grid), dim3(ROWS_WARPS * 32), 0, stream, x, ldx, w, ldw, b, out, ldc, M, N, K);
     return true;
   }
@@ -350,3 +528,41 @@ bool gemm_skinny(const void* X, const void* W, void* C, int M, int N, int K, lon
 }
 
 }  // namespace ssm
+
+using namespace ssm;
+
+static int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  return sms;
+}
+
+// out[M, N] = rmsnorm(x + res) W^T (+ bias) and res_out = x + res, M <= 8.  x [M, K] bf16 (row stride ldx); res contiguous
+// [M, K] of the residual type or null; 1 where the shape is not this kernel's.
+extern "C" int ssm_add_norm_linear(const void* x, long long ldx, const void* res, void* res_out, int res_fp32, const void* wn,
+                                   float eps, const void* w, long long ldw, const void* bias, void* out, long long ldo, int M,
+                                   int N, int K, cudaStream_t st) {
+  NormLinearParams p = {};
+  p.a = reinterpret_cast<const __nv_bfloat16*>(x); p.lda = ldx; p.b = res; p.ldb = K;
+  p.wn = reinterpret_cast<const __nv_bfloat16*>(wn); p.res_out = res_out; p.w = reinterpret_cast<const __nv_bfloat16*>(w);
+  p.ldw = ldw; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.out = reinterpret_cast<__nv_bfloat16*>(out); p.ldo = ldo;
+  p.M = M; p.N = N; p.K = K; p.groups = 1; p.eps = eps;
+  return res_fp32 ? launch_norm_linear<NORM_ADD_FP32>(p, true, device_sms(), st) : launch_norm_linear<NORM_ADD_BF16>(p, false, device_sms(), st);
+}
+
+// out[M, N] = gated_rmsnorm(y, z) W^T (+ bias) behind ssm_decode_mixer_step, M <= 8; also rolls channels [c0, C) of the conv
+// windows [M][C][4] with the new token xnew (row stride xs).
+extern "C" int ssm_gated_norm_linear(const void* y, long long ldy, const void* z, long long ldz, const void* wn, int gs, float eps,
+                                     const void* w, long long ldw, const void* bias, void* out, long long ldo, int M, int N, int K,
+                                     void* window, const void* xnew, long long xs, int c0, int C, cudaStream_t st) {
+  if (gs < 1 || K % gs) return -SSM_ERR_BAD_ARG;
+  NormLinearParams p = {};
+  p.a = reinterpret_cast<const __nv_bfloat16*>(y); p.lda = ldy; p.b = z; p.ldb = ldz;
+  p.wn = reinterpret_cast<const __nv_bfloat16*>(wn); p.w = reinterpret_cast<const __nv_bfloat16*>(w);
+  p.ldw = ldw; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.out = reinterpret_cast<__nv_bfloat16*>(out); p.ldo = ldo;
+  p.M = M; p.N = N; p.K = K; p.groups = K / gs; p.eps = eps;
+  p.window = reinterpret_cast<__nv_bfloat16*>(window); p.xnew = reinterpret_cast<const __nv_bfloat16*>(xnew); p.xs = xs;
+  p.c0 = c0; p.C = C;
+  if (z == nullptr) return -SSM_ERR_BAD_ARG;
+  return launch_norm_linear<NORM_GATED>(p, false, device_sms(), st);
+}

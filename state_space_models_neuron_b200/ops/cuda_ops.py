@@ -7,6 +7,7 @@ reads it (this synchronises) and raises.
 from __future__ import annotations
 
 import ctypes
+import struct
 from typing import Optional
 
 import torch
@@ -993,6 +994,65 @@ def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_lo
          _p(-torch.exp(A_log.float()).contiguous()), _p(D.float().contiguous()), _p(ssm_state), _p(y), B, C, H, head_dim, d_state,
          n_groups, d_inner, _st())
     return _gated_fwd(y, zxBCdt[:, :d_inner], norm_w, eps, gs)
+
+
+_BLOCK = struct.Struct("=20Qq11i2f")
+
+
+def _norms_in_products(B: int, width: int, d_inner: int, gs: int):
+    """Which norms of a decoding block are computed inside the product behind them (norm_linear_kernel): (first, gated).  Up to
+    eight rows, and groups that whole warps of that kernel can share.  Every block of it reads all rows, so narrow products
+    gain and wide ones lose (one kernel / two, us, one row: in_proj from 768 columns 3.4 / 3.4, 1024 3.8 / 4.1, 1536 9.7 / 6.6;
+    out_proj from 1536 3.3 / 4.4, 3072 5.1 / 6.6, 4096 7.2 / 7.8, 5120 10.9 / 9.2; five rows the same within 0.5)."""
+    groups = d_inner // gs
+    return (B <= 8 and width <= 1024,
+            B <= 8 and d_inner <= 4096 and (groups == 1 or (groups in (2, 4, 8) and gs % 64 == 0)))
+
+
+def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w, conv_b, dt_bias, A_log,
+                 D, gate_w, out_w, d_inner, n_groups, d_state, head_dim, eps, norm_group_size):
+    """One token of a pre-norm block, `out_proj(mixer(norm(residual + hidden)))`, by one native call of three to five kernels.
+    Returns (branch output, new residual), or None where a tensor is not as the kernels read it; the
+    caller then takes the separate operations, which convert or refuse it."""
+    B, _, width = hidden.shape
+    C, H, bf16 = d_inner + 2 * n_groups * d_state, d_inner // head_dim, torch.bfloat16
+    W = d_inner + C + H
+    rd = residual_dtype or bf16
+    gs = d_inner if norm_group_size is None else norm_group_size
+    mask = _head_param_mask(A_log, D, dt_bias, H)
+    operands = [hidden, norm_w, in_w, conv_w, gate_w, out_w]
+    operands += [t for t in (in_b, conv_b) if t is not None]
+    if (mask is None or 2 * d_state + head_dim > 12288 or d_state % 4 or H % n_groups or width % 8 or d_inner % 8
+            or d_inner % gs or gs % 8 or max(width, gs) > 8192 or B > 65535
+            or any(t.dtype is not bf16 or not t.is_contiguous() for t in operands)
+            or not (rd is bf16 or rd is torch.float32)
+            or conv_state.dtype is not bf16 or ssm_state.dtype is not torch.float32
+            or conv_state.shape != (B, C, 4) or ssm_state.shape != (B, H, head_dim, d_state)
+            or not conv_state.is_contiguous() or not ssm_state.is_contiguous()
+            or in_w.shape != (W, width) or out_w.shape != (width, d_inner) or norm_w.numel() != width or gate_w.numel() != d_inner
+            or conv_w.numel() != 4 * C or (in_b is not None and in_b.numel() != W) or (conv_b is not None and conv_b.numel() != C)):
+        return None
+    if residual is not None and (residual.dtype is not rd or not residual.is_contiguous() or residual.shape != hidden.shape):
+        return None
+    dev = hidden.device
+    ld, ldd = _ceil8(W), max(width, d_inner)
+    scratch = torch.empty(B * (ld + d_inner + ldd), dtype=bf16, device=dev)
+    out, res_out = torch.empty_like(hidden), torch.empty(hidden.shape, dtype=rd, device=dev)
+    zx = scratch.data_ptr()
+    pointers = [hidden.data_ptr(), 0 if residual is None else residual.data_ptr(), res_out.data_ptr(), norm_w.data_ptr(), in_w.data_ptr(),
+                0 if in_b is None else in_b.data_ptr(), conv_w.data_ptr(), 0 if conv_b is None else conv_b.data_ptr(),
+                A_log.data_ptr(), D.data_ptr(), dt_bias.data_ptr(), gate_w.data_ptr(), out_w.data_ptr(), conv_state.data_ptr(),
+                ssm_state.data_ptr(), zx, zx + 2 * B * ld, zx + 2 * B * (ld + d_inner), out.data_ptr(), status_tensor(dev).data_ptr()]
+    aligned = 0
+    for i in (0, 1, 2, 3, 4, 11, 12, 14):
+        aligned |= pointers[i]
+    if aligned & 15 or (pointers[6] | pointers[13]) & 7:
+        return None
+    first, gated = _norms_in_products(B, width, d_inner, gs)
+    _run("ssm_decode_block", _BLOCK.pack(*pointers, ld, B, width, d_inner, H, head_dim, d_state, n_groups, gs,
+                                         int(rd is torch.float32), mask, int(first) | 2 * int(gated), norm_eps, eps), _st())
+    _launches[0] += 4 - first - gated
+    return out, res_out
 
 
 # ======================================================================================

@@ -171,6 +171,18 @@ def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_lo
     return oracle.gated_rmsnorm(y.to(zxBCdt.dtype), z, norm_w, eps, norm_group_size)
 
 
+def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w, conv_b, dt_bias,
+                 A_log, D, gate_w, out_w, *, d_inner: int, n_groups: int, d_state: int, head_dim: int, eps: float,
+                 norm_group_size: Optional[int]):
+    """One token of a whole pre-norm block (residual add and norm, in_proj, mixer step, out_proj) over cached states:
+    (branch output, new residual), or None where only the separate operations take these tensors."""
+    if not _native(hidden) or _cuda()._recording():
+        return None
+    return _cuda().decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w,
+                                conv_b, dt_bias, A_log, D, gate_w, out_w, d_inner, n_groups, d_state, head_dim, eps,
+                                norm_group_size)
+
+
 # ---- attention ----------------------------------------------------------------------------
 def attention(q, k, v, causal: bool = True):
     """GQA flash attention; q [B,L,Hq,Dh], k/v [B,L,Hkv,Dh]."""

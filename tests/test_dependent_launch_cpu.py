@@ -30,4 +30,4 @@ def test_no_read_only_loads_in_dependent_kernels():
                 assert not ("const" in p and "__restrict__" in p), (kernel, p)
             assert "ld.global.nc" not in source and "__ldg" not in body, kernel
     assert {"gemm_rows_kernel", "gemm_cols_kernel", "decode_mixer_kernel", "decode_ssm_step_kernel", "decode_conv_step_kernel",
-            "gated_rmsnorm_fwd_kernel", "add_rmsnorm_fwd_kernel"} <= set(seen)
+            "gated_rmsnorm_fwd_kernel", "add_rmsnorm_fwd_kernel", "norm_linear_kernel"} <= set(seen)

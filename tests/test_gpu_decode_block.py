@@ -1,0 +1,85 @@
+"""One token of a whole block by one native call, against the operations one by one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# rows of 64-column chunks and a remainder; both, one and no norm inside a product; parts of a head; groups of several warps
+@pytest.mark.parametrize("B,width,H,P,G,gs,fp32", [(1, 256, 8, 64, 1, 512, False), (8, 768, 24, 64, 8, 192, True),
+                                                   (5, 1000, 16, 128, 2, 1024, False), (2, 1032, 8, 64, 4, 128, True),
+                                                   (3, 2560, 80, 64, 1, 5120, False), (9, 256, 8, 64, 1, 512, True),
+                                                   (2, 256, 12, 64, 2, 96, False)])
+def test_block_equals_separate_operations(B, width, H, P, G, gs, fp32):
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    d, N = H * P, 128
+    C = d + 2 * G * N
+    gen = torch.Generator(device="cuda").manual_seed(B + width)
+    make = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=gen) * scale).bfloat16()
+    norm_w, gate_w = make(width), make(d)
+    in_w, in_b, out_w = make(d + C + H, width, scale=width ** -0.5), make(d + C + H), make(width, d, scale=d ** -0.5)
+    conv_w, conv_b, head = make(C, 1, 4), make(C), [make(H).float(), make(H).abs(), make(H)]
+    window, state = make(B, C, 4), torch.randn(B, H, P, N, device="cuda", generator=gen)
+    rd = torch.float32 if fp32 else None
+    kw = dict(d_inner=d, n_groups=G, d_state=N, head_dim=P, eps=1e-5, norm_group_size=gs)
+    w0, s0 = window.clone(), state.clone()
+    hidden, residual = make(B, 1, width), None
+    with torch.no_grad():
+        for _ in range(3):
+            window.copy_(w0), state.copy_(s0)                   # both sides from the same states
+            out, res = ops.decode_block(hidden, residual, rd, window, state, norm_w, 1e-5, in_w, in_b, conv_w, conv_b, *head, gate_w,
+                                        out_w, **kw)
+            normed, want_res = ops.add_rmsnorm(hidden, residual, norm_w, 1e-5, rd)
+            zx = ops.linear(normed, in_w, in_b)[:, 0]
+            y = ops.ssm_decode_step(zx, w0, s0, conv_w, conv_b, *head, gate_w, **kw)
+            want = ops.linear(y[:, None], out_w)
+            torch.cuda.synchronize()
+            cuda_ops.check_status()
+            assert torch.equal(res, want_res) and out.shape == hidden.shape
+            # in_proj's operands and results are rounded to bf16 once on both sides, of equal values in another order: what
+            # follows from them differs by a few steps of bf16, spread over sums of hundreds of terms
+            near = lambda a, b: ((a.double() - b.double()).norm() / b.double().norm()).item() < 2.0 ** -7
+            assert near(window, w0) and torch.equal(window[..., :3], w0[..., :3]) and near(state, s0) and near(out, want)
+            hidden, residual = want, want_res
+
+
+def test_block_refuses_what_it_cannot_read():
+    from state_space_models_neuron_b200 import ops
+    B, width, H, P, N = 1, 256, 8, 64, 128
+    d, C = H * P, H * P + 2 * N
+    make = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    good = dict(hidden=make(B, 1, width), residual=None, residual_dtype=None, conv_state=make(B, C, 4),
+                ssm_state=torch.zeros(B, H, P, N, device="cuda"), norm_w=make(width), norm_eps=1e-5, in_w=make(d + C + H, width), in_b=None,
+                conv_w=make(C, 1, 4), conv_b=None, dt_bias=make(H), A_log=make(H), D=make(H), gate_w=make(d), out_w=make(width, d))
+    kw = dict(d_inner=d, n_groups=1, d_state=N, head_dim=P, eps=1e-5, norm_group_size=None)
+    bad = dict(hidden=make(B, 1, width).float(), residual=make(B, 1, width).float(), conv_state=make(B, C, 8)[..., ::2],
+               ssm_state=torch.zeros(B, H, N, P, device="cuda").transpose(2, 3), norm_w=make(width + 1)[1:], in_w=make(width, d + C + H).t(),
+               in_b=make(3), out_w=make(width, d).float(), D=make(2 * H)[::2], gate_w=make(d + 8))
+    with torch.no_grad():
+        assert ops.decode_block(**good, **kw) is not None
+        for name, value in bad.items():
+            assert ops.decode_block(**{**good, name: value}, **kw) is None, name
+    assert ops.decode_block(**good, **kw) is None               # recorded: autograd's operations stay
+
+
+def test_hooks_and_replaced_modules_keep_their_calls():
+    from state_space_models_neuron_b200.models import Mamba2Cache, Mamba2Config, Mamba2ForCausalLM
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    cfg = Mamba2Config(num_heads=8, head_dim=64, vocab_size=512, hidden_size=256, state_size=128, num_hidden_layers=2, n_groups=1,
+                       initializer_range=0.02, dtype=torch.bfloat16)
+    model = Mamba2ForCausalLM(cfg, device="cuda").to(torch.bfloat16).eval()
+    token = torch.tensor([[3]], device="cuda")
+    plain = model.step(token, Mamba2Cache(cfg, 1, dtype=torch.bfloat16, device="cuda"))
+    seen = []
+    block = model.backbone.layers[1]
+    handle = block.mixer.out_proj.register_forward_hook(lambda *a: seen.append(a[2].shape))
+    hooked = model.step(token, Mamba2Cache(cfg, 1, dtype=torch.bfloat16, device="cuda"))
+    handle.remove()
+    assert len(seen) == 1
+    block.mixer.in_proj.forward = lambda x, f=block.mixer.in_proj.forward: seen.append(x.shape) or f(x)
+    model.step(token, Mamba2Cache(cfg, 1, dtype=torch.bfloat16, device="cuda"))
+    assert len(seen) == 2
+    assert ((hooked - plain).norm() / plain.norm()).item() < 2.0 ** -6
