@@ -228,10 +228,34 @@ ssd_state_pass_kernel(const float* __restrict__ local, const float* __restrict__
 // buffers) while this one's state is stored and updated.
 // Bound by latency per chunk (wait, scale V, products, update) at few heads, by HBM at many (V in, bf16 states out): the
 // fp32 states, written and read back, were two thirds of the bytes.
+// Few head slices leave most SMs idle while each walks all its chunks, so the chunks are cut into segments: a first launch
+// finds the state behind every segment but the last from a zero state (`finals`), and the launch that wants the states
+// (this kernel backwards, ssd_walk_scan_kernel forwards) starts a segment from those behind the earlier ones.
+// 32 slices x 64 chunks (us): forward 178 in one walk, 137 with a CTA per chunk, 79 in four segments; backward states 93, 78, 54.
 // =====================================================================================
+struct Segments {
+  int count, len;                        // of consecutive steps, `len` chunks each (the last one may be shorter)
+  float* fin;                            // [B, Hv, count][128 n][64 p] state behind a segment that began with zeros
+  float* decay;                          // [B, Hv, count] decay over a segment
+};
+// the state that enters segment `seg`: V consecutive channels of row `row` from `at` on, entered with `run`
+template <int V>
+__device__ __forceinline__ void segment_entry(const Segments& sg, long long slice, int seg, int row, int at, float (&run)[V]) {
+  for (int r = 0; r < seg; ++r) {
+    const float d = sg.decay[slice * sg.count + r];
+    const float4* f = reinterpret_cast<const float4*>(sg.fin + ((slice * sg.count + r) * NS + row) * PS + at);
+    #pragma unroll
+    for (int e = 0; e < V; e += 4) {
+      const float4 v = f[e / 4];
+      run[e] = d * run[e] + v.x; run[e + 1] = d * run[e + 1] + v.y; run[e + 2] = d * run[e + 2] + v.z; run[e + 3] = d * run[e + 3] + v.w;
+    }
+  }
+}
 struct StateWalkParams {
-  const float* l;                        // [B, H, L]
+  const float* dt; const float* l;       // [B, H, L]; dt forwards only
   int L, H, Hv, G, nc, w_col0;
+  int forward, finals;                   // forward: W = B, V = x, ascending; finals: no states, only what Segments wants
+  Segments seg;
   int* status;
 };
 constexpr int WALK_STAGES = 3;
@@ -247,11 +271,13 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   uint64_t* full = reinterpret_cast<uint64_t*>(sOut + 2 * TILE64);       // [stage] loads landed
   uint64_t* done = full + WALK_STAGES;                                   // [2] products of a TMEM buffer complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 2);
-  const int hv = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5;
+  const int hv = blockIdx.x, b = blockIdx.y, seg = blockIdx.z, tid = threadIdx.x, warp = tid >> 5;
+  const int first = seg * p.seg.len, n = p.nc - first < p.seg.len ? p.nc - first : p.seg.len;      // steps of this segment
   const int row = tid & 127, half = tid >> 7;
   const int h = hv / (p.Hv / p.H), g = h / (p.H / p.G);
   const float* lh = p.l + ((long long)b * p.H + h) * p.L;
-  auto chunk = [&](int k) { return p.nc - 1 - k; };                      // chunk of step k
+  const float* dth = p.dt + ((long long)b * p.H + h) * p.L;
+  auto chunk = [&](int k) { return p.forward ? first + k : p.nc - 1 - first - k; };      // chunk of step k
 
   if (tid == 0) {
     for (int s = 0; s < WALK_STAGES; ++s) mbar_init(&full[s], 1);
@@ -275,13 +301,15 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   };
   int loaded = 0;                                                        // steps whose loads have been issued (thread 0)
   if (tid == 0)
-    for (; loaded < WALK_STAGES && loaded < p.nc; ++loaded) load(loaded);
-  // scaling of a step: l_j of this thread's row and l_T, fetched a step ahead
-  float lj = 0.f, lT = 0.f;
+    for (; loaded < WALK_STAGES && loaded < n; ++loaded) load(loaded);
+  // scaling of a step: l_j and dt_j of this thread's row and l_T, fetched a step ahead
+  float lj = 0.f, lT = 0.f, dj = 1.f, lsum = 0.f;
   auto fetch = [&](int k) {
-    if (k >= p.nc) return;
+    if (k >= n) return;
     const long long o = (long long)chunk(k) * CT;
     lj = lh[o + row]; lT = lh[o + CT - 1];
+    if (p.forward) dj = dth[o + row];
+    lsum += lT;
   };
   // V rows of step k scaled in place, then its products issued into TMEM buffer k & 1
   bool ok = true;
@@ -289,7 +317,7 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     const int st = k % WALK_STAGES;
     uint8_t* sw = smem + st * WALK_STAGE_BYTES;
     uint8_t* sv = sw + TILE128;
-    const float s = __expf(lj);
+    const float s = p.forward ? __expf(lT - lj) * dj : __expf(lj);
     ok = mbar_wait(&full[st], (k / WALK_STAGES) & 1, p.status);
     if (ok) {
       #pragma unroll
@@ -319,22 +347,26 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   float run[32];
   #pragma unroll
   for (int e = 0; e < 32; ++e) run[e] = 0.f;
+  const long long slice = (long long)b * p.Hv + hv;
+  if (!p.finals) segment_entry<32>(p.seg, slice, seg, row, half * 32, run);
   fetch(0);
   float dec = __expf(lT);                                                // of the step whose products are in flight
   scale_and_issue(0);
   fetch(1);
-  for (int k = 0; k < p.nc && ok; ++k) {
+  for (int k = 0; k < n && ok; ++k) {
     const float dec_k = dec;
     // the state that enters step k's chunk
     uint8_t* so = sOut + (k & 1) * TILE64;
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float f[8];
+    if (!p.finals) {
       #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = run[q * 8 + e];
-      *reinterpret_cast<uint4*>(so + sw128_offset(row, half * 4 + q)) = pack8(f);
+      for (int q = 0; q < 4; ++q) {
+        float f[8];
+        #pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = run[q * 8 + e];
+        *reinterpret_cast<uint4*>(so + sw128_offset(row, half * 4 + q)) = pack8(f);
+      }
     }
-    if (k + 1 < p.nc) {
+    if (k + 1 < n) {
       dec = __expf(lT);
       scale_and_issue(k + 1);                                            // its barrier also covers the staging tile
       if (!ok) break;
@@ -343,14 +375,14 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       fence_proxy_async_smem();
       __syncthreads();
     }
-    if (tid == 0) {
+    if (tid == 0 && !p.finals) {
       tma_store_2d(&tm_in, so, 0, ((b * p.Hv + hv) * p.nc + chunk(k)) * NS);
       tma_store_commit();
     }
     ok = mbar_wait(&done[k & 1], (k >> 1) & 1, p.status);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after_sync();
-    if (tid == 0 && ok && loaded < p.nc) { load(loaded); ++loaded; }     // step k's stage is free again
+    if (tid == 0 && ok && loaded < n) { load(loaded); ++loaded; }        // step k's stage is free again
     if (ok) {
       uint32_t v[32];
       tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, (k & 1) * 64 + half * 32), v);
@@ -361,6 +393,12 @@ ssd_state_walk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     tc_fence_before_sync();
     if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // step k - 1's tile has been read
     ok = __syncthreads_and(ok);                                          // TMEM buffer and staging tile are free again
+  }
+  if (p.finals && ok) {
+    float4* f = reinterpret_cast<float4*>(p.seg.fin + ((slice * p.seg.count + seg) * NS + row) * PS + half * 32);
+    #pragma unroll
+    for (int e = 0; e < 32; e += 4) f[e / 4] = make_float4(run[e], run[e + 1], run[e + 2], run[e + 3]);
+    if (tid == 0) p.seg.decay[slice * p.seg.count + seg] = __expf(lsum);
   }
   if (tid == 0) {
     tma_store_wait_all();
@@ -547,6 +585,7 @@ struct WalkScanParams {
   const float* init; float* fin;         // fp32 [B, Hv, 128 n, 64 p] in, [B, Hv, 64 p, 128 n] out, or null
   int store_states;                      // write the bf16 state entering every chunk
   int L, H, Hv, G, nc, d_in;
+  Segments seg;                          // one CTA per (head slice, batch, segment)
   int* status;
 };
 constexpr int WS_THREADS = 18 * 32;
@@ -572,6 +611,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
     return;
   }
   const int hv = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int c0 = blockIdx.z * p.seg.len, n = p.nc - c0 < p.seg.len ? p.nc - c0 : p.seg.len;        // this segment's chunks
   const int h = hv / (p.Hv / p.H), g = h / (p.H / p.G);
 
   if (tid == 0) {
@@ -589,11 +629,11 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
 
   if (warp == 17) {
     if (lane == 0) {
-      const long long lo = ((long long)b * p.H + h) * p.L;
+      const long long lo = ((long long)b * p.H + h) * p.L + (long long)c0 * CT;
       auto load = [&](int k) {
         uint8_t* sb = smem + (k & 1) * WS_STAGE;
         uint64_t* bar = &full[k & 1];
-        const int r = b * p.L + k * CT, cB = p.d_in + g * NS, cC = p.d_in + p.G * NS + g * NS;
+        const int r = b * p.L + (c0 + k) * CT, cB = p.d_in + g * NS, cC = p.d_in + p.G * NS + g * NS;
         mbar_expect_tx(bar, WS_STAGE + 2 * CT * 4);
         tma_load_2d(sb, &tm_xbc, cB, r, bar);
         tma_load_2d(sb + TILE128 / 2, &tm_xbc, cB + 64, r, bar);
@@ -604,13 +644,13 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
         bulk_load(sLD + (k & 1) * 2 * CT + CT, p.dt + lo + (long long)k * CT, CT * 4, bar);
       };
       int loaded = 0;
-      for (; loaded < 2 && loaded < p.nc; ++loaded) load(loaded);
+      for (; loaded < 2 && loaded < n; ++loaded) load(loaded);
       bool ok = true;
-      for (int k = -1; k < p.nc && ok; ++k) {
-        if (p.store_states && k + 1 < p.nc) {          // the state entering chunk k + 1 is in shared memory
+      for (int k = -1; k < n && ok; ++k) {
+        if (p.store_states && k + 1 < n) {          // the state entering chunk k + 1 is in shared memory
           ok = mbar_wait(xs_ready, (k + 1) & 1, p.status);
           if (!ok) break;
-          tma_store_2d(&tm_in, sS, 0, ((b * p.Hv + hv) * p.nc + k + 1) * NS);
+          tma_store_2d(&tm_in, sS, 0, ((b * p.Hv + hv) * p.nc + c0 + k + 1) * NS);
           tma_store_commit();
           tma_store_wait_read();
           mbar_arrive(s_free);
@@ -618,9 +658,9 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
         if (k >= 0) {                                  // y of chunk k stands in its x tile
           ok = mbar_wait(&y_ready[k & 1], (k >> 1) & 1, p.status);
           if (!ok) break;
-          tma_store_2d(&tm_y, smem + (k & 1) * WS_STAGE + 2 * TILE128, hv * PS, b * p.L + k * CT);
+          tma_store_2d(&tm_y, smem + (k & 1) * WS_STAGE + 2 * TILE128, hv * PS, b * p.L + (c0 + k) * CT);
           tma_store_commit();
-          if (loaded < p.nc) { tma_store_wait_read(); load(loaded); ++loaded; }
+          if (loaded < n) { tma_store_wait_read(); load(loaded); ++loaded; }
         }
       }
       tma_store_wait_all();
@@ -659,7 +699,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
         umma_commit(st_done);
       };
       if (ok) issue_state(0);
-      for (int k = 0; k < p.nc && ok; ++k) {
+      for (int k = 0; k < n && ok; ++k) {
         ok = mbar_wait(m_ready, k & 1, p.status);
         if (!ok) break;
         tc_fence_after_sync();
@@ -669,7 +709,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
         for (int kk = 0; kk < 8; ++kk)                 // Y_diag[i][p] = sum_j M[i][j] x[j][p]
           umma_bf16(tmem + 384, dM + kstep(kk), dX + (uint64_t)(kk * 128), id_off, kk != 0);
         umma_commit(y_done);
-        if (k + 1 < p.nc) {
+        if (k + 1 < n) {
           ok = mbar_wait(&full[(k + 1) & 1], ((k + 1) >> 1) & 1, p.status);
           if (!ok) break;
           tc_fence_after_sync();
@@ -691,6 +731,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
         v = *reinterpret_cast<const float4*>(p.init + ((long long)b * p.Hv + hv) * (NS * PS) + row * PS + wq * 16 + e);
       run[e] = v.x; run[e + 1] = v.y; run[e + 2] = v.z; run[e + 3] = v.w;
     }
+    segment_entry<16>(p.seg, (long long)b * p.Hv + hv, blockIdx.z, row, wq * 16, run);
     bool ok = true;
     // what the other warps do with these writes starts when all sixteen warps have arrived
     auto arrive = [&](uint64_t* bar) {
@@ -727,7 +768,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
       arrive(xs_ready);
     };
     prepare(0);
-    for (int k = 0; k < p.nc && ok; ++k) {
+    for (int k = 0; k < n && ok; ++k) {
       const float lik = li, dec = __expf(lT);
       const float* sl = sLD + (k & 1) * 2 * CT + wq * 32;
       // ---- c
@@ -764,7 +805,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
       #pragma unroll
       for (int e = 0; e < 16; ++e) run[e] = dec * run[e] + __uint_as_float(v[e]);
       // ---- a of the next chunk
-      if (k + 1 < p.nc) { prepare(k + 1); if (!ok) break; }
+      if (k + 1 < n) { prepare(k + 1); if (!ok) break; }
       // ---- f
       wait(y_done, k);
       if (!ok) break;
@@ -784,7 +825,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
       }
       arrive(&y_ready[k & 1]);                         // two barriers: the store of a chunk may lag one chunk behind
     }
-    if (ok && p.fin != nullptr) {                      // channel rows, as a decoding cache holds them
+    if (ok && p.fin != nullptr && c0 + n == p.nc) {                      // channel rows, as a decoding cache holds them
       float* fin = p.fin + ((long long)b * p.Hv + hv) * (NS * PS) + (wq * 16) * NS + row;
       #pragma unroll
       for (int e = 0; e < 16; ++e) fin[e * NS] = run[e];
@@ -1287,12 +1328,25 @@ extern "C" int ssm_ssd_state_pass(const void* local, const void* l, const void* 
   return (int)cudaGetLastError();
 }
 
-// mode 1 of ssm_ssd_chunk_state (w_src: C) and ssm_ssd_state_pass in one; v: bf16 [B*L, Hv*64] (row stride v_stride).  in16 bf16
-// [B,Hv,nc,128,64] is written.
-extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_cols, int w_col0, const void* v,
-                                  long long v_stride, const void* l, void* in16, int B, int L, int H, int Hv, int G,
-                                  int* status, cudaStream_t st) {
-  if (L % CT || Hv % H || H % G || w_stride % 8 || v_stride % 8 || B < 1 || B > 65535) return -SSM_ERR_BAD_ARG;
+// `count` segments cover the nc chunks; the buffers are wanted for more than one
+static bool segments_ok(int nc, int count, const void* fin, const void* decay, Segments* sg) {
+  if (count < 1 || count > nc || count > 64 || (count > 1 && (fin == nullptr || decay == nullptr || (reinterpret_cast<uintptr_t>(fin) & 15))))
+    return false;
+  sg->count = count; sg->len = (nc + count - 1) / count;
+  sg->fin = reinterpret_cast<float*>(const_cast<void*>(fin)); sg->decay = reinterpret_cast<float*>(const_cast<void*>(decay));
+  return (count - 1) * sg->len < nc;               // none is empty
+}
+
+// Backwards (forward = 0): mode 1 of ssm_ssd_chunk_state (w_src: C) and ssm_ssd_state_pass in one; v: bf16 [B*L, Hv*64] (row
+// stride v_stride); in16 bf16 [B,Hv,nc,128,64] is written.  Without in16: the states behind the first `count` - 1 segments
+// from zero states, seg_fin fp32 [B,Hv,count,128,64] and seg_decay fp32 [B,Hv,count], either way (forward: w_src B, v x).
+extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_cols, int w_col0, const void* v, long long v_stride,
+                                  const void* dt, const void* l, void* in16, int B, int L, int H, int Hv, int G, int forward,
+                                  int count, void* seg_fin, void* seg_decay, int* status, cudaStream_t st) {
+  Segments sg;
+  if (L % CT || Hv % H || H % G || w_stride % 8 || v_stride % 8 || B < 1 || B > 65535 || (forward && (in16 != nullptr || dt == nullptr)) ||
+      !segments_ok(L / CT, count, seg_fin, seg_decay, &sg) || (in16 == nullptr && count < 2))
+    return -SSM_ERR_BAD_ARG;
   static bool cfg = false;
   if (!cfg) { int e = smem_opt_in((const void*)ssd_state_walk_kernel, WALK_SMEM); if (e) return e; cfg = true; }
   const int nc = L / CT;
@@ -1301,21 +1355,27 @@ extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_c
   if (r) return -100 - r;
   r = make_tmap_2d_bf16(&tv, v, (uint64_t)Hv * PS, (uint64_t)B * L, (uint64_t)v_stride * 2, 64, 128);
   if (r) return -200 - r;
-  r = make_tmap_2d_bf16(&ti, in16, 64, (uint64_t)B * Hv * nc * NS, 128, 64, 128);
+  ti = tv;
+  if (in16 != nullptr) r = make_tmap_2d_bf16(&ti, in16, 64, (uint64_t)B * Hv * nc * NS, 128, 64, 128);
   if (r) return -300 - r;
   StateWalkParams p;
-  p.l = reinterpret_cast<const float*>(l);
+  p.dt = reinterpret_cast<const float*>(dt); p.l = reinterpret_cast<const float*>(l);
   p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.w_col0 = w_col0; p.status = status;
-  ssd_state_walk_kernel<<<dim3(Hv, B), 256, WALK_SMEM, st>>>(tw, tv, ti, p);
+  p.forward = forward; p.finals = in16 == nullptr; p.seg = sg;
+  ssd_state_walk_kernel<<<dim3(Hv, B, p.finals ? count - 1 : count), 256, WALK_SMEM, st>>>(tw, tv, ti, p);
   return (int)cudaGetLastError();
 }
 
 // The whole forward scan.  xbc as in ssm_ssd_chunk_scan_fwd; s_in (bf16 [B,Hv,nc,128,64], written) or null; init fp32
-// [B,Hv,128 n,64 p] and fin fp32 [B,Hv,64 p,128 n] are optional; y as in ssm_ssd_chunk_scan_fwd.
+// [B,Hv,128 n,64 p] and fin fp32 [B,Hv,64 p,128 n] are optional; y as in ssm_ssd_chunk_scan_fwd; more than one segment wants
+// what ssm_ssd_state_walk left in seg_fin and seg_decay.
 extern "C" int ssm_ssd_walk_scan(const void* xbc, long long xbc_stride, int xbc_cols, void* s_in, void* y, long long y_stride,
                                  const void* dt, const void* l, const void* D, const void* init, void* fin, int B, int L,
-                                 int H, int Hv, int G, int d_in, int* status, cudaStream_t st) {
+                                 int H, int Hv, int G, int d_in, int count, const void* seg_fin, const void* seg_decay, int* status,
+                                 cudaStream_t st) {
+  Segments sg;
   if (L % CT || Hv % H || H % G || xbc_stride % 8 || y_stride % 8 || B < 1 || B > 65535 ||
+      !segments_ok(L / CT, count, seg_fin, seg_decay, &sg) ||
       ((reinterpret_cast<uintptr_t>(dt) | reinterpret_cast<uintptr_t>(l)) & 15))
     return -SSM_ERR_BAD_ARG;
   static bool cfg = false;
@@ -1334,8 +1394,8 @@ extern "C" int ssm_ssd_walk_scan(const void* xbc, long long xbc_stride, int xbc_
   p.D = reinterpret_cast<const float*>(D);
   p.init = reinterpret_cast<const float*>(init); p.fin = reinterpret_cast<float*>(fin);
   p.store_states = s_in != nullptr;
-  p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.d_in = d_in; p.status = status;
-  ssd_walk_scan_kernel<<<dim3(Hv, B), WS_THREADS, WS_SMEM, st>>>(tx, ts, ty, p);
+  p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.d_in = d_in; p.status = status; p.seg = sg;
+  ssd_walk_scan_kernel<<<dim3(Hv, B, count), WS_THREADS, WS_SMEM, st>>>(tx, ts, ty, p);
   return (int)cudaGetLastError();
 }
 

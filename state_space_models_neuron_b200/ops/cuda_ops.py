@@ -7,6 +7,7 @@ reads it (this synchronises) and raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import struct
 from typing import Optional
 
@@ -658,8 +659,10 @@ def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, 
     dev, nc, st = conv_out.device, L // _CT, status_tensor(conv_out.device)
     states = torch.empty(B, Hv, nc, 128, 64, dtype=torch.bfloat16, device=dev)
     if mode == 1 and _walk_states(B * Hv, nc):         # forwards, ssm_ssd_walk_scan walks and scans at once
-        _run("ssm_ssd_state_walk", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(l), _p(states), B, L, H, Hv, G,
-             _p(st), _st())
+        count = _segments(B * Hv, nc, _PER_CHUNK[1])
+        ends = _segment_ends(conv_out, C, w_col0, v, v_stride, None, l, B, L, H, Hv, G, 0, count)
+        _run("ssm_ssd_state_walk", _p(conv_out), _ll(C), C, w_col0, _p(v), _ll(v_stride), _p(None), _p(l), _p(states), B, L, H, Hv, G,
+             0, count, _p(ends[0]), _p(ends[1]), _p(st), _st())
         return states, None
     final = torch.empty(B, Hv, 128, 64, dtype=torch.float32, device=dev) if want_final else None
     local = torch.empty(B, Hv, nc, 128, 64, dtype=torch.float32, device=dev)
@@ -671,14 +674,46 @@ def _chunk_states(conv_out, C, w_col0, v, v_stride, dt, l, init, want_final, B, 
     return states, final
 
 
+def _walk_cost(slices: int, nc: int, count: int, per_chunk: float, sms: int = 148) -> float:
+    """us of a walk of `count` segments: 5 us and the chunks of a segment for as many CTAs as there are SMs at once; with more
+    than one segment also the launch that finds the states behind all but the last (1.35 us per chunk) and 0.7 us for each of
+    these that a segment starts from."""
+    length = -(-nc // count)
+    cost = -(-slices * count // sms) * (5.0 + length * per_chunk)
+    return cost if count == 1 else cost + -(-slices * (count - 1) // sms) * (5.0 + length * 1.35) + 0.7 * (count - 1)
+
+
+_PER_CHUNK = (2.9, 1.35)               # us of a chunk of the forward walk, of the walk of the backward states
+
+
+@functools.lru_cache(maxsize=4096)
+def _segments(slices: int, nc: int, per_chunk: float) -> int:
+    """Segments that the chunks of a walk are cut into (none of them empty).  Measured (us, with 4 us of other kernels forwards;
+    slices x chunks: one / the count taken here): forward 16 x 64 165 / 51, 32 x 64 182 / 83, 64 x 16 47 / 44, 160 x 64 392 / 376,
+    1 x 512 1189 / 101; backward states 16 x 64 90 / 36, 32 x 64 93 / 54."""
+    return min((c for c in range(1, min(32, nc) + 1) if (c - 1) * -(-nc // c) < nc),
+               key=lambda c: _walk_cost(slices, nc, c, per_chunk))
+
+
+def _segment_ends(w, w_cols, w_col0, v, v_stride, dt, l, B, L, H, Hv, G, forward, count):
+    """(states behind the segments from zero states, decays over them), or (None, None) for one segment."""
+    if count == 1:
+        return None, None
+    fin = torch.empty(B, Hv, count, 128, 64, dtype=torch.float32, device=w.device)
+    decay = torch.empty(B, Hv, count, dtype=torch.float32, device=w.device)
+    _run("ssm_ssd_state_walk", _p(w), _ll(w_cols), w_cols, w_col0, _p(v), _ll(v_stride), _p(dt), _p(l), _p(None), B, L, H, Hv, G,
+         forward, count, _p(fin), _p(decay), _p(status_tensor(w.device)), _st())
+    return fin, decay
+
+
+@functools.lru_cache(maxsize=4096)
 def _walk_states(slices: int, nc: int) -> bool:
-    """Kernels that walk the chunks of a head slice, or one CTA per chunk and a recurrence kernel between.  Walking takes 3.3 us
-    per chunk forwards and 1.5 us for the backward states, for up to 148 slices at once; the separate kernels take about 50
-    and 23 us and 57 and 34 ns per slice and chunk (us at 64 chunks, forward / backward states: 32 slices walk 207 / 97, separate
-    168 / 91; 48 slices 210 / 99, 226 / 122; 64 slices 215 / 99, 279 / 145; 160 slices, the start of a second wave, 414 / 186,
-    638 / 366).  They cross at 44 slices forwards and 35 for the backward states, which follow the forward's line: between the
-    two they lose up to a sixth.  Up to four chunks the launches saved decide."""
-    return slices >= 44 or nc <= 4
+    """Kernels that walk the chunks of a head slice in segments, or one CTA per chunk and a recurrence kernel between, which take
+    about 6 us, 55 ns per slice and chunk and 0.2 us per chunk forwards.  The separate kernels win for few chunks in all (us,
+    separate / walk: 16 x 16 24 / 26, 2 x 64 30 / 42) and lose elsewhere (32 x 64 141 / 83, 48 x 64 198 / 106, 24 x 8 23 / 22, 1 x 512
+    134 / 101).  The backward states follow the forward's line (16 x 16 14 / 20, 32 x 64 78 / 54).  Up to four chunks the launches
+    saved decide."""
+    return nc <= 4 or _walk_cost(slices, nc, _segments(slices, nc, _PER_CHUNK[0]), _PER_CHUNK[0]) < 6.0 + 0.055 * slices * nc + 0.2 * nc
 
 
 def _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a):
@@ -717,8 +752,10 @@ def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner,
         final = None
         if want_final:
             final = torch.empty(B, H, Hv // H * 64, 128, dtype=torch.float32, device=dev) if final_out is None else final_out
+        count = _segments(B * Hv, nc, _PER_CHUNK[0])
+        ends = _segment_ends(conv_out, C, d_inner, conv_out, C, dt, l, B, L, H, Hv, G, 1, count)
         _run("ssm_ssd_walk_scan", _p(conv_out), _ll(C), C, _p(s_in), _p(y), _ll(d_inner), _p(dt), _p(l), _p(D),
-             _p(init_state), _p(final), B, L, H, Hv, G, d_inner, _p(st), _st())
+             _p(init_state), _p(final), B, L, H, Hv, G, d_inner, count, _p(ends[0]), _p(ends[1]), _p(st), _st())
         return y, dt, l, s_in, final, params
     s_in, final = _chunk_states(conv_out, C, d_inner, conv_out, C, dt, l, init_state, want_final, B, L, H, Hv, G, 0)
     if want_final:

@@ -54,6 +54,34 @@ def test_walk_scan_equals_separate_kernels(monkeypatch, nc, H, P, G):
     assert bare[3] is None and torch.equal(bare[0], y1) and torch.equal(bare[4], f1)
 
 
+@pytest.mark.parametrize("nc,count", [(2, 2), (5, 2), (7, 3), (7, 7), (11, 4)])       # equal segments, a short last one, one chunk each
+@pytest.mark.parametrize("H,P,G", [(4, 64, 1), (6, 128, 2)])
+def test_segments_equal_one_walk(monkeypatch, nc, count, H, P, G):
+    from state_space_models_neuron_b200.ops import cuda_ops
+    B, L, d, Hv = 2, nc * 128, H * P, H * P // 64
+    gen = torch.Generator(device="cuda").manual_seed(nc * 10 + H)
+    xbc = torch.randn(B * L, d + 2 * G * 128, device="cuda", generator=gen).bfloat16()
+    dy = torch.randn(B * L, d, device="cuda", generator=gen).bfloat16()
+    raw = torch.randn(B * L, 8, device="cuda", generator=gen).bfloat16() - 4           # decays that reach over several chunks
+    A, D, bias = -torch.rand(H, device="cuda", generator=gen) * 0.5, torch.rand(H, device="cuda"), torch.zeros(H, device="cuda")
+    init = torch.randn(B, Hv, 128, 64, device="cuda", generator=gen)
+    monkeypatch.setattr(cuda_ops, "_walk_states", lambda slices, n: True)
+    out = []
+    for segments in (1, count):
+        monkeypatch.setattr(cuda_ops, "_segments", lambda *a: segments)
+        y, dt, l, s, f, _ = cuda_ops._ssd_forward(xbc, raw, 8, A, D, bias, B, L, d, G, H, Hv, init, True)
+        back = cuda_ops._chunk_states(xbc, d + 2 * G * 128, d + G * 128, dy, d, dt, l, None, False, B, L, H, Hv, G, 1)[0]
+        out.append((s, f, y, back))
+    torch.cuda.synchronize()
+    cuda_ops.check_status()
+    (s0, f0, y0, b0), (s1, f1, y1, b1) = out
+    # the recurrence in fp32, associated otherwise: at most one bf16 step of a state, of values that may have cancelled
+    for a, b in ((s0, s1), (b0, b1)):
+        assert ((a.float() - b.float()).abs() <= 2.0 ** -7 * a.float().abs() + 1e-5 * a.float().abs().max()).all()
+    assert torch.allclose(f0, f1, rtol=1e-5, atol=1e-5 * f0.abs().max().item())
+    assert ((y0.float() - y1.float()).abs() <= 2.0 ** -7 * (y0.float().abs() + y0.float().abs().mean())).all()
+
+
 @pytest.mark.parametrize("B,H,P,G,fp32", [(1, 8, 64, 1, False), (3, 24, 64, 8, True), (5, 16, 128, 2, False)])
 def test_decode_step_equals_separate_kernels(monkeypatch, B, H, P, G, fp32):
     """Conv, state update and window roll in the fused decoding kernels against one kernel each."""
