@@ -7,11 +7,20 @@ first), `ssm_states[layer]` is `[B, H, P, N]`; sizes are per tensor-parallel ran
 """
 from __future__ import annotations
 
+import math
 from typing import Optional
 
 import torch
 
 from ..parallel import state as ps
+
+
+def _zeros(count: int, shape, dtype, device):
+    """`count` zero tensors of one shape with one allocation and one fill where their sizes are whole 16-byte vectors (48 fills
+    took 250 us of the host in front of a prompt through 24 layers).  Each has a version counter of its own."""
+    if math.prod(shape) * dtype.itemsize % 16 or count < 2:
+        return [torch.zeros(shape, device=device, dtype=dtype) for _ in range(count)]
+    return [t.data for t in torch.zeros((count, *shape), device=device, dtype=dtype).unbind(0)]
 
 
 class Mamba2Cache:
@@ -25,10 +34,10 @@ class Mamba2Cache:
         conv_dim = (config.intermediate_size + 2 * config.n_groups * config.state_size) // tp
         heads = config.num_heads // tp
         layers = range(config.num_hidden_layers) if layer_indices is None else layer_indices
-        self.conv_states = {i: torch.zeros(batch_size, conv_dim, config.conv_kernel, device=device, dtype=dtype)
-                            for i in layers}
-        self.ssm_states = {i: torch.zeros(batch_size, heads, config.head_dim, config.state_size,
-                                          device=device, dtype=ssm_dtype) for i in layers}
+        layers = list(layers)
+        self.conv_states = dict(zip(layers, _zeros(len(layers), (batch_size, conv_dim, config.conv_kernel), dtype, device)))
+        self.ssm_states = dict(zip(layers, _zeros(len(layers), (batch_size, heads, config.head_dim, config.state_size), ssm_dtype,
+                                                  device)))
 
     def update_conv_state(self, layer_idx: int, new_conv_state: torch.Tensor) -> torch.Tensor:
         self.conv_states[layer_idx].copy_(new_conv_state.to(self.conv_states[layer_idx].dtype))

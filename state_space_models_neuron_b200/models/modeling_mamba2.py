@@ -48,11 +48,8 @@ class Mamba2RMSNorm(nn.Module):
         return ops.add_rmsnorm(hidden_states, residual, self.weight, self.variance_epsilon, residual_dtype)
 
 
-def _is_untouched(module, cls) -> bool:
-    """True for a module of exactly this class, with no hook and no forward of its own: calling it is its class's forward."""
-    return (type(module) is cls and "forward" not in vars(module)
-            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
-                     or _has_any_global_hook()))
+def _hooked(module) -> bool:
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
 
 
 class Mamba2Block(nn.Module):
@@ -73,27 +70,42 @@ class Mamba2Block(nn.Module):
                                   dtype=config.dtype or torch.float32, device=device)
         self.mixer = Mamba2Mixer(config, layer_idx=layer_idx, device=device)
 
-    def _is_plain(self) -> bool:
-        """True where the block is made of the plain modules on one rank, so that one native call can stand for theirs: any other
-        class, a hook, a method set on a module, or a bias behind out_proj keeps the calls one by one."""
-        m = self.mixer
-        return (type(m) is Mamba2Mixer and type(self.norm) is Mamba2RMSNorm and type(m.norm) is MambaRMSNormGated
-                and m.out_proj.bias is None and _is_untouched(m.in_proj, ColumnParallelLinear)
-                and _is_untouched(m.out_proj, RowParallelLinear) and "step" not in vars(m) and "forward_add" not in vars(self.norm)
-                and ps.get_tensor_model_parallel_size() == 1)
+    def _in_one_call(self, op, method: str, hidden_states, residual, residual_dtype, conv_state, ssm_state):
+        """`op`, one native call that stands for `method` of the mixer and what surrounds it, where the block is made of the
+        plain modules on one rank.  None where any is of another class, has a hook or a method set on it, or out_proj has a bias:
+        these keep the calls one by one.  (The modules' own dictionaries: attribute lookups of a module cost the host more than
+        the launches.)"""
+        norm, m = self._modules["norm"], self._modules["mixer"]
+        if type(m) is not Mamba2Mixer or type(norm) is not Mamba2RMSNorm:
+            return None
+        parts, own = m._modules, m._parameters
+        gate, conv, first, last = parts["norm"], parts["conv1d"]._parameters, parts["in_proj"], parts["out_proj"]
+        if (method in vars(m) or "forward_add" in vars(norm) or (method == "forward" and _hooked(m)) or _has_any_global_hook()
+                or type(gate) is not MambaRMSNormGated or type(first) is not ColumnParallelLinear or type(last) is not RowParallelLinear
+                or "forward" in vars(first) or "forward" in vars(last) or _hooked(first) or _hooked(last)
+                or last._parameters["bias"] is not None or ps.get_tensor_model_parallel_size() != 1):
+            return None
+        return op(hidden_states, residual, residual_dtype, conv_state, ssm_state, norm._parameters["weight"], norm.variance_epsilon,
+                  first._parameters["weight"], first._parameters["bias"], conv["weight"], conv["bias"], own["dt_bias"], own["A_log"],
+                  own["D"], gate._parameters["weight"], last._parameters["weight"], m.intermediate_size_tp, m.n_groups_tp,
+                  m.ssm_state_size, m.head_dim, m.layer_norm_epsilon, gate.group_size)
 
     def forward(self, hidden_states, residual=None, cache_params=None):
         rd = torch.float32 if self.residual_in_fp32 else None
+        if (not torch.is_grad_enabled() and hidden_states.dim() == 3 and (cache_params is None or type(cache_params) is Mamba2Cache)):
+            states = (None, None) if cache_params is None else (cache_params.conv_states[self.layer_idx],
+                                                                cache_params.ssm_states[self.layer_idx])
+            done = self._in_one_call(ops.block_forward, "forward", hidden_states, residual, rd, *states)
+            if done is not None:
+                return done
         normed, residual = self.norm.forward_add(hidden_states, residual, rd)
         return self.mixer(normed, cache_params=cache_params), residual
 
     def step(self, hidden_states, residual, cache_params):
         rd = torch.float32 if self.residual_in_fp32 else None
-        if self._is_plain() and hidden_states.dim() == 3 and hidden_states.shape[1] == 1:
-            m, i = self.mixer, self.layer_idx
-            done = ops.decode_block(hidden_states, residual, rd, cache_params.conv_states[i], cache_params.ssm_states[i],
-                                    self.norm.weight, self.norm.variance_epsilon, m.in_proj.weight, m.in_proj.bias, m.conv1d.weight,
-                                    m.conv1d.bias, m.dt_bias, m.A_log, m.D, m.norm.weight, m.out_proj.weight, **m._core_kwargs())
+        if hidden_states.dim() == 3 and hidden_states.shape[1] == 1:
+            done = self._in_one_call(ops.decode_block, "step", hidden_states, residual, rd, cache_params.conv_states[self.layer_idx],
+                                     cache_params.ssm_states[self.layer_idx])
             if done is not None:
                 return done
         normed, residual = self.norm.forward_add(hidden_states, residual, rd)
@@ -212,7 +224,8 @@ class Mamba2Model(Mamba2PreTrainedModel):
 def _delivers_statistics(head) -> bool:
     """True for the plain head, whose GEMM can take the cross-entropy statistics along.  Any other module, a bias or a
     gathered output has no such form; a hook, or a forward set on the module, gets the tensor that the head returns."""
-    return _is_untouched(head, ColumnParallelLinear) and head.bias is None and not head.gather_output
+    return (type(head) is ColumnParallelLinear and head.bias is None and not head.gather_output and "forward" not in vars(head)
+            and not (_hooked(head) or _has_any_global_hook()))
 
 
 def _shift_labels(labels):

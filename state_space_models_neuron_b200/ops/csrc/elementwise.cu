@@ -4,6 +4,7 @@
 // all arithmetic fp32.  Reference counterparts: mamba2/conv1d_grouped.py:65-194 (conv),
 // mamba2/fused_kernel.py:76-175 (gated norm), mamba2/modeling_mamba2.py:94-103 (RMSNorm).
 #include "common.cuh"
+#include "dt_prep.cuh"
 #include <type_traits>
 
 namespace ssm {
@@ -85,15 +86,13 @@ __device__ __forceinline__ void conv_params(const __nv_bfloat16* w, const __nv_b
 
 // x [B, L, C] with row stride xs (elements); out row stride os.  init [B, 3, C] (tokens preceding x) or null.
 template <int TOK>
-__global__ void __launch_bounds__(128, 8)
-conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const __nv_bfloat16* __restrict__ w,
-                       const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ init,
-                       __nv_bfloat16* __restrict__ out, long long os, int L, int C) {
-  const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * CONV_CPT;
+__device__ __forceinline__ void conv_fwd_tile(const __nv_bfloat16* __restrict__ x, long long xs, const __nv_bfloat16* __restrict__ w,
+                                              const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ init,
+                                              __nv_bfloat16* __restrict__ out, long long os, int L, int C, int bx, int tile, int b) {
+  const int c0 = (bx * 128 + threadIdx.x) * CONV_CPT;
   if (c0 >= C) return;
   if (!SSM_INDEX_OK(c0 + CONV_CPT - 1, C) || !SSM_INDEX_OK(C - 1, xs) || !SSM_INDEX_OK(C - 1, os)) return;   // whole vectors inside a row
-  const int t0 = blockIdx.y * TOK;
-  const int b = blockIdx.z;
+  const int t0 = tile * TOK;
   uint64_t wt[CONV_K][CONV_PAIRS], bs[CONV_PAIRS];
   const __nv_bfloat16* xb = x + (long long)b * L * xs + c0;
   __nv_bfloat16* ob = out + (long long)b * L * os + c0;
@@ -133,6 +132,48 @@ conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
       }
       *reinterpret_cast<uint2*>(ob + (long long)t * os) = make_uint2(pack_bf16_pair(o[0]), pack_bf16_pair(o[1]));
     }
+  }
+}
+
+template <int TOK>
+__global__ void __launch_bounds__(128, 8)
+conv1d_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const __nv_bfloat16* __restrict__ w,
+                       const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ init,
+                       __nv_bfloat16* __restrict__ out, long long os, int L, int C) {
+  conv_fwd_tile<TOK>(x, xs, w, bias, init, out, os, L, C, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// last four inputs of the conv, [B, C, 4], from x [B, L, C] (row stride xs), L >= 4
+__device__ __forceinline__ void conv_window_tile(const __nv_bfloat16* __restrict__ x, long long xs, uint2* __restrict__ out, int L, int C, int c, int b) {
+  if (c >= C) return;
+  const __nv_bfloat16* p = x + ((long long)b * L + L - 4) * xs + c;
+  uint32_t v[4];
+  #pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = __bfloat16_as_ushort(p[k * xs]);
+  out[(long long)b * C + c] = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+}
+
+// What a mixer does with the output of in_proj in front of its scan, in one launch: conv of x | B | C, the step sizes, and where a
+// prompt fills a cache the conv window.  The blocks of the three parts stand one behind the other in grid.x, the small parts
+// first, which run beside the conv (us in three kernels -> one: 128 x 1792 with 24 heads 7.5 -> 5.9).
+struct ConvDt {
+  const __nv_bfloat16 *x, *w, *bias; long long xs; __nv_bfloat16* out; long long os; int L, C;
+  DtPrep dt;
+  uint2* window;
+  int conv_x, conv_tiles, dt_groups, dt_blocks, window_x, window_blocks;     // conv: conv_x column blocks x conv_tiles x B
+};
+template <int TOK>
+__global__ void __launch_bounds__(128, 8) conv_dt_kernel(const ConvDt a) {
+  int i = blockIdx.x;
+  if (i < a.dt_blocks) {
+    const int chunks = a.L / DT_CHUNK, per = chunks * a.dt_groups, b = i / per, r = i - b * per;
+    dt_prep_block(a.dt, r / a.dt_groups, r % a.dt_groups * DT_HEADS, b);
+  } else if ((i -= a.dt_blocks) < a.window_blocks) {
+    conv_window_tile(a.x, a.xs, a.window, a.L, a.C, (i % a.window_x) * 128 + threadIdx.x, i / a.window_x);
+  } else {
+    i -= a.window_blocks;
+    const int per = a.conv_x * a.conv_tiles, b = i / per, r = i - b * per;
+    conv_fwd_tile<TOK>(a.x, a.xs, a.w, a.bias, nullptr, a.out, a.os, a.L, a.C, r % a.conv_x, r / a.conv_x, b);
   }
 }
 
@@ -978,6 +1019,30 @@ extern "C" int ssm_conv1d_silu_fwd(const void* x, long long xs, const void* w, c
   return (int)cudaGetLastError();
 }
 
+// ssm_conv1d_silu_fwd without initial tokens, ssm_ssd_dt_prep and, with a window, ssm_conv_window in one launch
+extern "C" int ssm_conv_dt(const void* x, long long xs, const void* w, const void* bias, void* out, long long os, const void* dt_raw,
+                           const void* dt_bias, const void* A, const void* D, int mask, void* params_out, void* dt_out, void* l_out,
+                           void* window, int B, int L, int C, int H, cudaStream_t st) {
+  if (C % 8 || xs % 8 || os % 8 || L < DT_CHUNK || L % DT_CHUNK || B < 1 || H < 1 || (reinterpret_cast<uintptr_t>(dt_raw) & 15) ||
+      (reinterpret_cast<uintptr_t>(window) & 7))
+    return -SSM_ERR_BAD_ARG;
+  const int tok = conv_tok_for(B, L, C, CONV_CPT, 8);
+  ConvDt a;
+  a.x = BF(x); a.w = BF(w); a.bias = BF(bias); a.xs = xs; a.out = BFM(out); a.os = os; a.L = L; a.C = C;
+  a.dt = DtPrep{BF(dt_raw), xs, {A, D, dt_bias, mask, reinterpret_cast<float*>(params_out)}, reinterpret_cast<float*>(dt_out),
+                reinterpret_cast<float*>(l_out), L, H};
+  a.window = reinterpret_cast<uint2*>(window);
+  a.conv_x = (C / CONV_CPT + 127) / 128; a.conv_tiles = (L + tok - 1) / tok;
+  a.dt_groups = (H + DT_HEADS - 1) / DT_HEADS; a.window_x = (C + 127) / 128;
+  const long long conv = (long long)a.conv_x * a.conv_tiles * B, dt = (long long)(L / DT_CHUNK) * a.dt_groups * B,
+                  last = window != nullptr ? (long long)a.window_x * B : 0, total = conv + dt + last;
+  if (total > 0x7fffffffll) return -SSM_ERR_BAD_ARG;
+  a.dt_blocks = (int)dt; a.window_blocks = (int)last;
+  auto kern = tok == 32 ? conv_dt_kernel<32> : tok == 16 ? conv_dt_kernel<16> : conv_dt_kernel<8>;
+  kern<<<(unsigned)total, 128, 0, st>>>(a);
+  return (int)cudaGetLastError();
+}
+
 // tokens per partial-sum tile of the backward kernel for this problem size
 extern "C" int ssm_conv_bwd_tok_tile(int B, int L, int C) { return conv_tok_for(B, L, C, CONV_CPT, 16); }
 
@@ -1205,22 +1270,15 @@ extern "C" int ssm_ce_backward(const void* logits, long long ld, int is_fp32, co
   return (int)cudaGetLastError();
 }
 
-// last four inputs of the conv, [B, C, 4], from x [B, L, C] (row stride xs), L >= 4
 namespace ssm {
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 conv_window_kernel(const __nv_bfloat16* __restrict__ x, long long xs, uint2* __restrict__ out, int L, int C) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-  if (c >= C) return;
-  const __nv_bfloat16* p = x + ((long long)b * L + L - 4) * xs + c;
-  uint32_t v[4];
-  #pragma unroll
-  for (int k = 0; k < 4; ++k) v[k] = __bfloat16_as_ushort(p[k * xs]);
-  out[(long long)b * C + c] = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+  conv_window_tile(x, xs, out, L, C, blockIdx.x * 128 + threadIdx.x, blockIdx.y);
 }
 }  // namespace ssm
 extern "C" int ssm_conv_window(const void* x, long long xs, void* out, int B, int L, int C, cudaStream_t st) {
   if (L < 4 || B < 1 || B > 65535 || C < 1 || (reinterpret_cast<uintptr_t>(out) & 7)) return -SSM_ERR_BAD_ARG;
-  conv_window_kernel<<<dim3((C + 255) / 256, B), 256, 0, st>>>(BF(x), xs, reinterpret_cast<uint2*>(out), L, C);
+  conv_window_kernel<<<dim3((C + 127) / 128, B), 128, 0, st>>>(BF(x), xs, reinterpret_cast<uint2*>(out), L, C);
   return (int)cudaGetLastError();
 }
 

@@ -11,6 +11,7 @@
 // cumulative sums, never as a ratio of exponentials.
 // Reference math: mamba2/mamba2_kernel.py:15-62,138-169 (forward), :358-480 (backward).
 #include "common.cuh"
+#include "dt_prep.cuh"
 
 namespace ssm {
 
@@ -57,45 +58,9 @@ __device__ __forceinline__ float block_sum128(float v, float* red) {
 }
 
 // =====================================================================================
-// dt = softplus(dt_raw + bias), l = inclusive cumsum of A*dt within each chunk.   grid (nc, H, B), 128 threads
+// dt and its running sums (dt_prep.cuh).   grid (nc, heads / 8, B), 128 threads
 // =====================================================================================
-// Parameters as they are (bf16 where bit 0, 1, 2 of the mask is set for A, D, dt_bias; bit 3: A holds A_log); `out`
-// (optional) receives (A, D, dt_bias) in fp32, [3][H], for the kernels behind this one.
-struct HeadParams { const void* A; const void* D; const void* dt_bias; int mask; float* out; };
-__device__ __forceinline__ float head_param(const void* p, int h, bool bf16) {
-  return bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[h]) : reinterpret_cast<const float*>(p)[h];
-}
-__global__ void __launch_bounds__(128)
-ssd_dt_prep_kernel(const __nv_bfloat16* __restrict__ dt_raw, long long row_stride, const HeadParams prm,
-                   float* __restrict__ dt_out, float* __restrict__ l_out, int L, int H) {
-  __shared__ float wsum[4];
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, j = threadIdx.x;
-  const long long t = (long long)c * CT + j;
-  float A = head_param(prm.A, h, prm.mask & 1);
-  if (prm.mask & 8) A = -expf(A);
-  const float bias = head_param(prm.dt_bias, h, prm.mask & 4);
-  if (prm.out != nullptr && c == 0 && b == 0 && j == 0) {
-    prm.out[h] = A;
-    prm.out[H + h] = head_param(prm.D, h, prm.mask & 2);
-    prm.out[2 * H + h] = bias;
-  }
-  const float v = __bfloat162float(dt_raw[((long long)b * L + t) * row_stride + h]) + bias;
-  const float dt = softplus_f(v);
-  float a = A * dt;
-  const int lane = j & 31, w = j >> 5;
-  #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float n = __shfl_up_sync(0xffffffffu, a, o);
-    if (lane >= o) a += n;
-  }
-  if (lane == 31) wsum[w] = a;
-  __syncthreads();
-  float off = 0.f;
-  for (int k = 0; k < w; ++k) off += wsum[k];
-  const long long o = ((long long)b * H + h) * L + t;
-  dt_out[o] = dt;
-  l_out[o] = a + off;
-}
+__global__ void __launch_bounds__(DT_CHUNK) ssd_dt_prep_kernel(const DtPrep p) { dt_prep_block(p, blockIdx.x, blockIdx.y * DT_HEADS, blockIdx.z); }
 
 // =====================================================================================
 // chunk states:  S[n][p] = sum_j W[j][n] * s_j * V[j][p]
@@ -1288,11 +1253,10 @@ static int smem_opt_in(const void* fn, int bytes) {
 // A, D, dt_bias, mask, params_out: see HeadParams
 extern "C" int ssm_ssd_dt_prep(const void* dt_raw, long long row_stride, const void* dt_bias, const void* A, const void* D,
                                int mask, void* params_out, void* dt_out, void* l_out, int B, int L, int H, cudaStream_t st) {
-  if (L % CT) return -SSM_ERR_BAD_ARG;
-  dim3 grid(L / CT, H, B);
-  const HeadParams prm{A, D, dt_bias, mask, reinterpret_cast<float*>(params_out)};
-  ssd_dt_prep_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(dt_raw), row_stride, prm,
-                                           reinterpret_cast<float*>(dt_out), reinterpret_cast<float*>(l_out), L, H);
+  if (L % CT || row_stride % 8 || (reinterpret_cast<uintptr_t>(dt_raw) & 15)) return -SSM_ERR_BAD_ARG;
+  const DtPrep p{reinterpret_cast<const __nv_bfloat16*>(dt_raw), row_stride, {A, D, dt_bias, mask, reinterpret_cast<float*>(params_out)},
+                 reinterpret_cast<float*>(dt_out), reinterpret_cast<float*>(l_out), L, H};
+  ssd_dt_prep_kernel<<<dim3(L / CT, (H + DT_HEADS - 1) / DT_HEADS, B), DT_CHUNK, 0, st>>>(p);
   return (int)cudaGetLastError();
 }
 

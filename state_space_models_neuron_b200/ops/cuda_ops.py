@@ -736,15 +736,15 @@ def _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a):
 
 
 def _ssd_forward(conv_out, dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, d_inner, G, H, Hv, init_state=None,
-                 want_final=False, want_states=True, log_a=False, final_out=None):
+                 want_final=False, want_states=True, log_a=False, final_out=None, prepared=None):
     """conv_out [B*L, C] bf16 contiguous.  Returns y [B*L, d_inner], dt, l, S_in (None without want_states), final (or
     None), and (A, D, dt_bias) in fp32.  The backward pass wants S_in, the states entering the chunks.  final_out: contiguous
-    fp32 [B, H, P, 128] that receives the final state."""
+    fp32 [B, H, P, 128] that receives the final state.  prepared: what _dt_prep would return."""
     dev = conv_out.device
     C = conv_out.shape[1]
     nc = L // _CT
     st = status_tensor(dev)
-    dt, l, params = _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a)
+    dt, l, params = prepared or _dt_prep(dt_raw2, dt_raw_stride, A, D, dt_bias, B, L, H, log_a)
     D = params[1]
     y = torch.empty(B * L, d_inner, dtype=torch.bfloat16, device=dev)
     if _walk_states(B * Hv, nc):
@@ -806,16 +806,22 @@ def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, 
     return dx, dBC, hp[:, 0], hp[:, 1], hp[:, 2]
 
 
-def _conv_window(xBC, K, out=None):
-    """Last K inputs of the conv, [B, C, K]."""
+def _conv_dt(xBC, w2, bias, dt_raw2, dt_raw_stride, A_log, D, dt_bias, window=None):
+    """(conv output [B L, C], what _dt_prep returns for A_log) and, into `window` [B, C, 4], the last inputs of the conv."""
     B, L, C = xBC.shape
-    if K == 4 and L >= 4:
-        if out is None:
-            out = torch.empty(B, C, 4, dtype=xBC.dtype, device=xBC.device)
-        _run("ssm_conv_window", _p(xBC), _ll(xBC.stride(1)), _p(out), B, L, C, _st())
-        return out
-    tail = xBC[:, -K:, :] if L >= K else torch.cat([xBC.new_zeros(B, K - L, C), xBC], dim=1)
-    return tail.transpose(1, 2).contiguous()
+    H, dev = dt_raw2.shape[1], xBC.device
+    mask = _head_param_mask(A_log, D, dt_bias, H)
+    if mask is None:
+        if window is not None:
+            _run("ssm_conv_window", _p(xBC), _ll(xBC.stride(1)), _p(window), B, L, C, _st())
+        return _conv_fwd(xBC, w2, bias, None).view(B * L, C), _dt_prep(dt_raw2, dt_raw_stride, A_log, D, dt_bias, B, L, H, True)
+    out = torch.empty(B * L, C, dtype=xBC.dtype, device=dev)
+    params = torch.empty(3, H, dtype=torch.float32, device=dev)
+    dt = torch.empty(B, H, L, dtype=torch.float32, device=dev)
+    l = torch.empty_like(dt)
+    _run("ssm_conv_dt", _p(xBC), _ll(xBC.stride(1)), _p(w2), _p(bias), _p(out), _ll(C), _p(dt_raw2), _p(dt_bias), _p(A_log), _p(D),
+         mask | 8, _p(params), _p(dt), _p(l), _p(window), B, L, C, H, _st())
+    return out, (dt, l, params.unbind(0))
 
 
 def _head_param_mask(A, D, dt_bias, H):
@@ -851,11 +857,14 @@ class _MixerCore(torch.autograd.Function):
         flat = zxBCdt.as_strided((B * L, W), (ld, 1))
         z2, xBC, dt_raw2 = flat[:, :d_inner], zxBCdt[..., d_inner:d_inner + C], flat[:, d_inner + C:]
         w2 = conv_w.reshape(C, -1).contiguous()
-        conv_out = _conv_fwd(xBC, w2, conv_b, None).view(B * L, C)
         window_out, final_out = state_out or (None, None)
+        conv_state = None
+        if want_final:
+            conv_state = torch.empty(B, C, 4, dtype=zxBCdt.dtype, device=zxBCdt.device) if window_out is None else window_out
+        conv_out, prepared = _conv_dt(xBC, w2, conv_b, dt_raw2, ld, A_log, D, dt_bias, conv_state)
         y, dt, l, s_in, final, (A, Df, bf) = _ssd_forward(
             conv_out, dt_raw2, ld, A_log, D, dt_bias, B, L, d_inner, G, H, Hv, want_final=want_final,
-            want_states=recorded and not recompute, log_a=True, final_out=final_out)
+            want_states=recorded and not recompute, log_a=True, final_out=final_out, prepared=prepared)
         out = _gated_fwd(y, z2, norm_w, eps, gs)
         ctx.dims = (B, L, W, C, d_inner, G, N, P, H, Hv, eps, gs, recompute)
         if recompute:
@@ -866,7 +875,6 @@ class _MixerCore(torch.autograd.Function):
         ctx.conv_w_param = conv_w if conv_w.is_leaf else None
         out = out.view(B, L, d_inner)
         if want_final:
-            conv_state = _conv_window(xBC, w2.shape[1], window_out)
             ctx.mark_non_differentiable(conv_state, final)
             return out, conv_state, final
         return out
@@ -1033,6 +1041,91 @@ def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_lo
     return _gated_fwd(y, zxBCdt[:, :d_inner], norm_w, eps, gs)
 
 
+def _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D, gate_w, out_w):
+    """Addresses of a block's weights and the mask of its bf16 per-head parameters, or None where one of them is not as the
+    kernels read it."""
+    C, H, bf16 = d_inner + 2 * n_groups * d_state, d_inner // head_dim, torch.bfloat16
+    W = d_inner + C + H
+    mask = _head_param_mask(A_log, D, dt_bias, H)
+    given = [t for t in (norm_w, in_w, conv_w, gate_w, out_w, in_b, conv_b) if t is not None]
+    if (mask is None or H % n_groups or width % 8 or d_inner % 8 or d_inner % gs or gs % 8 or max(width, gs) > 8192
+            or any(t.dtype is not bf16 or not t.is_contiguous() for t in given)
+            or in_w.shape != (W, width) or out_w.shape != (width, d_inner) or norm_w.numel() != width or gate_w.numel() != d_inner
+            or conv_w.numel() != 4 * C or (in_b is not None and in_b.numel() != W) or (conv_b is not None and conv_b.numel() != C)):
+        return None
+    at = [norm_w.data_ptr(), in_w.data_ptr(), 0 if in_b is None else in_b.data_ptr(), conv_w.data_ptr(),
+          0 if conv_b is None else conv_b.data_ptr(), A_log.data_ptr(), D.data_ptr(), dt_bias.data_ptr(), gate_w.data_ptr(),
+          out_w.data_ptr()]
+    if (at[0] | at[1] | at[8] | at[9]) & 15 or at[3] & 7:
+        return None
+    return at, mask
+
+
+def _block_rows(hidden, residual, rd):
+    """Addresses of a block's input rows, or None where they are not as the kernels read them."""
+    if (hidden.dtype is not torch.bfloat16 or not hidden.is_contiguous() or not (rd is torch.bfloat16 or rd is torch.float32)
+            or (residual is not None and (residual.dtype is not rd or not residual.is_contiguous() or residual.shape != hidden.shape))):
+        return None
+    at = [hidden.data_ptr(), 0 if residual is None else residual.data_ptr()]
+    return None if (at[0] | at[1]) & 15 else at
+
+
+def _block_states(B, C, H, P, N, conv_state, ssm_state):
+    """Addresses of a layer's cached states, or None where the kernels cannot use them in place."""
+    if (conv_state.dtype is not torch.bfloat16 or ssm_state.dtype is not torch.float32 or conv_state.shape != (B, C, 4)
+            or ssm_state.shape != (B, H, P, N) or not conv_state.is_contiguous() or not ssm_state.is_contiguous()):
+        return None
+    at = [conv_state.data_ptr(), ssm_state.data_ptr()]
+    return None if at[0] & 7 or at[1] & 15 else at
+
+
+@functools.lru_cache(maxsize=256)
+def _scratch_offsets(*sizes):
+    """Offsets of buffers of these sizes (bytes) in one allocation, on 256-byte boundaries, and its size."""
+    at, end = [], 0
+    for size in sizes:
+        at.append(end)
+        end += (size + 255) // 256 * 256
+    return at, end
+
+
+_BLOCK_FORWARD = struct.Struct("=26Qq11i2f")
+
+
+def block_forward(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w, conv_b, dt_bias, A_log,
+                  D, gate_w, out_w, d_inner, n_groups, d_state, head_dim, eps, norm_group_size):
+    """A pre-norm block over whole sequences, `out_proj(mixer(norm(residual + hidden)))`, by one native call.  conv_state and
+    ssm_state, which may be None, receive the states behind the last token.  Returns (branch output, new residual), or None
+    where a tensor is not as the kernels read it; the caller then takes the separate operations."""
+    B, L, width = hidden.shape
+    C, H = d_inner + 2 * n_groups * d_state, d_inner // head_dim
+    rd = residual_dtype or hidden.dtype
+    gs = d_inner if norm_group_size is None else norm_group_size
+    if L % _CT or L == 0 or B == 0 or B > 65535 or d_state != 128 or head_dim % 64 or hidden.numel() >= 2 ** 31:
+        return None
+    weights = _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D,
+                             gate_w, out_w)
+    rows = _block_rows(hidden, residual, rd)
+    states = [0, 0] if conv_state is None else _block_states(B, C, H, head_dim, d_state, conv_state, ssm_state)
+    if weights is None or rows is None or states is None:
+        return None
+    dev, ld, T = hidden.device, _ceil8(d_inner + C + H), B * L
+    count = _segments(T // L * d_inner // 64, L // _CT, _PER_CHUNK[0])
+    segments = 0 if count == 1 else B * (d_inner // 64) * count
+    at, end = _scratch_offsets(2 * T * max(width, d_inner), 2 * T * ld, 2 * T * C, 2 * T * d_inner, 12 * H, 4 * T * H, 4 * T * H,
+                               segments * 4 * 128 * 64, segments * 4)
+    scratch = torch.empty(end, dtype=torch.uint8, device=dev)
+    base = scratch.data_ptr()
+    out, res_out = torch.empty_like(hidden), torch.empty(hidden.shape, dtype=rd, device=dev)
+    _run("ssm_block_forward", _BLOCK_FORWARD.pack(*rows, res_out.data_ptr(), *weights[0], *states, *[base + o for o in at], out.data_ptr(),
+                                                  status_tensor(dev).data_ptr(), ld, B, L, width, d_inner, H, head_dim, n_groups, gs,
+                                                  int(rd is torch.float32), weights[1], count, norm_eps, eps), _st())
+    _launches[0] += 5 + (count > 1)
+    if conv_state is not None:             # written through their addresses: autograd learns of it here
+        torch.autograd.graph.increment_version((conv_state, ssm_state))
+    return out, res_out
+
+
 _BLOCK = struct.Struct("=20Qq11i2f")
 
 
@@ -1052,42 +1145,25 @@ def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w
     Returns (branch output, new residual), or None where a tensor is not as the kernels read it; the
     caller then takes the separate operations, which convert or refuse it."""
     B, _, width = hidden.shape
-    C, H, bf16 = d_inner + 2 * n_groups * d_state, d_inner // head_dim, torch.bfloat16
-    W = d_inner + C + H
-    rd = residual_dtype or bf16
+    C, H = d_inner + 2 * n_groups * d_state, d_inner // head_dim
+    rd = residual_dtype or hidden.dtype
     gs = d_inner if norm_group_size is None else norm_group_size
-    mask = _head_param_mask(A_log, D, dt_bias, H)
-    operands = [hidden, norm_w, in_w, conv_w, gate_w, out_w]
-    operands += [t for t in (in_b, conv_b) if t is not None]
-    if (mask is None or 2 * d_state + head_dim > 12288 or d_state % 4 or H % n_groups or width % 8 or d_inner % 8
-            or d_inner % gs or gs % 8 or max(width, gs) > 8192 or B > 65535
-            or any(t.dtype is not bf16 or not t.is_contiguous() for t in operands)
-            or not (rd is bf16 or rd is torch.float32)
-            or conv_state.dtype is not bf16 or ssm_state.dtype is not torch.float32
-            or conv_state.shape != (B, C, 4) or ssm_state.shape != (B, H, head_dim, d_state)
-            or not conv_state.is_contiguous() or not ssm_state.is_contiguous()
-            or in_w.shape != (W, width) or out_w.shape != (width, d_inner) or norm_w.numel() != width or gate_w.numel() != d_inner
-            or conv_w.numel() != 4 * C or (in_b is not None and in_b.numel() != W) or (conv_b is not None and conv_b.numel() != C)):
+    if 2 * d_state + head_dim > 12288 or d_state % 4 or B > 65535:
         return None
-    if residual is not None and (residual.dtype is not rd or not residual.is_contiguous() or residual.shape != hidden.shape):
+    weights = _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D,
+                             gate_w, out_w)
+    rows = _block_rows(hidden, residual, rd)
+    states = _block_states(B, C, H, head_dim, d_state, conv_state, ssm_state)
+    if weights is None or rows is None or states is None:
         return None
-    dev = hidden.device
-    ld, ldd = _ceil8(W), max(width, d_inner)
-    scratch = torch.empty(B * (ld + d_inner + ldd), dtype=bf16, device=dev)
+    dev, ld = hidden.device, _ceil8(d_inner + C + H)
+    scratch = torch.empty(B * (ld + d_inner + max(width, d_inner)), dtype=torch.bfloat16, device=dev)
     out, res_out = torch.empty_like(hidden), torch.empty(hidden.shape, dtype=rd, device=dev)
     zx = scratch.data_ptr()
-    pointers = [hidden.data_ptr(), 0 if residual is None else residual.data_ptr(), res_out.data_ptr(), norm_w.data_ptr(), in_w.data_ptr(),
-                0 if in_b is None else in_b.data_ptr(), conv_w.data_ptr(), 0 if conv_b is None else conv_b.data_ptr(),
-                A_log.data_ptr(), D.data_ptr(), dt_bias.data_ptr(), gate_w.data_ptr(), out_w.data_ptr(), conv_state.data_ptr(),
-                ssm_state.data_ptr(), zx, zx + 2 * B * ld, zx + 2 * B * (ld + d_inner), out.data_ptr(), status_tensor(dev).data_ptr()]
-    aligned = 0
-    for i in (0, 1, 2, 3, 4, 11, 12, 14):
-        aligned |= pointers[i]
-    if aligned & 15 or (pointers[6] | pointers[13]) & 7:
-        return None
     first, gated = _norms_in_products(B, width, d_inner, gs)
-    _run("ssm_decode_block", _BLOCK.pack(*pointers, ld, B, width, d_inner, H, head_dim, d_state, n_groups, gs,
-                                         int(rd is torch.float32), mask, int(first) | 2 * int(gated), norm_eps, eps), _st())
+    _run("ssm_decode_block", _BLOCK.pack(*rows, res_out.data_ptr(), *weights[0], *states, zx, zx + 2 * B * ld, zx + 2 * B * (ld + d_inner),
+                                         out.data_ptr(), status_tensor(dev).data_ptr(), ld, B, width, d_inner, H, head_dim, d_state,
+                                         n_groups, gs, int(rd is torch.float32), weights[1], int(first) | 2 * int(gated), norm_eps, eps), _st())
     _launches[0] += 4 - first - gated
     return out, res_out
 

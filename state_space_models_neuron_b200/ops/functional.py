@@ -19,9 +19,15 @@ from . import oracle
 _BASELINE = [False]
 
 
+_cuda_ops = None
+
+
 def _cuda():
-    from . import cuda_ops
-    return cuda_ops
+    global _cuda_ops
+    if _cuda_ops is None:
+        from . import cuda_ops
+        _cuda_ops = cuda_ops
+    return _cuda_ops
 
 
 def _native(t) -> bool:
@@ -171,16 +177,21 @@ def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_lo
     return oracle.gated_rmsnorm(y.to(zxBCdt.dtype), z, norm_w, eps, norm_group_size)
 
 
-def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w, conv_b, dt_bias,
-                 A_log, D, gate_w, out_w, *, d_inner: int, n_groups: int, d_state: int, head_dim: int, eps: float,
-                 norm_group_size: Optional[int]):
-    """One token of a whole pre-norm block (residual add and norm, in_proj, mixer step, out_proj) over cached states:
-    (branch output, new residual), or None where only the separate operations take these tensors."""
+def decode_block(hidden, *args, **kwargs):
+    """One token of a whole pre-norm block (residual add and norm, in_proj, mixer step, out_proj) over cached states; arguments
+    of `cuda_ops.decode_block`.  (branch output, new residual), or None where only the separate operations take these tensors."""
     if not _native(hidden) or _cuda()._recording():
         return None
-    return _cuda().decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w,
-                                conv_b, dt_bias, A_log, D, gate_w, out_w, d_inner, n_groups, d_state, head_dim, eps,
-                                norm_group_size)
+    return _cuda().decode_block(hidden, *args, **kwargs)
+
+
+def block_forward(hidden, *args, **kwargs):
+    """A whole pre-norm block over full sequences, leaving its final states in conv_state and ssm_state (both may be None); arguments
+    of `cuda_ops.block_forward`.  (branch output, new residual), or None where gradients are recorded or only the separate
+    operations take these tensors."""
+    if not _native(hidden) or _cuda()._recording():
+        return None
+    return _cuda().block_forward(hidden, *args, **kwargs)
 
 
 # ---- attention ----------------------------------------------------------------------------

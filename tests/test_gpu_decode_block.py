@@ -83,3 +83,63 @@ def test_hooks_and_replaced_modules_keep_their_calls():
     model.step(token, Mamba2Cache(cfg, 1, dtype=torch.bfloat16, device="cuda"))
     assert len(seen) == 2
     assert ((hooked - plain).norm() / plain.norm()).item() < 2.0 ** -6
+
+
+# one chunk; heads of two slices and groups; several segments and few slices; a width that is no multiple of 64
+@pytest.mark.parametrize("B,L,width,H,P,G,gs,fp32,cached", [(1, 128, 256, 8, 64, 1, 512, False, True), (2, 384, 512, 6, 128, 2, 384, True, True),
+                                                            (1, 2176, 264, 4, 64, 1, 256, False, True), (3, 256, 256, 8, 64, 4, 512, True, False)])
+def test_block_over_a_sequence_equals_separate_operations(B, L, width, H, P, G, gs, fp32, cached):
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    d, N = H * P, 128
+    C = d + 2 * G * N
+    gen = torch.Generator(device="cuda").manual_seed(B + L)
+    make = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=gen) * scale).bfloat16()
+    norm_w, gate_w = make(width), make(d)
+    in_w, in_b, out_w = make(d + C + H, width, scale=width ** -0.5), make(d + C + H), make(width, d, scale=d ** -0.5)
+    conv_w, conv_b, head = make(C, 1, 4), make(C), [make(H).float(), make(H).abs(), make(H)]
+    window, state = make(B, C, 4), torch.randn(B, H, P, N, device="cuda", generator=gen)
+    rd = torch.float32 if fp32 else None
+    kw = dict(d_inner=d, n_groups=G, d_state=N, head_dim=P, eps=1e-5, norm_group_size=gs)
+    hidden, residual = make(B, L, width), None
+    with torch.no_grad():
+        for _ in range(2):
+            versions = window._version, state._version
+            out, res = ops.block_forward(hidden, residual, rd, window if cached else None, state if cached else None, norm_w, 1e-5, in_w, in_b,
+                                         conv_w, conv_b, *head, gate_w, out_w, **kw)
+            normed, want_res = ops.add_rmsnorm(hidden, residual, norm_w, 1e-5, rd)
+            y, (w, s) = ops.mamba2_mixer_core(ops.linear(normed, in_w, in_b), conv_w, conv_b, *head, gate_w, return_final_states=True, **kw)
+            want = ops.linear(y, out_w)
+            torch.cuda.synchronize()
+            cuda_ops.check_status()
+            assert torch.equal(res, want_res) and out.shape == hidden.shape
+            # the same kernels, but for the chunks' route: states in the order of another association, one bf16 step of a value
+            near = lambda a, b: ((a.double() - b.double()).norm() / b.double().norm()).item() < 2.0 ** -8
+            assert near(out, want)
+            if cached:
+                assert torch.equal(window, w) and near(state, s) and window._version > versions[0] and state._version > versions[1]
+            hidden, residual = want, want_res
+    assert ops.block_forward(hidden, residual, rd, None, None, norm_w, 1e-5, in_w, in_b, conv_w, conv_b, *head, gate_w, out_w, **kw) is None
+
+
+def test_prompts_with_hooks_and_odd_caches_keep_their_calls():
+    from state_space_models_neuron_b200.models import Mamba2Cache, Mamba2Config, Mamba2ForCausalLM
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    cfg = Mamba2Config(num_heads=8, head_dim=64, vocab_size=512, hidden_size=256, state_size=128, num_hidden_layers=2, n_groups=1,
+                       initializer_range=0.02, dtype=torch.bfloat16)
+    model = Mamba2ForCausalLM(cfg, device="cuda").to(torch.bfloat16).eval()
+    ids = torch.randint(0, 512, (2, 128), device="cuda")
+    plain, cache = model.prefill(ids)
+    seen = []
+    mixer = model.backbone.layers[1].mixer
+    handles = [mixer.register_forward_hook(lambda *a: seen.append("mixer")), mixer.in_proj.register_forward_hook(lambda *a: seen.append("in"))]
+    hooked, other = model.prefill(ids)
+    [h.remove() for h in handles]
+    assert seen == ["in", "mixer"] and torch.equal(hooked, plain)
+    odd = Mamba2Cache(cfg, 2, dtype=torch.bfloat16, device="cuda", ssm_dtype=torch.bfloat16)
+    again, _ = model.prefill(ids, odd)
+    assert torch.equal(again, plain) and torch.equal(odd.ssm_states[1], cache.ssm_states[1].bfloat16())
+    for i in range(2):
+        assert torch.equal(cache.conv_states[i], other.conv_states[i]) and torch.equal(cache.ssm_states[i], other.ssm_states[i])

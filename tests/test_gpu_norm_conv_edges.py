@@ -63,3 +63,29 @@ def test_conv(L, C, init):
         ref.backward(dy.double())
         for got, want in ((x, X), (w, W), (b, Bs)):
             _near(got.grad, want.grad)
+
+
+@pytest.mark.parametrize("B,L,C,H", [(1, 128, 264, 3), (2, 256, 520, 8), (1, 1024, 5376, 13), (3, 2048, 2560, 80)])     # 8, 16 and 32 tokens a tile
+@pytest.mark.parametrize("fp32", [False, True])
+def test_conv_and_step_sizes_in_one_launch(B, L, C, H, fp32):
+    """Conv, step sizes and conv window of ssm_conv_dt against one kernel each and against 64 bits."""
+    from state_space_models_neuron_b200.ops import cuda_ops
+    gen = torch.Generator(device="cuda").manual_seed(B + H)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+    ld = (C + H + 7) // 8 * 8
+    rows = make(B, L, ld)
+    xbc, raw = rows[..., :C], rows.view(B * L, ld)[:, C:C + H]
+    w, bias = make(C, 4), make(C)
+    A_log, D, dt_bias = (t.float() if fp32 else t for t in (make(H).abs(), make(H), make(H)))
+    window = torch.empty(B, C, 4, dtype=torch.bfloat16, device="cuda")
+    out, (dt, l, params) = cuda_ops._conv_dt(xbc, w, bias, raw, ld, A_log, D, dt_bias, window)
+    assert torch.equal(out.view(B, L, C), cuda_ops._conv_fwd(xbc, w, bias, None))
+    assert torch.equal(window, xbc[:, -4:].transpose(1, 2))
+    dt2, l2, params2 = cuda_ops._dt_prep(raw, ld, A_log, D, dt_bias, B, L, H, True)
+    assert torch.equal(dt, dt2) and torch.equal(l, l2) and all(torch.equal(a, b.float()) for a, b in zip(params, params2))
+    A = -A_log.double().exp()
+    want = torch.nn.functional.softplus(raw.double().view(B, L, H) + dt_bias.double()).permute(0, 2, 1)
+    sums = (want * A[:, None]).view(B, H, L // 128, 128).cumsum(-1).view(B, H, L)
+    # exponential and logarithm to a few ulp, sums of 128 in chains of 5 and 3
+    assert torch.allclose(dt.double(), want, rtol=1e-5, atol=1e-6) and torch.allclose(l.double(), sums, rtol=2e-5, atol=1e-5)
+    assert torch.allclose(params[0].double(), A, rtol=1e-6) and torch.equal(params[1], D.float()) and torch.equal(params[2], dt_bias.float())
