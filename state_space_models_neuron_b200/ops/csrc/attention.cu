@@ -293,16 +293,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // ---------------------------------------------------------------------------------------------------
 // Backward: one CTA per (128-key tile, kv head, batch) walks its group's query heads and their 64-query tiles at or below
 // the diagonal.  Everything is transposed, TMEM lane = key (or channel for dQ): S^T = K Q^T and dP^T = V dO^T take 64
-// columns each, which leaves room for dQ^T (64), dV and dK (128 each) without sharing, and a query tile is small enough for
-// two stages of Q / dO and of P / dS in shared memory.
-//   warps 0-15   P and dS of a tile (row = key, 16 queries per warpgroup)
-//   warps 16-19  read dQ^T back and add it to fp32 dQ with one bulk reduction per tile
-//   warp 20      issues all products;  warp 21  loads
-// The scores of the next tile are issued before the three gradient products of this one, so the arithmetic of a tile and the
-// products of the tile before it overlap.  Bound by these two in turn.  One 128-thread group doing everything in turn, with a
-// reduction instruction per 16 bytes of dQ, took 3390 us with its fills and conversions for 8192 queries of 32 heads, this
-// 2343 (4096 x 32: 1046 -> 647; one box, back to back).  The kernel alone takes 2131 us (2863 with eight warps for P and dS, 2670
-// without packed arithmetic and with masks on every tile).
+// columns each, twice, next to dV and dK (128 each): two tiles are under way, and the arithmetic of one runs under the
+// products of the other.
+//   warps 0-15   P and dS of a tile (row = key, 16 queries per warpgroup), back into the S^T columns they came from: P^T and
+//                dS^T are the A operands of dV and dK there.  dS^T also goes to shared memory, as B operand of dQ^T
+//   warps 16-19  read dQ^T back (it stands where dP^T was) and add it to fp32 dQ with one bulk reduction per tile
+//   warp 20      issues all products, of whichever tile has its operands;  warp 21  loads, three tiles of Q and dO deep
+// Bound by shared memory (288 KB per 64 x 128 tile, 2250 of about 2870 clocks: K and V as A operands 96, Q and dO as B 64, dS
+// and dQ the rest).  us of the whole backward pass, 8192 queries of 32 heads / 4096 x 32: one 128-thread group doing everything
+// in turn 3390 / 1046; these warps with one tile of scores 2362 / 651, two 1987 / 571, P and dS in TMEM 1913 / 563, and a third
+// stage of Q and dO in the room they left 1701 / 561.  (dQ by a reduction per value instead of the staged bulk ones: +5 %.)
 struct AttnBwdParams {
   const float* lse; const float* delta;     // [B, Hq, L]
   __nv_bfloat16* dk; __nv_bfloat16* dv;     // [B*L, Hkv*128]
@@ -314,8 +314,9 @@ constexpr int AQ = 64;                               // queries of a tile
 constexpr int QTILE = AQ * AD * 2;                   // [64][128] bf16: two 8 KiB swizzle blocks
 constexpr int PTILE = AT * AQ * 2;                   // [128 keys][64 queries] bf16
 constexpr int BWD_STAGE = 2 * QTILE;                 // Q and dO
+constexpr int BWD_RING = 3;
 constexpr int ATTN_BWD_THREADS = 22 * 32;
-constexpr int ATTN_BWD_SMEM = 2 * ATILE + 2 * BWD_STAGE + 4 * PTILE + AQ * AD * 4 + 2 * 2 * AQ * 4 + 256 + 1024;
+constexpr int ATTN_BWD_SMEM = 2 * ATILE + BWD_RING * BWD_STAGE + 2 * PTILE + AQ * AD * 4 + BWD_RING * 2 * AQ * 4 + 256 + 1024;
 
 __global__ void __launch_bounds__(ATTN_BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -325,14 +326,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + ATILE;
-  uint8_t* sStage = sV + ATILE;                        // [2] Q | dO
-  uint8_t* sPS = sStage + 2 * BWD_STAGE;               // [2] P^T | dS^T
-  float* sdQ = reinterpret_cast<float*>(sPS + 4 * PTILE);              // [64 queries][128 channels]
-  float* sStat = sdQ + AQ * AD;                        // [2] lse[64] | delta[64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * 2 * AQ);
-  uint64_t *kv_full = bars, *full = bars + 1, *empty = bars + 3, *s_full = bars + 5, *ds_ready = bars + 6,
-           *done = bars + 7, *dq_full = bars + 9, *dq_free = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint8_t* sStage = sV + ATILE;                        // [3] Q | dO
+  uint8_t* sDS = sStage + BWD_RING * BWD_STAGE;        // [2] dS^T
+  float* sdQ = reinterpret_cast<float*>(sDS + 2 * PTILE);              // [64 queries][128 channels]
+  float* sStat = sdQ + AQ * AD;                        // [3] lse[64] | delta[64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + BWD_RING * 2 * AQ);
+  uint64_t *kv_full = bars, *full = bars + 1, *empty = full + BWD_RING, *s_full = empty + BWD_RING, *ds_ready = s_full + 2,
+           *dq_full = ds_ready + 2, *dq_free = dq_full + 2, *done = dq_free + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   const int hk = blockIdx.x % p.Hkv, b = blockIdx.x / p.Hkv, kt = blockIdx.y;      // longest walks first
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ratio = p.Hq / p.Hkv, per_head = p.L / AQ - 2 * kt, n = ratio * per_head;
@@ -340,8 +341,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   if (tid == 0) {
     mbar_init(kv_full, 1);
-    for (int k = 0; k < 2; ++k) { mbar_init(&full[k], 1); mbar_init(&empty[k], 1); mbar_init(&done[k], 1); }
-    mbar_init(s_full, 1); mbar_init(ds_ready, 16); mbar_init(dq_full, 1); mbar_init(dq_free, 128);
+    for (int k = 0; k < BWD_RING; ++k) { mbar_init(&full[k], 1); mbar_init(&empty[k], 1); }
+    for (int k = 0; k < 2; ++k) {
+      mbar_init(&s_full[k], 1); mbar_init(&ds_ready[k], 16);
+      mbar_init(&dq_full[k], 1); mbar_init(&dq_free[k], 4);
+    }
+    mbar_init(done, 1);
     mbar_fence_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_dq);
@@ -350,7 +355,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = *tmem_slot;                    // S^T 0, dP^T 64, dQ^T 128, dV 256, dK 384
+  const uint32_t tmem = *tmem_slot;                    // stage s: S^T (then dQ^T) 128 s, dP^T 128 s + 64; dV 256, dK 384
 
   if (warp == 21) {
     if (lane == 0) {
@@ -362,8 +367,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       bool ok = true;
       int it = 0;
       for (; it < n; ++it) {
-        const int st = it & 1, h = hk * ratio + it / per_head, q = (2 * kt + it % per_head) * AQ;
-        ok = mbar_wait(&empty[st], ((it >> 1) & 1) ^ 1, p.status);
+        const int st = it % BWD_RING, h = hk * ratio + it / per_head, q = (2 * kt + it % per_head) * AQ;
+        ok = mbar_wait(&empty[st], ((it / BWD_RING) & 1) ^ 1, p.status);
         if (!ok) break;
         uint8_t* sq = sStage + st * BWD_STAGE;
         mbar_expect_tx(&full[st], BWD_STAGE + 2 * AQ * 4);
@@ -377,7 +382,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (!ok) {                                       // copies still in flight land before the CTA goes
         mbar_wait(kv_full, 0, nullptr);
-        for (int k = it > 2 ? it - 2 : 0; k < it; ++k) mbar_wait(&full[k & 1], (k >> 1) & 1, nullptr);
+        for (int k = it > BWD_RING ? it - BWD_RING : 0; k < it; ++k) mbar_wait(&full[k % BWD_RING], (k / BWD_RING) & 1, nullptr);
       }
     }
     __syncwarp();
@@ -393,42 +398,59 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       auto mstep = [](int kk) { return (uint64_t)(kk * 128); };
       const uint64_t dKk = adesc_k(aK, 0), dVk = adesc_k(aV, 0), dKm = adesc_mn(aK, 0);
       auto scores = [&](int it) {
-        const uint32_t aQ = smem_u32(sStage + (it & 1) * BWD_STAGE);
+        const uint32_t aQ = smem_u32(sStage + it % BWD_RING * BWD_STAGE), to = tmem + (it & 1) * 128;
         const uint64_t dQk = make_smem_desc_sw128(aQ, 16, 1024), dOk = make_smem_desc_sw128(aQ + QTILE, 16, 1024);
         #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem, dKk + kstep(kk), dQk + qstep(kk), id_s, kk != 0);
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(to, dKk + kstep(kk), dQk + qstep(kk), id_s, kk != 0);
         #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem + 64, dVk + kstep(kk), dOk + qstep(kk), id_s, kk != 0);
-        umma_commit(s_full);
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(to + 64, dVk + kstep(kk), dOk + qstep(kk), id_s, kk != 0);
+        umma_commit(&s_full[it & 1]);
       };
-      bool ok = mbar_wait(kv_full, 0, p.status) && mbar_wait(&full[0], 0, p.status);
-      if (ok) { tc_fence_after_sync(); scores(0); }
-      for (int it = 0; it < n && ok; ++it) {
-        ok = mbar_wait(ds_ready, it & 1, p.status);
-        if (ok && it + 1 < n) {
-          ok = mbar_wait(&full[(it + 1) & 1], ((it + 1) >> 1) & 1, p.status);
-          tc_fence_after_sync();
-          if (ok) scores(it + 1);
-        }
-        if (ok && it > 0) ok = mbar_wait(dq_free, (it - 1) & 1, p.status);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint32_t aQ = smem_u32(sStage + (it & 1) * BWD_STAGE), aP = smem_u32(sPS + (it & 1) * 2 * PTILE);
+      auto gradients = [&](int it) {
+        const uint32_t aQ = smem_u32(sStage + it % BWD_RING * BWD_STAGE);
         const uint64_t dQm = make_smem_desc_sw128(aQ, QTILE / 2, 1024), dOm = make_smem_desc_sw128(aQ + QTILE, QTILE / 2, 1024);
-        const uint64_t dP = make_smem_desc_sw128(aP, 16, 1024), dDS = make_smem_desc_sw128(aP + PTILE, 16, 1024);
-        #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dQ^T[d][i] = sum_key K[key][d] dS^T[key][i]
-          umma_bf16(tmem + 128, dKm + mstep(kk), dDS + mstep(kk), id_q, kk != 0);
-        umma_commit(dq_full);
+        const uint64_t dDS = make_smem_desc_sw128(smem_u32(sDS + (it & 1) * PTILE), 16, 1024);
+        const uint32_t ts = tmem + (it & 1) * 128;
+        // k-step kk of P^T and dS^T is what warpgroup kk left in its own columns of S^T
         #pragma unroll
         for (int kk = 0; kk < 4; ++kk)      // dV[key][d] += sum_i P^T[key][i] dO[i][d]
-          umma_bf16(tmem + 256, dP + kstep(kk), dOm + mstep(kk), id_g, (it | kk) != 0);
+          umma_bf16_ta(tmem + 256, ts + kk * 16, dOm + mstep(kk), id_g, (it | kk) != 0);
         #pragma unroll
         for (int kk = 0; kk < 4; ++kk)      // dK[key][d] += sum_i dS^T[key][i] Q[i][d]
-          umma_bf16(tmem + 384, dDS + kstep(kk), dQm + mstep(kk), id_g, (it | kk) != 0);
-        umma_commit(&done[it & 1]);
-        umma_commit(&empty[it & 1]);
+          umma_bf16_ta(tmem + 384, ts + kk * 16 + 8, dQm + mstep(kk), id_g, (it | kk) != 0);
+        #pragma unroll
+        for (int kk = 0; kk < 8; ++kk)      // dQ^T[d][i] = sum_key K[key][d] dS^T[key][i], where dP^T of this tile was
+          umma_bf16(ts + 64, dKm + mstep(kk), dDS + mstep(kk), id_q, kk != 0);
+        umma_commit(&dq_full[it & 1]);      // also behind the readers of P^T and dS^T: their columns take the scores of it + 2
+        umma_commit(&empty[it % BWD_RING]);
+      };
+      // Whatever is ready goes next: the scores of tile s (its operands have landed, its TMEM stage has been read for the last
+      // time) or the gradients of tile g (P and dS are in shared memory).  The other of two stages stands for work meanwhile.
+      bool ok = mbar_wait(kv_full, 0, p.status);
+      uint64_t last = 0;
+      int s = 0, g = 0;
+      for (uint32_t idle = 1; g < n && ok; ++idle) {
+        bool moved = false;
+        if (s < n && s < g + 2 && mbar_test(&full[s % BWD_RING], (s / BWD_RING) & 1) && (s < 2 || mbar_test(&dq_free[s & 1], ((s >> 1) - 1) & 1))) {
+          tc_fence_after_sync();
+          scores(s++);
+          moved = true;
+        }
+        if (g < s && mbar_test(&ds_ready[g & 1], (g >> 1) & 1)) {
+          tc_fence_after_sync();
+          gradients(g++);
+          moved = true;
+        }
+        if (moved) {
+          idle = 0;
+        } else if ((idle & 1023u) == 0u) {             // bounded, as every wait here
+          if (p.status != nullptr && *((volatile int*)p.status) != 0) ok = false;
+          const uint64_t now = global_timer_ns();
+          if (idle == 1024u) last = now;
+          else if (now - last > SSM_WAIT_NS) { if (p.status != nullptr) atomicCAS(p.status, 0, SSM_ERR_TIMEOUT_MBAR); ok = false; }
+        }
       }
+      if (ok) umma_commit(done);
     }
     __syncwarp();
   } else if (warp >= 16) {
@@ -437,21 +459,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     for (int it = 0; it < n && ok; ++it) {
       const int h = hk * ratio + it / per_head, q = (2 * kt + it % per_head) * AQ;
-      ok = __all_sync(0xffffffffu, mbar_wait(dq_full, it & 1, p.status));
+      ok = __all_sync(0xffffffffu, mbar_wait(&dq_full[it & 1], (it >> 1) & 1, p.status));
       tc_fence_after_sync();
+      uint32_t v[2][32];
+      if (ok) {
+        tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, (it & 1) * 128 + 64), v[0]);
+        tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, (it & 1) * 128 + 96), v[1]);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&dq_free[it & 1]);  // the stage takes the scores of tile it + 2
+      }
       if (d == 0) tma_store_wait_read();               // the previous tile has left the staging rows
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (ok) {
         #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          uint32_t v[32];
-          tmem_ld32(tmem_addr(tmem, (warp & 3) * 32, 128 + i * 32), v);
-          tmem_ld_wait();
+        for (int i = 0; i < 2; ++i)
           #pragma unroll
-          for (int e = 0; e < 32; ++e) sdQ[(i * 32 + e) * AD + d] = __uint_as_float(v[e]);
-        }
-        tc_fence_before_sync();
-        mbar_arrive(dq_free);
+          for (int e = 0; e < 32; ++e) sdQ[(i * 32 + e) * AD + d] = __uint_as_float(v[i][e]);
       }
       fence_proxy_async_smem();
       ok = barrier_and<1, 128>(ok);                    // the four warps meet at barriers: they leave together
@@ -468,19 +493,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const float c = p.scale * LOG2E;
     bool ok = true;
     for (int it = 0; it < n && ok; ++it) {
-      const int st = it & 1, rel = (it % per_head) * AQ;      // first query relative to the key tile's first key
-      ok = __all_sync(0xffffffffu, mbar_wait(s_full, it & 1, p.status));
+      const int st = it & 1, ring = it % BWD_RING, rel = (it % per_head) * AQ;      // first query relative to the key tile's first key
+      // the loads of this stage (statistics included) complete on `full`, long before the scores; this thread observes the
+      // phase before it reads what they wrote.  The scores are complete behind the gradients of tile it - 2, which were issued
+      // in front of them: P, dS and the statistics of that tile have been read.
+      ok = mbar_wait(&full[ring], (it / BWD_RING) & 1, p.status);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&s_full[st], (it >> 1) & 1, p.status));
       if (!ok) break;
       tc_fence_after_sync();
       uint32_t sv[16], dp[16];
-      tmem_ld16(tmem_addr(tmem, lanes, wg * 16), sv);
-      tmem_ld16(tmem_addr(tmem, lanes, 64 + wg * 16), dp);
-      // the loads of this stage (statistics included) have completed on `full`, which the products of s_full waited for;
-      // this thread observes the same phase before it reads what they wrote
-      ok = __all_sync(0xffffffffu, mbar_wait(&full[st], (it >> 1) & 1, p.status));
+      tmem_ld16(tmem_addr(tmem, lanes, st * 128 + wg * 16), sv);
+      tmem_ld16(tmem_addr(tmem, lanes, st * 128 + 64 + wg * 16), dp);
       tmem_ld_wait();
-      if (!ok) break;
-      const float* lse = sStat + st * 2 * AQ + wg * 16;
+      const float* lse = sStat + ring * 2 * AQ + wg * 16;
       const float* delta = lse + AQ;
       uint32_t pk[8], dk[8];
       #pragma unroll
@@ -504,23 +529,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         pk[e4 * 2] = pack_bf16(pv[0], pv[1]); pk[e4 * 2 + 1] = pack_bf16(pv[2], pv[3]);
         dk[e4 * 2] = pack_bf16(ds[0], ds[1]); dk[e4 * 2 + 1] = pack_bf16(ds[2], ds[3]);
       }
-      if (it >= 2) {                                          // the products of tile it - 2 have read these buffers
-        ok = __all_sync(0xffffffffu, mbar_wait(&done[st], ((it >> 1) - 1) & 1, p.status));
-        if (!ok) break;
-      }
-      uint8_t* sp = sPS + st * 2 * PTILE;
+      tmem_st8(tmem_addr(tmem, lanes, st * 128 + wg * 16), pk);
+      tmem_st8(tmem_addr(tmem, lanes, st * 128 + wg * 16 + 8), dk);
+      uint8_t* sp = sDS + st * PTILE;
       #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const uint32_t off = sw128_offset(row, wg * 2 + q);
-        *reinterpret_cast<uint4*>(sp + off) = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
-        *reinterpret_cast<uint4*>(sp + PTILE + off) = make_uint4(dk[q * 4], dk[q * 4 + 1], dk[q * 4 + 2], dk[q * 4 + 3]);
-      }
+      for (int q = 0; q < 2; ++q)
+        *reinterpret_cast<uint4*>(sp + sw128_offset(row, wg * 2 + q)) = make_uint4(dk[q * 4], dk[q * 4 + 1], dk[q * 4 + 2], dk[q * 4 + 3]);
+      tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ds_ready);
+      if (lane == 0) mbar_arrive(&ds_ready[st]);
     }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&done[(n - 1) & 1], ((n - 1) >> 1) & 1, p.status));
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(done, 0, p.status));
     if (ok) {
       tc_fence_after_sync();
       __nv_bfloat16* dst = (wg < 2 ? p.dv : p.dk) + (long long)(krow0 + row) * (p.Hkv * AD) + hk * AD + (wg & 1) * 64;
