@@ -598,28 +598,58 @@ add_rmsnorm_bwd_kernel(const RT* __restrict__ res, const __nv_bfloat16* __restri
 // =====================================================================================
 // GELU (erf) forward / backward, 8 elements per thread
 // =====================================================================================
-__global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n8) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
-    float a[8];
-    load8(x + i * 8, a);
-    #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = 0.5f * a[e] * (1.f + erff(a[e] * 0.70710678118654752f));
-    store8(y + i * 8, a);
+// Gaussian distribution function of a pair, and exp(-x^2 / 2) on the way.  With t = 1 / (1 + 0.34 |x|), the tail
+// 0.5 erfc(|x| / sqrt 2) is exp(-x^2 / 2) times a polynomial of degree 9 in t (least-squares fit of 0.5 erfcx on |x| <= 14,
+// weighted towards equal relative errors: 1.3e-8 in the fit, 3e-7 in fp32), which is one division and one exponential per value, shared
+// with the density that the backward pass wants; erff() takes two polynomials behind a branch on |x| < 1.  Below zero the tail
+// itself is the result, so no digits cancel as they do in 1 + erf.
+// These kernels were bound by that arithmetic, twice to three times what moving their rows takes:
+//   us, 8192 x 16384, before -> now: forward 143 -> 108, backward 180 -> 138 (82 and 123 at copy bandwidth)
+__device__ __forceinline__ uint64_t gauss_cdf2(uint64_t x, uint64_t& gauss) {
+  float a, b;
+  unpack2(mul2(mul2(x, x), pack2(-0.72134752f, -0.72134752f)), a, b);
+  gauss = pack2(exp2f(a), exp2f(b));
+  unpack2(x, a, b);
+  const uint64_t t = pack2(1.f / fmaf(0.34f, fabsf(a), 1.f), 1.f / fmaf(0.34f, fabsf(b), 1.f));
+  constexpr float c[10] = {2.20011179e-06f, 0.135569155f, 0.136619806f, 0.112408914f, 0.124749377f, -0.0648477748f, 0.229716182f,
+                           -0.296367794f, 0.150507778f, -0.0283578485f};
+  uint64_t p = pack2(c[9], c[9]);
+  #pragma unroll
+  for (int k = 8; k >= 0; --k) p = fma2(p, t, pack2(c[k], c[k]));
+  float u, v;
+  unpack2(mul2(gauss, p), u, v);
+  return pack2(a < 0.f ? u : 1.f - u, b < 0.f ? v : 1.f - v);
+}
+// x Phi(x), and its derivative Phi(x) + x phi(x)
+__device__ __forceinline__ uint64_t gelu2(uint64_t x) {
+  uint64_t gauss;
+  return mul2(x, gauss_cdf2(x, gauss));
+}
+__device__ __forceinline__ uint64_t gelu_grad2(uint64_t x) {
+  uint64_t gauss;
+  const uint64_t cdf = gauss_cdf2(x, gauss);
+  return fma2(mul2(x, pack2(0.3989422804014327f, 0.3989422804014327f)), gauss, cdf);
+}
+__global__ void __launch_bounds__(256) gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n8) {
+  const long long step = (long long)gridDim.x * blockDim.x;
+  #pragma unroll 2
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += step) {
+    uint4 u = load_raw8(x + i * 8);
+    u.x = pack_bf16_pair(gelu2(bf16x2_pair(u.x))); u.y = pack_bf16_pair(gelu2(bf16x2_pair(u.y)));
+    u.z = pack_bf16_pair(gelu2(bf16x2_pair(u.z))); u.w = pack_bf16_pair(gelu2(bf16x2_pair(u.w)));
+    *reinterpret_cast<uint4*>(y + i * 8) = u;
   }
 }
-__global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                                __nv_bfloat16* __restrict__ dx, long long n8) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
-    float a[8], g[8];
-    load8(x + i * 8, a);
-    load8(dy + i * 8, g);
-    #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float cdf = 0.5f * (1.f + erff(a[e] * 0.70710678118654752f));
-      const float pdf = 0.3989422804014327f * __expf(-0.5f * a[e] * a[e]);
-      g[e] *= cdf + a[e] * pdf;
-    }
-    store8(dx + i * 8, g);
+__global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+                                                       __nv_bfloat16* __restrict__ dx, long long n8) {
+  const long long step = (long long)gridDim.x * blockDim.x;
+  #pragma unroll 2
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += step) {
+    uint4 u = load_raw8(x + i * 8);
+    const uint4 g = load_raw8(dy + i * 8);
+    u.x = pack_bf16_pair(mul2(bf16x2_pair(g.x), gelu_grad2(bf16x2_pair(u.x)))); u.y = pack_bf16_pair(mul2(bf16x2_pair(g.y), gelu_grad2(bf16x2_pair(u.y))));
+    u.z = pack_bf16_pair(mul2(bf16x2_pair(g.z), gelu_grad2(bf16x2_pair(u.z)))); u.w = pack_bf16_pair(mul2(bf16x2_pair(g.w), gelu_grad2(bf16x2_pair(u.w))));
+    *reinterpret_cast<uint4*>(dx + i * 8) = u;
   }
 }
 
@@ -1145,64 +1175,82 @@ extern "C" int ssm_add_rmsnorm_bwd(const void* res, const void* w, const void* d
 // (the reference's gated variant is mamba2hybrid/mamba2hybrid_mlp.py:118-134 in ATen ops)
 // -------------------------------------------------------------------------------------
 namespace ssm {
-__device__ __forceinline__ float glu_act(float x, int act) {
-  return act == 0 ? 0.5f * x * (1.f + erff(x * 0.70710678118654752f)) : x / (1.f + __expf(-x));
+// (activation, derivative) of a pair
+template <int ACT>
+__device__ __forceinline__ uint64_t glu_act2(uint64_t x) {
+  return ACT == 0 ? gelu2(x) : mul2(x, sigmoid2(x));
 }
-__device__ __forceinline__ float glu_act_grad(float x, int act) {
-  if (act == 0) return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.3989422804014327f * __expf(-0.5f * x * x);
-  const float sg = 1.f / (1.f + __expf(-x));
-  return sg * (1.f + x * (1.f - sg));
-}
-__global__ void __launch_bounds__(256)
-glu_fwd_kernel(const __nv_bfloat16* __restrict__ h, long long ld, __nv_bfloat16* __restrict__ out, long long rows, int S, int act) {
-  const int vec = S / 8;
-  const long long total = rows * vec;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / vec;
-    const int c = (int)(i - r * vec) * 8;
-    float g[8], u[8];
-    load8(h + r * ld + c, g);
-    load8(h + r * ld + S + c, u);
-    #pragma unroll
-    for (int e = 0; e < 8; ++e) g[e] = glu_act(g[e], act) * u[e];
-    store8(out + r * S + c, g);
+template <int ACT>
+__device__ __forceinline__ void glu_act_grad2(uint64_t x, uint64_t& act, uint64_t& grad) {
+  if (ACT == 0) {
+    uint64_t gauss;
+    const uint64_t cdf = gauss_cdf2(x, gauss);
+    act = mul2(x, cdf);
+    grad = fma2(mul2(x, pack2(0.3989422804014327f, 0.3989422804014327f)), gauss, cdf);
+  } else {
+    const uint64_t sg = sigmoid2(x), one = pack2(1.f, 1.f), minus = pack2(-1.f, -1.f);
+    act = mul2(x, sg);
+    grad = mul2(sg, fma2(x, fma2(sg, minus, one), one));
   }
 }
+// us, 4096 x 16384, before -> now: GELU forward 94 -> 72, backward 202 -> 109 (62 and 103 at copy bandwidth)
+template <int ACT>
 __global__ void __launch_bounds__(256)
-glu_bwd_kernel(const __nv_bfloat16* __restrict__ h, long long ld, const __nv_bfloat16* __restrict__ dout,
-               __nv_bfloat16* __restrict__ dh, long long rows, int S, int act) {
+glu_fwd_kernel(const __nv_bfloat16* __restrict__ h, long long ld, __nv_bfloat16* __restrict__ out, long long rows, int S) {
   const int vec = S / 8;
   const long long total = rows * vec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / vec;
     const int c = (int)(i - r * vec) * 8;
-    float g[8], u[8], d[8], dg[8], du[8];
-    load8(h + r * ld + c, g);
-    load8(h + r * ld + S + c, u);
-    load8(dout + r * S + c, d);
+    const uint4 g = load_raw8(h + r * ld + c), u = load_raw8(h + r * ld + S + c);
+    uint4 o;
+    o.x = pack_bf16_pair(mul2(glu_act2<ACT>(bf16x2_pair(g.x)), bf16x2_pair(u.x)));
+    o.y = pack_bf16_pair(mul2(glu_act2<ACT>(bf16x2_pair(g.y)), bf16x2_pair(u.y)));
+    o.z = pack_bf16_pair(mul2(glu_act2<ACT>(bf16x2_pair(g.z)), bf16x2_pair(u.z)));
+    o.w = pack_bf16_pair(mul2(glu_act2<ACT>(bf16x2_pair(g.w)), bf16x2_pair(u.w)));
+    *reinterpret_cast<uint4*>(out + r * S + c) = o;
+  }
+}
+template <int ACT>
+__global__ void __launch_bounds__(256)
+glu_bwd_kernel(const __nv_bfloat16* __restrict__ h, long long ld, const __nv_bfloat16* __restrict__ dout,
+               __nv_bfloat16* __restrict__ dh, long long rows, int S) {
+  const int vec = S / 8;
+  const long long total = rows * vec;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / vec;
+    const int c = (int)(i - r * vec) * 8;
+    const uint4 g = load_raw8(h + r * ld + c), u = load_raw8(h + r * ld + S + c), d = load_raw8(dout + r * S + c);
+    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w}, dw[4] = {d.x, d.y, d.z, d.w};
+    uint32_t dg[4], du[4];
     #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      dg[e] = d[e] * u[e] * glu_act_grad(g[e], act);
-      du[e] = d[e] * glu_act(g[e], act);
+    for (int e = 0; e < 4; ++e) {
+      uint64_t act, grad;
+      glu_act_grad2<ACT>(bf16x2_pair(gw[e]), act, grad);
+      const uint64_t dd = bf16x2_pair(dw[e]);
+      dg[e] = pack_bf16_pair(mul2(mul2(dd, bf16x2_pair(uw[e])), grad));
+      du[e] = pack_bf16_pair(mul2(dd, act));
     }
-    store8(dh + r * 2 * S + c, dg);
-    store8(dh + r * 2 * S + S + c, du);
+    *reinterpret_cast<uint4*>(dh + r * 2 * S + c) = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+    *reinterpret_cast<uint4*>(dh + r * 2 * S + S + c) = make_uint4(du[0], du[1], du[2], du[3]);
   }
 }
 }  // namespace ssm
+static int glu_blocks(long long rows, int S) {
+  const long long blocks = (rows * (S / 8) + 255) / 256;
+  return (int)(blocks < 148 * 16 ? blocks : 148 * 16);
+}
 extern "C" int ssm_glu_fwd(const void* h, long long ld, void* out, long long rows, int S, int act, cudaStream_t st) {
   if (S % 8 || ld % 8 || rows < 1 || act < 0 || act > 1) return -SSM_ERR_BAD_ARG;
-  const long long total = rows * (S / 8);
-  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  glu_fwd_kernel<<<blocks, 256, 0, st>>>(BF(h), ld, BFM(out), rows, S, act);
+  auto kern = act == 0 ? glu_fwd_kernel<0> : glu_fwd_kernel<1>;
+  kern<<<glu_blocks(rows, S), 256, 0, st>>>(BF(h), ld, BFM(out), rows, S);
   return (int)cudaGetLastError();
 }
 extern "C" int ssm_glu_bwd(const void* h, long long ld, const void* dout, void* dh, long long rows, int S, int act,
                            cudaStream_t st) {
   if (S % 8 || ld % 8 || rows < 1 || act < 0 || act > 1) return -SSM_ERR_BAD_ARG;
-  const long long total = rows * (S / 8);
-  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  glu_bwd_kernel<<<blocks, 256, 0, st>>>(BF(h), ld, BF(dout), BFM(dh), rows, S, act);
+  auto kern = act == 0 ? glu_bwd_kernel<0> : glu_bwd_kernel<1>;
+  kern<<<glu_blocks(rows, S), 256, 0, st>>>(BF(h), ld, BF(dout), BFM(dh), rows, S);
   return (int)cudaGetLastError();
 }
 

@@ -89,3 +89,39 @@ def test_conv_and_step_sizes_in_one_launch(B, L, C, H, fp32):
     # exponential and logarithm to a few ulp, sums of 128 in chains of 5 and 3
     assert torch.allclose(dt.double(), want, rtol=1e-5, atol=1e-6) and torch.allclose(l.double(), sums, rtol=2e-5, atol=1e-5)
     assert torch.allclose(params[0].double(), A, rtol=1e-6) and torch.equal(params[1], D.float()) and torch.equal(params[2], dt_bias.float())
+
+
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+@pytest.mark.parametrize("rows,S", [(1, 8), (3, 2056), (2371, 16)])          # one vector, a second column block, more rows than blocks
+def test_gated_linear_unit(rows, S, act):
+    from state_space_models_neuron_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(rows + S)
+    h = (torch.randn(rows, 2 * S, device="cuda", generator=gen) * 3).bfloat16().requires_grad_()
+    dout = torch.randn(rows, S, device="cuda", generator=gen).bfloat16()
+    H = h.detach().double().requires_grad_()
+    f = torch.nn.functional.gelu if act == "gelu" else torch.nn.functional.silu
+    out, ref = ops.glu(h, act), f(H[:, :S]) * H[:, S:]
+    _near(out, ref)
+    out.backward(dout)
+    ref.backward(dout.double())
+    _near(h.grad, H.grad)
+
+
+def test_gelu_of_every_bf16_value():
+    """All 65,536 values: below zero GELU is its Gaussian tail, where the result must not lose digits to 1 + erf."""
+    from state_space_models_neuron_b200 import ops
+    x = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16).requires_grad_()
+    X = x.detach().double()
+    y, cdf = ops.gelu(x), torch.special.erfc(-X / 2 ** 0.5) / 2
+    Y = X * cdf
+    d, = torch.autograd.grad(y, x, torch.ones_like(y))
+    D = cdf + X * torch.exp(-X.square() / 2) * 0.3989422804014327
+    ok = X.abs() < 12                                       # beyond: 0 or x, and a tail below what fp32 holds
+    # half a step of 8 significant bits, and 2^-16 of the arithmetic (an argument of the exponential up to 104, rounded twice to
+    # 2^-24 of itself)
+    assert ((y.double() - Y).abs() <= (2.0 ** -8 + 2.0 ** -16) * Y.abs() + 1e-36)[ok].all()
+    assert ((d.double() - D).abs() <= (2.0 ** -8 + 2.0 ** -16) * D.abs() + 2.0 ** -22)[ok].all()     # terms of the gradient cancel near -0.75
+    big = (X.abs() >= 12) & X.isfinite()
+    up, down = big & (X > 0), big & (X < 0)                 # x and 1; the rest of the tail, 12 phi(12) = 2^-102 at most
+    assert torch.equal(y[up].double(), X[up]) and (d[up] == 1).all() and (y[down].abs() < 2.0 ** -101).all() and (d[down].abs() < 2.0 ** -97).all()
+    assert y[X.isnan()].isnan().all() and y[X == float("inf")].item() == float("inf")
