@@ -239,6 +239,8 @@ def wgrad_to_main_grad(dy2: torch.Tensor, x2: torch.Tensor, w) -> bool:
         return False
     stale = getattr(w, "grad_stale", False)
     acc = getattr(w, "norm_acc", None) if stale else None
+    if acc is not None and getattr(w, "scatter_added", False) and not _follow_norm(dy2.shape[0], w.shape[0]):
+        acc = None
     if not stale:
         untrack_norm(w)
     gemm(dy2, x2, a_mn=True, b_mn=True, out=mg, accumulate=not stale, sumsq=acc)
@@ -246,6 +248,14 @@ def wgrad_to_main_grad(dy2: torch.Tensor, x2: torch.Tensor, w) -> bool:
     if acc is not None:
         w.norm_tracked = True
     return True
+
+
+def _follow_norm(tokens: int, rows: int) -> bool:
+    """Whether the additions of an embedding's gradient carry the gradient norm on (ssm_embed_bwd with an accumulator), or the norm
+    of its rows is taken by a pass over all of them.  Following costs a third to double of the additions, the pass 4 bytes per
+    value of the table (us, additions with and without, pass: 2048 tokens of 4096 into 50288 rows 25, 13, 126; 8192 of 2560 83, 39, 79;
+    8192 of 1024 42, 14, 31; 2048 of 4096 into 6286 rows 31, 12, 16): they meet at about six rows per token."""
+    return tokens * 6 <= rows
 
 
 def untrack_norm(w) -> None:
@@ -530,17 +540,23 @@ def glu(h, act: str = "silu"):
 # ======================================================================================
 # embedding
 # ======================================================================================
-def embed_grad_target(w):
-    """(fp32 [V, D] buffer to accumulate into, direct).  With an optimizer-owned `main_grad` the embedding backward
-    adds into it in place (after the tied LM-head wgrad, which ran earlier in the backward pass)."""
+def embed_grad_target(w, follow_norm: bool = False, tokens: int = 0):
+    """(fp32 [V, D] buffer to accumulate into, direct, norm accumulator or None).  With an optimizer-owned `main_grad` the embedding
+    backward adds into it in place (after the tied LM-head wgrad, which ran earlier in the backward pass).  follow_norm: the
+    additions may go on with a gradient norm that the accumulator already holds (zeros, or what a GEMM stored and added);
+    otherwise they make it stale."""
     mg = getattr(w, "main_grad", None)
     if mg is not None and mg.dtype == torch.float32 and mg.is_contiguous():
+        acc = getattr(w, "norm_acc", None) if follow_norm and not getattr(w, "norm_dirty", False) else None
         if getattr(w, "grad_stale", False):
             mg.zero_()
             w.grad_stale = False
-        untrack_norm(w)                 # scatter-added rows change the norm of a gradient a GEMM may have stored
-        return mg, True
-    return torch.zeros(w.shape, dtype=torch.float32, device=w.device), False
+            w.norm_tracked = acc is not None and _follow_norm(tokens, w.shape[0])
+        if acc is None or not getattr(w, "norm_tracked", False):
+            untrack_norm(w)             # scatter-added rows change the norm of a gradient a GEMM may have stored
+            acc = None
+        return mg, True, acc
+    return torch.zeros(w.shape, dtype=torch.float32, device=w.device), False, None
 
 
 class _Embedding(torch.autograd.Function):
@@ -561,10 +577,10 @@ class _Embedding(torch.autograd.Function):
         g2 = g.reshape(-1, D)
         if g2.stride(1) != 1 or g2.stride(0) % 4:
             g2 = g2.contiguous()
-        tgt, direct = embed_grad_target(w)
+        tgt, direct, acc = embed_grad_target(w, follow_norm=True, tokens=ids.numel())
         n = ids.numel()
         _run("ssm_embed_bwd", _P(ids), _P(g2), _ll(g2.stride(0)), _P(tgt), _ll(ctx.vocab_start), _ll(w.shape[0]), 1, n, n,
-             D, 1, None, 0, 0, None, _P(status_tensor(w.device)), _st())
+             D, 1, None, 0, 0, None, _P(acc), _P(status_tensor(w.device)), _st())
         return None, (None if direct else tgt.to(w.dtype)), None
 
 

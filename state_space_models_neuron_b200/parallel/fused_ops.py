@@ -212,10 +212,10 @@ class _VocabEmbedScatter(torch.autograd.Function):
         _run("ssm_push_shard", _P(g2), _ll(g2.stride(0)), ws.peer_ptrs(off), _ll(D), _ll(ws.me * B * Ls), B * Ls, D, T,
              ws.me, ws.flag_ptr_array, base, seq, _P(ws.seq_base), _c.c_void_p(ws.counter_ptr(33)),
              min(148, max(1, B * Ls * D // 8 // 256)), _st())
-        tgt, direct = cuda_ops.embed_grad_target(w)
+        tgt, direct, _ = cuda_ops.embed_grad_target(w)
         _run("ssm_embed_bwd", _P(ids), _P(ws.local_view(off, B * L, D)), _ll(D), _P(tgt), _ll(ctx.vocab_start),
              _ll(w.shape[0]), B, L, Ls, D, T, _c.c_void_p(ws.base_ptrs[ws.me]), base, seq, _P(ws.seq_base),
-             _P(status_tensor(ws.device)), _st())
+             _P(None), _P(status_tensor(ws.device)), _st())
         return None, (None if direct else tgt.to(w.dtype)), None, None
 
 

@@ -355,9 +355,10 @@ class ParallelEmbedding(nn.Module):
         (init_method or normal_init(1.0))(full, generator=gen)
         self.weight = nn.Parameter(full[self.vocab_start:self.vocab_end].to(dtype).contiguous())
         _mark(self.weight, 0)
-        # the embedding gradient is scatter-added (and, when tied, lands on top of the LM head's): its share of the
-        # gradient norm is always taken from the buffer, never from a GEMM epilogue
-        self.weight.no_norm_tracking = True
+        # the embedding gradient is scatter-added (and, when tied, lands on top of the LM head's): on one rank the kernel that
+        # adds it carries the norm on; between ranks its share of the norm is taken from the buffer, never from a GEMM epilogue
+        self.weight.no_norm_tracking = tp > 1
+        self.weight.scatter_added = True
 
     def forward(self, ids: torch.Tensor, scatter_to_sequence_parallel: bool = False) -> torch.Tensor:
         tp = ps.get_tensor_model_parallel_size()
