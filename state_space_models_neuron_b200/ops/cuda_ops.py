@@ -633,6 +633,19 @@ def widen(x):
     return out
 
 
+def row_max(x):
+    """(largest value, its first index) of every row of fp32 x [..., V]; NaN counts as largest."""
+    V = x.shape[-1]
+    rows = x.numel() // V if V else 0
+    x2 = x.reshape(-1, V) if x.dim() != 2 and rows else x
+    if x.dtype != torch.float32 or rows == 0 or rows > 65535 or x2.stride(1) != 1 or V >= 2 ** 31 - 2 ** 16 or _observed():
+        return x.float().max(dim=-1)
+    val = torch.empty(x.shape[:-1], dtype=torch.float32, device=x.device)
+    idx = torch.empty(x.shape[:-1], dtype=torch.int64, device=x.device)
+    _run("ssm_row_max", _p(x2), _ll(x2.stride(0)), V, _ll(rows), _p(val), _p(idx), _st())
+    return val, idx
+
+
 # ======================================================================================
 # optimizer
 # ======================================================================================

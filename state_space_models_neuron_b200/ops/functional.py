@@ -242,6 +242,13 @@ def widen(x):
     return x.float()
 
 
+def row_max(x):
+    """(largest value, its index) over the last dimension, in fp32."""
+    if _native(x):
+        return _cuda().row_max(x)
+    return x.float().max(dim=-1)
+
+
 def ce_backward(logits, labels, row_max, row_sum, grad_rows, vocab_start: int, ignore_index: int):
     """d loss / d logits for the local vocab shard: (softmax - onehot) * grad_rows."""
     if _native(logits):

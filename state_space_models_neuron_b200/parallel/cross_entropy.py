@@ -67,7 +67,7 @@ def parallel_argmax(logits: torch.Tensor) -> torch.Tensor:
     ties), identical on every TP rank.  Two tiny all-reduces (max of the values, then max of the negated
     candidate index), through the fused small all-reduce when it is available."""
     tp, r = ps.get_tensor_model_parallel_size(), ps.get_tensor_model_parallel_rank()
-    val, idx = logits.float().max(dim=-1)
+    val, idx = ops.row_max(logits)
     if tp == 1:
         return idx
     from . import fused

@@ -107,3 +107,23 @@ def test_statistics_at_the_edges_of_a_column_block(N):
     # exponentials within 2 ulp and an argument below 2^7 rounded to 2^-24 of itself; sums of at most 1001 positive terms in
     # chains of at most 16 per block and 16 blocks
     assert torch.allclose(s.double(), (ref - ref.max(1, keepdim=True).values).exp().sum(1), rtol=2 ** -17 + 40 * 2 ** -24)
+
+
+@pytest.mark.parametrize("V", [1, 3, 255, 2048, 8195, 50288])
+@pytest.mark.parametrize("pad", [0, 4, 1])                   # rows on 16-byte boundaries, with a gap, and not on them
+def test_row_maximum(V, pad):
+    from state_space_models_neuron_b200.ops import cuda_ops
+    gen = torch.Generator(device="cuda").manual_seed(V + pad)
+    x = torch.randn(9, V + pad, device="cuda", generator=gen)[:, :V].clone(memory_format=torch.preserve_format) if pad == 0 else \
+        torch.randn(9, V + pad, device="cuda", generator=gen)[:, :V]
+    x[1] = float("-inf")
+    x[2], x[2, V // 2:] = 1.0, 2.0                            # equal values: the first index
+    x[3], x[3, V - 1] = -3.0, -2.0                            # all negative, the last one
+    x[4], x[4, V // 3] = 0.0, -0.0                            # zeros of both signs are equal
+    x[5, V // 4], x[5, V // 2] = float("nan"), float("nan")
+    x[6, V - 1] = float("inf")
+    val, idx = cuda_ops.row_max(x)
+    want = x.cpu().max(dim=1)
+    assert torch.equal(idx.cpu(), want.indices) and torch.equal(val.cpu().nan_to_num(7.0), want.values.nan_to_num(7.0))
+    v3, i3 = cuda_ops.row_max(x.reshape(3, 3, V))
+    assert torch.equal(i3.view(-1), idx) and v3.shape == (3, 3)
