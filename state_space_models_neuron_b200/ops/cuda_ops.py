@@ -619,6 +619,17 @@ def ce_backward(logits, labels, row_max, row_sum, grad_rows, vocab_start, ignore
     return grad
 
 
+def ce_row_loss(m, s, tgt, labels, ignore_index):
+    """log(s) + m - tgt per row, 0 where the label is ignored (fp32 statistics as ce_partials delivers them)."""
+    rows = labels.numel()
+    if (rows == 0 or labels.dtype != torch.int64 or _observed()
+            or not all(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == rows for t in (m, s, tgt))):
+        return torch.where(labels != ignore_index, torch.log(s) + m - tgt, torch.zeros_like(s))
+    loss = torch.empty_like(s)
+    _run("ssm_ce_row_loss", _p(m), _p(s), _p(tgt), _p(labels.contiguous()), _ll(ignore_index), _ll(rows), _p(loss), _st())
+    return loss
+
+
 def widen(x):
     """fp32 copy of bf16 `x` [..., n] (rows may be padded); inference only, the gradient path keeps `x.float()`."""
     if _observed():
@@ -658,6 +669,14 @@ def adamw_step(master, m, v, g, out, clip, lr, b1, b2, eps, wd, step, lr_dev=Non
     _run("ssm_adamw", _p(master), _p(m), _p(v), _p(g), int(g.dtype == torch.float32), _p(out16), _p(out32),
          _ll(master.numel()), _p(clip), _c.c_float(lr), _c.c_float(b1), _c.c_float(b2), _c.c_float(eps),
          _c.c_float(wd), int(step), _p(lr_dev), _p(step_dev), _st())
+
+
+def clip_coefficient(total, max_norm, step, skipped):
+    """(gradient norm, clip coefficient or -1 where it is not finite) as fp32 [1] tensors from the norm's square; counts the step
+    as applied (`step`) or skipped (int32 [1] tensors)."""
+    norm, clip = torch.empty(1, dtype=torch.float32, device=total.device), torch.empty(1, dtype=torch.float32, device=total.device)
+    _run("ssm_clip_coefficient", _p(total), _c.c_float(max_norm), _p(norm), _p(clip), _p(step), _p(skipped), _st())
+    return norm, clip
 
 
 def sumsq_accumulate(g, total):

@@ -242,6 +242,13 @@ def widen(x):
     return x.float()
 
 
+def ce_row_loss(m, s, tgt, labels, ignore_index: int):
+    """Cross entropy of every row from its (max, sum of exponentials, target logit); 0 where the label is ignored."""
+    if _native(s):
+        return _cuda().ce_row_loss(m, s, tgt, labels, ignore_index)
+    return torch.where(labels != ignore_index, torch.log(s) + m - tgt, torch.zeros_like(s))
+
+
 def row_max(x):
     """(largest value, its index) over the last dimension, in fp32."""
     if _native(x):

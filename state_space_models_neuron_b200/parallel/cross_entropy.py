@@ -36,8 +36,7 @@ class _ParallelCrossEntropy(torch.autograd.Function):
             if not fused.small_allreduce(packed.view(-1), "sum"):
                 dist.all_reduce(packed, group=grp)
             s, tgt, m = packed[0], packed[1], gm
-        valid = lb != ignore_index
-        loss = torch.where(valid, torch.log(s) + m - tgt, torch.zeros_like(s))
+        loss = ops.ce_row_loss(m, s, tgt, lb, ignore_index)
         ctx.save_for_backward(lg, lb, m, s)
         ctx.vocab_start, ctx.ignore_index, ctx.shape = vocab_start, ignore_index, shape
         return loss.reshape(shape[:-1])

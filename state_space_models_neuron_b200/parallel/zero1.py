@@ -273,8 +273,7 @@ class Zero1Optimizer(torch.optim.Optimizer):
             flat = [v for sp in spans for v in sp]
             self._norm_ranges[key] = (torch.tensor(flat, dtype=torch.int64, device=self.device), len(spans))
         ranges, n = self._norm_ranges[key]
-        total = self._norm_buf.zero_()
-        total += self._norm_acc
+        total = self._norm_buf.copy_(self._norm_acc)
         if n:
             from ..ops import cuda_ops
             cuda_ops._run("ssm_sumsq_ranges", cuda_ops._P(g), cuda_ops._P(ranges), n, cuda_ops._P(total), cuda_ops._st())
@@ -356,7 +355,13 @@ class Zero1Optimizer(torch.optim.Optimizer):
         if self.max_grad_norm is None:
             self._dev_step.add_(1)
             return torch.ones(1, dtype=torch.float32, device=self.device)
-        norm = torch.sqrt(norm_sq_fn()).reshape(1)
+        total = norm_sq_fn()
+        from ..ops.functional import _native
+        if _native(total) and total.dtype == torch.float32:
+            from ..ops import cuda_ops
+            self.last_grad_norm, clip = cuda_ops.clip_coefficient(total, float(self.max_grad_norm), self._dev_step, self._dev_skipped)
+            return clip
+        norm = torch.sqrt(total).reshape(1)
         self.last_grad_norm = norm
         finite = torch.isfinite(norm)
         clip = torch.where(finite, torch.clamp(self.max_grad_norm / (norm + 1e-6), max=1.0), -torch.ones_like(norm))

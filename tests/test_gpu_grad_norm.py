@@ -32,3 +32,30 @@ def test_norm_follows_the_embedding(tied, ids_below, passes, vocab):
         want = opt.flat_grads.double().square().sum().item()
         # fp32 sums of up to 2^18 squares in trees of threads, warps and blocks
         assert abs(total - want) <= 2e-5 * want
+
+
+@pytest.mark.parametrize("total", [0.0, 1e-20, 0.25, 1.0, 3.7e9, float("inf"), float("nan"), -1.0])
+def test_clip_coefficient_equals_separate_operations(total):
+    from state_space_models_neuron_b200.ops import cuda_ops
+    sq = torch.tensor([total], device="cuda")
+    step, skipped = torch.tensor([5], dtype=torch.int32, device="cuda"), torch.tensor([2], dtype=torch.int32, device="cuda")
+    norm, clip = cuda_ops.clip_coefficient(sq, 0.7, step, skipped)
+    want = torch.sqrt(sq)
+    finite = torch.isfinite(want)
+    assert torch.equal(norm.nan_to_num(9.0, 8.0), want.nan_to_num(9.0, 8.0))
+    assert torch.equal(clip, torch.where(finite, torch.clamp(0.7 / (want + 1e-6), max=1.0), -torch.ones_like(want)))
+    assert (step.item(), skipped.item()) == ((6, 2) if finite else (5, 3))
+
+
+@pytest.mark.parametrize("rows", [1, 256, 257])
+def test_row_loss_equals_separate_operations(rows):
+    from state_space_models_neuron_b200.ops import cuda_ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    m, s, t = (torch.randn(rows, device="cuda", generator=gen) * 9 for _ in range(3))
+    s = s.abs() + 1
+    s[0], m[0] = (0.0, float("-inf")) if rows > 1 else (1.0, 0.0)
+    labels = torch.randint(0, 3, (rows,), device="cuda", generator=gen)
+    loss = cuda_ops.ce_row_loss(m, s, t, labels, 2)
+    want = torch.where(labels != 2, torch.log(s) + m - t, torch.zeros_like(s))
+    # the logarithm may be rounded to the other side: one step of it
+    assert torch.allclose(loss, want, rtol=2.0 ** -23, atol=2.0 ** -23 * 6, equal_nan=True)
