@@ -982,10 +982,12 @@ __global__ void __launch_bounds__(256) mixer_small_grads_kernel(const SmallGradA
   float s = 0.f;
   if (i < n_conv) {
     seg = 0;
+    #pragma unroll 8
     for (int t = tg; t < a.T1; t += CS_GROUPS) s += a.conv_part[(long long)t * n_conv + i];
   } else if (i - n_conv < n_gated) {
     seg = 1;
     i -= n_conv;
+    #pragma unroll 8
     for (int t = tg; t < a.S; t += CS_GROUPS) s += a.gated_part[(long long)t * n_gated + i];
   } else if (i - n_conv - n_gated < n_h) {
     seg = 2;
@@ -1017,8 +1019,10 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ p
   const int tx = threadIdx.x & (CS_COLS - 1), tg = threadIdx.x / CS_COLS;
   const int c = blockIdx.x * CS_COLS + tx;
   float s = 0.f;
-  if (c < n)
+  if (c < n) {
+    #pragma unroll 8
     for (int t = tg; t < S; t += CS_GROUPS) s += part[(long long)t * n + c];
+  }
   s = colsum_groups(s, red);
   if (tg == 0 && c < n) dst[c] = acc ? dst[c] + s : s;
 }

@@ -823,7 +823,7 @@ ssd_walk_scan_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __grid_co
 // dB and dC, 4 under the next head's 1.  Bound by the per-pair arithmetic of 2 and the hand-overs between the steps: with
 // 128-token tiles and four operands per head in shared memory there is room for one head only.
 // TMEM: [0,128) CB then dU_diag | dU_state, [128,256) dM then C S_in, [256,384) dB, [384,512) dC
-// (dB, dC accumulate over the CTA's heads and are added to the fp32 output by bulk reductions).
+// (dB, dC accumulate over the CTA's heads and go to the fp32 output by bulk stores, or reductions where CTAs share a group).
 // =====================================================================================
 struct ScanBwdParams {
   const float* dt; const float* l; const float* D; const float* A; const float* dt_bias;
@@ -1231,7 +1231,8 @@ ssd_chunk_scan_bwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __gr
     ok = all_ok(ok);
     if (tid == 0 && ok) {
       for (int k = 0; k < 8; ++k)
-        tma_add_2d(&tm_dbc, smem + k * TILE64, (k >> 2) * GN + g * NS + (k & 3) * 32, row0);
+        if (splits > 1) tma_add_2d(&tm_dbc, smem + k * TILE64, (k >> 2) * GN + g * NS + (k & 3) * 32, row0);
+        else tma_store_2d(&tm_dbc, smem + k * TILE64, (k >> 2) * GN + g * NS + (k & 3) * 32, row0);
       tma_store_commit();
       tma_store_wait_all();
     }
@@ -1390,7 +1391,7 @@ extern "C" int ssm_ssd_chunk_scan_fwd(const void* xbc, long long xbc_stride, int
 }
 
 // dy: bf16 [B*L, Hv*64] (row stride dy_stride).  dx: bf16 [B*L, Hv*64] written (row stride dx_stride).
-// dBC: fp32 [B*L, 2*G*128], must be zero on entry.  hpart: fp32 [B*nc, Hv, 3].
+// dBC: fp32 [B*L, 2*G*128], written whole.  hpart: fp32 [B*nc, Hv, 3].
 // ddt: if ddt32 != null it receives fp32 [B,Hv,L]; else bf16 values are written to ddt_raw rows.
 extern "C" int ssm_ssd_chunk_scan_bwd(const void* xbc, long long xbc_stride, int xbc_cols, const void* dy,
                                       long long dy_stride, const void* s_in,
@@ -1430,6 +1431,10 @@ extern "C" int ssm_ssd_chunk_scan_bwd(const void* xbc, long long xbc_stride, int
   p.ddt32 = reinterpret_cast<float*>(ddt32);
   p.hpart = reinterpret_cast<float*>(hpart);
   p.L = L; p.H = H; p.Hv = Hv; p.G = G; p.nc = nc; p.d_in = d_in; p.hpc = hpc; p.status = status;
+  if (hpc < hv_per_group) {                            // CTAs of a group add to it
+    const cudaError_t e = cudaMemsetAsync(dBC, 0, (size_t)B * L * 2 * G * NS * sizeof(float), st);
+    if (e != cudaSuccess) return (int)e;
+  }
   dim3 grid(nc, G * (hv_per_group / hpc), B);
   ssd_chunk_scan_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(tx, tdy, ts, tds, tdx, tdbc, p);
   return (int)cudaGetLastError();

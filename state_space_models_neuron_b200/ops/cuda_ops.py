@@ -837,7 +837,7 @@ def _ssd_backward(conv_out, dy2, y2, dt, l, s_in, dt_raw2, dt_raw_stride, A, D, 
     psplit = Hv // H
     ds_out, _ = _chunk_states(conv_out, C, d_inner + G * 128, dy2, dy2.stride(0), dt, l, None, False, B, L, H, Hv, G, 1)
     dx = torch.empty(B * L, d_inner, dtype=torch.bfloat16, device=dev)
-    dBC = torch.zeros(B * L, 2 * G * 128, dtype=torch.float32, device=dev)
+    dBC = torch.empty(B * L, 2 * G * 128, dtype=torch.float32, device=dev)
     hpart = torch.empty(B * nc, Hv, 3, dtype=torch.float32, device=dev)
     ddt32 = torch.empty(B, Hv, L, dtype=torch.float32, device=dev) if psplit > 1 else None
     hpc = _pick_hpc(Hv // G, nc * G * B)
