@@ -293,11 +293,11 @@ conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long xs, const 
 // one block per (row, group); thread handles vectors v = tid, tid + blockDim, ... of 8 elements
 // =====================================================================================
 // MAXV = 16-byte vectors per thread (norm_threads picks it).  All four norm kernels are bound by moving their rows once;
-// what a block waits for is one round of loads and the block-wide sums.  The backward kernels therefore keep the raw rows
-// in registers instead of reading them a second time, fetch the next row before they reduce the present one, and reduce
+// what a block waits for is one round of loads and the block-wide sums.  The add backward kernel therefore keeps the raw rows
+// in registers instead of reading them a second time, fetches the next row before it reduces the present one, and reduces
 // both sums of a row together behind one barrier.
 // Measured (us, before -> now): gated forward 32768 x 5120 318 -> 143, 2048 x 8192 24.8 -> 16.8; add forward 32768 x 2560
-// 118 -> 94; gated backward 4608 x 1536 38.2 -> 31.1, 2048 x 8192 65.7 -> 62.1; add backward 4608 x 768 25.5 -> 14.3.
+// 118 -> 94; add backward 4608 x 768 25.5 -> 14.3.
 // The forward kernels also fetch the weights in front of the sum, since ordinary loads behind pdl_wait() are not moved there
 // by the compiler (130M, one sequence, 49 norms and gates per token: 467 -> 433 us with all weights fetched there).
 
@@ -386,79 +386,114 @@ gated_rmsnorm_fwd_kernel(const __nv_bfloat16* y, long long ys, const __nv_bfloat
 
 // grid (row_slices, groups); each block walks rows r = blockIdx.x, blockIdx.x + gridDim.x, ...; one vector per thread.
 // dwpart [gridDim.x, d] fp32 partial sums of dout * h * rstd.
-__global__ void __launch_bounds__(1024)
-gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ y, long long ys, const __nv_bfloat16* __restrict__ z,
-                         long long zs, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dout,
-                         long long dos, __nv_bfloat16* __restrict__ dy, long long dys, __nv_bfloat16* __restrict__ dz,
-                         long long dzs, float* __restrict__ dwpart, long long rows, int d, int gs, float eps) {
+// Bound by moving five rows per row.  Rows of y, z and dout come by bulk copies into a ring in shared memory, where both passes
+// over a row read them: held in registers (with the next row's), they left room for one block per SM, which waited for its
+// loads and its barrier in turn.  Arithmetic in pairs; the sigmoids of the first pass stay in registers for the second.
+// us, before -> now: 8192 x 5120 146 -> 93, 4096 x 8192 104 -> 76, 2048 x 8192 58 -> 38, 4608 x 1536 26 -> 20 (64, 51, 26, 11 at copy
+// bandwidth)
+constexpr int GATED_RING_MAX = 4;
+template <bool GATE, int THREADS, int PER_SM>
+__global__ void __launch_bounds__(THREADS, PER_SM)
+gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ y, long long ys, const __nv_bfloat16* __restrict__ z, long long zs,
+                         const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dout, long long dos,
+                         __nv_bfloat16* __restrict__ dy, long long dys, __nv_bfloat16* __restrict__ dz, long long dzs,
+                         float* __restrict__ dwpart, long long rows, int d, int gs, float eps, int ring, int* __restrict__ status) {
+  extern __shared__ __align__(128) uint8_t stages[];       // [ring] y | dout | z rows of this group
   __shared__ float2 red[64];
+  __shared__ uint64_t full[GATED_RING_MAX];
+  const uint32_t bytes = (uint32_t)gs * 2, stage_bytes = (GATE ? 3 : 2) * bytes;
   const bool mine = (int)threadIdx.x < gs / 8;
-  const long long c = (long long)blockIdx.y * gs + (mine ? threadIdx.x * 8 : 0);      // first column of this thread
-  const uint4 none = make_uint4(0, 0, 0, 0);
-  uint4 yn = none, zn = none, gn = none;
-  auto fetch = [&](long long row) {
-    if (mine && row < rows) {
-      yn = load_raw8(y + row * ys + c);
-      gn = load_raw8(dout + row * dos + c);
-      if (z) zn = load_raw8(z + row * zs + c);
-    }
+  const long long c0 = (long long)blockIdx.y * gs, c = c0 + (mine ? threadIdx.x * 8 : 0);      // first column of group, of thread
+  auto load = [&](long long row, int stage) {
+    uint8_t* at = stages + stage * stage_bytes;
+    mbar_expect_tx(&full[stage], stage_bytes);
+    bulk_load(at, y + row * ys + c0, bytes, &full[stage]);
+    bulk_load(at + bytes, dout + row * dos + c0, bytes, &full[stage]);
+    if (GATE) bulk_load(at + 2 * bytes, z + row * zs + c0, bytes, &full[stage]);
   };
-  float dwacc[8];
-  #pragma unroll
-  for (int e = 0; e < 8; ++e) dwacc[e] = 0.f;
-  fetch(blockIdx.x);
-  int turn = 0;
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < ring; ++k) mbar_init(&full[k], 1);
+    mbar_fence_init();
+    for (int k = 0; k < ring; ++k)
+      if (blockIdx.x + (long long)k * gridDim.x < rows) load(blockIdx.x + (long long)k * gridDim.x, k);
+  }
+  uint4 wq = make_uint4(0, 0, 0, 0);
+  if (mine) wq = load_raw8(w + c);
+  const uint32_t wr[4] = {wq.x, wq.y, wq.z, wq.w};
+  uint64_t dw[4] = {0, 0, 0, 0};
+  __syncthreads();
+  int turn = 0, stage = 0;
+  uint32_t phase = 0;
+  bool ok = true;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x, ++turn) {
-    const uint4 yq = yn, zq = zn, gq = gn;
-    fetch(row + gridDim.x);
-    float ss = 0.f, dot = 0.f;
+    ok = mbar_wait(&full[stage], phase, ok ? status : nullptr) && ok;     // also behind a failure: copies land before the block goes
+    const uint4* at = reinterpret_cast<const uint4*>(stages + stage * stage_bytes) + threadIdx.x;
+    uint64_t sg[4];
+    float2 t = make_float2(0.f, 0.f);
     if (mine) {
-      float a[8], go[8], ww[8];
-      unpack8(yq, a);
-      unpack8(gq, go);
-      load8(w + c, ww);
-      if (z) {
-        float zz[8];
-        unpack8(zq, zz);
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] *= silu_f(zz[e]);
-      }
+      const uint4 yq = at[0], gq = at[bytes / 16];
+      uint4 zq = make_uint4(0, 0, 0, 0);
+      if (GATE) zq = at[2 * (bytes / 16)];
+      const uint32_t yr[4] = {yq.x, yq.y, yq.z, yq.w}, gr[4] = {gq.x, gq.y, gq.z, gq.w}, zr[4] = {zq.x, zq.y, zq.z, zq.w};
+      uint64_t ss = 0, dot = 0;
       #pragma unroll
-      for (int e = 0; e < 8; ++e) { ss += a[e] * a[e]; dot += go[e] * ww[e] * a[e]; }
+      for (int e = 0; e < 4; ++e) {
+        uint64_t h = bf16x2_pair(yr[e]);
+        if (GATE) {
+          const uint64_t zz = bf16x2_pair(zr[e]);
+          sg[e] = sigmoid2(zz);
+          h = mul2(h, mul2(zz, sg[e]));
+        }
+        ss = fma2(h, h, ss);
+        dot = fma2(mul2(bf16x2_pair(gr[e]), bf16x2_pair(wr[e])), h, dot);
+      }
+      float a, b;
+      unpack2(ss, a, b);
+      t.x = a + b;
+      unpack2(dot, a, b);
+      t.y = a + b;
     }
-    const float2 t = block_sum2(ss, dot, red, turn);
+    t = block_sum2(t.x, t.y, red, turn);
+    if (threadIdx.x == 0 && turn > 0) {                     // everybody is past the stage of the row before
+      const long long next = row + (long long)(ring - 1) * gridDim.x;
+      if (next < rows) load(next, stage == 0 ? ring - 1 : stage - 1);
+    }
     const float rstd = rsqrtf(t.x / gs + eps);
     const float mdot = t.y * rstd / gs;                     // mean(dn * n), n = h * rstd
-    if (mine) {
-      float yy[8], go[8], ww[8], oy[8];
-      unpack8(yq, yy);
-      unpack8(gq, go);
-      load8(w + c, ww);
-      if (z) {
-        float zz[8], oz[8];
-        unpack8(zq, zz);
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float s = sigmoid_f(zz[e]), gate = zz[e] * s;
-          const float n = yy[e] * gate * rstd;
-          const float dh = rstd * (go[e] * ww[e] - n * mdot);
-          oy[e] = dh * gate;
-          oz[e] = dh * yy[e] * s * (1.f + zz[e] * (1.f - s));
-          dwacc[e] += go[e] * n;
-        }
-        store8(dz + row * dzs + c, oz);
-      } else {
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float n = yy[e] * rstd;
-          oy[e] = rstd * (go[e] * ww[e] - n * mdot);
-          dwacc[e] += go[e] * n;
+    if (mine && ok) {
+      const uint4 yq = at[0], gq = at[bytes / 16];
+      uint4 zq = make_uint4(0, 0, 0, 0);
+      if (GATE) zq = at[2 * (bytes / 16)];
+      const uint32_t yr[4] = {yq.x, yq.y, yq.z, yq.w}, gr[4] = {gq.x, gq.y, gq.z, gq.w}, zr[4] = {zq.x, zq.y, zq.z, zq.w};
+      const uint64_t r2 = pack2(rstd, rstd), m2 = pack2(-mdot, -mdot), one = pack2(1.f, 1.f), minus = pack2(-1.f, -1.f);
+      uint32_t oy[4], oz[4];
+      #pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint64_t yy = bf16x2_pair(yr[e]), g = bf16x2_pair(gr[e]);
+        if (GATE) {
+          const uint64_t zz = bf16x2_pair(zr[e]), gate = mul2(zz, sg[e]);
+          const uint64_t n = mul2(mul2(yy, gate), r2);
+          const uint64_t dh = mul2(r2, fma2(n, m2, mul2(g, bf16x2_pair(wr[e]))));
+          oy[e] = pack_bf16_pair(mul2(dh, gate));
+          oz[e] = pack_bf16_pair(mul2(mul2(dh, yy), mul2(sg[e], fma2(zz, fma2(sg[e], minus, one), one))));
+          dw[e] = fma2(g, n, dw[e]);
+        } else {
+          const uint64_t n = mul2(yy, r2);
+          oy[e] = pack_bf16_pair(mul2(r2, fma2(n, m2, mul2(g, bf16x2_pair(wr[e])))));
+          dw[e] = fma2(g, n, dw[e]);
         }
       }
-      store8(dy + row * dys + c, oy);
+      *reinterpret_cast<uint4*>(dy + row * dys + c) = make_uint4(oy[0], oy[1], oy[2], oy[3]);
+      if (GATE) *reinterpret_cast<uint4*>(dz + row * dzs + c) = make_uint4(oz[0], oz[1], oz[2], oz[3]);
     }
+    if (++stage == ring) { stage = 0; phase ^= 1; }
   }
-  if (mine) store8f(dwpart + (long long)blockIdx.x * d + c, dwacc);
+  if (mine) {
+    float f[8];
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) unpack2(dw[e], f[2 * e], f[2 * e + 1]);
+    store8f(dwpart + (long long)blockIdx.x * d + c, f);
+  }
 }
 
 // =====================================================================================
@@ -1130,18 +1165,39 @@ extern "C" int ssm_gated_rmsnorm_roll(const void* y, long long ys, const void* z
                                       long long xs, int c0, int C, cudaStream_t st) {
   return gated_fwd<true>(y, ys, z, zs, w, out, os, rows, d, gs, eps, WindowRoll{BFM(window), BF(x), xs, c0, C}, st);
 }
+template <bool GATE, int THREADS, int PER_SM>
+static int launch_gated_bwd(dim3 grid, int t, int gs, cudaStream_t st, const void* y, long long ys, const void* z, long long zs, const void* w,
+                            const void* dout, long long dos, void* dy, long long dys, void* dz, long long dzs, void* dwpart, long long rows,
+                            int d, float eps, int* status) {
+  auto kern = gated_rmsnorm_bwd_kernel<GATE, THREADS, PER_SM>;
+  // as many rows ahead as fit beside the other block of the SM
+  const int stage = (GATE ? 6 : 4) * gs, room = (PER_SM == 1 ? 200 : 100) * 1024;
+  const int ring = room / stage < GATED_RING_MAX ? room / stage : GATED_RING_MAX;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  kern<<<grid, t, ring * stage, st>>>(BF(y), ys, BF(z), zs, BF(w), BF(dout), dos, BFM(dy), dys, BFM(dz), dzs,
+                                      reinterpret_cast<float*>(dwpart), rows, d, gs, eps, ring, status);
+  return (int)cudaGetLastError();
+}
 // dwpart must hold row_slices * d floats.
 extern "C" int ssm_gated_rmsnorm_bwd(const void* y, long long ys, const void* z, long long zs, const void* w,
                                      const void* dout, long long dos, void* dy, long long dys, void* dz, long long dzs,
-                                     void* dwpart, int row_slices, long long rows, int d, int gs, float eps,
+                                     void* dwpart, int row_slices, long long rows, int d, int gs, float eps, int* status,
                                      cudaStream_t st) {
   int mv = 1;
   const int t = norm_threads(gs, &mv, true);
-  if (gs % 8 || d % gs || t < 0 || ys % 8 || zs % 8 || dos % 8 || dys % 8 || dzs % 8) return -SSM_ERR_BAD_ARG;
+  if (gs % 8 || d % gs || t < 0 || ys % 8 || zs % 8 || dos % 8 || dys % 8 || dzs % 8 ||
+      ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(dout)) & 15))
+    return -SSM_ERR_BAD_ARG;
   dim3 grid(row_slices, d / gs);
-  gated_rmsnorm_bwd_kernel<<<grid, t, 0, st>>>(BF(y), ys, BF(z), zs, BF(w), BF(dout), dos, BFM(dy), dys, BFM(dz), dzs,
-                                               reinterpret_cast<float*>(dwpart), rows, d, gs, eps);
-  return (int)cudaGetLastError();
+  #define GATED_BWD(GATE, THREADS, PER_SM) launch_gated_bwd<GATE, THREADS, PER_SM>(grid, t, gs, st, y, ys, z, zs, w, dout, dos, dy, dys, dz, dzs, dwpart, rows, d, eps, status)
+  if (z != nullptr) return t <= 640 ? GATED_BWD(true, 640, 2) : GATED_BWD(true, 1024, 1);
+  return t <= 640 ? GATED_BWD(false, 640, 2) : GATED_BWD(false, 1024, 1);
+  #undef GATED_BWD
 }
 
 extern "C" int ssm_add_rmsnorm_fwd(const void* x, const void* res, const void* w, void* out, void* res_out,

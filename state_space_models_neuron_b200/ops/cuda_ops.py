@@ -387,11 +387,14 @@ def _gated_fwd(y2, z2, w, eps, gs, out=None):
 
 def _gated_bwd(y2, z2, w, dout2, eps, gs, dy_out, dz_out, raw=False):
     rows, d = y2.shape
-    slices = int(min(rows, _ROW_SLICES))
+    # one block per SM of the widest groups, two, or four of narrow rows (us with 148 / 296 / 592 slices, column sums included:
+    # 2048 x 8192 43 / 52 / 61, 8192 x 5120 121 / 99 / 103, 2688 x 3072 35 / 28 / 32, 8192 x 2048 88 / 57 / 47, 4608 x 1536 42 / 31 / 25)
+    slices = int(min(rows, _ROW_SLICES // 2 if gs > 5120 else _ROW_SLICES if d >= 2560 else _ROW_SLICES * 2))
     part = torch.empty(slices, d, dtype=torch.float32, device=y2.device)
     _run("ssm_gated_rmsnorm_bwd", _p(y2), _ll(y2.stride(0)), _p(z2), _ll(z2.stride(0) if z2 is not None else 0), _p(w),
          _p(dout2), _ll(dout2.stride(0)), _p(dy_out), _ll(dy_out.stride(0)), _p(dz_out),
-         _ll(dz_out.stride(0) if dz_out is not None else 0), _p(part), slices, _ll(rows), d, gs, _c.c_float(eps), _st())
+         _ll(dz_out.stride(0) if dz_out is not None else 0), _p(part), slices, _ll(rows), d, gs, _c.c_float(eps),
+         _p(status_tensor(y2.device)), _st())
     return part if raw else part.sum(0)
 
 
