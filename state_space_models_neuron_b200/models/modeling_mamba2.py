@@ -72,9 +72,9 @@ class Mamba2Block(nn.Module):
 
     def _in_one_call(self, op, method: str, hidden_states, residual, residual_dtype, conv_state, ssm_state):
         """`op`, one native call that stands for `method` of the mixer and what surrounds it, where the block is made of the
-        plain modules on one rank.  None where any is of another class, has a hook or a method set on it, or out_proj has a bias:
-        these keep the calls one by one.  (The modules' own dictionaries: attribute lookups of a module cost the host more than
-        the launches.)"""
+        plain modules on one rank.  None where any is of another class, has a hook or a method set on it, holds a weight that is no
+        parameter of its own (parametrised, pruned), or out_proj has a bias: these keep the calls one by one.  (The modules' own
+        dictionaries: attribute lookups of a module cost the host more than the launches.)"""
         norm, m = self._modules["norm"], self._modules["mixer"]
         if type(m) is not Mamba2Mixer or type(norm) is not Mamba2RMSNorm:
             return None
@@ -83,11 +83,15 @@ class Mamba2Block(nn.Module):
         if (method in vars(m) or "forward_add" in vars(norm) or (method == "forward" and _hooked(m)) or _has_any_global_hook()
                 or type(gate) is not MambaRMSNormGated or type(first) is not ColumnParallelLinear or type(last) is not RowParallelLinear
                 or "forward" in vars(first) or "forward" in vars(last) or _hooked(first) or _hooked(last)
-                or last._parameters["bias"] is not None or ps.get_tensor_model_parallel_size() != 1):
+                or last._parameters.get("bias", last) is not None or ps.get_tensor_model_parallel_size() != 1):
             return None
-        return op(hidden_states, residual, residual_dtype, conv_state, ssm_state, norm._parameters["weight"], norm.variance_epsilon,
-                  first._parameters["weight"], first._parameters["bias"], conv["weight"], conv["bias"], own["dt_bias"], own["A_log"],
-                  own["D"], gate._parameters["weight"], last._parameters["weight"], m.intermediate_size_tp, m.n_groups_tp,
+        try:
+            weights = (norm._parameters["weight"], norm.variance_epsilon, first._parameters["weight"], first._parameters["bias"],
+                       conv["weight"], conv["bias"], own["dt_bias"], own["A_log"], own["D"], gate._parameters["weight"],
+                       last._parameters["weight"])
+        except KeyError:
+            return None
+        return op(hidden_states, residual, residual_dtype, conv_state, ssm_state, *weights, m.intermediate_size_tp, m.n_groups_tp,
                   m.ssm_state_size, m.head_dim, m.layer_norm_epsilon, gate.group_size)
 
     def forward(self, hidden_states, residual=None, cache_params=None):

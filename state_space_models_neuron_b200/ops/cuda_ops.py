@@ -625,7 +625,7 @@ def ce_backward(logits, labels, row_max, row_sum, grad_rows, vocab_start, ignore
 def ce_row_loss(m, s, tgt, labels, ignore_index):
     """log(s) + m - tgt per row, 0 where the label is ignored (fp32 statistics as ce_partials delivers them)."""
     rows = labels.numel()
-    if (rows == 0 or labels.dtype != torch.int64 or _observed()
+    if (rows == 0 or labels.dtype != torch.int64 or labels.device != s.device or _observed()
             or not all(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == rows for t in (m, s, tgt))):
         return torch.where(labels != ignore_index, torch.log(s) + m - tgt, torch.zeros_like(s))
     loss = torch.empty_like(s)
@@ -1092,15 +1092,17 @@ def ssm_decode_step(zxBCdt, conv_state, ssm_state, conv_w, conv_b, dt_bias, A_lo
     return _gated_fwd(y, zxBCdt[:, :d_inner], norm_w, eps, gs)
 
 
-def _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D, gate_w, out_w):
+def _block_weights(dev, width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D, gate_w,
+                   out_w):
     """Addresses of a block's weights and the mask of its bf16 per-head parameters, or None where one of them is not as the
-    kernels read it."""
+    kernels read it, or not on the GPU of this index."""
     C, H, bf16 = d_inner + 2 * n_groups * d_state, d_inner // head_dim, torch.bfloat16
     W = d_inner + C + H
     mask = _head_param_mask(A_log, D, dt_bias, H)
     given = [t for t in (norm_w, in_w, conv_w, gate_w, out_w, in_b, conv_b) if t is not None]
     if (mask is None or H % n_groups or width % 8 or d_inner % 8 or d_inner % gs or gs % 8 or max(width, gs) > 8192
-            or any(t.dtype is not bf16 or not t.is_contiguous() for t in given)
+            or any(t.dtype is not bf16 or not t.is_contiguous() or t.get_device() != dev for t in given)
+            or A_log.get_device() != dev or D.get_device() != dev or dt_bias.get_device() != dev
             or in_w.shape != (W, width) or out_w.shape != (width, d_inner) or norm_w.numel() != width or gate_w.numel() != d_inner
             or conv_w.numel() != 4 * C or (in_b is not None and in_b.numel() != W) or (conv_b is not None and conv_b.numel() != C)):
         return None
@@ -1115,16 +1117,19 @@ def _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w
 def _block_rows(hidden, residual, rd):
     """Addresses of a block's input rows, or None where they are not as the kernels read them."""
     if (hidden.dtype is not torch.bfloat16 or not hidden.is_contiguous() or not (rd is torch.bfloat16 or rd is torch.float32)
-            or (residual is not None and (residual.dtype is not rd or not residual.is_contiguous() or residual.shape != hidden.shape))):
+            or (residual is not None and (residual.dtype is not rd or not residual.is_contiguous() or residual.shape != hidden.shape
+                                          or residual.get_device() != hidden.get_device()))):
         return None
     at = [hidden.data_ptr(), 0 if residual is None else residual.data_ptr()]
     return None if (at[0] | at[1]) & 15 else at
 
 
-def _block_states(B, C, H, P, N, conv_state, ssm_state):
-    """Addresses of a layer's cached states, or None where the kernels cannot use them in place."""
+def _block_states(dev, B, C, H, P, N, conv_state, ssm_state):
+    """Addresses of a layer's cached states, or None where the kernels cannot use them in place (a cache in host memory, which a
+    prompt's states are copied into, is one such case)."""
     if (conv_state.dtype is not torch.bfloat16 or ssm_state.dtype is not torch.float32 or conv_state.shape != (B, C, 4)
-            or ssm_state.shape != (B, H, P, N) or not conv_state.is_contiguous() or not ssm_state.is_contiguous()):
+            or ssm_state.shape != (B, H, P, N) or not conv_state.is_contiguous() or not ssm_state.is_contiguous()
+            or conv_state.get_device() != dev or ssm_state.get_device() != dev):
         return None
     at = [conv_state.data_ptr(), ssm_state.data_ptr()]
     return None if at[0] & 7 or at[1] & 15 else at
@@ -1154,10 +1159,10 @@ def block_forward(hidden, residual, residual_dtype, conv_state, ssm_state, norm_
     gs = d_inner if norm_group_size is None else norm_group_size
     if L % _CT or L == 0 or B == 0 or B > 65535 or d_state != 128 or head_dim % 64 or hidden.numel() >= 2 ** 31:
         return None
-    weights = _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D,
-                             gate_w, out_w)
+    weights = _block_weights(hidden.get_device(), width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b,
+                             dt_bias, A_log, D, gate_w, out_w)
     rows = _block_rows(hidden, residual, rd)
-    states = [0, 0] if conv_state is None else _block_states(B, C, H, head_dim, d_state, conv_state, ssm_state)
+    states = [0, 0] if conv_state is None else _block_states(hidden.get_device(), B, C, H, head_dim, d_state, conv_state, ssm_state)
     if weights is None or rows is None or states is None:
         return None
     dev, ld, T = hidden.device, _ceil8(d_inner + C + H), B * L
@@ -1199,12 +1204,12 @@ def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w
     C, H = d_inner + 2 * n_groups * d_state, d_inner // head_dim
     rd = residual_dtype or hidden.dtype
     gs = d_inner if norm_group_size is None else norm_group_size
-    if 2 * d_state + head_dim > 12288 or d_state % 4 or B > 65535:
+    if 2 * d_state + head_dim > 12288 or d_state % 4 or not 0 < B <= 65535:
         return None
-    weights = _block_weights(width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b, dt_bias, A_log, D,
-                             gate_w, out_w)
+    weights = _block_weights(hidden.get_device(), width, d_inner, n_groups, d_state, head_dim, gs, norm_w, in_w, in_b, conv_w, conv_b,
+                             dt_bias, A_log, D, gate_w, out_w)
     rows = _block_rows(hidden, residual, rd)
-    states = _block_states(B, C, H, head_dim, d_state, conv_state, ssm_state)
+    states = _block_states(hidden.get_device(), B, C, H, head_dim, d_state, conv_state, ssm_state)
     if weights is None or rows is None or states is None:
         return None
     dev, ld = hidden.device, _ceil8(d_inner + C + H)

@@ -143,3 +143,6 @@ def test_prompts_with_hooks_and_odd_caches_keep_their_calls():
     assert torch.equal(again, plain) and torch.equal(odd.ssm_states[1], cache.ssm_states[1].bfloat16())
     for i in range(2):
         assert torch.equal(cache.conv_states[i], other.conv_states[i]) and torch.equal(cache.ssm_states[i], other.ssm_states[i])
+    host = Mamba2Cache(cfg, 2, dtype=torch.bfloat16, device="cpu")          # states of a prompt are copied into host memory
+    again, _ = model.prefill(ids, host)
+    assert torch.equal(again, plain) and all(torch.equal(host.ssm_states[i], cache.ssm_states[i].cpu()) for i in range(2))

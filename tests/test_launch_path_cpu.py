@@ -74,3 +74,56 @@ def test_traced_without_grad():
         # the widening of logits takes the operation that a tracer can record
         traced = torch.jit.trace(lambda x: cuda_ops.widen(x) + 1, torch.ones(2, 8).bfloat16(), check_trace=False)
         assert torch.equal(traced(torch.full((2, 8), 5.0).bfloat16()), torch.full((2, 8), 6.0))
+
+
+def _block_parts(width=64, H=2, P=64, N=128):
+    C, W = H * P + 2 * N, 2 * H * P + 2 * N + H
+    make = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    weights = dict(norm_w=make(width), in_w=make(W, width), in_b=make(W), conv_w=make(C, 1, 4), conv_b=make(C), dt_bias=make(H),
+                   A_log=make(H), D=make(H), gate_w=make(H * P), out_w=make(width, H * P))
+    return weights, make(1, C, 4), torch.zeros(1, H, P, N)
+
+
+class _Elsewhere(torch.Tensor):
+    """A tensor that answers as one of another device."""
+
+    def get_device(self):
+        return 1
+
+
+def test_blocks_by_one_call_keep_to_one_device():
+    """Addresses are passed on only where every tensor lies on the rows' device."""
+    weights, window, state = _block_parts()
+    here = window.get_device()
+    given = lambda **kw: cuda_ops._block_weights(here, 64, 128, 1, 128, 64, 128, **{**weights, **kw})
+    assert given() is not None and cuda_ops._block_states(here, 1, 384, 2, 64, 128, window, state) is not None
+    for name, t in weights.items():
+        assert given(**{name: t.as_subclass(_Elsewhere)}) is None, name
+    assert cuda_ops._block_weights(0, 64, 128, 1, 128, 64, 128, **weights) is None
+    assert cuda_ops._block_states(here, 1, 384, 2, 64, 128, window.as_subclass(_Elsewhere), state) is None
+    assert cuda_ops._block_states(here, 1, 384, 2, 64, 128, window, state.as_subclass(_Elsewhere)) is None
+    assert cuda_ops._block_states(0, 1, 384, 2, 64, 128, window, state) is None
+    hidden = torch.zeros(1, 1, 64, dtype=torch.bfloat16)
+    assert cuda_ops._block_rows(hidden, hidden.clone(), torch.bfloat16) is not None
+    assert cuda_ops._block_rows(hidden, hidden.as_subclass(_Elsewhere), torch.bfloat16) is None
+
+
+@pytest.mark.parametrize("module,name", [("norm", "weight"), ("mixer.conv1d", "weight"), ("mixer.conv1d", "bias"), ("mixer", "D"),
+                                         ("mixer.norm", "weight"), ("mixer.in_proj", "weight"), ("mixer.out_proj", "weight"),
+                                         ("mixer.out_proj", "bias")])
+def test_blocks_by_one_call_want_plain_parameters(module, name):
+    """A weight that is no parameter of its module (computed by a parametrisation or a pruning mask) keeps the calls one by one."""
+    from state_space_models_neuron_b200.models import Mamba2Config
+    from state_space_models_neuron_b200.models.modeling_mamba2 import Mamba2Block
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    cfg = Mamba2Config(num_heads=2, head_dim=64, vocab_size=64, hidden_size=64, state_size=128, num_hidden_layers=1, n_groups=1)
+    block = Mamba2Block(cfg, 0)
+    op = lambda *a: "one call"
+    assert block._in_one_call(op, "step", None, None, None, None, None) == "one call"
+    owner = block.get_submodule(module)
+    value = getattr(owner, name)
+    delattr(owner, name)
+    setattr(owner, name, None if value is None else value.detach())
+    assert block._in_one_call(op, "step", None, None, None, None, None) is None
