@@ -389,7 +389,7 @@ gated_rmsnorm_fwd_kernel(const __nv_bfloat16* y, long long ys, const __nv_bfloat
 // Bound by moving five rows per row.  Rows of y, z and dout come by bulk copies into a ring in shared memory, where both passes
 // over a row read them: held in registers (with the next row's), they left room for one block per SM, which waited for its
 // loads and its barrier in turn.  Arithmetic in pairs; the sigmoids of the first pass stay in registers for the second.
-// us, before -> now: 8192 x 5120 146 -> 93, 4096 x 8192 104 -> 76, 2048 x 8192 58 -> 38, 4608 x 1536 26 -> 20 (64, 51, 26, 11 at copy
+// us, before -> now: 8192 x 5120 146 -> 93, 4096 x 8192 104 -> 71, 2048 x 8192 58 -> 40, 4608 x 1536 26 -> 20 (64, 51, 26, 11 at copy
 // bandwidth)
 constexpr int GATED_RING_MAX = 4;
 template <bool GATE, int THREADS, int PER_SM>
@@ -1473,7 +1473,8 @@ namespace ssm {
 // steps.  Correctly rounded operations, as the library's.
 __global__ void clip_kernel(const float* __restrict__ sumsq, float max_norm, float* __restrict__ norm, float* __restrict__ clip,
                             int* __restrict__ step, int* __restrict__ skipped) {
-  const float n = __fsqrt_rn(*sumsq);
+  const float square = *sumsq;              // where an embedding's additions took back what a product had added, rounding may leave
+  const float n = __fsqrt_rn(square < 0.f ? 0.f : square);        // a value just below zero
   const bool finite = (__float_as_uint(n) & 0x7f800000u) != 0x7f800000u;
   *norm = n;
   *clip = finite ? fminf(__fdiv_rn(max_norm, __fadd_rn(n, 1e-6f)), 1.f) : -1.f;
