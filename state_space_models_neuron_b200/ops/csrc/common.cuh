@@ -475,6 +475,17 @@ inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, si
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
+// Threads per block and vectors per thread of a norm's row (or group) of n elements; -1 if unsupported.  Whole warps, not
+// powers of two (5120 columns need 640 threads, not 1024).  Forward kernels take two vectors per thread above 256, so that
+// blocks of at most 512 threads leave room for several per SM; backward kernels, which hold two rows, take one.
+inline int norm_threads(int n, int* maxv, bool backward) {
+  const int v = n / 8;
+  if (v > 1024) return -1;
+  const int mv = backward || v <= 256 ? 1 : 2;
+  const int t = ((v + mv - 1) / mv + 31) / 32 * 32;
+  *maxv = mv;
+  return t < 32 ? 32 : t;
+}
 }  // namespace ssm
 #include <cudaTypedefs.h>
 #include <stdio.h>

@@ -1133,18 +1133,6 @@ extern "C" int ssm_conv1d_silu_bwd(const void* x, long long xs, const void* w, c
   return (int)cudaGetLastError();
 }
 
-// threads per block and vectors per thread for a row (or group) of n elements; -1 if unsupported.  Whole warps, not
-// powers of two (5120 columns need 640 threads, not 1024).  Forward kernels take two vectors per thread above 256, so that
-// blocks of at most 512 threads leave room for several per SM; backward kernels, which hold two rows, take one.
-static int norm_threads(int n, int* maxv, bool backward) {
-  const int v = n / 8;
-  if (v > 1024) return -1;
-  const int mv = backward || v <= 256 ? 1 : 2;
-  const int t = ((v + mv - 1) / mv + 31) / 32 * 32;
-  *maxv = mv;
-  return t < 32 ? 32 : t;
-}
-
 template <bool ROLL>
 static int gated_fwd(const void* y, long long ys, const void* z, long long zs, const void* w, void* out, long long os,
                      long long rows, int d, int gs, float eps, const WindowRoll& roll, cudaStream_t st) {

@@ -124,16 +124,15 @@ gemm_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, 
 }
 
 // ------------------------------------------------------------------------------------------------ norm and product, M <= 8
-// A norm in front of a product with at most eight rows: out[m, n] = sum_g rstd[m, g] sum_{k in g} bf16(h[m, k] wn[k]) W[n, k].
-// The factor rstd of a row (and group) is known only when the whole row has been read, but it can be applied to the sums, so
-// every warp forms the operand of its own k from the inputs of the norm while it waits for its weights, and neither a kernel
-// nor a barrier stands in front of the product.  One rounding to bf16 per operand, as with a norm kernel of its own.
-//   add    h = x + residual, the new residual is stored by the blocks in turn (chunk c by block c mod gridDim.x)
+// A norm in front of a product with at most eight rows, in one kernel with every rounding of the two that it stands for
+// (the forward norms of elementwise.cu and gemm_rows_kernel): the sums of squares are taken in the order of a norm kernel's
+// threads, an operand is bf16((wn h) rstd), and the products add up as in gemm_rows_kernel, so results are the same bits.
+//   add    h = x + residual, the new residual is stored by the blocks in turn (64 columns c by block c mod gridDim.x)
 //   gated  h = y silu(z); also rolls the conv windows of a decoding step (see WindowRoll in elementwise.cu)
+// While a warp waits for its first weights it forms wn h of its share of the rows, in fp32 in shared memory, and its part of
+// the sums; behind one barrier the operands are read from there.
 // Every block reads the M rows for itself (from L2) next to 32 K bytes of weights, so this pays for narrow products, where a
-// kernel's start and end cost more than its work (us per call behind another call, norm and product -> this: one row, gated
-// 768 x 1536 4.4 -> 3.3, 2048 x 4096 7.8 -> 7.2, add 4384 x 1024 4.1 -> 3.8), and not for wide ones (add 10576 x 2560 12.9 ->
-// 19.8); the caller has the rule.
+// kernel's start and end cost more than its work, and not for wide ones; the caller has the rule and the times.
 enum { NORM_ADD_BF16 = 0, NORM_ADD_FP32 = 1, NORM_GATED = 2 };
 
 struct NormLinearParams {
@@ -144,28 +143,28 @@ struct NormLinearParams {
   const __nv_bfloat16* w; long long ldw;
   const __nv_bfloat16* bias;
   __nv_bfloat16* out; long long ldo;
-  int M, N, K, groups;                        // groups: 1, 2, 4 or 8 equal parts of K, each a multiple of ROWS_CHUNK if more than one
+  int M, N, K, groups;                        // groups: equal parts of K, each a multiple of ROWS_CHUNK if more than one
+  int threads;                                // a norm kernel's threads for one group
   float eps;
   __nv_bfloat16* window; const __nv_bfloat16* xnew; long long xs; int c0, C;      // gated: windows [M][C][4], channels [c0, C)
 };
+constexpr int NORM_PARTS = 8;                 // warps of a norm kernel's block at most 4096 columns
+// floats of a row of wn h: four beyond the columns, so that two rows of a fragment meet no bank twice
+__host__ __device__ constexpr int norm_row(int K) { return K + 4; }
 
 __device__ __forceinline__ uint4 ld16_if(bool in, const void* p) { return ld8_if(in, reinterpret_cast<const __nv_bfloat16*>(p)); }
 
-template <int KIND, int UNROLL>
-__global__ void __launch_bounds__(ROWS_WARPS * 32)
+// VECS: 16-byte vectors of a row (or group) per thread of the norm kernel
+template <int KIND, int UNROLL, int VECS>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, KIND == NORM_GATED ? 1 : 2)
 norm_linear_kernel(const NormLinearParams p) {
+  extern __shared__ __align__(16) float rows[];          // [M][norm_row(K)] wn h
+  __shared__ float parts[8][8][NORM_PARTS];              // [row][group][warp of a norm kernel] sums of squares
   __shared__ float red[ROWS_WARPS][8][16 + 1];
-  __shared__ float sums[ROWS_WARPS][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * 16;
-  // the warps of a group share its chunks
-  const int per_group = ROWS_WARPS / p.groups, width = p.K / p.groups;
-  const int k_first = (warp / per_group) * width + (warp % per_group) * ROWS_CHUNK, k_end = (warp / per_group + 1) * width;
-  const int k_step = per_group * ROWS_CHUNK;
+  const int n0 = blockIdx.x * 16, width = p.K / p.groups, chunks = (p.K + ROWS_CHUNK - 1) / ROWS_CHUNK;
   const __nv_bfloat16* wl = p.w + (long long)(n0 + g < p.N ? n0 + g : 0) * p.ldw + t * 8;
   const __nv_bfloat16* wh = p.w + (long long)(n0 + g + 8 < p.N ? n0 + g + 8 : 0) * p.ldw + t * 8;
-  const bool mine = g < p.M;                  // lanes of rows beyond M bring zeros
-  const int row = mine ? g : 0;
   pdl_trigger();
   {
     // this warp's first weights on their way to L2 while the predecessor finishes: a 128-byte line per row and chunk
@@ -173,81 +172,131 @@ norm_linear_kernel(const NormLinearParams p) {
     if (r < p.N) {
       #pragma unroll
       for (int u = 0; u < UNROLL; u += 2) {
-        const int k = k_first + (u + (lane >> 4)) * k_step;
-        if (k < k_end) prefetch_l2(p.w + (long long)r * p.ldw + k);
+        const int k = (warp + (u + (lane >> 4)) * ROWS_WARPS) * ROWS_CHUNK;
+        if (k < p.K) prefetch_l2(p.w + (long long)r * p.ldw + k);
       }
     }
   }
   pdl_wait();
-  float acc[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.f;
-  for (int k0 = k_first; k0 < k_end; k0 += k_step * UNROLL) {
-    uint4 wa[UNROLL][2], wb[UNROLL][2], xa[UNROLL][2], xb[UNROLL][2], xc[UNROLL][2], nw[UNROLL][2];
+  uint4 wa[UNROLL][2], wb[UNROLL][2];
+  auto fetch = [&](int c0) {
     #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
       #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int k = k0 + u * k_step + s * 32, kk = k + t * 8;
-        const bool in = kk < k_end;           // a group's width is a multiple of 8
-        xa[u][s] = ld16_if(in && mine, p.a + row * p.lda + kk);
-        if (KIND == NORM_ADD_FP32) {
-          const float* r = reinterpret_cast<const float*>(p.b) + row * p.ldb + kk;
-          xb[u][s] = ld16_if(in && mine && p.b != nullptr, r);
-          xc[u][s] = ld16_if(in && mine && p.b != nullptr, r + 4);
-        } else {
-          xb[u][s] = ld16_if(in && mine && p.b != nullptr, reinterpret_cast<const __nv_bfloat16*>(p.b) + row * p.ldb + kk);
-        }
-        nw[u][s] = ld16_if(in && mine, p.wn + kk);
+        const int k = (c0 + u * ROWS_WARPS) * ROWS_CHUNK + s * 32;
+        const bool in = k + t * 8 < p.K;                 // K is a multiple of 8
         wa[u][s] = ld8_if(in, wl + k);
         wb[u][s] = ld8_if(in, wh + k);
       }
     }
-    __syncwarp();                             // all loads go out in front of it
+    __syncwarp();                                        // all loads go out in front of it
+  };
+  fetch(warp);
+  // ---- wn h and the sums of squares: an item stands for one warp of a norm kernel's block of one row and group; the vectors
+  // of ITEMS of them are under way at once
+  const int warps = p.threads >> 5, per_row = p.groups * warps, items = p.M * per_row;
+  constexpr int ITEMS = KIND == NORM_GATED && VECS == 1 ? 3 : 1;
+  for (int i0 = warp; i0 < items; i0 += ROWS_WARPS * ITEMS) {
+    uint4 xa[ITEMS][VECS], xb[ITEMS][VECS], xc[ITEMS][VECS], nw[ITEMS][VECS];
     #pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
+    for (int j = 0; j < ITEMS; ++j) {
+      const int i = i0 + j * ROWS_WARPS, m = i / per_row, rest = i - m * per_row, grp = rest / warps;
       #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        float h[8], n[8];
-        unpack8(xa[u][s], h);
-        unpack8(nw[u][s], n);
-        if (KIND == NORM_GATED) {
-          float z[8];
-          unpack8(xb[u][s], z);
-          #pragma unroll
-          for (int e = 0; e < 8; ++e) h[e] *= silu_f(z[e]);
+      for (int q = 0; q < VECS; ++q) {
+        const int v = (rest - grp * warps) * 32 + lane + q * p.threads, k = grp * width + v * 8;
+        const bool in = i < items && v * 8 < width;
+        xa[j][q] = ld16_if(in, p.a + m * p.lda + k);
+        if (KIND == NORM_ADD_FP32) {
+          const float* r = reinterpret_cast<const float*>(p.b) + m * p.ldb + k;
+          xb[j][q] = ld16_if(in && p.b != nullptr, r);
+          xc[j][q] = ld16_if(in && p.b != nullptr, r + 4);
         } else {
-          float r[8];
-          if (KIND == NORM_ADD_FP32) {
-            const uint4 lo = xb[u][s], hi = xc[u][s];
-            r[0] = __uint_as_float(lo.x); r[1] = __uint_as_float(lo.y); r[2] = __uint_as_float(lo.z); r[3] = __uint_as_float(lo.w);
-            r[4] = __uint_as_float(hi.x); r[5] = __uint_as_float(hi.y); r[6] = __uint_as_float(hi.z); r[7] = __uint_as_float(hi.w);
+          xb[j][q] = ld16_if(in && p.b != nullptr, reinterpret_cast<const __nv_bfloat16*>(p.b) + m * p.ldb + k);
+        }
+        nw[j][q] = ld16_if(in, p.wn + k);
+      }
+    }
+    __syncwarp();                                        // all loads go out in front of it
+    #pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int i = i0 + j * ROWS_WARPS, m = i / per_row, rest = i - m * per_row, grp = rest / warps, vw = rest - grp * warps;
+      if (i >= items) break;
+      float ss = 0.f;
+      #pragma unroll
+      for (int q = 0; q < VECS; ++q) {
+        const int v = vw * 32 + lane + q * p.threads, k = grp * width + v * 8;
+        float h[8], n[8], r[8];
+        unpack8(xa[j][q], h);
+        unpack8(nw[j][q], n);
+        if (KIND == NORM_ADD_FP32) {
+          const uint4 lo = xb[j][q], hi = xc[j][q];
+          r[0] = __uint_as_float(lo.x); r[1] = __uint_as_float(lo.y); r[2] = __uint_as_float(lo.z); r[3] = __uint_as_float(lo.w);
+          r[4] = __uint_as_float(hi.x); r[5] = __uint_as_float(hi.y); r[6] = __uint_as_float(hi.z); r[7] = __uint_as_float(hi.w);
+        } else {
+          unpack8(xb[j][q], r);
+        }
+        if (v * 8 < width) {
+          if (KIND == NORM_GATED) {
+            #pragma unroll
+            for (int e = 0; e < 8; ++e) h[e] *= silu_f(r[e]);
           } else {
-            unpack8(xb[u][s], r);
-          }
-          #pragma unroll
-          for (int e = 0; e < 8; ++e) h[e] += r[e];
-          const int kk = k0 + u * k_step + s * 32 + t * 8;
-          if (mine && kk < k_end && (kk / ROWS_CHUNK) % gridDim.x == blockIdx.x) {
-            if (KIND == NORM_ADD_FP32) {
-              float* o = reinterpret_cast<float*>(p.res_out) + (long long)row * p.K + kk;
-              *reinterpret_cast<float4*>(o) = make_float4(h[0], h[1], h[2], h[3]);
-              *reinterpret_cast<float4*>(o + 4) = make_float4(h[4], h[5], h[6], h[7]);
-            } else {
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.res_out) + (long long)row * p.K + kk) =
-                  make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
+            if (p.b != nullptr) {
+              #pragma unroll
+              for (int e = 0; e < 8; ++e) h[e] += r[e];
+            }
+            if ((k / ROWS_CHUNK) % gridDim.x == blockIdx.x) {
+              if (KIND == NORM_ADD_FP32) {
+                float* o = reinterpret_cast<float*>(p.res_out) + (long long)m * p.K + k;
+                *reinterpret_cast<float4*>(o) = make_float4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<float4*>(o + 4) = make_float4(h[4], h[5], h[6], h[7]);
+              } else {
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.res_out) + (long long)m * p.K + k) =
+                    make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
+              }
             }
           }
+          #pragma unroll
+          for (int e = 0; e < 8; ++e) ss += h[e] * h[e];
+          float4* o = reinterpret_cast<float4*>(rows + m * norm_row(p.K) + k);
+          o[0] = make_float4(n[0] * h[0], n[1] * h[1], n[2] * h[2], n[3] * h[3]);
+          o[1] = make_float4(n[4] * h[4], n[5] * h[5], n[6] * h[6], n[7] * h[7]);
         }
-        #pragma unroll
-        for (int e = 0; e < 8; ++e) ss += h[e] * h[e];
+      }
+      __syncwarp();
+      #pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane < NORM_PARTS && (lane == vw || lane >= warps)) parts[m][grp][lane] = lane == vw ? ss : 0.f;
+    }
+  }
+  __syncthreads();
+  // ---- the product
+  const bool mine = g < p.M;                             // lanes of rows beyond M bring zeros
+  const float* row = rows + (mine ? g : 0) * norm_row(p.K);
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, rstd = 0.f;
+  int have = -1;                                         // group of rstd
+  for (int c0 = warp; c0 < chunks; c0 += ROWS_WARPS * UNROLL) {
+    if (c0 != warp) fetch(c0);
+    #pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int k0 = (c0 + u * ROWS_WARPS) * ROWS_CHUNK, grp = p.groups == 1 ? 0 : k0 / width;
+      if (k0 >= p.K) break;
+      if (grp != have) {                                 // the sum over the warps as block_sum forms it
+        const float* q = parts[mine ? g : 0][grp];
+        rstd = rsqrtf((((q[0] + q[4]) + (q[2] + q[6])) + ((q[1] + q[5]) + (q[3] + q[7]))) / width + p.eps);
+        have = grp;
+      }
+      #pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int k = k0 + s * 32 + t * 8;
+        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+        if (mine && k < p.K) { lo = *reinterpret_cast<const float4*>(row + k); hi = *reinterpret_cast<const float4*>(row + k + 4); }
         const uint4 q = wa[u][s], v = wb[u][s];
-        mma_16x8x16(acc, q.x, v.x, q.y, v.y, pack_bf16(h[0] * n[0], h[1] * n[1]), pack_bf16(h[2] * n[2], h[3] * n[3]));
-        mma_16x8x16(acc, q.z, v.z, q.w, v.w, pack_bf16(h[4] * n[4], h[5] * n[5]), pack_bf16(h[6] * n[6], h[7] * n[7]));
+        mma_16x8x16(acc, q.x, v.x, q.y, v.y, pack_bf16(lo.x * rstd, lo.y * rstd), pack_bf16(lo.z * rstd, lo.w * rstd));
+        mma_16x8x16(acc, q.z, v.z, q.w, v.w, pack_bf16(hi.x * rstd, hi.y * rstd), pack_bf16(hi.z * rstd, hi.w * rstd));
       }
     }
   }
-  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-  if (t == 0) sums[warp][g] = ss;
   red[warp][2 * t][g] = acc[0];
   red[warp][2 * t + 1][g] = acc[1];
   red[warp][2 * t][g + 8] = acc[2];
@@ -265,30 +314,33 @@ norm_linear_kernel(const NormLinearParams p) {
   __syncthreads();
   const int m = threadIdx.x >> 4, r = threadIdx.x & 15;
   if (m < p.M && n0 + r < p.N) {
-    float v = 0.f;
-    for (int i = 0; i < ROWS_WARPS; i += per_group) {
-      float part = red[i][m][r], square = sums[i][m];
-      for (int k = 1; k < per_group; ++k) { part += red[i + k][m][r]; square += sums[i + k][m]; }
-      v += part * rsqrtf(square / width + p.eps);
-    }
+    float v = red[0][m][r];
+    #pragma unroll
+    for (int k = 1; k < ROWS_WARPS; ++k) v += red[k][m][r];
     if (p.bias != nullptr) v += __bfloat162float(p.bias[n0 + r]);
     p.out[(long long)m * p.ldo + n0 + r] = __float2bfloat16(v);
   }
 }
 
 template <int KIND>
-static int launch_norm_linear(const NormLinearParams& p, bool fp32, int sms, cudaStream_t stream) {
-  // bases and strides of 16-byte vectors, groups that whole warps can share
+static int launch_norm_linear(NormLinearParams p, bool fp32, int sms, cudaStream_t stream) {
+  // bases and strides of 16-byte vectors, groups of whole chunks, rows that fit the shared memory of any kernel
   const uintptr_t a = reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.b) | reinterpret_cast<uintptr_t>(p.wn) |
                       reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.res_out);
-  if (p.M < 1 || p.M > 8 || p.N < 1 || p.K < 8 || p.K % 8 || (a & 15) || p.lda % 8 || p.ldw % 8 || p.ldb % (fp32 ? 4 : 8) ||
-      !(p.groups == 1 || ((p.groups == 2 || p.groups == 4 || p.groups == 8) && p.K % (p.groups * ROWS_CHUNK) == 0)))
+  const size_t smem = (size_t)p.M * norm_row(p.K) * sizeof(float);
+  if (p.M < 1 || p.M > 8 || p.N < 1 || p.K < 8 || p.K > 4096 || p.K % 8 || (a & 15) || p.lda % 8 || p.ldw % 8 || p.ldb % (fp32 ? 4 : 8) ||
+      smem > 41 * 1024 || !(p.groups == 1 || ((p.groups == 2 || p.groups == 4 || p.groups == 8) && p.K % (p.groups * ROWS_CHUNK) == 0)))
     return -SSM_ERR_BAD_ARG;
+  int vecs = 1;
+  p.threads = norm_threads(p.K / p.groups, &vecs, false);
+  if (p.threads < 0 || p.threads > 32 * NORM_PARTS || (vecs == 2 && KIND != NORM_GATED)) return -SSM_ERR_BAD_ARG;
   const unsigned grid = (unsigned)((p.N + 15) / 16);
   const int unroll = rows_unroll(((p.K + ROWS_CHUNK - 1) / ROWS_CHUNK + ROWS_WARPS - 1) / ROWS_WARPS);
-  auto kern = unroll == 1 ? norm_linear_kernel<KIND, 1> : unroll == 2 || grid > (unsigned)sms ? norm_linear_kernel<KIND, 2>
-            : norm_linear_kernel<KIND, 3>;
-  return launch_dependent(kern, dim3(grid), dim3(ROWS_WARPS * 32), 0, stream, p);
+  const bool few = unroll <= 2 || grid > (unsigned)sms;
+  auto kern = unroll == 1 && vecs == 1 ? norm_linear_kernel<KIND, 1, 1> : few ? norm_linear_kernel<KIND, 2, 1> : norm_linear_kernel<KIND, 3, 1>;
+  if constexpr (KIND == NORM_GATED)
+    if (vecs == 2) kern = few ? norm_linear_kernel<KIND, 2, 2> : norm_linear_kernel<KIND, 3, 2>;
+  return launch_dependent(kern, dim3(grid), dim3(ROWS_WARPS * 32), smem, stream, p);
 }
 
 // ------------------------------------------------------------------------------------------------ M <= 128
@@ -538,7 +590,7 @@ static int device_sms() {
 }
 
 // out[M, N] = rmsnorm(x + res) W^T (+ bias) and res_out = x + res, M <= 8.  x [M, K] bf16 (row stride ldx); res contiguous
-// [M, K] of the residual type or null; 1 where the shape is not this kernel's.
+// [M, K] of the residual type or null.  -SSM_ERR_BAD_ARG where the shape is not this kernel's.
 extern "C" int ssm_add_norm_linear(const void* x, long long ldx, const void* res, void* res_out, int res_fp32, const void* wn,
                                    float eps, const void* w, long long ldw, const void* bias, void* out, long long ldo, int M,
                                    int N, int K, cudaStream_t st) {

@@ -1185,14 +1185,18 @@ def block_forward(hidden, residual, residual_dtype, conv_state, ssm_state, norm_
 _BLOCK = struct.Struct("=20Qq11i2f")
 
 
-def _norms_in_products(B: int, width: int, d_inner: int, gs: int):
-    """Which norms of a decoding block are computed inside the product behind them (norm_linear_kernel): (first, gated).  Up to
-    eight rows, and groups that whole warps of that kernel can share.  Every block of it reads all rows, so narrow products
-    gain and wide ones lose (one kernel / two, us, one row: in_proj from 768 columns 3.4 / 3.4, 1024 3.8 / 4.1, 1536 9.7 / 6.6;
-    out_proj from 1536 3.3 / 4.4, 3072 5.1 / 6.6, 4096 7.2 / 7.8, 5120 10.9 / 9.2; five rows the same within 0.5)."""
+def _norms_in_products(B: int, width: int, in_cols: int, d_inner: int, gs: int, captured: bool):
+    """Which norms of a decoding block are computed inside the product behind them (norm_linear_kernel, the same bits as two
+    kernels): (first, gated).  Every block of it forms all rows, so few columns in all gain and many lose; two blocks of the first
+    kind fit an SM, and a second wave of them costs what the launch saved (one kernel / two, us: in_proj 1 x 3352 x 768 3.0 / 3.8,
+    1 x 4384 x 1024 3.5 / 4.5, 1 x 6176 x 1024 6.3 / 4.7, 2 x 4384 x 1024 3.7 / 4.5, 3 x 4384 x 1024 4.4 / 4.6, 5 x 4384 x 1024 5.4 / 4.7;
+    out_proj from 1 x 1536 columns 3.5 / 4.6, 1 x 4096 7.5 / 8.4, 3 x 2048 5.5 / 5.7, 2 x 4096 8.9 / 8.7, 5 x 1536 5.7 / 5.6, 5 x 2048
+    6.9 / 5.9; with eight groups 1 x 2048 5.0 / 5.2, 2 x 2048 5.4 / 5.3, 1 x 4096 8.5 / 8.2).  Where no graph is captured the host is
+    the limit, which a launch less saves 3 us (370M, 5 sequences: 723 us a token with two kernels each, 642 with one)."""
     groups = d_inner // gs
-    return (B <= 8 and width <= 1024,
-            B <= 8 and d_inner <= 4096 and (groups == 1 or (groups in (2, 4, 8) and gs % 64 == 0)))
+    first, gated = (2048, 6144 if groups == 1 else 2048) if captured else (8192, 10240)
+    return (B <= 8 and width <= 1024 and B * width <= first and (in_cols <= 16 * 2 * 148 or not captured),
+            B <= 8 and d_inner <= 4096 and B * d_inner <= gated and (groups == 1 or (groups in (2, 4, 8) and gs % 64 == 0)))
 
 
 def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w, norm_eps, in_w, in_b, conv_w, conv_b, dt_bias, A_log,
@@ -1216,7 +1220,7 @@ def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w
     scratch = torch.empty(B * (ld + d_inner + max(width, d_inner)), dtype=torch.bfloat16, device=dev)
     out, res_out = torch.empty_like(hidden), torch.empty(hidden.shape, dtype=rd, device=dev)
     zx = scratch.data_ptr()
-    first, gated = _norms_in_products(B, width, d_inner, gs)
+    first, gated = _norms_in_products(B, width, d_inner + C + H, d_inner, gs, torch.cuda.is_current_stream_capturing())
     _run("ssm_decode_block", _BLOCK.pack(*rows, res_out.data_ptr(), *weights[0], *states, zx, zx + 2 * B * ld, zx + 2 * B * (ld + d_inner),
                                          out.data_ptr(), status_tensor(dev).data_ptr(), ld, B, width, d_inner, H, head_dim, d_state,
                                          n_groups, gs, int(rd is torch.float32), weights[1], int(first) | 2 * int(gated), norm_eps, eps), _st())

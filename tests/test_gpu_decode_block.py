@@ -44,6 +44,44 @@ def test_block_equals_separate_operations(B, width, H, P, G, gs, fp32):
             hidden, residual = want, want_res
 
 
+# norms inside the products (of the last case the gated one alone): one and two vectors per thread of the norm kernel, whole and partial warps and chunks, groups of
+# whole chunks, one to eight rows, several turns of the rows, no residual at first and then one of either type
+@pytest.mark.parametrize("B,width,H,P,G,gs,fp32", [(1, 768, 24, 64, 1, 1536, True), (1, 1000, 8, 272, 1, 2176, False),
+                                                   (8, 1024, 16, 64, 2, 1024, True), (5, 256, 32, 64, 1, 2048, False),
+                                                   (1, 264, 16, 128, 1, 2048, True), (2, 64, 16, 64, 2, 512, False),
+                                                   (1, 72, 8, 192, 4, 192, True), (4, 8, 8, 64, 1, 512, False),
+                                                   (7, 104, 13, 64, 1, 832, True), (1, 1000, 8, 480, 1, 3840, False)])
+def test_block_has_the_bits_of_separate_operations(B, width, H, P, G, gs, fp32):
+    """Which norms run inside the products is a matter of time only: every sum and rounding is that of the separate kernels."""
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    d, N = H * P, 128
+    C = d + 2 * G * N
+    assert cuda_ops._norms_in_products(B, width, d + C + H, d, gs, False) == (d < 3840, True)
+    gen = torch.Generator(device="cuda").manual_seed(B + width)
+    make = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=gen) * scale).bfloat16()
+    norm_w, gate_w = make(width), make(d)
+    in_w, in_b, out_w = make(d + C + H, width, scale=width ** -0.5), make(d + C + H), make(width, d, scale=d ** -0.5)
+    conv_w, conv_b, head = make(C, 1, 4), make(C), [make(H).float(), make(H).abs(), make(H)]
+    window, state = make(B, C, 4), torch.randn(B, H, P, N, device="cuda", generator=gen)
+    rd = torch.float32 if fp32 else None
+    kw = dict(d_inner=d, n_groups=G, d_state=N, head_dim=P, eps=1e-5, norm_group_size=gs)
+    w0, s0 = window.clone(), state.clone()
+    hidden, residual = make(B, 1, width), None
+    with torch.no_grad():
+        for _ in range(4):
+            out, res = ops.decode_block(hidden, residual, rd, window, state, norm_w, 1e-5, in_w, in_b, conv_w, conv_b, *head, gate_w,
+                                        out_w, **kw)
+            normed, want_res = ops.add_rmsnorm(hidden, residual, norm_w, 1e-5, rd)
+            y = ops.ssm_decode_step(ops.linear(normed, in_w, in_b)[:, 0], w0, s0, conv_w, conv_b, *head, gate_w, **kw)
+            want = ops.linear(y[:, None], out_w)
+            torch.cuda.synchronize()
+            cuda_ops.check_status()
+            for a, b in ((out, want), (res, want_res), (window, w0), (state, s0)):
+                assert torch.equal(a, b)
+            hidden, residual = out, res
+
+
 def test_block_refuses_what_it_cannot_read():
     from state_space_models_neuron_b200 import ops
     B, width, H, P, N = 1, 256, 8, 64, 128
