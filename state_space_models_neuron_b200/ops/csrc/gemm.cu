@@ -27,6 +27,7 @@
 // Replaces the XLA-compiled `dot` of every Linear layer of the reference (mamba2/mamba2_mixer.py:228,233,
 // mamba2/modeling_mamba2.py:498, mamba2hybrid/mamba2hybrid_attn.py:411-413,463, mamba2hybrid/mamba2hybrid_mlp.py:121,134).
 #include "common.cuh"
+#include "gemm_scratch.h"
 #include <stdlib.h>
 #include <string.h>
 
@@ -38,7 +39,7 @@ constexpr int GEMM_THREADS = 224;                       // warp 0: TMA (A), 1: M
 constexpr int EPI_BLOCK_COLS = 64;                       // bf16 columns per TMA store block (128 bytes)
 constexpr int EPI_BUF_BYTES = GEMM_BM * EPI_BLOCK_COLS * 2;  // 16 KiB
 constexpr int MAX_SPLIT = 8;                             // K slices of a tail tile (upper bound of GemmParams::split)
-constexpr int MAX_UNITS = 160;                           // scheduling units (CTAs or pairs) the scratch is sized for
+constexpr int MAX_UNITS = 160;                           // CTAs of a launch with split tiles that the scratch is sized for
 constexpr int AG_MAX_GROUPS = 4;                         // column (K) groups of a shard with a ready flag of their own
 
 struct GemmParams {
@@ -1024,25 +1025,6 @@ static int gemm_forced_bn() {
   return g_opt_bn;
 }
 
-// Scratch for the split tail (allocated once per device, on first use): partial sums and arrival counters.
-struct Scratch { float* ws; int* counters; };
-static Scratch g_scratch[16] = {};
-static int scratch_for_current_device(Scratch* out) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return -1;
-  if (g_scratch[dev].ws == nullptr) {
-    const size_t ws_bytes = (size_t)MAX_UNITS * 2 * GEMM_BM * 256 * sizeof(float);   // one slice per CTA and launch
-    void* a = nullptr; void* b = nullptr;
-    if (cudaMalloc(&a, ws_bytes) != cudaSuccess) return -1;
-    if (cudaMalloc(&b, MAX_UNITS * 2 * sizeof(int)) != cudaSuccess) { cudaFree(a); return -1; }
-    if (cudaMemset(b, 0, MAX_UNITS * 2 * sizeof(int)) != cudaSuccess) { cudaFree(a); cudaFree(b); return -1; }
-    g_scratch[dev].ws = reinterpret_cast<float*>(a);
-    g_scratch[dev].counters = reinterpret_cast<int*>(b);
-  }
-  *out = g_scratch[dev];
-  return 0;
-}
-
 struct TileChoice { int bn; int pair; };
 
 // Tile shape.  The cost of a tiling is (full waves + the split tail) x time of one tile; tile times relative to a
@@ -1163,17 +1145,20 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     }
     if (max_units > max_clusters) max_units = max_clusters;
   }
-  if (max_units > MAX_UNITS) max_units = MAX_UNITS;
+  if (max_units > MAX_UNITS / (PAIR ? 2 : 1)) max_units = MAX_UNITS / (PAIR ? 2 : 1);
   const int kblocks = (p.K + GEMM_BK - 1) / GEMM_BK;
   Schedule sc = plan_schedule(tiles, max_units, kblocks, p.mode, PAIR ? 1 : 0, BN);
   p.ws = nullptr; p.ws_counters = nullptr;
-  if (sc.split > 1 && p.mode != 2) {             // slices exchange fp32 partial sums through a per-device scratch buffer
+  std::unique_lock<std::mutex> scratch_held;
+  if (sc.split > 1 && p.mode != 2) {             // slices exchange fp32 partial sums through the stream's scratch
     Scratch s;
-    if (scratch_for_current_device(&s) != 0) {
+    ScratchPool& pool = ScratchPool::get();
+    scratch_held = std::unique_lock<std::mutex>(pool.lock);
+    if (pool.take(stream, (size_t)MAX_UNITS * GEMM_BM * 256 * sizeof(float), MAX_UNITS, &s)) {
+      p.ws = s.ws; p.ws_counters = s.counters;
+    } else {
       if (tiles < max_units) sc.units = sc.rem;   // no scratch: whole tail tiles, one per unit
       sc.split = 1;
-    } else {
-      p.ws = s.ws; p.ws_counters = s.counters;
     }
   }
   const int units = sc.units;
@@ -1243,6 +1228,9 @@ extern "C" int ssm_gemm_ce_tiles(int M, int N, int K, int rows_per_shard) {
   return (N + c.bn - 1) / c.bn;
 }
 
+// out[3]: scratches of split tiles that are kept for streams, that belong to graphs, and that are spare
+extern "C" int ssm_gemm_scratch_count(int* out) { ssm::ScratchPool::get().count(out); return 0; }
+
 // The tiling and work distribution that a plain GEMM of this shape gets, without launching anything (host only; also
 // callable without a GPU, where 148 SMs are assumed): out[8] = {tile width BN, 1 if CTA-pair tiles, tiles along M,
 // tiles along N, units launched, whole tiles in the full waves, tail tiles, K slices per tail tile}.
@@ -1255,7 +1243,7 @@ extern "C" int ssm_gemm_plan(int M, int N, int K, int mode, int allow_pair, int*
   const int tile_m = c.pair ? 256 : 128;
   const int tiles_m = (M + tile_m - 1) / tile_m, tiles_n = (N + c.bn - 1) / c.bn;
   int max_units = c.pair ? sms / 2 : sms;
-  if (max_units > MAX_UNITS) max_units = MAX_UNITS;
+  if (max_units > MAX_UNITS / (c.pair ? 2 : 1)) max_units = MAX_UNITS / (c.pair ? 2 : 1);
   const Schedule sc = plan_schedule(tiles_m * tiles_n, max_units, (K + GEMM_BK - 1) / GEMM_BK, mode, c.pair, c.bn);
   out[0] = c.bn; out[1] = c.pair; out[2] = tiles_m; out[3] = tiles_n;
   out[4] = sc.units; out[5] = sc.full_tiles; out[6] = sc.rem; out[7] = sc.split;
