@@ -363,10 +363,16 @@ class _Conv(torch.autograd.Function):
         return dx, dw.to(w2.dtype).reshape(ctx.wshape), (None if bias is None else db.to(bias.dtype)), None
 
 
+def _require_four_taps(weight, channels: int) -> None:
+    if weight.numel() != 4 * channels:
+        raise ValueError(f"the conv kernels are written for 4 taps of {channels} channels, got {tuple(weight.shape)}")
+
+
 def causal_conv1d_silu(x, weight, bias, initial_state=None):
     _require_bf16(x, weight, bias)
     if weight.shape[-1] != 4:
-        raise ValueError("the conv kernel is written for 4 taps")
+        raise ValueError("the conv kernels are written for 4 taps")
+    _require_four_taps(weight, x.shape[-1])
     return _apply(_Conv, x, weight, bias, initial_state)
 
 
@@ -898,6 +904,7 @@ class _MixerCore(torch.autograd.Function):
         C = d_inner + 2 * G * N
         if W != d_inner + C + H or L % _CT or d_inner % 8 or (G * N) % 8:
             raise ValueError("bad zxBCdt shape for the mixer core")
+        _require_four_taps(conv_w, C)
         # rows may carry padding (row stride ld >= W, multiple of 8): that is how the GEMM epilogue writes them
         if (zxBCdt.stride(2) != 1 or zxBCdt.stride(1) % 8 or zxBCdt.stride(0) != L * zxBCdt.stride(1)
                 or zxBCdt.data_ptr() % 16):

@@ -127,3 +127,19 @@ def test_blocks_by_one_call_want_plain_parameters(module, name):
     delattr(owner, name)
     setattr(owner, name, None if value is None else value.detach())
     assert block._in_one_call(op, "step", None, None, None, None, None) is None
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 5])
+def test_other_numbers_of_taps_are_refused(taps):
+    """The conv kernels read four taps per channel: any other weight is refused before a launch, in the mixer as in the conv itself."""
+    H, P, N, L = 2, 64, 128, 128
+    d, C = H * P, H * P + 2 * N
+    make = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    for cached in (False, True):
+        with torch.no_grad(), pytest.raises(ValueError, match="taps"):
+            cuda_ops.mamba2_mixer_core(make(1, L, d + C + H), make(C, 1, taps), make(C), make(H), make(H), make(H), make(d), d, 1, N, P,
+                                       1e-5, None, 128, False, cached)
+    with torch.no_grad(), pytest.raises(ValueError, match="taps"):
+        cuda_ops.causal_conv1d_silu(make(1, L, C), make(C, 1, taps), make(C))
+    with torch.no_grad(), pytest.raises(ValueError, match="taps"):         # four taps of fewer channels
+        cuda_ops.causal_conv1d_silu(make(1, L, C), make(C // 2, 1, 4), make(C))
