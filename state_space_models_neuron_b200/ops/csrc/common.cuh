@@ -108,8 +108,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// Full barrier over all threads of all CTAs of the cluster, with release/acquire ordering of shared memory.
+// Full barrier over all threads of all CTAs of the cluster, with release/acquire ordering of shared memory.  The aligned form
+// wants whole warps, which a branch for one thread in front of it may have split.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
