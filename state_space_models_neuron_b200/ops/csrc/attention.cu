@@ -602,13 +602,9 @@ static int attn_maps(CUtensorMap* tq, CUtensorMap* tk, CUtensorMap* tv, CUtensor
 extern "C" int ssm_attn_fwd(const void* q, const void* k, const void* v, void* out, void* lse, int B, int L, int Hq,
                             int Hkv, int D, float scale, int* status, cudaStream_t st) {
   if (D != AD || L % AT || Hq % Hkv) return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
   const int smem = ATTN_FWD_SMEM;
-  if (!cfg) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    cfg = true;
-  }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(attn_fwd_kernel), smem)) return e;
   CUtensorMap tq, tk, tv, to;
   int r = attn_maps(&tq, &tk, &tv, &to, q, k, v, out, B, L, Hq, Hkv, AT);
   if (r) return r;
@@ -635,12 +631,8 @@ extern "C" int ssm_attn_bwd(const void* q, const void* k, const void* v, const v
   if (D != AD || L % AT || Hq % Hkv || L / AT > 65535 ||
       ((reinterpret_cast<uintptr_t>(lse) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(dq32)) & 15))
     return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
-  if (!cfg) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_BWD_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    cfg = true;
-  }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(attn_bwd_kernel), ATTN_BWD_SMEM)) return e;
   CUtensorMap tq, tk, tv, tdo, tdq;
   int r = attn_maps(&tq, &tk, &tv, &tdo, q, k, v, dout, B, L, Hq, Hkv, AQ);
   if (r) return r;

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <cuda.h>
 #include <stdint.h>
+#include <atomic>
 
 #define SSM_OK 0
 #define SSM_ERR_TIMEOUT_MBAR 1      // an mbarrier phase never completed
@@ -477,6 +478,21 @@ inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, si
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
+// A kernel's opt-in to more than 48 KB of dynamic shared memory, which every device keeps for itself: asked for once per
+// device.  One static object per kernel; threads that meet here at once ask for the same bytes twice.
+struct SmemOptIn {
+  std::atomic<uint64_t> asked{0};                          // bit: device
+  int ask(const void* kern, int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;          // beyond 64 devices: at every launch
+    if (asked.load(std::memory_order_acquire) & bit) return 0;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) asked.fetch_or(bit, std::memory_order_release);
+    return (int)e;
+  }
+};
 // Threads per block and vectors per thread of a norm's row (or group) of n elements; -1 if unsupported.  Whole warps, not
 // powers of two (5120 columns need 640 threads, not 1024).  Forward kernels take two vectors per thread above 256, so that
 // blocks of at most 512 threads leave room for several per SM; backward kernels, which hold two rows, take one.

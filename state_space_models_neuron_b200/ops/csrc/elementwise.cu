@@ -1161,12 +1161,8 @@ static int launch_gated_bwd(dim3 grid, int t, int gs, cudaStream_t st, const voi
   // as many rows ahead as fit beside the other block of the SM
   const int stage = (GATE ? 6 : 4) * gs, room = (PER_SM == 1 ? 200 : 100) * 1024;
   const int ring = room / stage < GATED_RING_MAX ? room / stage : GATED_RING_MAX;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(kern), room)) return e;
   kern<<<grid, t, ring * stage, st>>>(BF(y), ys, BF(z), zs, BF(w), BF(dout), dos, BFM(dy), dys, BFM(dz), dzs,
                                       reinterpret_cast<float*>(dwpart), rows, d, gs, eps, ring, status);
   return (int)cudaGetLastError();

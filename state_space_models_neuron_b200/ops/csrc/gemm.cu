@@ -1112,13 +1112,9 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
                        cudaStream_t stream, const GemmComm* comm = nullptr, const RsMaps* maps = nullptr,
                        const CUtensorMap* ta_local = nullptr, const CUtensorMap* ta_push = nullptr) {
   using L = GemmSmem<BN, STAGES, PAIR>;
-  static bool configured = false;
   auto kern = gemm_bf16_tcgen05<BN, STAGES, PAIR>;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(kern), L::TOTAL)) return e;
   constexpr int TILE_M = PAIR ? 256 : 128;
   p.tiles_m = (p.M + TILE_M - 1) / TILE_M;
   p.tiles_n = (p.N + BN - 1) / BN;

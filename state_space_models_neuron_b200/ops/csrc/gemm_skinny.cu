@@ -518,12 +518,8 @@ static int launch_cols(const void* X, long long ldx, const void* W, long long ld
                        cudaStream_t stream) {
   using S = ColsSmem<NB, STAGES>;
   auto kern = gemm_cols_kernel<NB, STAGES, PER_SM>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(kern), S::TOTAL)) return e;
   CUtensorMap tw, tx;
   int r = make_tmap_2d_bf16(&tw, W, (uint64_t)K, (uint64_t)p.N, (uint64_t)ldw * 2, 64, 128);
   if (r) return -200 - r;

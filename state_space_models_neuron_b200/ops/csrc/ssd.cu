@@ -1247,10 +1247,6 @@ ssd_chunk_scan_bwd_kernel(const __grid_constant__ CUtensorMap tm_xbc, const __gr
 // ------------------------------------------------------------------------------------ C API
 using namespace ssm;
 
-static int smem_opt_in(const void* fn, int bytes) {
-  return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 // A, D, dt_bias, mask, params_out: see HeadParams
 extern "C" int ssm_ssd_dt_prep(const void* dt_raw, long long row_stride, const void* dt_bias, const void* A, const void* D,
                                int mask, void* params_out, void* dt_out, void* l_out, int B, int L, int H, cudaStream_t st) {
@@ -1267,9 +1263,9 @@ extern "C" int ssm_ssd_chunk_state(const void* w_src, long long w_stride, int w_
                                    long long v_stride, const void* dt, const void* l, void* out, int B, int L, int H,
                                    int Hv, int G, int mode, int* status, cudaStream_t st) {
   if (L % CT || Hv % H || H % G || w_stride % 8 || v_stride % 8) return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
   const int smem = TILE128 + TILE64 + 64 + 1024;
-  if (!cfg) { int e = smem_opt_in((const void*)ssd_chunk_state_kernel, smem); if (e) return e; cfg = true; }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(ssd_chunk_state_kernel), smem)) return e;
   CUtensorMap tm;
   int r = make_tmap_2d_bf16(&tm, w_src, (uint64_t)w_cols, (uint64_t)B * L, (uint64_t)w_stride * 2, 64, 128);
   if (r) return -100 - r;
@@ -1312,8 +1308,8 @@ extern "C" int ssm_ssd_state_walk(const void* w_src, long long w_stride, int w_c
   if (L % CT || Hv % H || H % G || w_stride % 8 || v_stride % 8 || B < 1 || B > 65535 || (forward && (in16 != nullptr || dt == nullptr)) ||
       !segments_ok(L / CT, count, seg_fin, seg_decay, &sg) || (in16 == nullptr && count < 2))
     return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
-  if (!cfg) { int e = smem_opt_in((const void*)ssd_state_walk_kernel, WALK_SMEM); if (e) return e; cfg = true; }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(ssd_state_walk_kernel), WALK_SMEM)) return e;
   const int nc = L / CT;
   CUtensorMap tw, tv, ti;
   int r = make_tmap_2d_bf16(&tw, w_src, (uint64_t)w_cols, (uint64_t)B * L, (uint64_t)w_stride * 2, 64, 128);
@@ -1343,8 +1339,8 @@ extern "C" int ssm_ssd_walk_scan(const void* xbc, long long xbc_stride, int xbc_
       !segments_ok(L / CT, count, seg_fin, seg_decay, &sg) ||
       ((reinterpret_cast<uintptr_t>(dt) | reinterpret_cast<uintptr_t>(l)) & 15))
     return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
-  if (!cfg) { int e = smem_opt_in((const void*)ssd_walk_scan_kernel, WS_SMEM); if (e) return e; cfg = true; }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(ssd_walk_scan_kernel), WS_SMEM)) return e;
   const int nc = L / CT;
   CUtensorMap tx, ts, ty;
   int r = make_tmap_2d_bf16(&tx, xbc, (uint64_t)xbc_cols, (uint64_t)B * L, (uint64_t)xbc_stride * 2, 64, 128);
@@ -1370,9 +1366,9 @@ extern "C" int ssm_ssd_chunk_scan_fwd(const void* xbc, long long xbc_stride, int
                                       long long y_stride, const void* dt, const void* l, const void* D, int B, int L,
                                       int H, int Hv, int G, int d_in, int* status, cudaStream_t st) {
   if (L % CT || Hv % H || H % G || xbc_stride % 8 || y_stride % 8) return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
   const int smem = 2 * TILE128 + 2 * TILE64 + 2 * CT * 4 + 64 + 1024;
-  if (!cfg) { int e = smem_opt_in((const void*)ssd_chunk_scan_fwd_kernel, smem); if (e) return e; cfg = true; }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(ssd_chunk_scan_fwd_kernel), smem)) return e;
   const int nc = L / CT;
   CUtensorMap tx, ts, ty;
   int r = make_tmap_2d_bf16(&tx, xbc, (uint64_t)xbc_cols, (uint64_t)B * L, (uint64_t)xbc_stride * 2, 64, 128);
@@ -1405,8 +1401,8 @@ extern "C" int ssm_ssd_chunk_scan_bwd(const void* xbc, long long xbc_stride, int
     return -SSM_ERR_BAD_ARG;
   const int hv_per_group = Hv / G;
   if (hpc <= 0 || hv_per_group % hpc) return -SSM_ERR_BAD_ARG;
-  static bool cfg = false;
-  if (!cfg) { int e = smem_opt_in((const void*)ssd_chunk_scan_bwd_kernel, BWD_SMEM); if (e) return e; cfg = true; }
+  static SmemOptIn opt_in;
+  if (const int e = opt_in.ask(reinterpret_cast<const void*>(ssd_chunk_scan_bwd_kernel), BWD_SMEM)) return e;
   const int nc = L / CT;
   CUtensorMap tx, tdy, ts, tds, tdx;
   int r = make_tmap_2d_bf16(&tx, xbc, (uint64_t)xbc_cols, (uint64_t)B * L, (uint64_t)xbc_stride * 2, 64, 128);
