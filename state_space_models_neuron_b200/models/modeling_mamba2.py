@@ -52,6 +52,16 @@ def _hooked(module) -> bool:
     return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
 
 
+def _stood_for():
+    """What a block's one native call stands for: methods of the classes and operations as they are now."""
+    return (Mamba2Mixer.forward, Mamba2Mixer.step, Mamba2Mixer._core_kwargs, Mamba2Mixer.__call__, Mamba2RMSNorm.forward_add,
+            ColumnParallelLinear.forward, ColumnParallelLinear.__call__, RowParallelLinear.forward, RowParallelLinear.__call__,
+            ops.add_rmsnorm, ops.linear, ops.mamba2_mixer_core, ops.ssm_decode_step)
+
+
+_STOOD_FOR = _stood_for()
+
+
 class Mamba2Block(nn.Module):
     """Pre-norm residual block: h <- h + mixer(norm(h)).
 
@@ -72,15 +82,16 @@ class Mamba2Block(nn.Module):
 
     def _in_one_call(self, op, method: str, hidden_states, residual, residual_dtype, conv_state, ssm_state):
         """`op`, one native call that stands for `method` of the mixer and what surrounds it, where the block is made of the
-        plain modules on one rank.  None where any is of another class, has a hook or a method set on it, holds a weight that is no
-        parameter of its own (parametrised, pruned), or out_proj has a bias: these keep the calls one by one.  (The modules' own
+        plain modules on one rank.  None where any is of another class, has a hook or a method set on it or on its class, holds a
+        weight that is no parameter of its own (parametrised, pruned), or out_proj has a bias: these keep the calls one by one.  (The modules' own
         dictionaries: attribute lookups of a module cost the host more than the launches.)"""
         norm, m = self._modules["norm"], self._modules["mixer"]
         if type(m) is not Mamba2Mixer or type(norm) is not Mamba2RMSNorm:
             return None
         parts, own = m._modules, m._parameters
         gate, conv, first, last = parts["norm"], parts["conv1d"]._parameters, parts["in_proj"], parts["out_proj"]
-        if (method in vars(m) or "forward_add" in vars(norm) or (method == "forward" and _hooked(m)) or _has_any_global_hook()
+        if (method in vars(m) or "_core_kwargs" in vars(m) or "forward_add" in vars(norm) or (method == "forward" and _hooked(m))
+                or _has_any_global_hook() or _stood_for() != _STOOD_FOR
                 or type(gate) is not MambaRMSNormGated or type(first) is not ColumnParallelLinear or type(last) is not RowParallelLinear
                 or "forward" in vars(first) or "forward" in vars(last) or _hooked(first) or _hooked(last)
                 or last._parameters.get("bias", last) is not None or ps.get_tensor_model_parallel_size() != 1):

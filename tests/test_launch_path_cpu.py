@@ -143,3 +143,25 @@ def test_other_numbers_of_taps_are_refused(taps):
         cuda_ops.causal_conv1d_silu(make(1, L, C), make(C, 1, taps), make(C))
     with torch.no_grad(), pytest.raises(ValueError, match="taps"):         # four taps of fewer channels
         cuda_ops.causal_conv1d_silu(make(1, L, C), make(C // 2, 1, 4), make(C))
+
+
+@pytest.mark.parametrize("where,name", [("Mamba2Mixer", "forward"), ("Mamba2Mixer", "step"), ("Mamba2Mixer", "_core_kwargs"),
+                                        ("Mamba2Mixer", "__call__"), ("Mamba2RMSNorm", "forward_add"), ("ColumnParallelLinear", "forward"),
+                                        ("RowParallelLinear", "forward"), ("RowParallelLinear", "__call__"), ("ops", "linear"),
+                                        ("ops", "add_rmsnorm"), ("ops", "ssm_decode_step"), ("ops", "mamba2_mixer_core")])
+def test_blocks_by_one_call_see_methods_replaced_on_classes(monkeypatch, where, name):
+    """A method that a program or a test has set on a class, or an operation set in the package, is called as before."""
+    from state_space_models_neuron_b200.models import Mamba2Config, modeling_mamba2
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    cfg = Mamba2Config(num_heads=2, head_dim=64, vocab_size=64, hidden_size=64, state_size=128, num_hidden_layers=1, n_groups=1)
+    block = modeling_mamba2.Mamba2Block(cfg, 0)
+    op = lambda *a: "one call"
+    assert block._in_one_call(op, "step", None, None, None, None, None) == "one call"
+    owner = getattr(modeling_mamba2, where)
+    plain = getattr(owner, name)
+    monkeypatch.setattr(owner, name, lambda *a, **kw: plain(*a, **kw))
+    assert block._in_one_call(op, "step", None, None, None, None, None) is None
+    monkeypatch.undo()
+    assert block._in_one_call(op, "step", None, None, None, None, None) == "one call"
