@@ -15,12 +15,20 @@ import torch
 from ..parallel import state as ps
 
 
+_PIECE = 64 << 20
+
+
 def _zeros(count: int, shape, dtype, device):
-    """`count` zero tensors of one shape with one allocation and one fill where their sizes are whole 16-byte vectors (48 fills
-    took 250 us of the host in front of a prompt through 24 layers).  Each has a version counter of its own."""
-    if math.prod(shape) * dtype.itemsize % 16 or count < 2:
+    """`count` zero tensors of one shape.  Small ones whose sizes are whole 16-byte vectors share allocations and fills of at most
+    64 MB (48 fills took 250 us of the host in front of a prompt through 24 layers); larger ones have one each, so that a cache needs
+    no more memory in one piece than a layer's state, and a layer's state that is kept holds no more than that.  Each has a version
+    counter of its own."""
+    size = math.prod(shape) * dtype.itemsize
+    each = _PIECE // size if size and size % 16 == 0 else 1
+    if each < 2:
         return [torch.zeros(shape, device=device, dtype=dtype) for _ in range(count)]
-    return [t.data for t in torch.zeros((count, *shape), device=device, dtype=dtype).unbind(0)]
+    return [t.data for first in range(0, count, each)
+            for t in torch.zeros((min(each, count - first), *shape), device=device, dtype=dtype).unbind(0)]
 
 
 class Mamba2Cache:

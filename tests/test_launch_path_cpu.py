@@ -165,3 +165,24 @@ def test_blocks_by_one_call_see_methods_replaced_on_classes(monkeypatch, where, 
     assert block._in_one_call(op, "step", None, None, None, None, None) is None
     monkeypatch.undo()
     assert block._in_one_call(op, "step", None, None, None, None, None) == "one call"
+
+
+@pytest.mark.parametrize("batch", [0, 1, 7, 9, 130])
+def test_cache_pieces(monkeypatch, batch):
+    """Layers share memory in pieces of a limited size; a state above it has memory of its own."""
+    from state_space_models_neuron_b200.models import Mamba2Cache, Mamba2Config, cache
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    monkeypatch.setattr(cache, "_PIECE", 1 << 20)
+    cfg = Mamba2Config(num_heads=2, head_dim=64, vocab_size=64, hidden_size=64, state_size=128, num_hidden_layers=5, n_groups=1)
+    c = Mamba2Cache(cfg, batch, dtype=torch.bfloat16)
+    for states, shape in ((c.conv_states, (batch, 384, 4)), (c.ssm_states, (batch, 2, 64, 128))):
+        assert list(states) == list(range(5))
+        for i, t in states.items():
+            assert tuple(t.shape) == shape and t.is_contiguous() and not t.any()
+            assert t.untyped_storage().nbytes() <= max(1 << 20, t.numel() * t.element_size())
+            version = states[(i + 1) % 5]._version
+            t.fill_(i + 1)
+            assert states[(i + 1) % 5]._version == version
+        assert all(torch.equal(t, torch.full_like(t, i + 1)) for i, t in states.items())
