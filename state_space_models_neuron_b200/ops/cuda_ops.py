@@ -247,6 +247,8 @@ def wgrad_to_main_grad(dy2: torch.Tensor, x2: torch.Tensor, w) -> bool:
     w.grad_stale = False
     if acc is not None:
         w.norm_tracked = True
+        if getattr(w, "scatter_added", False):
+            w.norm_version = mg._version
     return True
 
 
@@ -264,6 +266,14 @@ def untrack_norm(w) -> None:
     if getattr(w, "norm_tracked", False):
         w.norm_tracked = False
         w.norm_dirty = True
+
+
+def untrack_edited(w) -> None:
+    """The same where operations of the program have written into the embedding's gradient since a kernel last added to the norm
+    (rows of frozen tokens set to zero, say).  They are seen by the version counter, which the optimizer's flat buffer and all
+    gradients in it share; writes through `.data` have a counter of their own and are not seen."""
+    if getattr(w, "norm_tracked", False) and w.main_grad._version != w.norm_version:
+        untrack_norm(w)
 
 
 class _Linear(torch.autograd.Function):
@@ -556,6 +566,7 @@ def embed_grad_target(w, follow_norm: bool = False, tokens: int = 0):
     otherwise they make it stale."""
     mg = getattr(w, "main_grad", None)
     if mg is not None and mg.dtype == torch.float32 and mg.is_contiguous():
+        untrack_edited(w)
         acc = getattr(w, "norm_acc", None) if follow_norm and not getattr(w, "norm_dirty", False) else None
         if getattr(w, "grad_stale", False):
             mg.zero_()
@@ -564,6 +575,7 @@ def embed_grad_target(w, follow_norm: bool = False, tokens: int = 0):
         if acc is None or not getattr(w, "norm_tracked", False):
             untrack_norm(w)             # scatter-added rows change the norm of a gradient a GEMM may have stored
             acc = None
+        w.norm_version = mg._version
         return mg, True, acc
     return torch.zeros(w.shape, dtype=torch.float32, device=w.device), False, None
 

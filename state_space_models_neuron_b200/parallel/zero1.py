@@ -250,6 +250,18 @@ class Zero1Optimizer(torch.optim.Optimizer):
             if p.dim() == 2 and not rep and not getattr(p, "no_norm_tracking", False):
                 p.norm_acc = self._norm_acc
 
+    def _untrack_edited(self, all_of_them: bool = False) -> None:
+        """Kernels have added the norm of what they wrote; where the program has written into an embedding's gradient since (or,
+        all_of_them, into any), the norm is read from the buffers."""
+        if self._norm_acc is None:
+            return
+        from ..ops import cuda_ops
+        for p, *_ in self.layout:
+            if all_of_them:
+                cuda_ops.untrack_norm(p)
+            elif getattr(p, "scatter_added", False):
+                cuda_ops.untrack_edited(p)
+
     def _tracked_norm_sq(self, g: torch.Tensor):
         """Gradient norm^2 from the GEMM epilogues plus one multi-range pass over everything they did not cover;
         None when tracking is off or a tracked gradient was modified after its GEMM (then the full pass runs)."""
@@ -319,10 +331,14 @@ class Zero1Optimizer(torch.optim.Optimizer):
         capturing = self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()
         if not capturing:
             self.upload_learning_rates()
+        self._untrack_edited()
         self._finish_lazy_zero()
         self._allreduce_sequence_parallel_grads()
         if self.post_reduce_hook is not None and not capturing:
+            version = self.flat_grads._version
             self.post_reduce_hook(self)
+            if self.flat_grads._version != version:
+                self._untrack_edited(all_of_them=True)
         self.step_count += 1
         if self._fused_dp:
             return self._fused_step()

@@ -34,6 +34,38 @@ def test_norm_follows_the_embedding(tied, ids_below, passes, vocab):
         assert abs(total - want) <= 2e-5 * want
 
 
+@pytest.mark.parametrize("tied", [True, False])
+@pytest.mark.parametrize("edit", ["none", "after", "between", "hook", "unused"])
+def test_norm_of_edited_gradients(tied, edit):
+    """What a program writes into the embedding's gradient between the backward pass and the step counts in the norm that clips."""
+    from state_space_models_neuron_b200 import parallel as nxd
+    from state_space_models_neuron_b200.models import Mamba2Config, Mamba2ForCausalLM
+    from state_space_models_neuron_b200.parallel import state as ps
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1)
+    cfg = nxd.parallel_config(1, {"zero_one_enabled": True, "grad_clipping": True, "max_grad_norm": 1.0}, init_seed=3)
+    mc = Mamba2Config(num_heads=8, head_dim=64, vocab_size=4096, hidden_size=256, state_size=128, num_hidden_layers=1, n_groups=1,
+                      tie_word_embeddings=tied, initializer_range=0.02, dtype=torch.bfloat16)
+    model = nxd.initialize_parallel_model(cfg, lambda: Mamba2ForCausalLM(mc, device="cuda").to(torch.bfloat16))
+    more = [torch.nn.Parameter(torch.ones(64, 64, device="cuda", dtype=torch.bfloat16))] if edit == "unused" else []
+    opt = nxd.initialize_parallel_optimizer(cfg, nxd.AdamW_FP32OptimParams, [{"params": [*model.parameters(), *more]}], lr=1e-3)
+    weight = model.backbone.embeddings.weight
+    ids = torch.randint(0, 4096, (2, 256), device="cuda", generator=torch.Generator(device="cuda").manual_seed(4))
+    opt.zero_grad()
+    for k in range(2 if edit == "between" else 1):
+        model(input_ids=ids, labels=ids, return_logits=False).loss.backward()
+        assert weight.norm_tracked == (k == 0)
+        if edit in ("after", "between") and k == 0:
+            with torch.no_grad():
+                weight.main_grad[:2048] *= 8
+    if edit == "hook":
+        opt.post_reduce_hook = lambda o: weight.main_grad[:2048].mul_(8)
+    opt.step()
+    assert weight.norm_tracked == (edit in ("none", "unused"))
+    want = opt.flat_grads.double().norm().item()
+    assert abs(opt.last_grad_norm.item() - want) <= 1e-5 * want
+
+
 @pytest.mark.parametrize("total", [0.0, 1e-20, 0.25, 1.0, 3.7e9, float("inf"), float("nan"), -1.0])
 def test_clip_coefficient_equals_separate_operations(total):
     from state_space_models_neuron_b200.ops import cuda_ops
