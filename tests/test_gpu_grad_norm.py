@@ -34,6 +34,32 @@ def test_norm_follows_the_embedding(tied, ids_below, passes, vocab):
         assert abs(total - want) <= 2e-5 * want
 
 
+# columns in one, four and more than four vectors per thread (256 threads of four values), more tokens than blocks, equal ids, ids of
+# other ranks' rows
+@pytest.mark.parametrize("D", [256, 1028, 4096, 5120, 8196])
+@pytest.mark.parametrize("tokens", [1, 1300])
+def test_additions_carry_the_norm_on(D, tokens):
+    from state_space_models_neuron_b200.ops import cuda_ops as co
+    gen = torch.Generator(device="cuda").manual_seed(D + tokens)
+    rows = 96
+    grad = torch.randn(rows, D, device="cuda", generator=gen)
+    want = grad.double()
+    norm = want.square().sum().float().reshape(1)
+    moved = want.square().sum()                             # of all terms that enter the sum, without their signs
+    for _ in range(2):
+        ids = torch.randint(-3, rows + 3, (tokens,), device="cuda", generator=gen)
+        g = torch.randn(tokens, D, device="cuda", generator=gen).bfloat16()
+        co._run("ssm_embed_bwd", co._P(ids), co._P(g), co._ll(D), co._P(grad), co._ll(0), co._ll(rows), 1, tokens, tokens, D, 1, None, 0, 0,
+                None, co._P(norm), co._P(co.status_tensor(grad.device)), co._st())
+        mine = (ids >= 0) & (ids < rows)
+        old, want = want, want.index_add(0, ids[mine], g[mine].double())
+        moved = moved + (g[mine].double().abs() * (2 * torch.maximum(old.abs(), want.abs())[ids[mine]] + g[mine].double().abs())).sum()
+    co.check_status()
+    assert torch.allclose(grad.double(), want, rtol=0, atol=2.0 ** -24 * 64 * want.abs().max().item())     # up to 40 additions to a value
+    # chains of about 100 additions per thread and of a few thousand to the accumulator, which round to either side
+    assert abs(norm.item() - want.square().sum().item()) <= 2.0 ** -24 * 64 * moved.item()
+
+
 @pytest.mark.parametrize("tied", [True, False])
 @pytest.mark.parametrize("edit", ["none", "after", "between", "hook", "unused"])
 def test_norm_of_edited_gradients(tied, edit):

@@ -44,6 +44,27 @@ def test_norms(d, groups, rows, gate):
             _near(gx, gs + dres.double())
 
 
+# blocks of the gated norm's backward kernel that walk more rows than their ring holds: stages are loaded again and their phase
+# turns, by both thread counts (296, 592 and 148 blocks; rings of 3 or 4)
+@pytest.mark.parametrize("rows,d,gs", [(296 * 8 + 1, 5120, 5120), (592 * 9 + 1, 264, 264), (592 * 5 + 7, 2048, 256), (148 * 9 + 1, 5128, 5128)])
+@pytest.mark.parametrize("gate", [True, False])
+def test_gated_norm_backward_of_many_rows(rows, d, gs, gate):
+    from state_space_models_neuron_b200 import ops
+    from state_space_models_neuron_b200.ops import cuda_ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+    y, z, w, dout = make(rows, d).requires_grad_(), make(rows, d).requires_grad_(), make(d).requires_grad_(), make(rows, d)
+    ops.gated_rmsnorm(y, z if gate else None, w, 1e-5, gs).backward(dout)
+    Y, Z, W = (t.detach().double().requires_grad_() for t in (y, z, w))
+    h = (Y * torch.nn.functional.silu(Z) if gate else Y).view(rows, d // gs, gs)
+    ((h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-5)).view(rows, d) * W).backward(dout.double())
+    cuda_ops.check_status()
+    _near(y.grad, Y.grad)
+    _near(w.grad, W.grad)
+    if gate:
+        _near(z.grad, Z.grad)
+
+
 @pytest.mark.parametrize("L", [1, 3, 8, 33, 35, 130])        # remainders of the token tiles and of the batches of four
 @pytest.mark.parametrize("C", [8, 520, 10240])
 @pytest.mark.parametrize("init", [True, False])
