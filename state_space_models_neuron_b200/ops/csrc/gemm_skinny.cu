@@ -324,12 +324,12 @@ norm_linear_kernel(const NormLinearParams p) {
 
 template <int KIND>
 static int launch_norm_linear(NormLinearParams p, bool fp32, int sms, cudaStream_t stream) {
-  // bases and strides of 16-byte vectors, groups of whole chunks, rows that fit the shared memory of any kernel
+  // bases and strides of 16-byte vectors, groups of whole chunks
   const uintptr_t a = reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.b) | reinterpret_cast<uintptr_t>(p.wn) |
                       reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.res_out);
   const size_t smem = (size_t)p.M * norm_row(p.K) * sizeof(float);
   if (p.M < 1 || p.M > 8 || p.N < 1 || p.K < 8 || p.K > 4096 || p.K % 8 || (a & 15) || p.lda % 8 || p.ldw % 8 || p.ldb % (fp32 ? 4 : 8) ||
-      smem > 41 * 1024 || !(p.groups == 1 || ((p.groups == 2 || p.groups == 4 || p.groups == 8) && p.K % (p.groups * ROWS_CHUNK) == 0)))
+      !(p.groups == 1 || ((p.groups == 2 || p.groups == 4 || p.groups == 8) && p.K % (p.groups * ROWS_CHUNK) == 0)))
     return -SSM_ERR_BAD_ARG;
   int vecs = 1;
   p.threads = norm_threads(p.K / p.groups, &vecs, false);
@@ -338,8 +338,12 @@ static int launch_norm_linear(NormLinearParams p, bool fp32, int sms, cudaStream
   const int unroll = rows_unroll(((p.K + ROWS_CHUNK - 1) / ROWS_CHUNK + ROWS_WARPS - 1) / ROWS_WARPS);
   const bool few = unroll <= 2 || grid > (unsigned)sms;
   auto kern = unroll == 1 && vecs == 1 ? norm_linear_kernel<KIND, 1, 1> : few ? norm_linear_kernel<KIND, 2, 1> : norm_linear_kernel<KIND, 3, 1>;
+  int which = unroll == 1 && vecs == 1 ? 0 : few ? 1 : 2;
   if constexpr (KIND == NORM_GATED)
-    if (vecs == 2) kern = few ? norm_linear_kernel<KIND, 2, 2> : norm_linear_kernel<KIND, 3, 2>;
+    if (vecs == 2) { kern = few ? norm_linear_kernel<KIND, 2, 2> : norm_linear_kernel<KIND, 3, 2>; which = few ? 3 : 4; }
+  static SmemOptIn opt_in[5];
+  if (smem > 40 * 1024)                                  // more than a kernel has without asking, beside its own tables
+    if (const int e = opt_in[which].ask(reinterpret_cast<const void*>(kern), 8 * norm_row(4096) * (int)sizeof(float))) return e;
   return launch_dependent(kern, dim3(grid), dim3(ROWS_WARPS * 32), smem, stream, p);
 }
 

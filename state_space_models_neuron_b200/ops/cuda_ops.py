@@ -1204,6 +1204,7 @@ def block_forward(hidden, residual, residual_dtype, conv_state, ssm_state, norm_
 _BLOCK = struct.Struct("=20Qq11i2f")
 
 
+@functools.lru_cache(maxsize=4096)
 def _norms_in_products(B: int, width: int, in_cols: int, d_inner: int, gs: int, captured: bool):
     """Which norms of a decoding block are computed inside the product behind them (norm_linear_kernel, the same bits as two
     kernels): (first, gated).  Every block of it forms all rows, so few columns in all gain and many lose; two blocks of the first
@@ -1213,7 +1214,7 @@ def _norms_in_products(B: int, width: int, in_cols: int, d_inner: int, gs: int, 
     6.9 / 5.9; with eight groups 1 x 2048 5.0 / 5.2, 2 x 2048 5.4 / 5.3, 1 x 4096 8.5 / 8.2).  Where no graph is captured the host is
     the limit, which a launch less saves 3 us (370M, 5 sequences: 723 us a token with two kernels each, 642 with one)."""
     groups = d_inner // gs
-    first, gated = (2048, 6144 if groups == 1 else 2048) if captured else (8192, 10240)
+    first, gated = (2048, 6144 if groups == 1 else 2048) if captured else (8192, 32768)
     return (B <= 8 and width <= 1024 and B * width <= first and (in_cols <= 16 * 2 * 148 or not captured),
             B <= 8 and d_inner <= 4096 and B * d_inner <= gated and (groups == 1 or (groups in (2, 4, 8) and gs % 64 == 0)))
 
@@ -1239,7 +1240,9 @@ def decode_block(hidden, residual, residual_dtype, conv_state, ssm_state, norm_w
     scratch = torch.empty(B * (ld + d_inner + max(width, d_inner)), dtype=torch.bfloat16, device=dev)
     out, res_out = torch.empty_like(hidden), torch.empty(hidden.shape, dtype=rd, device=dev)
     zx = scratch.data_ptr()
-    first, gated = _norms_in_products(B, width, d_inner + C + H, d_inner, gs, torch.cuda.is_current_stream_capturing())
+    first, gated = _norms_in_products(B, width, d_inner + C + H, d_inner, gs, True)
+    if not (first and gated) and not torch.cuda.is_current_stream_capturing():
+        first, gated = _norms_in_products(B, width, d_inner + C + H, d_inner, gs, False)
     _run("ssm_decode_block", _BLOCK.pack(*rows, res_out.data_ptr(), *weights[0], *states, zx, zx + 2 * B * ld, zx + 2 * B * (ld + d_inner),
                                          out.data_ptr(), status_tensor(dev).data_ptr(), ld, B, width, d_inner, H, head_dim, d_state,
                                          n_groups, gs, int(rd is torch.float32), weights[1], int(first) | 2 * int(gated), norm_eps, eps), _st())

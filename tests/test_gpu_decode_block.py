@@ -50,7 +50,8 @@ def test_block_equals_separate_operations(B, width, H, P, G, gs, fp32):
                                                    (8, 1024, 16, 64, 2, 1024, True), (5, 256, 32, 64, 1, 2048, False),
                                                    (1, 264, 16, 128, 1, 2048, True), (2, 64, 16, 64, 2, 512, False),
                                                    (1, 72, 8, 192, 4, 192, True), (4, 8, 8, 64, 1, 512, False),
-                                                   (7, 104, 13, 64, 1, 832, True), (1, 1000, 8, 480, 1, 3840, False)])
+                                                   (7, 104, 13, 64, 1, 832, True), (1, 1000, 8, 480, 1, 3840, False),
+                                                   (8, 128, 64, 64, 1, 4096, False), (5, 128, 48, 64, 8, 384, True)])
 def test_block_has_the_bits_of_separate_operations(B, width, H, P, G, gs, fp32):
     """Which norms run inside the products is a matter of time only: every sum and rounding is that of the separate kernels."""
     from state_space_models_neuron_b200 import ops
