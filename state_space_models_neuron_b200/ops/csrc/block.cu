@@ -1,6 +1,6 @@
 // Whole pre-norm blocks over a full sequence, launched by one call.  No kernels of its own: at a few hundred tokens the kernels
 // of a block take 3 to 8 us each and a launch from Python about 20, so the chain is put together here.
-// 130M, one prompt of 128 tokens, 24 layers: 4717 us with ten launches per block from Python, 1329 (850 of them kernels) so.
+// 130M, one prompt of 128 tokens, 24 layers: 4717 us with ten launches per block from Python, 1380 to 1430 (830 of them kernels) so.
 #include "common.cuh"
 
 extern "C" {

@@ -475,8 +475,8 @@ embed_wait_copy_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __r
 
 // norm (one rank only): += what the additions change the sum of squares of grad32 by, g (2 old + g) each with the value that the
 // addition met, whose sum telescopes over equal ids in any order.  The product that stored a tied gradient has added its sum of
-// squares already, so no pass over all rows of the vocabulary is needed for the gradient norm (50288 x 4096: 138 us for the pass,
-// 13 -> 25 here for 2048 tokens; 8192 tokens of 2560 93 for the pass, 39 -> 83 here, 2048 x 4096 into 6286 rows 19, 12 -> 31).
+// squares already, so no pass over all rows of the vocabulary is needed for the gradient norm (50288 x 4096 and 2048
+// tokens: 144 us for the pass, 21 -> 49 here; 50288 x 2560 and 8192 tokens 100, 45 -> 84; the rule that chooses has the others).
 __global__ void __launch_bounds__(256)
 embed_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ g, long long g_ld,
                  float* __restrict__ grad32, long long vocab_start, long long vloc, int B, int L, int Ls, int D,

@@ -635,7 +635,8 @@ add_rmsnorm_bwd_kernel(const RT* __restrict__ res, const __nv_bfloat16* __restri
 // =====================================================================================
 // Gaussian distribution function of a pair, and exp(-x^2 / 2) on the way.  With t = 1 / (1 + 0.34 |x|), the tail
 // 0.5 erfc(|x| / sqrt 2) is exp(-x^2 / 2) times a polynomial of degree 9 in t (least-squares fit of 0.5 erfcx on |x| <= 14,
-// weighted towards equal relative errors: 1.3e-8 in the fit, 3e-7 in fp32), which is one division and one exponential per value, shared
+// weighted towards equal relative errors: 1.3e-8 in the fit; in fp32 3e-7 up to |x| = 2, then growing with the exponential's argument,
+// 4e-7 up to 4, 1e-6 up to 6, 3.4e-6 up to 12), which is one division and one exponential per value, shared
 // with the density that the backward pass wants; erff() takes two polynomials behind a branch on |x| < 1.  Below zero the tail
 // itself is the result, so no digits cancel as they do in 1 + erf.
 // These kernels were bound by that arithmetic, twice to three times what moving their rows takes:

@@ -254,9 +254,12 @@ def wgrad_to_main_grad(dy2: torch.Tensor, x2: torch.Tensor, w) -> bool:
 
 def _follow_norm(tokens: int, rows: int) -> bool:
     """Whether the additions of an embedding's gradient carry the gradient norm on (ssm_embed_bwd with an accumulator), or the norm
-    of its rows is taken by a pass over all of them.  Following costs a third to double of the additions, the pass 4 bytes per
-    value of the table (us, additions with and without, pass: 2048 tokens of 4096 into 50288 rows 25, 13, 126; 8192 of 2560 83, 39, 79;
-    8192 of 1024 42, 14, 31; 2048 of 4096 into 6286 rows 31, 12, 16): they meet at about six rows per token."""
+    of its rows is taken by a pass over all of them.  Additions that bring the old value back cost 25 to 40 us more, the pass reads 4
+    bytes per value of the table (tokens x columns into rows: additions with and without, pass; us, cold): 2048 x 4096 into 50288
+    49, 21, 144; 8192 x 4096 into 50288 96, 60, 143; 8192 x 2560 into 50288 84, 45, 100; 8192 x 1024 into 50288 53, 25, 45; 12288 x 2560
+    into 50288 105, 63, 100; 4096 x 2560 into 16384 59, 27, 39; 4096 x 1024 into 16384 41, 16, 21; 2048 x 4096 into 6286 47, 21, 29.
+    From six rows per token on following wins at every width; between three and six it wins or loses with the width and the table,
+    and the pass, which takes no atomic additions with results, is kept there."""
     return tokens * 6 <= rows
 
 

@@ -37,8 +37,7 @@ def test_block_equals_separate_operations(B, width, H, P, G, gs, fp32):
             torch.cuda.synchronize()
             cuda_ops.check_status()
             assert torch.equal(res, want_res) and out.shape == hidden.shape
-            # in_proj's operands and results are rounded to bf16 once on both sides, of equal values in another order: what
-            # follows from them differs by a few steps of bf16, spread over sums of hundreds of terms
+            # in_proj's operands and results are rounded to bf16 once on both sides; that they are the same bits is tested below
             near = lambda a, b: ((a.double() - b.double()).norm() / b.double().norm()).item() < 2.0 ** -7
             assert near(window, w0) and torch.equal(window[..., :3], w0[..., :3]) and near(state, s0) and near(out, want)
             hidden, residual = want, want_res
