@@ -1121,9 +1121,10 @@ def _block_weights(dev, width, d_inner, n_groups, d_state, head_dim, gs, norm_w,
     C, H, bf16 = d_inner + 2 * n_groups * d_state, d_inner // head_dim, torch.bfloat16
     W = d_inner + C + H
     mask = _head_param_mask(A_log, D, dt_bias, H)
-    given = [t for t in (norm_w, in_w, conv_w, gate_w, out_w, in_b, conv_b) if t is not None]
+    for t in (norm_w, in_w, conv_w, gate_w, out_w, in_b, conv_b):        # (a generator costs the host more than the tests)
+        if t is not None and (t.dtype is not bf16 or not t.is_contiguous() or t.get_device() != dev):
+            return None
     if (mask is None or H % n_groups or width % 8 or d_inner % 8 or d_inner % gs or gs % 8 or max(width, gs) > 8192
-            or any(t.dtype is not bf16 or not t.is_contiguous() or t.get_device() != dev for t in given)
             or A_log.get_device() != dev or D.get_device() != dev or dt_bias.get_device() != dev
             or in_w.shape != (W, width) or out_w.shape != (width, d_inner) or norm_w.numel() != width or gate_w.numel() != d_inner
             or conv_w.numel() != 4 * C or (in_b is not None and in_b.numel() != W) or (conv_b is not None and conv_b.numel() != C)):
